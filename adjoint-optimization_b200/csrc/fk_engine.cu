@@ -33,31 +33,34 @@ void set_error(const std::string& m) { g_err = m; }
 static DevModel make_model(const fkadj_params& p, double dt) {
     DevModel M;
     M.u_c = p.u_c;
-    M.u_v = p.u_v;
-    M.ksm = p.ksm;
-    M.k_fk = p.k_fk;
     M.u_csi = p.u_csi;
+    // -2 k 16 / ln2 in two parts: 16/ln2 as h + l, the product's own rounding
+    // error recovered by an fma
+    auto slope = [](double k, double* hi, double* lo) {
+        constexpr double h = 0x1.71547652b82fep+4, l = 0x1.777d0ffda0d24p-52;
+        const double c = -2.0 * k;
+        *hi = c * h;
+        *lo = std::fma(c, h, -*hi) + c * l;
+    };
+    slope(p.ksm, &M.sp_h, &M.sp_l);
+    slope(p.k_fk, &M.ss_h, &M.ss_l);
     M.r_tau_d = 1.0 / p.tau_d;
     M.r_tau_0 = 1.0 / p.tau_0;
     M.r_tau_r = 1.0 / p.tau_r;
-    M.r_2tau_si = 1.0 / (2 * p.tau_si);
+    M.r_tau_si = 1.0 / p.tau_si;
     M.tau_v1m = p.tau_v1_minus;
     M.tau_v2m = p.tau_v2_minus;
-    M.r_tau_v2m = 1.0 / p.tau_v2_minus;
-    M.m2ksm = -2.0 * p.ksm;
-    M.m2kfk = -2.0 * p.k_fk;
     M.r_tau_vp = 1.0 / p.tau_v_plus;
     M.r_tau_wm = 1.0 / p.tau_w_minus;
     M.r_tau_wp = 1.0 / p.tau_w_plus;
-    M.dv12 = p.tau_v2_minus - p.tau_v1_minus;
     M.eq = std::exp(-2.0 * (p.ksm * (p.u_c - p.u_v)));
     M.cu = p.Du / (p.h * p.h);
     M.cv = p.Dv / (p.h * p.h);
     M.cw = p.Dw / (p.h * p.h);
     M.dt = dt;
     M.two_ksm = 2.0 * p.ksm;
-    M.kfk_r2tsi = p.k_fk / (2 * p.tau_si);
-    M.hksm_dv12 = 0.5 * p.ksm * M.dv12;
+    M.kfk2_rsi = 2.0 * p.k_fk / p.tau_si;
+    M.two_ksm_dv12 = 2.0 * p.ksm * (p.tau_v2_minus - p.tau_v1_minus);
     return M;
 }
 
@@ -182,7 +185,7 @@ Problem::~Problem() {
     if (pool_) {
         // stream-ordered frees need the stream (the problem's own one is destroyed
         // below): release the buffers first
-        DevBuf* all[] = {&gh_, &wc_, &fcode_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
+        DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
                          &fcache_, &Ed_};
         for (DevBuf* b : all) b->release();
@@ -210,7 +213,7 @@ Problem::~Problem() {
     delete spline_;
     const auto t3 = clk::now();
     if (verbose_ > 1) {
-        DevBuf* all[] = {&gh_, &wc_, &fcode_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
+        DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
                          &fcache_, &Ed_};
         size_t bytes = 0;
@@ -389,7 +392,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     }
     for (auto& e : ev_) CK(cudaEventCreate(&e), "cudaEventCreate");
     if (pool_) {
-        DevBuf* all[] = {&gh_, &wc_, &fcode_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
+        DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
                          &fcache_, &Ed_};
         for (DevBuf* b : all) b->st = st_, b->pool = pool_;
@@ -489,28 +492,12 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
                                weight(i, j, 0, 1) << 6);
             pos[a - 1] = (long long)o2;
         }
-    // forward stencil codes (FC_*), unless an active cell has two opposite
-    // holes (then the kernels test values for NaN, as the reference does)
-    std::vector<uint8_t> fcode(pl, (uint8_t)FC_HOLE);
-    bool two_opposite = false;
-    for (int i = 0; i < nrows; ++i)
-        for (int j = 0; j < ncols; ++j) {
-            if (!act(i, j)) continue;
-            const bool mN = !act(i - 1, j), mS = !act(i + 1, j), mW = !act(i, j - 1), mE = !act(i, j + 1);
-            two_opposite = two_opposite || (mN && mS) || (mW && mE);
-            fcode[(size_t)(i + HALO) * g_.ld + (j + HALO)] =
-                (uint8_t)((mN ? FC_N : 0) | ((mS && !mN) ? FC_S : 0) | (mW ? FC_W : 0) | ((mE && !mW) ? FC_E : 0));
-        }
-    const bool use_codes = FKADJ_FWD_CODES && !two_opposite;
     CK(gh_.alloc(pl * sizeof(double)), "alloc gh");
     CK(wc_.alloc(pl), "alloc weights");
-    if (use_codes) CK(fcode_.alloc(pl), "alloc stencil codes");
     CK(pos_.alloc((size_t)n_num * sizeof(long long)), "alloc positions");
     // stream-ordered copies (from pageable memory they return once the data is staged)
     CK(cudaMemcpyAsync(gh_.p, gh.data(), pl * sizeof(double), cudaMemcpyHostToDevice, st_), "upload gh");
     CK(cudaMemcpyAsync(wc_.p, wc.data(), pl, cudaMemcpyHostToDevice, st_), "upload weights");
-    if (use_codes) CK(cudaMemcpyAsync(fcode_.p, fcode.data(), pl, cudaMemcpyHostToDevice, st_), "upload codes");
-    g_.fcode = use_codes ? fcode_.as<uint8_t>() : nullptr;
     CK(cudaMemcpyAsync(pos_.p, pos.data(), (size_t)n_num * sizeof(long long), cudaMemcpyHostToDevice, st_),
        "upload positions");
 

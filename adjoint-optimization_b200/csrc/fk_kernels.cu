@@ -266,7 +266,7 @@ __device__ __forceinline__ void fwd_stage(const DevModel& P, const double* __res
                                           const double* __restrict__ y0g, const double* __restrict__ ghs,
                                           int ld, long long plane, double Ev, double cY, double cD,
                                           double* __restrict__ out, double* __restrict__ stage_out, int rows,
-                                          double* __restrict__ k_out, const uint8_t* __restrict__ fcs) {
+                                          double* __restrict__ k_out) {
     constexpr int RW = TX + 2 * HALO, RH = TY + 2 * HALO, RN = RW * RH;
     constexpr int W = TX + 2 * E;
     constexpr int IN = TX * TY;
@@ -277,11 +277,11 @@ __device__ __forceinline__ void fwd_stage(const DevModel& P, const double* __res
         const bool inner = (E == 0) || (r >= HALO && r < HALO + rows && c >= HALO && c < HALO + TX);
         const int d = (r - HALO) * TX + (c - HALO);
         if (MODE == 2) {
-            out[o] = (a + D[d]) + cD * ku;
-            out[plane + o] = (b + D[IN + d]) + cD * kv;
-            out[2 * plane + o] = (e + D[2 * IN + d]) + cD * kw;
+            out[o] = fma(cD, ku, a + D[d]);
+            out[plane + o] = fma(cD, kv, b + D[IN + d]);
+            out[2 * plane + o] = fma(cD, kw, e + D[2 * IN + d]);
         } else {
-            const double nu = a + cY * ku, nv = b + cY * kv, nw = e + cY * kw;
+            const double nu = fma(cY, ku, a), nv = fma(cY, kv, b), nw = fma(cY, kw, e);
             dst[s] = nu;
             dst[RN + s] = nv;
             dst[2 * RN + s] = nw;
@@ -291,9 +291,9 @@ __device__ __forceinline__ void fwd_stage(const DevModel& P, const double* __res
                     D[IN + d] = cD * kv;
                     D[2 * IN + d] = cD * kw;
                 } else {
-                    D[d] = D[d] + cD * ku;
-                    D[IN + d] = D[IN + d] + cD * kv;
-                    D[2 * IN + d] = D[2 * IN + d] + cD * kw;
+                    D[d] = fma(cD, ku, D[d]);
+                    D[IN + d] = fma(cD, kv, D[IN + d]);
+                    D[2 * IN + d] = fma(cD, kw, D[2 * IN + d]);
                 }
                 if (stage_out) {  // stage state kept for the discrete adjoint
                     stage_out[o] = nu;
@@ -314,13 +314,11 @@ __device__ __forceinline__ void fwd_stage(const DevModel& P, const double* __res
         // loaded while this cell computes.
         struct Ops {
             double gv, a, b, e;
-            int code;
         };
         auto fetch = [&](int r, int c, Ops& x) {
             const long long o = (long long)r * ld + c;
             x.gv = __ldg(ghs + o);
             if (MODE != 0) x.a = __ldg(y0g + o), x.b = __ldg(y0g + plane + o), x.e = __ldg(y0g + 2 * plane + o);
-            x.code = fcs ? (int)__ldg(fcs + o) : -1;
         };
         Ops cur;
         if ((int)threadIdx.x < N) fetch(rc.r, rc.c, cur);
@@ -334,7 +332,7 @@ __device__ __forceinline__ void fwd_stage(const DevModel& P, const double* __res
             double a = cur.a, b = cur.b, e = cur.e;
             if (MODE == 0) a = src[s], b = src[RN + s], e = src[2 * RN + s];
             double ku, kv, kw;
-            rhs_at<RW, RN>(P, src, s, Ev * cur.gv, ku, kv, kw, cur.code);
+            rhs_at<RW, RN>(P, src, s, Ev, cur.gv, ku, kv, kw);
             finish(r, c, s, o, a, b, e, ku, kv, kw);
             cur = nxt;
         }
@@ -354,7 +352,7 @@ __device__ __forceinline__ void fwd_stage(const DevModel& P, const double* __res
                 a = __ldg(y0g + o), b = __ldg(y0g + plane + o), e = __ldg(y0g + 2 * plane + o);
             }
             double ku, kv, kw;
-            rhs_at<RW, RN>(P, src, s, Ev * gv, ku, kv, kw, fcs ? (int)__ldg(fcs + o) : -1);
+            rhs_at<RW, RN>(P, src, s, Ev, gv, ku, kv, kw);
             finish(r, c, s, o, a, b, e, ku, kv, kw);
         }
     }
@@ -393,15 +391,14 @@ __device__ __forceinline__ void fwd_step_tile(const DevModel& P, const DevGrid& 
     double* s2 = stages ? stages + off : nullptr;
     double* s3 = stages ? stages + sst + off : nullptr;
     double* s4 = stages ? stages + 2 * sst + off : nullptr;
-    const uint8_t* fcs = g.fcode ? g.fcode + off : nullptr;
     fwd_stage<3, TX, TY, NT, 0, PF>(P, A, B, D, y0g, ghs, g.ld, g.plane, E0, dt * 0.5, 1.0 / 6.0 * dt, nullptr, s2,
-                                rows, k1 ? k1 + off : nullptr, fcs);
+                                rows, k1 ? k1 + off : nullptr);
     fwd_stage<2, TX, TY, NT, 1, PF>(P, B, A, D, y0g, ghs, g.ld, g.plane, Eh, dt * 0.5, 1.0 / 3.0 * dt, nullptr, s3,
-                                rows, nullptr, fcs);
+                                rows, nullptr);
     fwd_stage<1, TX, TY, NT, 1, PF>(P, A, B, D, y0g, ghs, g.ld, g.plane, Eh, dt * 1.0, 1.0 / 3.0 * dt, nullptr, s4,
-                                rows, nullptr, fcs);
+                                rows, nullptr);
     fwd_stage<0, TX, TY, NT, 2, PF>(P, B, A, D, y0g, ghs, g.ld, g.plane, E1, 0.0, dt * 1.0 / 6.0, yout + off, nullptr,
-                                rows, nullptr, fcs);
+                                rows, nullptr);
 }
 
 template <int TX, int TY, int NT>
@@ -437,6 +434,11 @@ __device__ __forceinline__ void store_jac(double* __restrict__ Jb, long long pla
     Jb[4 * plane + o] = J.a4;
     Jb[5 * plane + o] = J.a5;
     Jb[6 * plane + o] = J.a6;
+}
+
+// Hermite combination c0 x0 + c1 m0 + c2 x1 + c3 m1, in this order
+__device__ __forceinline__ double hermite4(const double (&c)[4], double x0, double m0, double x1, double m1) {
+    return fma(c[3], m1, fma(c[2], x1, fma(c[1], m0, c[0] * x0)));
 }
 
 // Midpoint state of step [t_{i-1}, t_i] (cu-G:1244-1301): y3 = cubic Hermite
@@ -490,10 +492,10 @@ __device__ __forceinline__ void adj_mid_tile(const DevModel& P, const DevGrid& g
             for (int f = 0; f < 3; ++f) {
                 const double m0 = a0[f] * dt, m1 = a1[f] * dt;
                 const double x0 = A[f * RN + s], x1 = B[f * RN + s];
-                C[f * RN + s] = ((hw.c3[0] * x0 + hw.c3[1] * m0) + hw.c3[2] * x1) + hw.c3[3] * m1;
+                C[f * RN + s] = hermite4(hw.c3, x0, m0, x1, m1);
                 if (inner) {
                     Q[f * TX * TY + (r - H2) * TX + (c - H2)] =
-                        ((hw.c4[0] * x0 + hw.c4[1] * m0) + hw.c4[2] * x1) + hw.c4[3] * m1;
+                        hermite4(hw.c4, x0, m0, x1, m1);
                 }
             }
         };
@@ -520,9 +522,8 @@ __device__ __forceinline__ void adj_mid_tile(const DevModel& P, const DevGrid& g
                 if (q + NT < N) fetch(rc.r, rc.c, nxt);
                 const int s = r * RW + c;
                 const long long o = off + (long long)r * g.ld + c;
-                const int code = g.fcode ? (int)__ldg(g.fcode + o) : -1;
-                if (!fa) rhs_at<RW, RN>(P, A, s, Ea * cur.gg, cur.a0[0], cur.a0[1], cur.a0[2], code);
-                if (!fin) rhs_at<RW, RN>(P, B, s, Eb * cur.gg, cur.a1[0], cur.a1[1], cur.a1[2], code);
+                if (!fa) rhs_at<RW, RN>(P, A, s, Ea, cur.gg, cur.a0[0], cur.a0[1], cur.a0[2]);
+                if (!fin) rhs_at<RW, RN>(P, B, s, Eb, cur.gg, cur.a1[0], cur.a1[1], cur.a1[2]);
                 hermite(r, c, s, o, cur.a0, cur.a1);
                 cur = nxt;
             }
@@ -539,14 +540,14 @@ __device__ __forceinline__ void adj_mid_tile(const DevModel& P, const DevGrid& g
                     a0[1] = __ldg(fa + g.plane + o);
                     a0[2] = __ldg(fa + 2 * g.plane + o);
                 } else {
-                    rhs_at<RW, RN>(P, A, s, Ea * gg, a0[0], a0[1], a0[2], g.fcode ? (int)__ldg(g.fcode + o) : -1);
+                    rhs_at<RW, RN>(P, A, s, Ea, gg, a0[0], a0[1], a0[2]);
                 }
                 if (fin) {
                     a1[0] = __ldg(fin + o);
                     a1[1] = __ldg(fin + g.plane + o);
                     a1[2] = __ldg(fin + 2 * g.plane + o);
                 } else {
-                    rhs_at<RW, RN>(P, B, s, Eb * gg, a1[0], a1[1], a1[2], g.fcode ? (int)__ldg(g.fcode + o) : -1);
+                    rhs_at<RW, RN>(P, B, s, Eb, gg, a1[0], a1[1], a1[2]);
                 }
                 hermite(r, c, s, o, a0, a1);
             }
@@ -563,10 +564,10 @@ __device__ __forceinline__ void adj_mid_tile(const DevModel& P, const DevGrid& g
             const int s = r * RW + c;
             const long long o = off + (long long)r * g.ld + c;
             double m2[3], yv[3];
-            rhs_at<RW, RN>(P, C, s, E3 * __ldg(gh + o), m2[0], m2[1], m2[2], g.fcode ? (int)__ldg(g.fcode + o) : -1);
+            rhs_at<RW, RN>(P, C, s, E3, __ldg(gh + o), m2[0], m2[1], m2[2]);
 #pragma unroll
             for (int f = 0; f < 3; ++f) {
-                yv[f] = Q[f * TX * TY + (r - H2) * TX + (c - H2)] + hw.c2 * (m2[f] * dt);
+                yv[f] = fma(hw.c2, m2[f] * dt, Q[f * TX * TY + (r - H2) * TX + (c - H2)]);
                 if (yh) yh[o + f * g.plane] = yv[f];
             }
             if (jh && !isnan(yv[0])) store_jac(jh, g.plane, o, fk_jacT(P, yv[0], yv[1], yv[2]));
@@ -614,25 +615,25 @@ __device__ __forceinline__ void adj_stage(const DevModel& P, const DevGrid& g, c
         const bool inner = (E == 0) || (r >= HALO && r < HALO + rows && c >= HALO && c < HALO + TX);
         const int d = (r - HALO) * TX + (c - HALO);
         if (MODE == 2) {
-            const double nu = (a + D[d]) + cD * ku;
+            const double nu = fma(cD, ku, a + D[d]);
             out[o] = nu;
-            out[g.plane + o] = (b + D[IN + d]) + cD * kv;
-            out[2 * g.plane + o] = (e + D[2 * IN + d]) + cD * kw;
+            out[g.plane + o] = fma(cD, kv, b + D[IN + d]);
+            out[2 * g.plane + o] = fma(cD, kw, e + D[2 * IN + d]);
             const double t = nu * __ldg(gh + o);
             D[d] = isnan(t) ? 0.0 : t;
         } else {
-            dst[s] = a + cZ * ku;
-            dst[RN + s] = b + cZ * kv;
-            dst[2 * RN + s] = e + cZ * kw;
+            dst[s] = fma(cZ, ku, a);
+            dst[RN + s] = fma(cZ, kv, b);
+            dst[2 * RN + s] = fma(cZ, kw, e);
             if (inner) {
                 if (MODE == 0) {
                     D[d] = cD * ku;
                     D[IN + d] = cD * kv;
                     D[2 * IN + d] = cD * kw;
                 } else {
-                    D[d] = D[d] + cD * ku;
-                    D[IN + d] = D[IN + d] + cD * kv;
-                    D[2 * IN + d] = D[2 * IN + d] + cD * kw;
+                    D[d] = fma(cD, ku, D[d]);
+                    D[IN + d] = fma(cD, kv, D[IN + d]);
+                    D[2 * IN + d] = fma(cD, kw, D[2 * IN + d]);
                 }
             }
         }
@@ -685,7 +686,7 @@ __device__ __forceinline__ void adj_stage(const DevModel& P, const DevGrid& g, c
                 if (jload) {
                     J = {cur.j[0], cur.j[1], cur.j[2], cur.j[3], cur.j[4], cur.j[5], cur.j[6]};
                 } else {
-                    J = fk_jacT(P, finite_u(cur.j[0]), cur.j[1], cur.j[2]);
+                    J = fk_jacT(P, cur.j[0], cur.j[1], cur.j[2]);
                     if (jstore) store_jac(jstore, g.plane, o, J);
                 }
                 adj_at<RW, RN>(P, src, s, cur.code, J, ku, kv, kw);
@@ -712,17 +713,14 @@ __device__ __forceinline__ void adj_stage(const DevModel& P, const DevGrid& g, c
             }
             const int code = __ldg(wc + o);
             double ku, kv, kw;
-#if FKADJ_HOLE_BRANCH
             if (isnan(src[s])) {  // holes and the NaN ring: the result is NaN
                 ku = kv = kw = src[s];
-            } else
-#endif
-            {
+            } else {
                 JacT J;
                 if (jload) {
                     J = load_jac(jload, g.plane, o);
                 } else {
-                    J = fk_jacT(P, finite_u(__ldg(ys + o)), __ldg(ys + g.plane + o), __ldg(ys + 2 * g.plane + o));
+                    J = fk_jacT(P, __ldg(ys + o), __ldg(ys + g.plane + o), __ldg(ys + 2 * g.plane + o));
                     if (jstore) store_jac(jstore, g.plane, o, J);
                 }
                 adj_at<RW, RN>(P, src, s, code, J, ku, kv, kw);
@@ -834,37 +832,34 @@ __device__ __forceinline__ void fused_stage(const DevModel& P, const DevGrid& g,
         const double a = Zw[s], b = Zw[RN + s], e = Zw[2 * RN + s];
         const int code = __ldg(wc + o);
         double ku, kv, kw;
-#if FKADJ_HOLE_BRANCH
         if (isnan(src[s])) {  // holes and the NaN ring: the result is NaN
             ku = kv = kw = src[s];
-        } else
-#endif
-        {
+        } else {
             const JacT J = jac(r, c, o);
             adj_at<RW, RN>(P, src, s, code, J, ku, kv, kw);
         }
         const bool inner = (E == 0) || (r >= HALO && r < HALO + TY && c >= HALO && c < HALO + TX);
         const int d = (r - HALO) * TX + (c - HALO);
         if (MODE == 2) {
-            const double nu = (a + D[d]) + cD * ku;
+            const double nu = fma(cD, ku, a + D[d]);
             out[o] = nu;
-            out[g.plane + o] = (b + D[IN + d]) + cD * kv;
-            out[2 * g.plane + o] = (e + D[2 * IN + d]) + cD * kw;
+            out[g.plane + o] = fma(cD, kv, b + D[IN + d]);
+            out[2 * g.plane + o] = fma(cD, kw, e + D[2 * IN + d]);
             const double t = nu * __ldg(gh + o);
             D[d] = isnan(t) ? 0.0 : t;
         } else {
-            dst[s] = a + cZ * ku;
-            dst[RN + s] = b + cZ * kv;
-            dst[2 * RN + s] = e + cZ * kw;
+            dst[s] = fma(cZ, ku, a);
+            dst[RN + s] = fma(cZ, kv, b);
+            dst[2 * RN + s] = fma(cZ, kw, e);
             if (inner) {
                 if (MODE == 0) {
                     D[d] = cD * ku;
                     D[IN + d] = cD * kv;
                     D[2 * IN + d] = cD * kw;
                 } else {
-                    D[d] = D[d] + cD * ku;
-                    D[IN + d] = D[IN + d] + cD * kv;
-                    D[2 * IN + d] = D[2 * IN + d] + cD * kw;
+                    D[d] = fma(cD, ku, D[d]);
+                    D[IN + d] = fma(cD, kv, D[IN + d]);
+                    D[2 * IN + d] = fma(cD, kw, D[2 * IN + d]);
                 }
             }
         }
@@ -925,14 +920,14 @@ __device__ __forceinline__ void adj_fused_tile(const DevModel& P, const DevGrid&
                 a0[1] = __ldg(fa + g.plane + o);
                 a0[2] = __ldg(fa + 2 * g.plane + o);
             } else {
-                rhs_at<RW, RN>(P, YA, s, Ea * gg, a0[0], a0[1], a0[2], g.fcode ? (int)__ldg(g.fcode + o) : -1);
+                rhs_at<RW, RN>(P, YA, s, Ea, gg, a0[0], a0[1], a0[2]);
             }
             if (fb) {
                 a1[0] = __ldg(fb + o);
                 a1[1] = __ldg(fb + g.plane + o);
                 a1[2] = __ldg(fb + 2 * g.plane + o);
             } else {
-                rhs_at<RW, RN>(P, YB, s, Eb * gg, a1[0], a1[1], a1[2], g.fcode ? (int)__ldg(g.fcode + o) : -1);
+                rhs_at<RW, RN>(P, YB, s, Eb, gg, a1[0], a1[1], a1[2]);
             }
             if (fout && r >= HALO && r < HALO + TY && c >= HALO && c < HALO + TX) {
                 fout[o] = a0[0];
@@ -946,8 +941,8 @@ __device__ __forceinline__ void adj_fused_tile(const DevModel& P, const DevGrid&
             for (int f = 0; f < 3; ++f) {
                 const double m0 = a0[f] * dt, m1 = a1[f] * dt;
                 const double x0 = YA[f * RN + s], x1 = YB[f * RN + s];
-                Y3[f * RN3 + s3] = ((hw.c3[0] * x0 + hw.c3[1] * m0) + hw.c3[2] * x1) + hw.c3[3] * m1;
-                if (qcell) Q[f * RNQ + sq] = ((hw.c4[0] * x0 + hw.c4[1] * m0) + hw.c4[2] * x1) + hw.c4[3] * m1;
+                Y3[f * RN3 + s3] = hermite4(hw.c3, x0, m0, x1, m1);
+                if (qcell) Q[f * RNQ + sq] = hermite4(hw.c4, x0, m0, x1, m1);
             }
         }
     }
@@ -964,10 +959,9 @@ __device__ __forceinline__ void adj_fused_tile(const DevModel& P, const DevGrid&
             const int s3 = (r - 1) * W3 + (c - 1);
             const int sq = (r - 2) * WQ + (c - 2);
             double m2[3];
-            rhs_at<W3, RN3>(P, Y3, s3, E3 * __ldg(gh + o), m2[0], m2[1], m2[2],
-                            g.fcode ? (int)__ldg(g.fcode + o) : -1);
+            rhs_at<W3, RN3>(P, Y3, s3, E3, __ldg(gh + o), m2[0], m2[1], m2[2]);
 #pragma unroll
-            for (int f = 0; f < 3; ++f) Q[f * RNQ + sq] = Q[f * RNQ + sq] + hw.c2 * (m2[f] * dt);
+            for (int f = 0; f < 3; ++f) Q[f * RNQ + sq] = fma(hw.c2, m2[f] * dt, Q[f * RNQ + sq]);
         }
     }
     __syncthreads();
@@ -975,14 +969,14 @@ __device__ __forceinline__ void adj_fused_tile(const DevModel& P, const DevGrid&
     auto j_yb = [&](int r, int c, long long o) -> JacT {
         if (jb) return load_jac(jb, g.plane, o);
         const int s = r * RW + c;
-        return fk_jacT(P, finite_u(YB[s]), YB[RN + s], YB[2 * RN + s]);
+        return fk_jacT(P, YB[s], YB[RN + s], YB[2 * RN + s]);
     };
     auto j_yh = [&](int r, int c, long long) -> JacT {
         const int sq = (r - 2) * WQ + (c - 2);
         return fk_jacT(P, Q[sq], Q[RNQ + sq], Q[2 * RNQ + sq]);
     };
     auto j_ya = [&](int, int, long long o) -> JacT {
-        const JacT J = fk_jacT(P, finite_u(__ldg(ya + o)), __ldg(ya + g.plane + o), __ldg(ya + 2 * g.plane + o));
+        const JacT J = fk_jacT(P, __ldg(ya + o), __ldg(ya + g.plane + o), __ldg(ya + 2 * g.plane + o));
         if (ja) store_jac(ja, g.plane, o, J);
         return J;
     };
@@ -1038,10 +1032,10 @@ __device__ __forceinline__ void exact_stage(const DevModel& P, const DevGrid& g,
             out[g.plane + o] = lb + (D[IN + d] + kv);
             out[2 * g.plane + o] = lc + (D[2 * IN + d] + kw);
         } else {
-            const double au = cL * la + cM * ku;
+            const double au = fma(cM, ku, cL * la);
             dst[s] = au;
-            dst[RN + s] = cL * lb + cM * kv;
-            dst[2 * RN + s] = cL * lc + cM * kw;
+            dst[RN + s] = fma(cM, kv, cL * lb);
+            dst[2 * RN + s] = fma(cM, kw, cL * lc);
             if (inner) {
                 if (MODE == 0) {
                     D[d] = ku;
@@ -1084,7 +1078,7 @@ __device__ __forceinline__ void exact_stage(const DevModel& P, const DevGrid& g,
             if (isnan(src[s])) {  // holes and the NaN ring: the result is NaN
                 ku = kv = kw = src[s];
             } else {
-                const JacT J = fk_jacT(P, finite_u(cur.y[0]), cur.y[1], cur.y[2]);
+                const JacT J = fk_jacT(P, cur.y[0], cur.y[1], cur.y[2]);
                 adj_at<RW, RN>(P, src, s, cur.code, J, ku, kv, kw);
             }
             finish(r, c, s, o, cur.l[0], cur.l[1], cur.l[2], ku, kv, kw);
@@ -1097,14 +1091,11 @@ __device__ __forceinline__ void exact_stage(const DevModel& P, const DevGrid& g,
             const int s = r * RW + c;
             const long long o = off + (long long)r * g.ld + c;
             double ku, kv, kw;
-#if FKADJ_HOLE_BRANCH
             if (isnan(src[s])) {  // holes and the NaN ring: the result is NaN
                 ku = kv = kw = src[s];
-            } else
-#endif
-            {
+            } else {
                 const JacT J =
-                    fk_jacT(P, finite_u(__ldg(ys + o)), __ldg(ys + g.plane + o), __ldg(ys + 2 * g.plane + o));
+                    fk_jacT(P, __ldg(ys + o), __ldg(ys + g.plane + o), __ldg(ys + 2 * g.plane + o));
                 adj_at<RW, RN>(P, src, s, __ldg(wc + o), J, ku, kv, kw);
             }
             const double la = __ldg(lamg + o), lb = __ldg(lamg + g.plane + o), lc = __ldg(lamg + 2 * g.plane + o);
