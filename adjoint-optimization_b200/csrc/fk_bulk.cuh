@@ -47,6 +47,17 @@ __device__ __forceinline__ void bulk_arrive(uint32_t bar, uint32_t bytes) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+// One row of WIDTH doubles.
+template <int WIDTH>
+__device__ __forceinline__ void bulk_row(uint32_t bar, double* dst, const double* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const size_t s = __cvta_generic_to_global(src);
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d), "l"(s),
+        "n"(WIDTH * 8), "r"(bar)
+        : "memory");
+}
+
 // Issues the copies of one window, spread over the NT threads.
 template <int RCAP, int WIDTH, int NT>
 __device__ __forceinline__ void bulk_issue(uint32_t bar, double* dst, const double* src, int ld, long long plane,
@@ -54,12 +65,7 @@ __device__ __forceinline__ void bulk_issue(uint32_t bar, double* dst, const doub
     constexpr int RN = RCAP * WIDTH;
     for (int t = threadIdx.x; t < 3 * rows; t += NT) {
         const int f = t / rows, r = t - f * rows;
-        const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + f * RN + r * WIDTH);
-        const size_t gsrc = __cvta_generic_to_global(src + f * plane + (long long)r * ld);
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-            "l"(gsrc), "n"(WIDTH * 8), "r"(bar)
-            : "memory");
+        bulk_row<WIDTH>(bar, dst + f * RN + r * WIDTH, src + f * plane + (long long)r * ld);
     }
 }
 

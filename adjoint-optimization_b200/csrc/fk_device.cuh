@@ -290,6 +290,11 @@ __device__ __forceinline__ void rhs_at(const DevModel& P, const double* __restri
     fk_field(P, y, t, E, gh, fu, fv, fw);
 }
 
+// Hermite combination c0 x0 + c1 m0 + c2 x1 + c3 m1, in this order
+__device__ __forceinline__ double hermite4(const double (&c)[4], double x0, double m0, double x1, double m1) {
+    return fma(c[3], m1, fma(c[2], x1, fma(c[1], m0, c[0] * x0)));
+}
+
 // Weight code of the transposed Laplacian at a cell: 2 bits per direction
 // (north, south, west, east), value 0 (neighbour missing), 1, or 2 (the
 // neighbour mirrored this cell); rule of cu-G:1004-1111.
@@ -297,9 +302,6 @@ __device__ __forceinline__ int wcode_n(int c) { return c & 3; }
 __device__ __forceinline__ int wcode_s(int c) { return (c >> 2) & 3; }
 __device__ __forceinline__ int wcode_w(int c) { return (c >> 4) & 3; }
 __device__ __forceinline__ int wcode_e(int c) { return (c >> 6) & 3; }
-
-// The code of a cell all of whose weights are 1
-constexpr int WCODE_PLAIN = 0x55;
 
 // J_F^T z plus D/h^2 times the transposed-Laplacian sums t.
 __device__ __forceinline__ void adj_field(const DevModel& P, const JacT& J, const double (&z)[3],
@@ -309,16 +311,22 @@ __device__ __forceinline__ void adj_field(const DevModel& P, const JacT& J, cons
     gw = fma(P.cw, t[2], fma(J.a5, z[0], J.a6 * z[2]));
 }
 
-// Weighted neighbour sum at shared-memory cell q of one field (missing
-// neighbours, weight 0, are not read into the sum: they hold NaN).  The
-// products with the weights 0, 1, 2 are exact, so weights of 1 give lap4's bits.
+// Weighted neighbour sum at shared-memory cell q of one field, minus four times
+// the centre: the plain sum, missing neighbours (weight 0; they hold NaN) as 0,
+// then those of weight 2 once more.
 template <int W>
 __device__ __forceinline__ double lapT_at(const double* __restrict__ Z, int q, int code) {
     const int cn = wcode_n(code), cs = wcode_s(code), cw = wcode_w(code), ce = wcode_e(code);
     const double vn = cn ? Z[q - W] : 0.0, vs = cs ? Z[q + W] : 0.0;  // integer tests: no FP64 compares
     const double vw = cw ? Z[q - 1] : 0.0, ve = ce ? Z[q + 1] : 0.0;
-    const double s = fma((double)ce, ve, fma((double)cw, vw, fma((double)cs, vs, (double)cn * vn)));
-    return fma(-4.0, Z[q], s);
+    double t = lap4(vn, vs, vw, ve, Z[q]);
+    if (code & 0xaa) {
+        if (cn == 2) t += vn;
+        if (cs == 2) t += vs;
+        if (cw == 2) t += vw;
+        if (ce == 2) t += ve;
+    }
+    return t;
 }
 
 // Adjoint vector field L^T z + J_F(y)^T z at shared-memory cell q.

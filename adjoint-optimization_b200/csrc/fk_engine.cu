@@ -187,7 +187,7 @@ Problem::~Problem() {
         // below): release the buffers first
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &xchg_, &pts_};
         for (DevBuf* b : all) b->release();
     }
     for (auto& r : prof_pool_) {
@@ -215,7 +215,7 @@ Problem::~Problem() {
     if (verbose_ > 1) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &xchg_, &pts_};
         size_t bytes = 0;
         for (DevBuf* b : all) bytes += b->bytes;
         for (DevBuf* b : all) b->release();
@@ -381,6 +381,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
         std::lock_guard<std::mutex> lk(g_init_mu);
         if (device_ < 64 && !g_init_done[device_]) {
             CK(kernels_init(), "kernel attribute setup");
+            CK(run_init(), "kernel attribute setup");
             g_init_done[device_] = true;
         }
     }
@@ -394,7 +395,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     if (pool_) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &xchg_, &pts_};
         for (DevBuf* b : all) b->st = st_, b->pool = pool_;
     }
     {
@@ -492,6 +493,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
                                weight(i, j, 0, 1) << 6);
             pos[a - 1] = (long long)o2;
         }
+    if (fkadj_status s = init_sweeps(ai, gh, wc)) return s;
     CK(gh_.alloc(pl * sizeof(double)), "alloc gh");
     CK(wc_.alloc(pl), "alloc weights");
     CK(pos_.alloc((size_t)n_num * sizeof(long long)), "alloc positions");
@@ -546,29 +548,75 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     return FKADJ_OK;
 }
 
+// Whether and how this problem's sweeps run as one launch each (fk_run.h): with
+// autotuned tiles, where the grid's tiles fit the device at once and every
+// active cell keeps a neighbour in both directions.  ai: the active index of
+// every cell; gh: the padded source plane.  FKADJ_SWEEPS=0 in the environment keeps one launch
+// per step.
+fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, const std::vector<uint8_t>& wc) {
+    run_ = RunShape();
+    CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "device attribute");
+    const char* v = getenv("FKADJ_SWEEPS");
+    if (!autotune_ || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ ||
+        (v && v[0] == '0')) return FKADJ_OK;
+    const char* sv = getenv("FKADJ_ZGH_SEGMENTS");  // the adjoint sweeps write row segments
+    if (sv && std::atoi(sv) == 0) return FKADJ_OK;
+    int coop = 0;
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_), "device attribute");
+    const RunShape shape = coop ? run_shape(g_, sms_) : RunShape();
+    if (shape.id < 0) return FKADJ_OK;
+    const int ld = g_.ld;
+    std::vector<uint8_t> cells((size_t)g_.plane, 0), adj((size_t)g_.plane, 0);
+    for (int i = 0; i < g_.nrows; ++i)
+        for (int j = 0; j < g_.ncols; ++j) {
+            const int k = i * g_.ncols + j;
+            if (ai[k] <= 0) continue;
+            const size_t o = (size_t)(i + HALO) * ld + (j + HALO);
+            const bool n = i == 0 || ai[k - g_.ncols] <= 0, s = i == g_.nrows - 1 || ai[k + g_.ncols] <= 0;
+            const bool w = j == 0 || ai[k - 1] <= 0, e = j == g_.ncols - 1 || ai[k + 1] <= 0;
+            if ((n && s) || (w && e)) return FKADJ_OK;
+            cells[o] = (uint8_t)(CELL_ACTIVE | (n ? CELL_N : 0) | (s ? CELL_S : 0) | (w ? CELL_W : 0) |
+                                 (e ? CELL_E : 0) | (gh[o] != 0.0 ? CELL_SOURCE : 0));
+            const int c = wc[o];
+            adj[o] = (uint8_t)(CELL_ACTIVE_ADJ | ((c & 3) == 2 ? CELL_2N : 0) | ((c >> 2 & 3) == 2 ? CELL_2S : 0) |
+                               ((c >> 4 & 3) == 2 ? CELL_2W : 0) | ((c >> 6 & 3) == 2 ? CELL_2E : 0));
+        }
+    CK(cells_.alloc(cells.size()), "alloc cell flags");
+    CK(cudaMemcpyAsync(cells_.p, cells.data(), cells.size(), cudaMemcpyHostToDevice, st_), "upload cell flags");
+    CK(adjf_.alloc(adj.size()), "alloc cell flags");
+    CK(cudaMemcpyAsync(adjf_.p, adj.data(), adj.size(), cudaMemcpyHostToDevice, st_), "upload cell flags");
+    CK(xchg_.alloc(run_exchange_bytes(g_)), "alloc edge exchange");
+    CK(cudaMemsetAsync(xchg_.p, 0, xchg_.bytes, st_), "clear edge exchange");
+    run_ = shape;
+    return FKADJ_OK;
+}
+
 int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t nnz, int grad_mode, int policy,
                                 bool want_grad) {
     const int64_t ld = round_up(round_up(ncols, 64) + 2 * HALO, 8);
     const int64_t rows = round_up(nrows, 64) + 2 * HALO;
     const int64_t plane = rows * ld * 8, state = 3 * plane;
-    int64_t b = plane + plane / 8 + (int64_t)n_num * (8 + 48) + nnz * 12 + 4 * state;  // geometry, compact, work
+    // geometry (and the sweeps' flags), compact, work, the sweeps' exchange
+    int64_t b = plane + 3 * (plane / 8) + (int64_t)n_num * (8 + 48) + nnz * 12 + 8 * state;
     if (!want_grad) return b;
     const int64_t nsb = (round_up(ncols, 64) / 16) * (round_up(nrows, 64) / 16);
     b += 2 * state + (int64_t)(3 * nt + 1) * (nsb + 1) * 8;  // adjoint pair, partials
-    b += grad_mode == FKADJ_GRAD_EXACT ? 3 * state : state + 27 * plane;  // stages | yh + caches
+    // stage states of a chunk | midpoint states of a chunk (more than yh and the caches)
+    b += grad_mode == FKADJ_GRAD_EXACT ? 3 * kSweepChunkExact * state : kSweepChunk * state;
     if (policy == FKADJ_CKPT_FULL) {
         b += (int64_t)(nt + 1) * state;
     } else {
         const int64_t c = std::max(2, (int)std::ceil(std::sqrt((double)nt)));
         b += ((nt + c - 1) / c + 1 + c - 1) * state;
-        if (grad_mode == FKADJ_GRAD_REF) b += (c - 1) * state;  // k1 kept by the segment recompute
+        b += grad_mode == FKADJ_GRAD_REF ? (c - 1) * state : 3 * c * state;  // kept by the segment recompute
     }
     return b;
 }
 
 int64_t Problem::device_bytes() const {
     const DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_,
-                           &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_, &fcache_};
+                           &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_, &fcache_,
+                           &cells_, &adjf_, &xchg_, &pts_};
     int64_t s = 0;
     for (auto* b : all) s += (int64_t)b->bytes;
     return s;
@@ -631,17 +679,19 @@ fkadj_status Problem::upload_state(const double* y_ini, double* d_state) {
     return FKADJ_OK;
 }
 
-cudaError_t Problem::prof_begin(int k) {
+cudaError_t Problem::prof_begin(int k, int steps) {
     prof_open_ = false;
-    if (!profiling_ || (kcount_[k]++ % prof_every_) != 0) return cudaSuccess;
+    // single steps are sampled, whole sweeps always timed
+    if (!profiling_ || (steps == 1 && (kcount_[k]++ % prof_every_) != 0)) return cudaSuccess;
     if (prof_used_ == prof_pool_.size()) {
-        ProfRec r{k, nullptr, nullptr};
+        ProfRec r{k, 1, nullptr, nullptr};
         cudaError_t e = cudaEventCreate(&r.a);
         if (e == cudaSuccess) e = cudaEventCreate(&r.b);
         if (e != cudaSuccess) return e;
         prof_pool_.push_back(r);
     }
     prof_pool_[prof_used_].k = k;
+    prof_pool_[prof_used_].n = steps;
     prof_open_ = true;
     return cudaEventRecord(prof_pool_[prof_used_].a, st_);
 }
@@ -656,8 +706,11 @@ cudaError_t Problem::prof_end(int k) {
 fkadj_status Problem::check_fault() {
     unsigned f = 0;
     CK(take_device_fault(st_, fault(), &f), "read the problem's fault word");
-    if (f) {
-        set_error("a bounded wait in a kernel expired (tile copy into shared memory); results are invalid");
+    nan_seen_ = (f & FAULT_NAN) != 0;
+    if (f & ~FAULT_NAN) {
+        nan_seen_ = false;
+        set_error("a bounded wait in a kernel expired (tile copy into shared memory, or a neighbouring tile's step); "
+                  "results are invalid");
         return FKADJ_ERR_TIMEOUT;
     }
     return FKADJ_OK;
@@ -670,7 +723,7 @@ fkadj_status Problem::prof_collect() {
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, prof_pool_[q].a, prof_pool_[q].b), "event time");
         kms_[prof_pool_[q].k] += ms;
-        ksamples_[prof_pool_[q].k]++;
+        ksamples_[prof_pool_[q].k] += prof_pool_[q].n;
     }
     prof_used_ = 0;
     return FKADJ_OK;
@@ -692,6 +745,108 @@ fkadj_status Problem::step_forward(int i, const double* yin, double* yout, doubl
     return FKADJ_OK;
 }
 
+fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* last, double* out, double* keep) {
+    if (n <= 0) return FKADJ_OK;
+    const long long stride = (long long)state_elems();
+    if (!sweeping()) {
+        // two states other than src for the steps in between
+        double* s0 = src == state_buf(1) ? state_buf(0) : state_buf(1);
+        double* s1 = src == state_buf(2) ? state_buf(0) : state_buf(2);
+        if (last == ((n & 1) ? s1 : s0)) std::swap(s0, s1);
+        const double* cur = src;
+        for (int k = 0; k < n; ++k) {
+            double* o = k == n - 1 ? last : (out ? out + k * stride : ((k & 1) ? s1 : s0));
+            if (fkadj_status s = step_forward(i + k, cur, o, keep ? keep + k * stride : nullptr)) return s;
+            cur = o;
+        }
+        return FKADJ_OK;
+    }
+    FwdRun r{};
+    r.src = src;
+    r.last = last;
+    r.out = out;
+    r.stages = keep;
+    r.stride = stride;
+    r.n = n;
+    r.Et = etab() + i;
+    r.Eh = etab() + (nt_ + 1) + i;
+    r.exchange = xchg_.p;
+    r.epoch = epoch_;
+    r.fault = fault();
+    epoch_ += (unsigned long long)n;
+    CK(prof_begin(K_FWD, n), "profiling event");
+    CK(launch_fwd_run(run_, P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), r, st_), "forward sweep");
+    CK(prof_end(K_FWD), "profiling event");
+    ++launches_;
+    return FKADJ_OK;
+}
+
+fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
+                                    const double* stages, double*& z, double*& z2) {
+    const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
+    const long long sz = (long long)state_elems();
+    auto state = [&](int t) { return t == hi ? y_hi : (t == lo ? y_lo : mid + (t - lo - 1) * sz); };
+    for (int top = hi; top > lo;) {
+        // a chunk's rows of partial sums (top - 1 down) stay within one window
+        const int n = std::min({top - lo, exact && !stages ? kSweepChunkExact : kSweepChunk, (top - 1) % pwin_ + 1});
+        AdjRun r{};
+        r.zin = z;
+        r.zout = z2;
+        r.y_hi = state(top);
+        r.y_mid = mid + (long long)(top - n - lo) * sz;
+        r.y_lo = state(top - n);
+        r.stride = sz;
+        r.n = n;
+        r.partial = partial_.as<double>();
+        r.nsb = nsb_;
+        r.nsbx = nsbx_;
+        r.row0 = top - 1;
+        r.window = pwin_;
+        r.exchange = xchg_.p;
+        r.epoch = epoch_;
+        r.fault = fault();
+        epoch_ += (unsigned long long)n;
+        r.pts = pts_.as<double>();
+        r.pts_step = exact ? 3 : 1;
+        if (exact && stages) {
+            r.pts = stages + 3 * (long long)(top - 1 - lo) * sz;
+            r.pts_step = -3;
+        } else if (exact) {
+            epoch_ += (unsigned long long)n;
+            for (int k = 0; k < n; ++k)
+                if (fkadj_status s = sweep_forward(top - 1 - k, 1, state(top - 1 - k), state_buf(1), nullptr,
+                                                   pts_.as<double>() + 3 * k * sz))
+                    return s;
+        } else {
+            MidRun m{};
+            m.y_hi = r.y_hi;
+            m.y_mid = r.y_mid;
+            m.y_lo = r.y_lo;
+            m.yh = pts_.as<double>();
+            m.stride = sz;
+            m.n = n;
+            m.Et = etab() + top;
+            m.E3 = etab() + (2 * nt_ + 1) + top - 1;
+            m.fault = fault();
+            CK(prof_begin(K_MID, n), "profiling event");
+            CK(launch_mid_run(P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), hw_, m, sms_, st_), "adjoint midpoints");
+            CK(prof_end(K_MID), "profiling event");
+            ++launches_;
+        }
+        CK(prof_begin(K_ADJ, n), "profiling event");
+        CK(launch_adj_run(run_, exact, P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), adjf_.as<uint8_t>(), r, st_),
+           "adjoint sweep");
+        CK(prof_end(K_ADJ), "profiling event");
+        ++launches_;
+        std::swap(z, z2);
+        top -= n;
+        // as in the per-step sweeps: a sqrt store reduces at the end of each segment
+        if (traj_plan_.policy != FKADJ_CKPT_SQRT && top % pwin_ == 0)
+            for (int g = 0; g < (exact ? 3 : 1); ++g) CK(flush_rows(g, top, exact ? nt_ : nt_ + 1), "reduce z.gh");
+    }
+    return FKADJ_OK;
+}
+
 fkadj_status Problem::download_grid(const double* d_state, double* host) {
     const size_t n = (size_t)g_.nrows * g_.ncols;
     for (int f = 0; f < 3; ++f) {
@@ -704,7 +859,7 @@ fkadj_status Problem::download_grid(const double* d_state, double* host) {
     return FKADJ_OK;
 }
 
-fkadj_status Problem::forward(const double* Et, const double* y_ini, int nstep, int ns, double* ys, double* yf) {
+fkadj_status Problem::forward_call(const double* Et, const double* y_ini, int nstep, int ns, double* ys, double* yf) {
     fkadj_status s;
     launches_ = 0;
     if ((s = prepare_E(Et))) return s;
@@ -715,20 +870,20 @@ fkadj_status Problem::forward(const double* Et, const double* y_ini, int nstep, 
     CK(cudaEventRecord(ev_[0], st_), "event");
     double* b0 = state_buf(0);
     if ((s = upload_state(y_ini, b0))) return s;
-    if (autotune_ && !tuned_fwd_) {
+    if (autotune_ && !tuned_fwd_ && !sweeping()) {
         if ((s = autotune())) return s;
         tuned_fwd_ = true;
     }
     double* cur = b0;
     const size_t n3 = (size_t)3 * g_.nrows * g_.ncols;
-    for (int i = 0; i < nt_; ++i) {
+    for (int i = 0, ks = 0; i < nt_;) {
+        // up to the next snapshot (cu-F:794-814), or to the end
+        const int n = ks < ns ? std::min(nstep, nt_ - i) : nt_ - i;
         double* out = (cur == state_buf(1)) ? state_buf(2) : state_buf(1);
-        if ((s = step_forward(i, cur, out))) return s;
+        if ((s = sweep_forward(i, n, cur, out))) return s;
         cur = out;
-        if (nstep > 0 && (i + 1) % nstep == 0) {  // snapshots (cu-F:794-814)
-            const int ks = (i + 1) / nstep - 1;
-            if (ks < ns && (s = download_grid(cur, ys + (size_t)ks * n3))) return s;
-        }
+        i += n;
+        if (ks < ns && i == (ks + 1) * nstep && (s = download_grid(cur, ys + (size_t)ks++ * n3))) return s;
     }
     CK(cudaEventRecord(ev_[1], st_), "event");
     CK(cudaEventRecord(ev_[2], st_), "event");
@@ -772,23 +927,20 @@ fkadj_status Problem::run_objective(const double* yT, double* L0) {
     return FKADJ_OK;
 }
 
-fkadj_status Problem::objective(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
-                                double* yf) {
+fkadj_status Problem::objective_call(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
+                                     double* yf) {
     fkadj_status s;
     launches_ = 0;
     if ((s = prepare_E(Et))) return s;
     CK(cudaEventRecord(ev_[0], st_), "event");
     double* cur = state_buf(0);
     if ((s = upload_state(y_ini, cur))) return s;
-    if (autotune_ && !tuned_fwd_) {
+    if (autotune_ && !tuned_fwd_ && !sweeping()) {
         if ((s = autotune())) return s;
         tuned_fwd_ = true;
     }
-    for (int i = 0; i < nt_; ++i) {
-        double* out = (cur == state_buf(1)) ? state_buf(2) : state_buf(1);
-        if ((s = step_forward(i, cur, out))) return s;
-        cur = out;
-    }
+    if ((s = sweep_forward(0, nt_, cur, state_buf(1)))) return s;
+    cur = state_buf(1);
     CK(cudaEventRecord(ev_[1], st_), "event");
     double l0 = 0;
     if ((s = run_objective(cur, &l0))) return s;
@@ -872,12 +1024,18 @@ fkadj_status Problem::plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only) {
     }
     // reference mode: keep k1 = f(y) beside the states the backward sweep walks
     // (the midpoint kernel then reads it instead of evaluating it) when that
-    // also fits the budget
-    if (grad_mode_ == FKADJ_GRAD_REF && pol != FKADJ_CKPT_BINOMIAL) {
-        const double kslots = pol == FKADJ_CKPT_FULL ? (double)nt_ : (double)tp.seg_slots;
-        tp.keep_f = need + kslots * sb <= (double)ckpt_budget_;
-    }
+    // also fits the budget; swept problems evaluate f in k_mid_run, and keep
+    // the stage states in the exact mode instead of replaying each step
+    const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
+    tp.keep_f = pol != FKADJ_CKPT_BINOMIAL && exact == sweeping() &&
+                need + (double)kept_states(tp) * sb <= (double)ckpt_budget_;
     return FKADJ_OK;
+}
+
+// States that keep_f holds under plan tp.
+int64_t Problem::kept_states(const TrajPlan& tp) const {
+    if (grad_mode_ == FKADJ_GRAD_EXACT) return 3 * (int64_t)(tp.policy == FKADJ_CKPT_FULL ? nt_ : tp.stride);
+    return tp.policy == FKADJ_CKPT_FULL ? nt_ : tp.seg_slots;
 }
 
 fkadj_status Problem::ensure_traj(const TrajPlan& tp) {
@@ -899,8 +1057,7 @@ fkadj_status Problem::ensure_traj(const TrajPlan& tp) {
     }
     if (tp.keep_f) {
         // cells no tile writes (ring, padding) stay NaN, as f there is
-        const size_t k = tp.policy == FKADJ_CKPT_FULL ? (size_t)nt_ : (size_t)tp.seg_slots;
-        CK(kf_.alloc(k * state_bytes()), "alloc kept f");
+        CK(kf_.alloc((size_t)kept_states(tp) * state_bytes()), "alloc kept f");
         CK(cudaMemsetAsync(kf_.p, 0xff, kf_.bytes, st_), "init kept f");
     }
     traj_plan_ = tp;
@@ -912,7 +1069,18 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
         CK(zbuf_.alloc(2 * state_bytes()), "alloc adjoint states");
         CK(cudaMemsetAsync(zbuf_.p, 0xff, zbuf_.bytes, st_), "init adjoint states");
     }
-    if (grad_mode_ == FKADJ_GRAD_REF && !yh_.p) {
+    const bool sweep = sweeping() && !all_rows;
+    if (sweep) {
+        // midpoint states of a chunk, or the stage states of one where the plan keeps none
+        const size_t k = grad_mode_ == FKADJ_GRAD_REF ? (size_t)std::min(kSweepChunk, nt_)
+                         : traj_plan_.keep_f          ? 0
+                                                      : 3 * (size_t)std::min(kSweepChunkExact, nt_);
+        if (pts_.bytes < k * state_bytes()) {
+            CK(pts_.alloc(k * state_bytes()), "alloc adjoint points");
+            CK(cudaMemsetAsync(pts_.p, 0xff, pts_.bytes, st_), "init adjoint points");
+        }
+    }
+    if (grad_mode_ == FKADJ_GRAD_REF && !sweep && !yh_.p) {
         CK(yh_.alloc(state_bytes()), "alloc midpoint state");
         CK(cudaMemsetAsync(yh_.p, 0xff, yh_.bytes, st_), "init midpoint state");
         // Jacobian caches J(y) x2 and J(yh) (7 planes each), f(y) carry x2 (3 planes each)
@@ -921,7 +1089,7 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
         CK(fcache_.alloc(6 * (size_t)g_.plane * sizeof(double)), "alloc f cache");
         CK(cudaMemsetAsync(fcache_.p, 0xff, fcache_.bytes, st_), "init f cache");
     }
-    if (grad_mode_ == FKADJ_GRAD_EXACT && !stg_.p) {
+    if (grad_mode_ == FKADJ_GRAD_EXACT && !sweep && !stg_.p) {
         CK(stg_.alloc(3 * state_bytes()), "alloc stage states");
         CK(cudaMemsetAsync(stg_.p, 0xff, stg_.bytes, st_), "init stage states");
     }
@@ -946,30 +1114,27 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
         win = std::min(per_group, c >= kPartialWindow ? c : c * (kPartialWindow / c));
     }
     // Lattice of the partials: 16-cell row segments (16 times as many partials
-    // as 16x16 sub-blocks; the adjoint step's tiles may then take any height)
-    // for the reference-mode split step with windowed partials, where 64x32
-    // tiles fit the grid into one wave of CTAs, one per SM (512 x 512 and
-    // below: tiles of the one-wave height fill the wave, 512^2 x 2000 gradient
-    // 132.0 -> 129.4 ms; at 2048 x 2048, 14 waves, the 16-fold partials cost
-    // 1.4 %), and where a window of one sqrt segment of rows fits within the
-    // full rows of 16x16 partials that estimate_bytes counts; the window then
-    // shrinks, in whole segments under a sqrt store, to fit there.  The choice
-    // depends on the grid, the horizon and the device only, never on the store,
-    // so that every store gives the same bits.  The 16x16 lattice otherwise:
-    // the exact mode, the fused step, the batch engine's all-rows buffers, and
-    // under FKADJ_ZGH_SEGMENTS=0.
+    // as 16x16 sub-blocks; the adjoint tiles may then take any height) with
+    // windowed partials, where 64x32 tiles fit the grid into one wave of CTAs,
+    // one per SM, or sweeps could (512 x 512 and below: tiles of the one-wave
+    // height fill the wave, 512^2 x 2000 gradient 132.0 -> 129.4 ms; at 2048 x
+    // 2048, 14 waves, the 16-fold partials cost 1.4 %).  The window then
+    // shrinks, in whole segments under a sqrt store, towards the full rows of
+    // 16x16 partials, but holds a sqrt segment.  The choice depends on the grid
+    // and the device only, never on the store or the launches, so that all give
+    // the same bits.  The 16x16 lattice otherwise: the fused step, the batch
+    // engine's all-rows buffers, and under FKADJ_ZGH_SEGMENTS=0.
     const size_t nsb16 = (size_t)nsbx_ * (size_t)nsby_, nsbseg = (size_t)nsbx_ * (size_t)g_.nrows;
-    const size_t fit = prow * (nsb16 + 1) / nsbseg;  // rows of segment partials within that count
+    const size_t fit = prow * (nsb16 + 1) / nsbseg / (size_t)groups;  // rows of segment partials within that count
     const int c_sqrt = std::max(2, (int)std::ceil(std::sqrt((double)nt_)));  // plan_trajectory's stride
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_) != cudaSuccess) sms = 0;
-    const bool one_wave = (int64_t)((g_.nrows + 31) / 32) * ((g_.ncols + 63) / 64) <= (int64_t)sms;
-    bool segs = !all_rows && grad_mode_ == FKADJ_GRAD_REF && (forced_path_ < 0 || forced_path_ == ADJ_SPLIT) &&
-                one_wave && fit >= (size_t)std::min(per_group, c_sqrt);
+    const bool one_wave = (int64_t)((g_.nrows + 31) / 32) * ((g_.ncols + 63) / 64) <= (int64_t)sms_;
+    bool segs = !all_rows && (forced_path_ < 0 || forced_path_ == ADJ_SPLIT) &&
+                (one_wave || run_shape(g_, sms_).id >= 0);
     if (const char* sv = getenv("FKADJ_ZGH_SEGMENTS")) segs = segs && std::atoi(sv) != 0;
     if (segs && (size_t)win > fit) {
         const int c = sqrt_store ? traj_plan_.stride : 1;
-        win = (int)std::max<size_t>(std::min<size_t>((size_t)win, fit / (size_t)c * (size_t)c), (size_t)c);
+        win = (int)std::max<size_t>(std::min<size_t>((size_t)win, fit / (size_t)c * (size_t)c),
+                                    (size_t)(sqrt_store ? c : std::min({win, c_sqrt, kSweepChunk})));
     }
     if (all_rows) win = (int)prow;
     const size_t nsb = segs ? nsbseg : nsb16;
@@ -1097,8 +1262,8 @@ fkadj_status Problem::autotune_trials() {
         best = 1e30f;
         for (int t = 0; t < tile_count(); ++t) {
             int rows[2] = {0, 0}, nr = 1;  // 0 = the preset's height
-            if (kind == T_FWD || kind == T_MID || (kind == T_ADJ && segs_)) {
-                const int bal = balanced_rows(t, kind == T_FWD ? 0 : (kind == T_MID ? 1 : 2), g_);
+            if (kind == T_FWD || kind == T_MID || segs_) {
+                const int bal = balanced_rows(t, kind, g_);
                 if (bal > 0 && bal < tile_shape(t).ty) rows[nr++] = bal;
             }
             for (int k = 0; k < nr; ++k) {
@@ -1166,10 +1331,10 @@ fkadj_status Problem::autotune_trials() {
                             stg_.as<double>(),
                             ty_[T_FWD]);
         if (!e)
-            e = pick(T_EXACT, [&](int t, int) {
+            e = pick(T_EXACT, [&](int t, int ty) {
                 double* p = partial_.as<double>();
                 return launch_adj_exact(t, P_, g_, y, z2, y, stg_.as<double>(), wc_.as<uint8_t>(),
-                                        gh_.as<double>(), p, p + nsb_, p + 2 * (size_t)nsb_, nsbx_, st_, fault());
+                                        gh_.as<double>(), p, p + nsb_, p + 2 * (size_t)nsb_, nsbx_, st_, fault(), ty, segs_);
             });
     }
     // the trial launches wrote scratch partials: clear them
@@ -1191,16 +1356,7 @@ static int64_t binom_small_k(int64_t n, int k) {
 }
 
 fkadj_status Problem::advance(int a, int m, const double* src, double* dst) {
-    fkadj_status s;
-    const double* cur = src;
-    double* s1 = state_buf(1);
-    double* s2 = state_buf(2);
-    for (int t = a; t < m; ++t) {
-        double* out = (t == m - 1) ? dst : ((cur == s1) ? s2 : s1);
-        if ((s = step_forward(t, cur, out))) return s;
-        cur = out;
-    }
-    return FKADJ_OK;
+    return sweep_forward(a, m - a, src, dst);
 }
 
 // Where the binomial (revolve) schedule puts the checkpoint of a part [a, b)
@@ -1321,7 +1477,7 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
         CK(prof_end(K_FWD), "profiling event");
         CK(prof_begin(K_ADJ), "profiling event");
         CK(launch_adj_exact(tk_[T_EXACT], P_, g_, lam, lam2, y, stg, wc_.as<uint8_t>(), gh_.as<double>(),
-                            prow(0, t), prow(1, t), prow(2, t), nsbx_, st_, fault()),
+                            prow(0, t), prow(1, t), prow(2, t), nsbx_, st_, fault(), ty_[T_EXACT], segs_),
            "exact adjoint step");
         CK(prof_end(K_ADJ), "profiling event");
         launches_ += 2;
@@ -1332,7 +1488,10 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
             for (int g = 0; g < 3; ++g) CK(flush_rows(g, t, nt), "reduce z.gh");
         return FKADJ_OK;
     };
+    const bool sweep = sweeping();
     if (tp.policy == FKADJ_CKPT_FULL) {
+        if (sweep)
+            return sweep_adjoint(nt, 0, slot(nt), slot(1), slot(0), tp.keep_f ? fslot(0) : nullptr, lam, lam2);
         for (int t = nt - 1; t >= 0; --t)
             if ((s = back(t, slot(t)))) return s;
         return FKADJ_OK;
@@ -1340,7 +1499,9 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
     if (tp.policy == FKADJ_CKPT_BINOMIAL) {
         std::vector<double*> free;
         for (int k = tp.nslots - 1; k >= 2; --k) free.push_back(slot(k));
-        return reverse_binomial(nt, slot(0), free, [&](int t, const double* y) { return back(t, y); });
+        return reverse_binomial(nt, slot(0), free, [&](int t, const double* y) {
+            return sweep ? sweep_adjoint(t + 1, t, y, nullptr, y, nullptr, lam, lam2) : back(t, y);
+        });
     }
     for (int k = K - 1; k >= 0; --k) {
         const int s0 = k * c, s1 = std::min(s0 + c, nt);
@@ -1349,9 +1510,16 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
             return segslot(t - s0 - 1);
         };
         if ((s = segment_begin())) return s;
-        for (int t = s0; t < s1 - 1; ++t)
-            if ((s = step_forward(t, st(t), st(t + 1)))) return s;
-        for (int t = s1 - 1; t >= s0; --t)
+        // with kept stage states the sweep takes the segment's last step too
+        const bool keep = sweep && tp.keep_f;
+        if ((s = sweep_forward(s0, keep ? s1 - s0 : s1 - 1 - s0, slot(k), keep ? state_buf(1) : st(s1 - 1), segslot(0),
+                               keep ? fslot(0) : nullptr)))
+            return s;
+        if (sweep) {
+            if ((s = sweep_adjoint(s1, s0, slot(k + 1), segslot(0), slot(k), keep ? fslot(0) : nullptr, lam, lam2)))
+                return s;
+        }
+        for (int t = s1 - 1; t >= s0 && !sweep; --t)
             if ((s = back(t, st(t)))) return s;
         for (int g = 0; g < 3; ++g) CK(flush_range(g, s0, s1 - s0), "reduce z.gh");
         if ((s = segment_launch())) return s;
@@ -1381,33 +1549,31 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
     auto record = [&](cudaEvent_t e) {
         return capturing_ ? cudaEventRecordWithFlags(e, st_, cudaEventRecordExternal) : cudaEventRecord(e, st_);
     };
-    double* cur = slot(0);
     const bool binomial = tp.policy == FKADJ_CKPT_BINOMIAL;
-    // binomial: the forward sweep stores the schedule's spine; its k-th state
-    // goes to the k-th slot the reversal takes (free slots are taken from the
-    // back of nslots-1 .. 2)
-    const std::vector<int> spine = binomial ? binomial_spine(nt, tp.nslots - 2) : std::vector<int>();
-    size_t next_spine = 0;
-    for (int i = 0; i < nt; ++i) {
-        double* out;
-        if (tp.policy == FKADJ_CKPT_FULL) out = slot(i + 1);
-        else if (binomial) {
-            if (i + 1 == nt) out = slot(1);
-            else if (next_spine < spine.size() && spine[next_spine] == i + 1) out = slot(2 + (int)next_spine++);
-            else out = (cur == state_buf(1)) ? state_buf(2) : state_buf(1);
+    const bool sweep = sweeping();
+    double* cur = slot(0);
+    if (tp.policy == FKADJ_CKPT_FULL) {
+        if ((s = sweep_forward(0, nt, slot(0), slot(nt), slot(1), tp.keep_f ? fslot(0) : nullptr))) return s;
+        cur = slot(nt);
+    } else {
+        // binomial: the forward sweep stores the schedule's spine; its k-th state
+        // goes to the k-th slot the reversal takes (free slots are taken from the
+        // back of nslots-1 .. 2), y(T) to slot 1; sqrt: every c-th state and y(T)
+        const std::vector<int> spine = binomial ? binomial_spine(nt, tp.nslots - 2) : std::vector<int>();
+        for (int i = 0, k = 0; i < nt; ++k) {
+            int stop = nt;
+            if (binomial ? k < (int)spine.size() : i + c < nt) stop = binomial ? spine[k] : i + c;
+            double* out = binomial ? (stop == nt ? slot(1) : slot(2 + k)) : slot(k + 1);
+            if ((s = sweep_forward(i, stop - i, cur, out))) return s;
+            cur = out;
+            i = stop;
         }
-        else if ((i + 1) % c == 0) out = slot((i + 1) / c);
-        else if (i + 1 == nt) out = slot(K);
-        else out = (cur == state_buf(1)) ? state_buf(2) : state_buf(1);
-        double* k1 = (tp.policy == FKADJ_CKPT_FULL && tp.keep_f) ? fslot(i) : nullptr;
-        if ((s = step_forward(i, cur, out, k1))) return s;
-        cur = out;
     }
     double* yT = cur;
     *yT_out = yT;
     CK(record(ev_[1]), "event");
     // sqrt-store segments from graphs when this sequence is not itself captured
-    seg_on_ = segment_graphs_wanted();
+    seg_on_ = segment_graphs_wanted() && !sweep;
     struct SegmentGuard {
         Problem* p;
         ~SegmentGuard() { p->segment_abort(); }
@@ -1494,6 +1660,8 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
     };
     if (exact) {
         // backward sweep done above
+    } else if (sweep && tp.policy == FKADJ_CKPT_FULL) {
+        if ((s = sweep_adjoint(nt, 0, slot(nt), slot(1), slot(0), nullptr, z, z2))) return s;
     } else if (binomial) {
         // visits j = nt-1 .. 0 in order; step i = j+1 needs y_j and y_{j+1}:
         // y_{j+1} is the previous visit's state, kept in state_buf(0)
@@ -1502,7 +1670,8 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
         const double* prev = slot(1);  // y(T)
         double* keep = state_buf(0);
         auto visit = [&](int j, const double* yj) -> fkadj_status {
-            fkadj_status r = back_step(j + 1, yj, prev, nullptr, nullptr);
+            fkadj_status r = sweep ? sweep_adjoint(j + 1, j, prev, nullptr, yj, nullptr, z, z2)
+                                   : back_step(j + 1, yj, prev, nullptr, nullptr);
             if (r) return r;
             CK(cudaMemcpyAsync(keep, yj, state_bytes(), cudaMemcpyDeviceToDevice, st_), "keep state");
             prev = keep;
@@ -1530,9 +1699,13 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
                 return (tp.keep_f && t >= s0 && t <= s1 - 2) ? fslot(t - s0) : nullptr;
             };
             if ((s = segment_begin())) return s;
-            for (int t = s0; t < s1 - 1; ++t)
-                if ((s = step_forward(t, st(t), st(t + 1), kept(t)))) return s;
-            for (int i = s1; i > s0; --i)
+            if ((s = sweep_forward(s0, s1 - 1 - s0, slot(k), st(s1 - 1), segslot(0),
+                                   !sweep && tp.keep_f ? fslot(0) : nullptr)))
+                return s;
+            if (sweep) {
+                if ((s = sweep_adjoint(s1, s0, slot(k + 1), segslot(0), slot(k), nullptr, z, z2))) return s;
+            }
+            for (int i = s1; i > s0 && !sweep; --i)
                 if ((s = back_step(i, st(i - 1), st(i), kept(i - 1), kept(i)))) return s;
             CK(flush_range(0, s0, s1 - s0), "reduce z.gh");  // rows s0 .. s1-1
             if ((s = segment_launch())) return s;
@@ -1603,8 +1776,8 @@ fkadj_status Problem::grad_replay(const TrajPlan& tp, bool exact, double** yT) {
     return FKADJ_OK;
 }
 
-fkadj_status Problem::grad(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
-                           double* gradE, double* yf) {
+fkadj_status Problem::grad_call(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
+                                double* gradE, double* yf) {
     fkadj_status s;
     launches_ = 0;
     if (!gradE) {
@@ -1641,7 +1814,7 @@ fkadj_status Problem::grad(const double* Et, const double* y_ini, double* L0, do
     CK(cudaEventRecord(ev_[0], st_), "event");
     // ---- forward sweep, storing states (cu-G:1689-1724 without the D2H copies)
     if ((s = upload_state(y_ini, slot(0)))) return s;
-    if (autotune_ && !tuned_) {
+    if (autotune_ && !tuned_ && !sweeping()) {
         if ((s = autotune())) return s;
         tuned_ = tuned_fwd_ = true;
     }
@@ -1650,7 +1823,8 @@ fkadj_status Problem::grad(const double* Et, const double* y_ini, double* L0, do
     // the drop-in fkadj_grad, never pays for capture and instantiation).
     double* yT = nullptr;
     const GraphKey key = graph_key(tp, exact);
-    const bool replay = graphs_ && !profiling_ && ((gexec_ && key == gkey_) || key == seen_key_);
+    // (sweeps are a few launches each, and their exchange counts steps on: not captured)
+    const bool replay = graphs_ && !profiling_ && !sweeping() && ((gexec_ && key == gkey_) || key == seen_key_);
     seen_key_ = key;
     if ((s = replay ? grad_replay(tp, exact, &yT) : grad_sequence(tp, exact, &yT))) return s;
     if (yf && (s = download_grid(yT, yf))) return s;

@@ -13,6 +13,7 @@
 
 #include "../../include/fkadj.h"
 #include "fk_kernels.h"
+#include "fk_run.h"
 #include "fk_spline.h"
 
 namespace fkadj {
@@ -61,8 +62,9 @@ struct TrajPlan {
     int stride = 1;                // steps between stored states (SQRT)
     int nslots = 0;                // stored state slots
     int seg_slots = 0;             // recompute buffer slots
-    bool keep_f = false;           // k1 = f(y_t, Et[t]) kept beside the states the
-                                   // backward sweep walks (FULL: all, SQRT: the segment)
+    bool keep_f = false;           // kept beside the states the backward sweep walks (FULL: all,
+                                   // SQRT: the segment): k1 = f(y_t, Et[t]) (reference mode, per-step
+                                   // launches) or the three stage states (exact mode, sweeps)
     int64_t recompute = 0;         // forward steps the backward sweep recomputes
 };
 
@@ -78,10 +80,22 @@ public:
                       const int64_t* S_colptr, const int64_t* S_rowidx, const double* S_val, double alpha,
                       const fkadj_options* opt, bool need_objective);
 
-    fkadj_status forward(const double* Et, const double* y_ini, int nstep, int ns, double* ys, double* yf);
+    fkadj_status forward(const double* Et, const double* y_ini, int nstep, int ns, double* ys, double* yf) {
+        return with_sweeps([&] { return forward_call(Et, y_ini, nstep, ns, ys, yf); });
+    }
     fkadj_status objective(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
-                           double* yf);
+                           double* yf) {
+        return with_sweeps([&] { return objective_call(Et, y_ini, L0, LE, Lcost, yf); });
+    }
     fkadj_status grad(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
+                      double* gradE, double* yf) {
+        return with_sweeps([&] { return grad_call(Et, y_ini, L0, LE, Lcost, gradE, yf); });
+    }
+
+    fkadj_status forward_call(const double* Et, const double* y_ini, int nstep, int ns, double* ys, double* yf);
+    fkadj_status objective_call(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
+                                double* yf);
+    fkadj_status grad_call(const double* Et, const double* y_ini, double* L0, double* LE, double* Lcost,
                       double* gradE, double* yf);
 
     int64_t device_bytes() const;
@@ -113,7 +127,10 @@ public:
     int adjoint_path() const { return adj_path_; }
     int fused_tile() const { return tkf_; }
     // Stream-ordered device memory from `pool` (call before init).
-    void use_pool(cudaMemPool_t pool) { pool_ = pool; }
+    void use_pool(cudaMemPool_t pool) {
+        pool_ = pool;
+        own_sweeps_ = false;
+    }
     // A problem of a one-shot entry point (call before init): device memory
     // from `pool` (null: cudaMalloc), pinned staging from the process's cache.
     void set_oneshot(cudaMemPool_t pool) {
@@ -143,6 +160,22 @@ public:
     // standalone kernels read (the batched kernels take E by value).
     fkadj_status prepare_E(const double* Et, bool upload = true);
     fkadj_status step_forward(int i, const double* yin, double* yout, double* k1 = nullptr);
+    // n forward steps from step i, src -> last; the states between go to out +
+    // k * state_elems() (k = 0 .. n-2) when out is non-null; `keep` receives per
+    // step k1 = f of the state before it (reference mode: per-step launches) or
+    // the three stage states (exact mode: sweeps).  One launch where the grid
+    // is swept (sweeping()), n launches otherwise.
+    fkadj_status sweep_forward(int i, int n, const double* src, double* last, double* out = nullptr,
+                               double* keep = nullptr);
+    // Backward steps hi .. lo + 1 of a swept problem, z -> z (the pair is
+    // swapped as it goes): y_hi, y_lo the states at both ends, mid the states
+    // lo + 1 .. hi - 1 in a row, stages (exact mode; null: replayed) the stage
+    // states of steps lo .. hi - 1 in a row.
+    fkadj_status sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
+                               const double* stages, double*& z, double*& z2);
+    fkadj_status init_sweeps(const int* ai, const std::vector<double>& gh, const std::vector<uint8_t>& wc);
+    // whether sweeps run as one launch (fk_run.h) on this problem
+    bool sweeping() const { return run_.id >= 0 && !run_off_; }
     double* state_buf(int k) const { return work_.as<double>() + (size_t)k * state_elems(); }
     size_t state_elems() const { return (size_t)3 * g_.plane; }
     size_t state_bytes() const { return state_elems() * sizeof(double); }
@@ -150,11 +183,13 @@ public:
 private:
     fkadj_status fail_cuda(cudaError_t e, const char* what);
     // brackets a launch of kernel kind k with sampled events when profiling
-    cudaError_t prof_begin(int k);
+    cudaError_t prof_begin(int k, int steps = 1);
     cudaError_t prof_end(int k);
     fkadj_status prof_collect();
     // FKADJ_ERR_TIMEOUT when a kernel's bounded wait expired since the last check
     fkadj_status check_fault();
+    // a call that sweeps, repeated with per-step launches where check_fault found FAULT_NAN
+    template <class Call> fkadj_status with_sweeps(Call&& call);
     // Resolves the checkpoint policy.  AUTO takes FULL when the budget holds
     // every state, else whichever of SQRT and BINOMIAL fits and recomputes
     // fewer forward steps (costed in forward-step equivalents, the binomial
@@ -163,6 +198,7 @@ private:
     // sqrt_or_full_only (the batch engine, which runs no binomial schedule)
     // BINOMIAL only when SQRT does not fit.
     fkadj_status plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only = false);
+    int64_t kept_states(const TrajPlan& tp) const;
     fkadj_status ensure_traj(const TrajPlan& tp);
     fkadj_status run_objective(const double* yT, double* L0);
     fkadj_status objective_async(const double* yT);
@@ -247,6 +283,19 @@ private:
     DevBuf gh_, wc_, pos_, Srow_, Scol_, Sval_, yc_, zc_, opart_, osum_;
     DevBuf fault_;     // this problem's fault word: set by a step kernel whose bounded wait expired
     unsigned* fault() const { return fault_.as<unsigned>(); }
+    DevBuf cells_;     // geometry flags per padded cell (CELL_*), where the grid is swept
+    DevBuf adjf_;      // the adjoint sweeps' flags per padded cell
+    DevBuf xchg_;      // the sweeps' edge exchange
+    DevBuf pts_;       // points between the states of one chunk of an adjoint sweep
+    int sms_ = 0;
+    static constexpr int kSweepChunk = 16, kSweepChunkExact = 8;
+    RunShape run_;     // how the grid is swept (id -1: per-step launches)
+    unsigned long long epoch_ = 0;  // steps swept so far (the exchange's tags)
+    // per-step launches after all: a sweep met a NaN away from the holes
+    // (FAULT_NAN), which the per-step kernels contain
+    bool run_off_ = false;
+    bool nan_seen_ = false;
+    bool own_sweeps_ = true;  // false for a batch engine's problems, which run batched launches
     DevBuf work_;      // 4 states: two ping-pong, z pair is separate
     DevBuf zbuf_;      // 2 adjoint states
     DevBuf yh_;        // midpoint state
@@ -291,7 +340,7 @@ private:
     int64_t ksamples_[K_COUNT] = {0, 0, 0};
     double kms_[K_COUNT] = {0, 0, 0};
     struct ProfRec {
-        int k;
+        int k, n;
         cudaEvent_t a, b;
     };
     std::vector<ProfRec> prof_pool_;
@@ -304,6 +353,17 @@ private:
     Timing timing_{};
     int64_t launches_ = 0;
 };
+
+template <class Call>
+fkadj_status Problem::with_sweeps(Call&& call) {
+    nan_seen_ = false;
+    fkadj_status s = call();
+    if (!nan_seen_) return s;
+    run_off_ = true;
+    s = call();
+    run_off_ = false;
+    return s;
+}
 
 // The binomial schedule's first chain of checkpoints (the states the forward
 // sweep stores), and the forward steps its reversal then recomputes.

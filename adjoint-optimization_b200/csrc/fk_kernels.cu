@@ -436,11 +436,6 @@ __device__ __forceinline__ void store_jac(double* __restrict__ Jb, long long pla
     Jb[6 * plane + o] = J.a6;
 }
 
-// Hermite combination c0 x0 + c1 m0 + c2 x1 + c3 m1, in this order
-__device__ __forceinline__ double hermite4(const double (&c)[4], double x0, double m0, double x1, double m1) {
-    return fma(c[3], m1, fma(c[2], x1, fma(c[1], m0, c[0] * x0)));
-}
-
 // Midpoint state of step [t_{i-1}, t_i] (cu-G:1244-1301): y3 = cubic Hermite
 // at 1/3 from (ya, yb, dt*f(ya), dt*f(yb)); yh = partial quartic at 1/2 plus
 // (27/64) dt f(y3, E(t_{i-1}+dt/3)).  Halo 2: f(ya), f(yb) on the tile grown by
@@ -1018,14 +1013,17 @@ __device__ __forceinline__ void exact_stage(const DevModel& P, const DevGrid& g,
                                             double* __restrict__ dst, double* __restrict__ D,
                                             const double* __restrict__ lamg, const uint8_t* __restrict__ wc,
                                             const double* __restrict__ ys, long long off, double cL, double cM,
-                                            double* __restrict__ out, double* __restrict__ keep_u) {
+                                            double* __restrict__ out, double* __restrict__ keep_u, int rows,
+                                            double cS = 0.0) {
     constexpr int RW = TX + 2 * HALO, RH = TY + 2 * HALO, RN = RW * RH;
-    constexpr int W = TX + 2 * E, H = TY + 2 * E, N = W * H;
+    constexpr int W = TX + 2 * E;
     constexpr int IN = TX * TY;
+    const int N = W * (rows + 2 * E);
     // the stage update of cell (r, c) from its lambda and k
     auto finish = [&](int r, int c, int s, long long o, double la, double lb, double lc, double ku, double kv,
                       double kw) {
-        const bool inner = (E == 0) || (r >= HALO && r < HALO + TY && c >= HALO && c < HALO + TX);
+        const bool inner = (E == 0) || (r >= HALO && r < HALO + rows && c >= HALO && c < HALO + TX);
+        if (MODE == 0) ku = cS * ku, kv = cS * kv, kw = cS * kw;
         const int d = (r - HALO) * TX + (c - HALO);
         if (MODE == 2) {
             out[o] = la + (D[d] + ku);
@@ -1114,7 +1112,8 @@ __device__ __forceinline__ void adj_exact_tile(const DevModel& P, const DevGrid&
                                                const double* __restrict__ stages, const uint8_t* __restrict__ wc,
                                                const double* __restrict__ gh, double* __restrict__ r1,
                                                double* __restrict__ r23, double* __restrict__ r4, int nsbx, int tbx,
-                                               int tby, unsigned* fault = nullptr, uint32_t* phase = nullptr) {
+                                               int tby, unsigned* fault = nullptr, uint32_t* phase = nullptr,
+                                               int ty = TY, bool segments = false) {
     constexpr int RW = TX + 2 * HALO, RH = TY + 2 * HALO, RN = RW * RH;
     constexpr int IN = TX * TY;
     extern __shared__ double4 smem_raw[];
@@ -1122,36 +1121,40 @@ __device__ __forceinline__ void adj_exact_tile(const DevModel& P, const DevGrid&
     double* B = A + 3 * RN;
     double* D = B + 3 * RN;
     double* T3 = D + 3 * IN;  // a3_u on the tile
-    const int i0 = tby * TY, j0 = tbx * TX;
+    // rows as in adj_step_tile
+    const int i0 = tby * ty, j0 = tbx * TX;
+    const int rows = segments ? min(ty, g.nrows - i0) : TY;
     const long long off = (long long)i0 * g.ld + j0;
     const bool vec_ok = ((g.ld | j0) & 1) == 0;
-    if (!load_windows<RH, RW, NT, BULK>(A, lam + off, nullptr, nullptr, g.ld, g.plane, vec_ok, RH, fault, nullptr,
-                                        nullptr, phase))
+    if (!load_windows<RH, RW, NT, BULK>(A, lam + off, nullptr, nullptr, g.ld, g.plane, vec_ok, rows + 2 * HALO, fault,
+                                        nullptr, nullptr, phase))
         return;
     const double dt = P.dt;
     const double c6 = dt / 6.0, c3 = dt / 3.0, c2 = dt * 0.5;
-#pragma unroll 2
-    for (int q = threadIdx.x; q < 3 * RN; q += NT) A[q] = c6 * A[q];  // a4
-    __syncthreads();
     const long long sst = 3 * g.plane;
-    exact_stage<3, TX, TY, NT, 0, PF>(P, g, A, B, D, lam, wc, stages + 2 * sst, off, c3, dt, nullptr, T3);
-    exact_stage<2, TX, TY, NT, 1, PF>(P, g, B, A, D, lam, wc, stages + sst, off, c3, c2, nullptr, nullptr);
-    exact_stage<1, TX, TY, NT, 1, PF>(P, g, A, B, D, lam, wc, stages, off, c6, c2, nullptr, nullptr);
-    exact_stage<0, TX, TY, NT, 2, PF>(P, g, B, A, D, lam, wc, y, off, 0.0, 0.0, lamout, nullptr);
+    // the first stage takes g(a4) = c6 g(lambda), a4 = c6 lambda
+    exact_stage<3, TX, TY, NT, 0, PF>(P, g, A, B, D, lam, wc, stages + 2 * sst, off, c3, dt, nullptr, T3, rows, c6);
+    exact_stage<2, TX, TY, NT, 1, PF>(P, g, B, A, D, lam, wc, stages + sst, off, c3, c2, nullptr, nullptr, rows);
+    exact_stage<1, TX, TY, NT, 1, PF>(P, g, A, B, D, lam, wc, stages, off, c6, c2, nullptr, nullptr, rows);
+    exact_stage<0, TX, TY, NT, 2, PF>(P, g, B, A, D, lam, wc, y, off, 0.0, 0.0, lamout, nullptr, rows);
     __syncthreads();
     // now A holds a2 and B holds a1 on the tile
     auto ghv = [&](int r, int c) { return __ldg(gh + off + (long long)(r + HALO) * g.ld + (c + HALO)); };
     auto z0 = [](double t) { return isnan(t) ? 0.0 : t; };
-    subblock_sums<TX, TY, NT>([&](int r, int c) { return z0(B[(r + HALO) * RW + c + HALO] * ghv(r, c)); },
-                              r1, i0, j0, nsbx);
-    subblock_sums<TX, TY, NT>(
-        [&](int r, int c) { return z0((A[(r + HALO) * RW + c + HALO] + T3[r * TX + c]) * ghv(r, c)); }, r23, i0,
-        j0, nsbx);
-    subblock_sums<TX, TY, NT>(
-        [&](int r, int c) {
-            return z0(c6 * __ldg(lam + off + (long long)(r + HALO) * g.ld + (c + HALO)) * ghv(r, c));
-        },
-        r4, i0, j0, nsbx);
+    auto t1 = [&](int r, int c) { return z0(B[(r + HALO) * RW + c + HALO] * ghv(r, c)); };
+    auto t23 = [&](int r, int c) { return z0((A[(r + HALO) * RW + c + HALO] + T3[r * TX + c]) * ghv(r, c)); };
+    auto t4 = [&](int r, int c) {
+        return z0(c6 * __ldg(lam + off + (long long)(r + HALO) * g.ld + (c + HALO)) * ghv(r, c));
+    };
+    if (segments) {
+        segment_sums<TX, NT>(t1, r1, i0, j0, nsbx, rows);
+        segment_sums<TX, NT>(t23, r23, i0, j0, nsbx, rows);
+        segment_sums<TX, NT>(t4, r4, i0, j0, nsbx, rows);
+    } else {
+        subblock_sums<TX, TY, NT>(t1, r1, i0, j0, nsbx);
+        subblock_sums<TX, TY, NT>(t23, r23, i0, j0, nsbx);
+        subblock_sums<TX, TY, NT>(t4, r4, i0, j0, nsbx);
+    }
 }
 
 template <int TX, int TY, int NT>
@@ -1159,11 +1162,12 @@ __global__ void __launch_bounds__(NT, min_blocks(TX, TY, NT))
     k_adj_exact(DevModel P, DevGrid g, const double* __restrict__ lam, double* __restrict__ lamout,
                 const double* __restrict__ y, const double* __restrict__ stages, const uint8_t* __restrict__ wc,
                 const double* __restrict__ gh, double* __restrict__ r1, double* __restrict__ r23,
-                double* __restrict__ r4, int nsbx, unsigned* fault) {
+                double* __restrict__ r4, int nsbx, unsigned* fault, int ty, int segments) {
     pdl_enter();
     exp_table_init();
     adj_exact_tile<TX, TY, NT, true, FKADJ_ADJ_PREFETCH != 0>(P, g, lam, lamout, y, stages, wc, gh, r1, r23, r4, nsbx,
-                                                              blockIdx.x, blockIdx.y, fault);
+                                                              blockIdx.x, blockIdx.y, fault, nullptr, ty,
+                                                              segments != 0);
 }
 
 // ---------------------------------------------------------------- batched
@@ -1591,10 +1595,13 @@ cudaError_t launch_fwd_step(int tile, const DevModel& P, const DevGrid& g, const
 
 cudaError_t launch_adj_exact(int tile, const DevModel& P, const DevGrid& g, const double* lam, double* lamout,
                              const double* y, const double* stages, const uint8_t* wc, const double* gh,
-                             double* r1, double* r23, double* r4, int nsbx, cudaStream_t st, unsigned* fault) {
+                             double* r1, double* r23, double* r4, int nsbx, cudaStream_t st, unsigned* fault, int ty,
+                             bool segments) {
     DISPATCH(tile, {
-        const cudaError_t e = launch_pdl(k_adj_exact<TX, TY, NT>, tile_grid(g, TX, TY), NT, exact_smem<TX, TY>(), st,
-                                         P, g, lam, lamout, y, stages, wc, gh, r1, r23, r4, nsbx, fault);
+        const int rows = (segments && ty > 0 && ty < TY) ? ty : TY;
+        const cudaError_t e = launch_pdl(k_adj_exact<TX, TY, NT>, tile_grid(g, TX, rows), NT, exact_smem<TX, TY>(), st,
+                                         P, g, lam, lamout, y, stages, wc, gh, r1, r23, r4, nsbx, fault, rows,
+                                         segments ? 1 : 0);
         if (e != cudaSuccess) return e;
     });
     return cudaGetLastError();
@@ -1635,7 +1642,8 @@ int balanced_rows(int tile, int kind, const DevGrid& g) {
     DISPATCH(tile, {
         r = kind == 0   ? wave_rows(k_fwd_step<TX, TY, NT>, NT, stencil_smem<TX, TY>(NT), TX, TY, g)
             : kind == 1 ? wave_rows(k_adj_mid<TX, TY, NT>, NT, mid_smem<TX, TY>(), TX, TY, g)
-                        : wave_rows(k_adj_step<TX, TY, NT>, NT, stencil_smem<TX, TY>(NT), TX, TY, g);
+            : kind == 2 ? wave_rows(k_adj_step<TX, TY, NT>, NT, stencil_smem<TX, TY>(NT), TX, TY, g)
+                        : wave_rows(k_adj_exact<TX, TY, NT>, NT, exact_smem<TX, TY>(), TX, TY, g);
     });
     return r;
 }

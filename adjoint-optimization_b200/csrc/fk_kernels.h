@@ -126,19 +126,20 @@ cudaError_t launch_fwd_step(int tile, const DevModel& P, const DevGrid& g, const
 // (on by default; the engine turns it off while it captures a graph).
 void set_launch_pdl(bool on);
 // Rows per tile that fit grid g into one wave of CTAs of preset `tile` for
-// kernel kind 0 (forward step), 1 (adjoint midpoint) or 2 (adjoint step); the
+// kernel kind 0 (forward step), 1 (adjoint midpoint), 2 (adjoint step) or 3 (exact adjoint step); the
 // preset's height when it does not fit.
 int balanced_rows(int tile, int kind, const DevGrid& g);
 // The z.gh style reductions write one partial per 16x16 sub-block of the
 // grid's lattice (nsbx x nsby, covering the 64-padded grid); sub-blocks no
-// tile covers are never written and must be zero.  The reference-mode adjoint
-// step and launch_dot_gh can instead write one partial per 16-cell row segment
+// tile covers are never written and must be zero.  The adjoint steps and
+// launch_dot_gh can instead write one partial per 16-cell row segment
 // (segments = true: nsbx x nrows partials per row of results), which lets the
 // step's tiles take any number of rows.
 void subblock_lattice(const DevGrid& g, int* nsbx, int* nsby);
 cudaError_t launch_adj_exact(int tile, const DevModel& P, const DevGrid& g, const double* lam, double* lamout,
                              const double* y, const double* stages, const uint8_t* wc, const double* gh,
-                             double* r1, double* r23, double* r4, int nsbx, cudaStream_t st, unsigned* fault);
+                             double* r1, double* r23, double* r4, int nsbx, cudaStream_t st, unsigned* fault,
+                             int ty = 0, bool segments = false);
 cudaError_t launch_adj_mid(int tile, const DevModel& P, const DevGrid& g, const double* ya, const double* yb,
                            const double* gh, double* yh, const EStep& E, const HermiteW& hw, cudaStream_t st,
                            unsigned* fault, const double* fin = nullptr, double* fout = nullptr,

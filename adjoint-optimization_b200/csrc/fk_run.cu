@@ -1,0 +1,873 @@
+// fk_run.cu -- time sweeps as one launch each (sm_100a).
+//
+// A per-step launch of the forward step at 512 x 512 takes 15.2 us in a
+// replayed graph, of which about 4 us are the launch boundary and the tile
+// loads, and the rest runs the FP64 pipe half busy.  Where the grid's tiles
+// fit the device at once (one CTA per SM), a whole sweep runs as one
+// cooperative launch instead: each CTA keeps its tile in shared memory from
+// step to step and exchanges only the 4-cell edges with its eight neighbours
+// through L2, waiting for its own neighbours and no one else.
+//
+// The exchange carries its own arrival: every edge value travels as one
+// 16-byte store of the value and the step's number, and the reader polls the
+// value it needs until the number is right.  A flag per tile instead (stores,
+// barrier, fence, flag; poll, barrier, loads) measured 5 us a step: the fence
+// and the flag are round trips of their own.
+//
+// Inside a step, what bounds the work is the FP64 pipe (80 instructions per
+// evaluation, 2 cycles each per scheduler) and then the shared-memory data
+// path; so
+//  - a thread owns R rows of one column and walks down them, keeping the
+//    column's three values in registers: per field and cell the stencil reads
+//    (R + 2 + 2 R) / R values instead of 5;
+//  - the RK accumulator lives in registers (the owner never changes) and the
+//    step-start state stays in its own window, so no stage reads global memory;
+//  - missing neighbours come from per-cell flags, six bits per row held in one
+//    register for the whole sweep, as selects: the NaN test with its branch,
+//    taken by one warp in five, cost 2.4 us a step at 512 x 512, a separate
+//    pass over the flagged cells 1.5-2 us.
+#include "fk_run.h"
+
+#include <algorithm>
+
+#include "fk_bulk.cuh"
+
+namespace fkadj {
+
+namespace {
+
+// Kernel instances (id, TX, R, TYM): tiles of TX columns and up to TYM rows;
+// TYM + 6 is a multiple of R (the first stage's region, TYM + 6 rows of it).
+#define FKADJ_RUN_LIST(X) \
+    X(0, 64, 5, 29)       \
+    X(1, 64, 3, 15)       \
+    X(2, 32, 3, 30)       \
+    X(3, 32, 2, 18)       \
+    X(4, 16, 2, 34)       \
+    X(5, 16, 1, 14)
+
+template <int TX_, int R_, int TYM_>
+struct Shape {
+    static constexpr int TX = TX_, R = R_, TYM = TYM_;
+    static constexpr int RW = TX + 2 * HALO;  // window width = pitch of every buffer
+    // Buffers, three planes each, all addressed in window coordinates (row 0 =
+    // 4 rows above the tile): A, the step-start state, rows 0 .. TYM + 7; B,
+    // rows 1 .. TYM + 6; C, rows 2 .. TYM + 5; then one plane G of the source,
+    // rows 1 .. TYM + 6.  A thread's column may read two rows past C's last
+    // plane (for rows it does not keep): they lie in G.  Last, the ring's table
+    // (ring_table).
+    static constexpr int PA = (TYM + 8) * RW, PB = (TYM + 6) * RW, PC = (TYM + 4) * RW;
+    static constexpr int THREADS = ((RW * ((TYM + 6) / R) + 31) / 32) * 32;
+    static constexpr int RING = 8 * RW + 8 * TYM;  // cells around the largest tile
+    static constexpr size_t SMEM = sizeof(double) * (size_t)(3 * (PA + PB + PC) + PB) + RING * sizeof(int2);
+    static constexpr size_t SMEM_EXACT = SMEM + sizeof(double) * (size_t)PB;  // and one more plane
+    static_assert((TYM + 6) % R == 0, "the first stage's rows are whole columns of R");
+    static_assert(R <= 5, "six flag bits a row in one register");
+    static_assert(SMEM_EXACT + 768 <= 232448, "one CTA's shared memory");
+    static_assert(THREADS <= 512, "128 registers per thread");
+};
+
+// One exchanged value: the state's double and the number of the step it
+// belongs to, read and written as one 16-byte access.
+struct alignas(16) Tagged {
+    double v;
+    unsigned long long tag;
+};
+__device__ __forceinline__ void put_tagged(Tagged* p, double v, unsigned long long tag) {
+    asm volatile(
+        "{\n .reg .b128 q;\n mov.b128 q, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], q;\n}" ::"l"(p),
+        "l"(__double_as_longlong(v)), "l"(tag)
+        : "memory");
+}
+__device__ __forceinline__ Tagged get_tagged(const Tagged* p) {
+    long long v;
+    unsigned long long t;
+    asm volatile("{\n .reg .b128 q;\n ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}"
+                 : "=l"(v), "=l"(t)
+                 : "l"(p)
+                 : "memory");
+    return {__longlong_as_double(v), t};
+}
+
+// The 4-cell ring around the tile, one entry per cell: x = its place in
+// window A, y = its offset from the window's origin in a state plane, or -1
+// outside the grid's tiles.  Made once a sweep: working the places out at
+// every step took 2.5 us of it at 512 x 512.
+template <class S>
+__device__ __forceinline__ int ring_table(int2* ring, int ld, int rows, int i0, int j0, int nrows, int ncols_tiled) {
+    const int count = 8 * S::RW + 8 * rows;
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        int r, c;
+        if (i < 8 * S::RW) {
+            r = i / S::RW;
+            c = i - r * S::RW;
+            if (r >= 4) r += rows;
+        } else {
+            const int j = i - 8 * S::RW;
+            r = 4 + (j >> 3);
+            c = (j & 7) + ((j & 4) ? S::TX : 0);
+        }
+        const int gi = i0 + r - HALO, gj = j0 + c - HALO;
+        const bool on = gi >= 0 && gi < nrows && gj >= 0 && gj < ncols_tiled;
+        ring[i] = make_int2(r * S::RW + c, on ? r * ld + c : -1);
+    }
+    return count;
+}
+
+// Fills the ring of window A with the values of step `tag` (3 x grid planes of
+// Tagged at x, window origin included).  Each thread polls its own cells, the
+// six values of two of them in flight until all have arrived (one after the
+// other, each would cost its own round trip to L2); ring cells outside the
+// grid's tiles are left alone (NaN since the sweep's start).  One outcome for
+// the CTA, which ends synchronised: false when a wait expired, after 2 s of
+// wall time, or another CTA gave up; *fault is then set and the caller
+// returns.  All CTAs are resident (cooperative launch), so only a CTA that
+// gave up is ever waited for in vain.
+template <class S>
+__device__ __noinline__ bool read_ring(double* A, const int2* ring, int count, const Tagged* x, unsigned long long tag,
+                                       long long plane, unsigned* fault) {
+    constexpr int N = 2;
+    bool ok = true;
+    for (int base = threadIdx.x; base < count && ok; base += N * blockDim.x) {
+        int2 e[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int i = base + u * blockDim.x;
+            e[u] = i < count ? ring[i] : make_int2(0, -1);
+        }
+        uint64_t t0 = 0;
+        bool all = false;
+        for (int it = 0; !all && ok; ++it) {
+            Tagged got[N][3];
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+                if (e[u].y >= 0) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) got[u][f] = get_tagged(x + f * plane + e[u].y);
+                }
+            all = true;
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+                if (e[u].y >= 0) {
+                    if (got[u][0].tag == tag && got[u][1].tag == tag && got[u][2].tag == tag) {
+#pragma unroll
+                        for (int f = 0; f < 3; ++f) A[f * S::PA + e[u].x] = got[u][f].v;
+                        e[u].y = -1;
+                    } else {
+                        all = false;
+                    }
+                }
+            if ((it & 255) == 255) {
+                const uint64_t now = bulk_now_ns();
+                if (!t0) t0 = now;
+                unsigned f;
+                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(fault) : "memory");
+                ok = now - t0 <= 2000000000ull && !(f & FAULT_TIMEOUT);
+            }
+        }
+    }
+    if (!ok) atomicOr(fault, FAULT_TIMEOUT);
+    return !__syncthreads_or(!ok);
+}
+
+// What a thread knows of its column (constant over the sweep).
+struct Column {
+    int c, r0;      // window column, first window row
+    int o;          // offset of (r0, c) from the window's origin in a state plane
+    unsigned bits;  // CELL_* of row r0 + k at bit 6 k
+};
+
+// One forward stage on the tile grown by E cells, for the thread's own cells:
+// k = f(src), then
+//   MODE 0: dst = y0 + cY k, D  = cD k     (first stage: src is y0's window)
+//   MODE 1: dst = y0 + cY k, D += cD k     (middle stages)
+//   MODE 2: y0 <- (y0 + D) + cD k          (last stage)
+// with y0 in window A; the result of the tile's own cells also to `out` (null:
+// nowhere) and, in the last stage, the tile's edges to the exchange x (null:
+// nowhere).  A hole's own value is NaN in A and so in every result
+// that leaves the tile; what B and C hold there is never read as a neighbour.
+template <int E, class S, int MODE, int PS, int PT>
+__device__ __forceinline__ void fwd_rows(const DevModel& P, const Column& T, const double* src, double* dst, double* A,
+                                         const double* G, double (&D)[S::R][3], int rows, int ld, long long plane,
+                                         double Ev, double cY, double cD, double* __restrict__ out,
+                                         Tagged* __restrict__ x, unsigned long long tag, bool& bad) {
+    constexpr int RW = S::RW;
+    if (T.c < HALO - E || T.c >= HALO + S::TX + E) return;
+    const int q0 = T.r0 * RW + T.c;
+    const double* Y = src + q0;
+    // opaque: what follows from the flags is the same at every step, and the
+    // compiler would keep it in registers (and spill) from step to step
+    unsigned bits = T.bits;
+    asm volatile("" : "+r"(bits));
+    double n[3], m[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) n[f] = Y[f * PS - RW], m[f] = Y[f * PS];
+#pragma unroll
+    for (int k = 0; k < S::R; ++k) {
+        const int r = T.r0 + k;
+        const unsigned b = bits >> (6 * k);
+        // a missing neighbour is read where the opposite one is; the value
+        // below then stands in for a hole's, which no one uses
+        const double* ps = Y + ((b & CELL_S) ? k - 1 : k + 1) * RW;
+        const double* pw = Y + k * RW + ((b & CELL_W) ? 1 : -1);
+        const double* pe = Y + k * RW + ((b & CELL_E) ? -1 : 1);
+        double s[3];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) s[f] = ps[f * PS];
+        if (r >= HALO - E && r < HALO + rows + E) {
+            double t[3], kk[3];
+#pragma unroll
+            for (int f = 0; f < 3; ++f) t[f] = lap4((b & CELL_N) ? s[f] : n[f], s[f], pw[f * PS], pe[f * PS], m[f]);
+            double gv = 0.0;
+            if (b & CELL_SOURCE) gv = G[q0 + k * RW];
+            fk_field(P, m, t, Ev, gv, kk[0], kk[1], kk[2]);
+            double* a = A + q0 + k * RW;
+            if (MODE == 2) {
+                double o[3];
+#pragma unroll
+                for (int f = 0; f < 3; ++f) a[f * S::PA] = o[f] = fma(cD, kk[f], a[f * S::PA] + D[k][f]);
+                bad = bad || (isnan(o[0]) && (b & CELL_ACTIVE));
+                if (out) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) out[f * plane + T.o + k * ld] = o[f];
+                }
+                if (x && (r < 2 * HALO || r >= rows || T.c < 2 * HALO || T.c >= S::TX)) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) put_tagged(x + f * plane + T.o + k * ld, o[f], tag);
+                }
+            } else {
+double o[3];
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                    const double y0 = MODE == 0 ? m[f] : a[f * S::PA];
+                    dst[f * PT + q0 + k * RW] = o[f] = fma(cY, kk[f], y0);
+                    D[k][f] = MODE == 0 ? cD * kk[f] : fma(cD, kk[f], D[k][f]);
+                }
+                if (out && r >= HALO && r < HALO + rows && T.c >= HALO && T.c < HALO + S::TX) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f)
+                        out[f * plane + T.o + k * ld] = (b & CELL_ACTIVE) ? o[f] : __longlong_as_double(-1);
+                }
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < 3; ++f) n[f] = m[f], m[f] = s[f];
+    }
+}
+
+// A sweep of r.n forward steps (launch_fwd_run: cooperative, one CTA per
+// tile).  The exchange area is two 3-plane grids of Tagged, used in turn: a
+// tile writes step k + 2's edges over step k's only after it has read its
+// neighbours' step k + 1, which they published after they had read step k.
+template <int TX, int R, int TYM>
+__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
+    k_fwd_run(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
+              const FwdRun r, int ty) {
+    using S = Shape<TX, R, TYM>;
+    constexpr int RW = S::RW;
+    extern __shared__ double4 smem_raw[];
+    __shared__ uint64_t bar;
+    double* A = reinterpret_cast<double*>(smem_raw);
+    double* B = A + 3 * S::PA - RW;
+    double* C = A + 3 * (S::PA + S::PB) - 2 * RW;
+    double* G = A + 3 * (S::PA + S::PB + S::PC) - RW;
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const int i0 = by * ty, j0 = bx * TX;
+    const int rows = min(ty, g.nrows - i0);
+    const long long off = (long long)i0 * g.ld + j0;  // window origin: logical (i0 - 4, j0 - 4)
+
+    int2* ring = reinterpret_cast<int2*>(G + RW + S::PB);
+    const int nring = ring_table<S>(ring, g.ld, rows, i0, j0, g.nrows, (int)gridDim.x * TX);
+    exp_table_init();
+    const uint32_t b = bulk_begin(&bar);
+    __syncthreads();
+    bulk_arrive(b, bulk_bytes<RW>(rows + 2 * HALO));
+    __syncthreads();
+    {
+        const int nr = rows + 2 * HALO;
+        for (int t = threadIdx.x; t < 3 * nr; t += blockDim.x) {
+            const int f = t / nr, row = t - f * nr;
+            bulk_row<RW>(b, A + f * S::PA + row * RW, r.src + off + f * g.plane + (long long)row * g.ld);
+        }
+    }
+    Column T;
+    {
+        const int col = threadIdx.x / RW;
+        T.c = threadIdx.x - col * RW;
+        T.r0 = 1 + col * R;
+        T.o = T.r0 * g.ld + T.c;
+        T.bits = 0;
+        if (T.r0 >= rows + 7) T.c = -1;  // no rows: out of every stage's columns
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            if (T.c >= 1 && T.c < TX + 7 && T.r0 + k < rows + 7) {
+                const unsigned f = cells[off + T.o + k * g.ld];
+                T.bits |= f << (6 * k);
+                G[(T.r0 + k) * RW + T.c] = gh[off + T.o + k * g.ld];
+            }
+        }
+    }
+    if (!bulk_wait_cta(b, r.fault)) return;
+    __syncthreads();
+    double D[R][3];
+    bool bad = false;
+    for (int k = 0; k < r.n; ++k) {
+        // what a stage needs is worked out where it starts: registers are short
+        auto stage_out = [&](int st) { return r.stages ? r.stages + (3LL * k + st) * r.stride + off : nullptr; };
+        fwd_rows<3, S, 0, S::PA, S::PB>(P, T, A, B, A, G, D, rows, g.ld, g.plane, __ldg(r.Et + k), 0.5 * P.dt,
+                                        1.0 / 6.0 * P.dt, stage_out(0), nullptr, 0, bad);
+        __syncthreads();
+        fwd_rows<2, S, 1, S::PB, S::PC>(P, T, B, C, A, G, D, rows, g.ld, g.plane, __ldg(r.Eh + k), 0.5 * P.dt,
+                                        1.0 / 3.0 * P.dt, stage_out(1), nullptr, 0, bad);
+        __syncthreads();
+        fwd_rows<1, S, 1, S::PC, S::PB>(P, T, C, B, A, G, D, rows, g.ld, g.plane, __ldg(r.Eh + k), P.dt,
+                                        1.0 / 3.0 * P.dt, stage_out(2), nullptr, 0, bad);
+        __syncthreads();
+        const bool end = k == r.n - 1;
+        const unsigned long long tag = r.epoch + k + 1;
+        Tagged* x = static_cast<Tagged*>(r.exchange) + (tag & 1) * (3 * g.plane) + off;
+        {
+            double* out = end ? r.last : (r.out ? r.out + k * r.stride : nullptr);
+            fwd_rows<0, S, 2, S::PB, S::PB>(P, T, B, nullptr, A, G, D, rows, g.ld, g.plane, __ldg(r.Et + k + 1), 0.0,
+                                            P.dt / 6.0, out ? out + off : nullptr, end ? nullptr : x, tag, bad);
+        }
+        if (end) break;
+        if (!read_ring<S>(A, ring, nring, x, tag, g.plane, r.fault)) return;
+    }
+    // A NaN in an active cell came from the inputs or from a state that blew
+    // up: the per-step kernels contain it (their stencil takes any NaN
+    // neighbour for missing), this sweep lets it spread.  The host repeats the
+    // call with them.
+    if (bad) atomicOr(r.fault, FAULT_NAN);
+}
+
+// ------------------------------------------------------------ adjoint sweeps
+//
+// A backward step of either mode is four stages k_s = L^T a_s + J_F(Y_s)^T a_s
+// of the same shape: stage s on the tile grown by 4 - s cells, each at its own
+// state Y_s, which no stage changes (the reference mode: y_i, the midpoint
+// twice, y_{i-1}; the exact mode: the step's stage states Y4, Y3, Y2 and y_s).
+// The sweep therefore is k_fwd_run's with the Jacobian evaluated at a state
+// read from global memory, one row ahead of its use.  Evaluating J on the
+// halo again (4.6 times a cell and step) costs 380 FP64 instructions a cell;
+// the per-step kernels read the seven entries cached by other kernels
+// instead, 250 B a cell and step through L2, and took 20 us for it at 512 x
+// 512.
+//
+// Holes hold 0 in the buffers here (and NaN in every state that leaves the
+// tile): a missing neighbour then adds nothing to the plain sum, and only the
+// neighbours that mirrored this cell are added once more.
+
+// Row k of a column's values of state y (its window's origin), 0 past the tile
+template <class S>
+__device__ __forceinline__ void load_point(const Column& T, int k, int rows, int ld, long long plane,
+                                           const double* __restrict__ y, double (&v)[3]) {
+    const bool on = T.c >= 1 && T.c < S::TX + 7 && T.r0 + k < rows + 7;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) v[f] = on ? __ldg(y + f * plane + T.o + k * ld) : 0.0;
+}
+
+// One backward stage on the tile grown by E cells, for the thread's own cells:
+// k = L^T src + J_F(y)^T src, then in the reference mode
+//   MODE 0: dst = z0 + cA k, D  = cB k
+//   MODE 1: dst = z0 + cA k, D += cB k
+//   MODE 2: z0 <- (z0 + D) + cB k
+// and in the exact mode, where src is z0 = lambda itself in the first stage
+// and k there is scaled by cS = dt/6 (a_4 = dt/6 lambda),
+//   MODE 0: dst = cB z0 + cA k, D  = k;  MODE 1: the same, D += k
+//   MODE 2: z0 <- z0 + (D + k)
+// with z0 in window A.  yv holds the first row of y; `keep` (exact mode, first
+// stage) receives a_3 on u.
+template <int E, class S, int MODE, int PS, int PT, bool EXACT>
+__device__ __forceinline__ void adj_rows(const DevModel& P, const Column& T, const double* src, double* dst, double* A,
+                                         double (&D)[S::R][3], double (&yv)[3], const double* __restrict__ y, int rows,
+                                         int ld, long long plane, double cA, double cB, double cS, double* keep,
+                                         double* __restrict__ out, Tagged* __restrict__ x, unsigned long long tag) {
+    constexpr int RW = S::RW;
+    if (T.c < HALO - E || T.c >= HALO + S::TX + E) return;
+    const int q0 = T.r0 * RW + T.c;
+    const double* Z = src + q0;
+    unsigned bits = T.bits;
+    asm volatile("" : "+r"(bits));  // as in fwd_rows
+    double n[3], m[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) n[f] = Z[f * PS - RW], m[f] = Z[f * PS];
+#pragma unroll
+    for (int k = 0; k < S::R; ++k) {
+        const int r = T.r0 + k;
+        const unsigned b = bits >> (6 * k);
+        double s[3], yn[3];
+        if (k + 1 < S::R) load_point<S>(T, k + 1, rows, ld, plane, y, yn);
+#pragma unroll
+        for (int f = 0; f < 3; ++f) s[f] = Z[f * PS + (k + 1) * RW];
+        if (r >= HALO - E && r < HALO + rows + E) {
+            double t[3], kk[3];
+#pragma unroll
+            for (int f = 0; f < 3; ++f)
+                t[f] = lap4(n[f], s[f], Z[f * PS + k * RW - 1], Z[f * PS + k * RW + 1], m[f]);
+            if (b & (CELL_2N | CELL_2S | CELL_2W | CELL_2E)) {
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                    if (b & CELL_2N) t[f] += n[f];
+                    if (b & CELL_2S) t[f] += s[f];
+                    if (b & CELL_2W) t[f] += Z[f * PS + k * RW - 1];
+                    if (b & CELL_2E) t[f] += Z[f * PS + k * RW + 1];
+                }
+            }
+            const JacT J = fk_jacT(P, yv[0], yv[1], yv[2]);
+            adj_field(P, J, m, t, kk[0], kk[1], kk[2]);
+            const bool act = b & CELL_ACTIVE_ADJ;
+            double* a = A + q0 + k * RW;
+            if (MODE == 2) {
+                double o[3];
+#pragma unroll
+                for (int f = 0; f < 3; ++f)
+                    o[f] = EXACT ? a[f * S::PA] + (D[k][f] + kk[f]) : fma(cB, kk[f], a[f * S::PA] + D[k][f]);
+                if (act) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) a[f * S::PA] = o[f];
+                }
+                if (out) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) out[f * plane + T.o + k * ld] = act ? o[f] : __longlong_as_double(-1);
+                }
+                if (x && (r < 2 * HALO || r >= rows || T.c < 2 * HALO || T.c >= S::TX)) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) put_tagged(x + f * plane + T.o + k * ld, act ? o[f] : 0.0, tag);
+                }
+            } else {
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                    const double z0 = MODE == 0 ? m[f] : a[f * S::PA];
+                    if (EXACT && MODE == 0) kk[f] = cS * kk[f];
+                    const double o = EXACT ? fma(cA, kk[f], cB * z0) : fma(cA, kk[f], z0);
+                    if (act) dst[f * PT + q0 + k * RW] = o;
+                    if (EXACT) D[k][f] = MODE == 0 ? kk[f] : D[k][f] + kk[f];
+                    else D[k][f] = MODE == 0 ? cB * kk[f] : fma(cB, kk[f], D[k][f]);
+                    if (EXACT && MODE == 0 && f == 0) keep[q0 + k * RW] = o;
+                }
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < 3; ++f) n[f] = m[f], m[f] = s[f], yv[f] = yn[f];
+    }
+}
+
+// The 16-cell row segments of the tile (lattice of segment_sums in
+// fk_kernels.cu) that hold a source cell, as row * (TX / 16) + segment: the
+// others' terms are all zero and their partial sums stay at the zero the
+// buffer was cleared to.
+template <class S>
+__device__ __forceinline__ void segment_list(uint16_t* list, int* count, const uint8_t* __restrict__ cells, int rows,
+                                             int ld) {
+    constexpr int SX = S::TX / 16;
+    for (int i = threadIdx.x; i < rows * SX; i += blockDim.x) {
+        const int r = i / SX, sx = i - r * SX;
+        const uint8_t* c = cells + (long long)(r + HALO) * ld + HALO + sx * 16;
+        bool any = false;
+        for (int l = 0; l < 16; ++l) any = any || (c[l] & CELL_SOURCE);
+        if (any) list[atomicAdd(count, 1)] = (uint16_t)i;
+    }
+}
+
+// Partial sums of the listed segments, each by a half-warp in segment_sums'
+// order; term(q) is the cell's term at window cell q, NaN counts as 0.  Every
+// thread runs every round (the shuffles take whole warps).
+template <class S, class Term>
+__device__ __forceinline__ void segment_terms(const uint16_t* list, int count, double* __restrict__ row, int i0, int j0,
+                                              int nsbx, Term term) {
+    constexpr int SX = S::TX / 16;
+    const int l = threadIdx.x & 15, h = threadIdx.x >> 4, nh = blockDim.x >> 4;
+    for (int b0 = 0; b0 < count; b0 += nh) {
+        if (b0 + (h & ~1) >= count) break;  // both halves of the warp are past the end
+        const bool on = b0 + h < count;
+        const int i = on ? list[b0 + h] : 0;
+        const int r = i / SX, sx = i - r * SX;
+        double s = 0.0;
+        if (on) {
+            const double t = term((r + HALO) * S::RW + HALO + sx * 16 + l);
+            s = isnan(t) ? 0.0 : t;
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (on && l == 0) row[(long long)(i0 + r) * nsbx + (j0 / 16 + sx)] = s;
+    }
+}
+
+template <int TX, int R, int TYM, bool EXACT>
+__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
+    k_adj_run(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
+              const uint8_t* __restrict__ adj, const AdjRun r, int ty) {
+    using S = Shape<TX, R, TYM>;
+    constexpr int RW = S::RW;
+    extern __shared__ double4 smem_raw[];
+    __shared__ uint64_t bar;
+    __shared__ int s_segs;
+    __shared__ uint16_t segs[TYM * TX / 16];
+    double* A = reinterpret_cast<double*>(smem_raw);
+    double* B = A + 3 * S::PA - RW;
+    double* C = A + 3 * (S::PA + S::PB) - 2 * RW;
+    double* G = A + 3 * (S::PA + S::PB + S::PC) - RW;
+    int2* ring = reinterpret_cast<int2*>(G + RW + S::PB);
+    double* K3 = reinterpret_cast<double*>(ring + S::RING) - RW;  // a_3 on u (exact mode), rows 1 ..
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const int i0 = by * ty, j0 = bx * TX;
+    const int rows = min(ty, g.nrows - i0);
+    const long long off = (long long)i0 * g.ld + j0;
+    const int nring = ring_table<S>(ring, g.ld, rows, i0, j0, g.nrows, (int)gridDim.x * TX);
+    exp_table_init();
+    if (threadIdx.x == 0) s_segs = 0;
+    const uint32_t b = bulk_begin(&bar);
+    __syncthreads();
+    bulk_arrive(b, bulk_bytes<RW>(rows + 2 * HALO));
+    __syncthreads();
+    {
+        const int nr = rows + 2 * HALO;
+        for (int t = threadIdx.x; t < 3 * nr; t += blockDim.x) {
+            const int f = t / nr, row = t - f * nr;
+            bulk_row<RW>(b, A + f * S::PA + row * RW, r.zin + off + f * g.plane + (long long)row * g.ld);
+        }
+    }
+    segment_list<S>(segs, &s_segs, cells + off, rows, g.ld);
+    for (int q = threadIdx.x; q < 3 * S::PB; q += blockDim.x) B[RW + q] = 0.0;
+    for (int q = threadIdx.x; q < 3 * S::PC; q += blockDim.x) C[2 * RW + q] = 0.0;
+    Column T;
+    {
+        const int col = threadIdx.x / RW;
+        T.c = threadIdx.x - col * RW;
+        T.r0 = 1 + col * R;
+        T.o = T.r0 * g.ld + T.c;
+        T.bits = 0;
+        if (T.r0 >= rows + 7) T.c = -1;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            if (T.c >= 1 && T.c < TX + 7 && T.r0 + k < rows + 7) {
+                T.bits |= (unsigned)adj[off + T.o + k * g.ld] << (6 * k);
+                G[(T.r0 + k) * RW + T.c] = gh[off + T.o + k * g.ld];
+            }
+        }
+    }
+    if (!bulk_wait_cta(b, r.fault)) return;
+    __syncthreads();
+    for (int q = threadIdx.x; q < (rows + 2 * HALO) * RW; q += blockDim.x) {
+        const int row = q / RW, c = q - row * RW;
+        if (!(adj[off + (long long)row * g.ld + c] & CELL_ACTIVE_ADJ)) {
+#pragma unroll
+            for (int f = 0; f < 3; ++f) A[f * S::PA + q] = 0.0;
+        }
+    }
+    __syncthreads();
+    const int nsegs = s_segs;
+    // the step's four states (k = 0 is the sweep's first, the latest in time)
+    auto yptr = [&](int j) {  // y after j steps back
+        return (j == 0 ? r.y_hi : (j == r.n ? r.y_lo : r.y_mid + (long long)(r.n - 1 - j) * r.stride)) + off;
+    };
+    auto point = [&](int k, int st) -> const double* {
+        if (EXACT) return st == 3 ? yptr(k + 1) : r.pts + ((long long)k * r.pts_step + (2 - st)) * r.stride + off;
+        return st == 0 ? yptr(k) : (st == 3 ? yptr(k + 1) : r.pts + (long long)k * r.pts_step * r.stride + off);
+    };
+    auto partial = [&](int group, int k) {
+        return r.partial + ((long long)group * r.window + (r.row0 - k) % r.window) * r.nsb;
+    };
+    double D[R][3], yv[3];
+    load_point<S>(T, 0, rows, g.ld, g.plane, point(0, 0), yv);
+    for (int k = 0; k < r.n; ++k) {
+        if (EXACT)
+            segment_terms<S>(segs, nsegs, partial(2, k), i0, j0, r.nsbx,
+                             [&](int q) { return ((P.dt / 6.0) * A[q]) * G[q]; });
+        adj_rows<3, S, 0, S::PA, S::PB, EXACT>(P, T, A, B, A, D, yv, point(k, 0), rows, g.ld, g.plane,
+                                               EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt / 3.0 : 1.0 / 6.0 * P.dt,
+                                               P.dt / 6.0, K3, nullptr, nullptr, 0);
+        load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 1), yv);
+        __syncthreads();
+        adj_rows<2, S, 1, S::PB, S::PC, EXACT>(P, T, B, C, A, D, yv, point(k, 1), rows, g.ld, g.plane, 0.5 * P.dt,
+                                               EXACT ? P.dt / 3.0 : 2.0 / 6.0 * P.dt, 0.0, nullptr, nullptr, nullptr,
+                                               0);
+        load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 2), yv);
+        __syncthreads();
+        adj_rows<1, S, 1, S::PC, S::PB, EXACT>(P, T, C, B, A, D, yv, point(k, 2), rows, g.ld, g.plane,
+                                               EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt / 6.0 : 2.0 / 6.0 * P.dt, 0.0,
+                                               nullptr, nullptr, nullptr, 0);
+        load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 3), yv);
+        __syncthreads();
+        if (EXACT) {
+            segment_terms<S>(segs, nsegs, partial(0, k), i0, j0, r.nsbx, [&](int q) { return B[q] * G[q]; });
+            segment_terms<S>(segs, nsegs, partial(1, k), i0, j0, r.nsbx, [&](int q) { return (C[q] + K3[q]) * G[q]; });
+        }
+        const bool end = k == r.n - 1;
+        const unsigned long long tag = r.epoch + k + 1;
+        Tagged* x = static_cast<Tagged*>(r.exchange) + (tag & 1) * (3 * g.plane) + off;
+        adj_rows<0, S, 2, S::PB, S::PB, EXACT>(P, T, B, nullptr, A, D, yv, point(k, 3), rows, g.ld, g.plane, 0.0,
+                                               1.0 / 6.0 * P.dt, 0.0, nullptr, end ? r.zout + off : nullptr,
+                                               end ? nullptr : x, tag);
+        if (end) {
+            __syncthreads();
+        } else {
+            load_point<S>(T, 0, rows, g.ld, g.plane, point(k + 1, 0), yv);
+            if (!read_ring<S>(A, ring, nring, x, tag, g.plane, r.fault)) return;
+        }
+        // z_u . gh of the new z: the window's interior stays as it is until
+        // the next step's last stage
+        if (!EXACT)
+            segment_terms<S>(segs, nsegs, partial(0, k), i0, j0, r.nsbx, [&](int q) { return A[q] * G[q]; });
+    }
+}
+
+// ------------------------------------------------------- midpoint states
+//
+// The midpoint states of r.n backward steps (cu-G:1244-1301) in one launch:
+// they depend on the stored states only, so the steps of a sweep's chunk are
+// all made before it.  A CTA takes one tile of one run of steps, walking back
+// in time: the state and f of a step's later end are the earlier end of the
+// step before it, so each step costs two evaluations and one window load,
+// issued a step ahead.  Per-step launches took 14 us a step at 512 x 512,
+// waiting for their operands.
+//   y(1/3) = cubic Hermite of (ya, fa, yb, fb) at 1/3,
+//   yh     = partial quartic at 1/2 + (27/64) dt f(y(1/3), E(t + dt/3)).
+struct MidShape {
+    static constexpr int TX = 64, R = 3, TY = 16, H = 2, RW = TX + 2 * HALO;
+    static constexpr int PW = (TY + 2 * H) * RW;      // a window: rows -2 .. TY + 1
+    static constexpr int THREADS = ((RW * (TY + 2) / R) + 31) / 32 * 32;
+    static constexpr size_t SMEM = sizeof(double) * (size_t)(3 * 3 * PW + 3 * PW + PW);
+};
+
+// f at the thread's cell of row k (window row r) of buffer Y from its column
+// values; as in fwd_rows
+__device__ __forceinline__ void mid_field(const DevModel& P, unsigned b, const double* Y, const double* g,
+                                          double E, double (&kk)[3]) {
+    constexpr int RW = MidShape::RW, PW = MidShape::PW;
+    const double* pn = Y + ((b & CELL_N) ? RW : -RW);
+    const double* ps = Y + ((b & CELL_S) ? -RW : RW);
+    const double* pw = Y + ((b & CELL_W) ? 1 : -1);
+    const double* pe = Y + ((b & CELL_E) ? -1 : 1);
+    double y[3], t[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) y[f] = Y[f * PW];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) t[f] = lap4(pn[f * PW], ps[f * PW], pw[f * PW], pe[f * PW], y[f]);
+    double gv = 0.0;
+    if (b & CELL_SOURCE) gv = *g;
+    fk_field(P, y, t, E, gv, kk[0], kk[1], kk[2]);
+}
+
+__global__ void __launch_bounds__(MidShape::THREADS, 1)
+    k_mid_run(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
+              const HermiteW hw, const MidRun r, int per) {
+    using S = MidShape;
+    constexpr int RW = S::RW, PW = S::PW, R = S::R;
+    extern __shared__ double4 smem_raw[];
+    __shared__ uint64_t bars[3];
+    double* W = reinterpret_cast<double*>(smem_raw);  // three windows in turn
+    double* Y3 = W + 9 * PW;
+    double* G = Y3 + 3 * PW;
+    const int i0 = blockIdx.y * S::TY, j0 = blockIdx.x * S::TX;
+    const int rows = min(S::TY, g.nrows - i0);
+    // window origin: logical (i0 - 2, j0 - 4) = padded (i0 + 2, j0)
+    const long long off = (long long)(i0 + HALO - S::H) * g.ld + j0;
+    const int k0 = blockIdx.z * per, k1 = min(k0 + per, r.n);  // steps k0 .. k1 - 1
+    if (k0 >= k1) return;
+    exp_table_init();
+    const uint32_t bar = bulk_begin(&bars[0]);
+    bulk_begin(&bars[1]);
+    bulk_begin(&bars[2]);
+    __syncthreads();
+    auto yptr = [&](int j) {  // y after j steps back
+        return (j == 0 ? r.y_hi : (j == r.n ? r.y_lo : r.y_mid + (long long)(r.n - 1 - j) * r.stride)) + off;
+    };
+    const int nr = rows + 2 * S::H;
+    // window of y after j steps back into buffer (j - k0) % 3; its barrier's
+    // parity is (j - k0) / 3 mod 2
+    auto fetch = [&](int j) {
+        const int u = (j - k0) % 3;
+        bulk_arrive(bar + 8 * u, bulk_bytes<RW>(nr));
+        __syncthreads();
+        const double* src = yptr(j);
+        for (int t = threadIdx.x; t < 3 * nr; t += blockDim.x) {
+            const int f = t / nr, row = t - f * nr;
+            bulk_row<RW>(bar + 8 * u, W + (3 * u + f) * PW + row * RW, src + f * g.plane + (long long)row * g.ld);
+        }
+    };
+    fetch(k0);
+    fetch(k0 + 1);
+    const int col = threadIdx.x / RW;
+    const int c = threadIdx.x - col * RW, r0 = 1 + col * R;
+    const bool in = c >= HALO - 1 && c < HALO + S::TX + 1;
+    unsigned bits = 0;
+    double fb[R][3];
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+        if (in && r0 + k < rows + 3) {
+            bits |= (unsigned)cells[off + (long long)(r0 + k) * g.ld + c] << (6 * k);
+            G[(r0 + k) * RW + c] = gh[off + (long long)(r0 + k) * g.ld + c];
+        }
+    if (!bulk_wait_cta(bar, r.fault)) return;
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+        if (in && r0 + k < rows + 3) {
+            const int q = (r0 + k) * RW + c;
+            mid_field(P, bits >> (6 * k), W + q, G + q, __ldg(r.Et - k0), fb[k]);
+        }
+    for (int k = k0; k < k1; ++k) {
+        const int ub = (k - k0) % 3, ua = (k + 1 - k0) % 3;
+        // the window after next into the buffer that the step before last used
+        if (k + 2 <= k1) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fetch(k + 2);
+        }
+        if (!bulk_wait_cta(bar + 8 * ua, r.fault, 1000000000ull, (unsigned)((k + 1 - k0) / 3) & 1u)) return;
+        const double* YA = W + 3 * ua * PW;
+        const double* YB = W + 3 * ub * PW;
+        const double Ea = __ldg(r.Et - k - 1);
+        double qv[R][3];
+#pragma unroll
+        for (int u = 0; u < R; ++u)
+            if (in && r0 + u < rows + 3) {
+                const int q = (r0 + u) * RW + c;
+                double fa[3];
+                mid_field(P, bits >> (6 * u), YA + q, G + q, Ea, fa);
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                    const double m0 = fa[f] * P.dt, m1 = fb[u][f] * P.dt;
+                    const double x0 = YA[f * PW + q], x1 = YB[f * PW + q];
+                    Y3[f * PW + q] = hermite4(hw.c3, x0, m0, x1, m1);
+                    qv[u][f] = hermite4(hw.c4, x0, m0, x1, m1);
+                    fb[u][f] = fa[f];
+                }
+            }
+        __syncthreads();
+        const double E3 = __ldg(r.E3 - k);
+        double* yh = r.yh + (long long)k * r.stride + off;
+#pragma unroll
+        for (int u = 0; u < R; ++u)
+            if (c >= HALO && c < HALO + S::TX && r0 + u >= S::H && r0 + u < S::H + rows) {
+                const int q = (r0 + u) * RW + c;
+                double m2[3];
+                mid_field(P, bits >> (6 * u), Y3 + q, G + q, E3, m2);
+#pragma unroll
+                for (int f = 0; f < 3; ++f)
+                    yh[f * g.plane + (long long)(r0 + u) * g.ld + c] = fma(hw.c2, m2[f] * P.dt, qv[u][f]);
+            }
+        __syncthreads();
+    }
+}
+
+}  // namespace
+
+#define X(id, a, b, c) \
+    case id: { using S = Shape<a, b, c>; DO(S); } break;
+
+RunShape run_shape(const DevGrid& g, int sms) {
+    RunShape best;
+    double best_cost = 0;
+    for (int id = 0; id < 6; ++id) {
+        int tx = 0, R = 0, tym = 0, rw = 0, threads = 0;
+        switch (id) {
+#define DO(S) tx = S::TX, R = S::R, tym = S::TYM, rw = S::RW, threads = S::THREADS
+            FKADJ_RUN_LIST(X)
+#undef DO
+        }
+        const int ntx = (g.ncols + tx - 1) / tx;
+        if (ntx > sms) continue;
+        // at least 4 rows: a tile's halo is its direct neighbours' cells
+        const int rows = std::max(HALO, (g.nrows + sms / ntx - 1) / (sms / ntx));
+        if (rows > tym) continue;
+        // a step's cost: per stage, the evaluations (a warp's row, by FP64
+        // issue) or the depth of a thread's column, whichever is longer
+        double cost = 0;
+        for (int e = 3; e >= 0; --e) {
+            const double warps = (double)rw * (rows + 2 * e) / 32.0;
+            cost += std::max(warps * 62.0, R * 420.0);
+        }
+        if (best.id < 0 || cost < best_cost) {
+            best_cost = cost;
+            best.id = id;
+            best.tx = tx;
+            best.rows = rows;
+            best.ntx = ntx;
+            best.nty = (g.nrows + rows - 1) / rows;
+            const int need = rw * ((rows + 6 + R - 1) / R);
+            best.threads = std::min(threads, (need + 31) / 32 * 32);
+        }
+    }
+    return best;
+}
+
+size_t run_exchange_bytes(const DevGrid& g) { return 2 * 3 * (size_t)g.plane * sizeof(Tagged); }
+
+cudaError_t run_init() {
+    cudaError_t e = cudaFuncSetAttribute(k_mid_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MidShape::SMEM);
+#undef X
+#define X(id, a, b, c)                                                                                     \
+    if (!e) e = cudaFuncSetAttribute(k_fwd_run<a, b, c>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                     (int)Shape<a, b, c>::SMEM);                                            \
+    if (!e) e = cudaFuncSetAttribute(k_adj_run<a, b, c, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                     (int)Shape<a, b, c>::SMEM);                                            \
+    if (!e) e = cudaFuncSetAttribute(k_adj_run<a, b, c, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                     (int)Shape<a, b, c>::SMEM_EXACT);
+    FKADJ_RUN_LIST(X)
+#undef X
+    return e;
+}
+
+template <class K, class... Args>
+static cudaError_t launch_run(K kernel, const RunShape& s, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s.ntx, s.nty);
+    cfg.blockDim = dim3(s.threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const DevGrid& g, const double* gh,
+                           const uint8_t* cells, const FwdRun& r, cudaStream_t st) {
+    if (r.n <= 0) return cudaSuccess;
+    switch (s.id) {
+#define X(id, a, b, c) \
+    case id: return launch_run(k_fwd_run<a, b, c>, s, Shape<a, b, c>::SMEM, st, P, g, gh, cells, r, s.rows);
+        FKADJ_RUN_LIST(X)
+#undef X
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_mid_run(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,
+                           const HermiteW& hw, const MidRun& r, int sms, cudaStream_t st) {
+    if (r.n <= 0) return cudaSuccess;
+    using S = MidShape;
+    const int ntx = (g.ncols + S::TX - 1) / S::TX, nty = (g.nrows + S::TY - 1) / S::TY, tiles = ntx * nty;
+    // runs of steps: the fewest evaluations (per steps cost 2 per + 1) over
+    // whole waves of CTAs, one per SM
+    int per = r.n;
+    long long best = -1;
+    for (int p = 1; p <= r.n; ++p) {
+        const long long ctas = (long long)tiles * ((r.n + p - 1) / p);
+        const long long cost = (ctas + sms - 1) / sms * (2 * p + 1);
+        if (best < 0 || cost <= best) best = cost, per = p;
+    }
+    k_mid_run<<<dim3(ntx, nty, (r.n + per - 1) / per), S::THREADS, S::SMEM, st>>>(P, g, gh, cells, hw, r, per);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adj_run(const RunShape& s, bool exact, const DevModel& P, const DevGrid& g, const double* gh,
+                           const uint8_t* cells, const uint8_t* adj, const AdjRun& r, cudaStream_t st) {
+    if (r.n <= 0) return cudaSuccess;
+    switch (s.id) {
+#define X(id, a, b, c)                                                                                            \
+    case id:                                                                                                      \
+        return exact ? launch_run(k_adj_run<a, b, c, true>, s, Shape<a, b, c>::SMEM_EXACT, st, P, g, gh, cells, adj, \
+                                  r, s.rows)                                                                      \
+                     : launch_run(k_adj_run<a, b, c, false>, s, Shape<a, b, c>::SMEM, st, P, g, gh, cells, adj, r, \
+                                  s.rows);
+        FKADJ_RUN_LIST(X)
+#undef X
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace fkadj
