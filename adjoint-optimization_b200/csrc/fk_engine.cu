@@ -187,7 +187,7 @@ Problem::~Problem() {
         // below): release the buffers first
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &xchg_, &pts_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_};
         for (DevBuf* b : all) b->release();
     }
     for (auto& r : prof_pool_) {
@@ -215,7 +215,7 @@ Problem::~Problem() {
     if (verbose_ > 1) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &xchg_, &pts_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_};
         size_t bytes = 0;
         for (DevBuf* b : all) bytes += b->bytes;
         for (DevBuf* b : all) b->release();
@@ -395,7 +395,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     if (pool_) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &xchg_, &pts_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_};
         for (DevBuf* b : all) b->st = st_, b->pool = pool_;
     }
     {
@@ -548,13 +548,15 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     return FKADJ_OK;
 }
 
-// Whether and how this problem's sweeps run as one launch each (fk_run.h): with
-// autotuned tiles, where the grid's tiles fit the device at once and every
-// active cell keeps a neighbour in both directions.  ai: the active index of
-// every cell; gh: the padded source plane.  FKADJ_SWEEPS=0 in the environment keeps one launch
-// per step.
+// Whether and how this problem's sweeps run (fk_run.h): with autotuned tiles,
+// where every active cell keeps a neighbour in both directions; one launch per
+// sweep where the grid's tiles fit the device at once, the tile kernels
+// otherwise.  ai: the active index of every cell; gh: the padded source plane;
+// wc: the transposed stencil's weight codes.  FKADJ_SWEEPS=0 in the
+// environment keeps the preset kernels.
 fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, const std::vector<uint8_t>& wc) {
     run_ = RunShape();
+    swept_ = false;
     CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "device attribute");
     const char* v = getenv("FKADJ_SWEEPS");
     if (!autotune_ || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ ||
@@ -564,9 +566,8 @@ fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, 
     int coop = 0;
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_), "device attribute");
     const RunShape shape = coop ? run_shape(g_, sms_) : RunShape();
-    if (shape.id < 0) return FKADJ_OK;
     const int ld = g_.ld;
-    std::vector<uint8_t> cells((size_t)g_.plane, 0), adj((size_t)g_.plane, 0);
+    std::vector<uint8_t> cells((size_t)g_.plane, 0), adj((size_t)g_.plane, 0), seg((size_t)nsbx_ * g_.nrows, 0);
     for (int i = 0; i < g_.nrows; ++i)
         for (int j = 0; j < g_.ncols; ++j) {
             const int k = i * g_.ncols + j;
@@ -578,16 +579,22 @@ fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, 
             cells[o] = (uint8_t)(CELL_ACTIVE | (n ? CELL_N : 0) | (s ? CELL_S : 0) | (w ? CELL_W : 0) |
                                  (e ? CELL_E : 0) | (gh[o] != 0.0 ? CELL_SOURCE : 0));
             const int c = wc[o];
-            adj[o] = (uint8_t)(CELL_ACTIVE_ADJ | ((c & 3) == 2 ? CELL_2N : 0) | ((c >> 2 & 3) == 2 ? CELL_2S : 0) |
+            if (gh[o] != 0.0) seg[(size_t)i * nsbx_ + j / 16] = 1;
+            adj[o] = (uint8_t)(CELL_ACTIVE_ADJ | (cells[o] & CELL_SOURCE) | ((c & 3) == 2 ? CELL_2N : 0) | ((c >> 2 & 3) == 2 ? CELL_2S : 0) |
                                ((c >> 4 & 3) == 2 ? CELL_2W : 0) | ((c >> 6 & 3) == 2 ? CELL_2E : 0));
         }
     CK(cells_.alloc(cells.size()), "alloc cell flags");
     CK(cudaMemcpyAsync(cells_.p, cells.data(), cells.size(), cudaMemcpyHostToDevice, st_), "upload cell flags");
     CK(adjf_.alloc(adj.size()), "alloc cell flags");
     CK(cudaMemcpyAsync(adjf_.p, adj.data(), adj.size(), cudaMemcpyHostToDevice, st_), "upload cell flags");
-    CK(xchg_.alloc(run_exchange_bytes(g_)), "alloc edge exchange");
-    CK(cudaMemsetAsync(xchg_.p, 0, xchg_.bytes, st_), "clear edge exchange");
+    CK(segf_.alloc(seg.size()), "alloc segment flags");
+    CK(cudaMemcpyAsync(segf_.p, seg.data(), seg.size(), cudaMemcpyHostToDevice, st_), "upload segment flags");
+    if (shape.id >= 0) {
+        CK(xchg_.alloc(run_exchange_bytes(g_)), "alloc edge exchange");
+        CK(cudaMemsetAsync(xchg_.p, 0, xchg_.bytes, st_), "clear edge exchange");
+    }
     run_ = shape;
+    swept_ = true;
     return FKADJ_OK;
 }
 
@@ -600,9 +607,12 @@ int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t
     int64_t b = plane + 3 * (plane / 8) + (int64_t)n_num * (8 + 48) + nnz * 12 + 8 * state;
     if (!want_grad) return b;
     const int64_t nsb = (round_up(ncols, 64) / 16) * (round_up(nrows, 64) / 16);
-    b += 2 * state + (int64_t)(3 * nt + 1) * (nsb + 1) * 8;  // adjoint pair, partials
+    // adjoint pair, partials (all rows of 16x16 ones, or the least window of row segments)
+    b += 2 * state + std::max<int64_t>((int64_t)(3 * nt + 1) * (nsb + 1),
+                                       (grad_mode == FKADJ_GRAD_EXACT ? 3 : 1) * std::min<int64_t>(nt + 1, std::max(32, (int)std::ceil(std::sqrt((double)nt)))) * 16 * nsb) * 8;
     // stage states of a chunk | midpoint states of a chunk (more than yh and the caches)
-    b += grad_mode == FKADJ_GRAD_EXACT ? 3 * kSweepChunkExact * state : kSweepChunk * state;
+    const bool ex = grad_mode == FKADJ_GRAD_EXACT;
+    b += (int64_t)std::min(nt, sweep_chunk_of(state, ex)) * (ex ? 3 : 1) * state;
     if (policy == FKADJ_CKPT_FULL) {
         b += (int64_t)(nt + 1) * state;
     } else {
@@ -616,7 +626,7 @@ int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t
 int64_t Problem::device_bytes() const {
     const DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_,
                            &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_, &fcache_,
-                           &cells_, &adjf_, &xchg_, &pts_};
+                           &cells_, &adjf_, &segf_, &xchg_, &pts_};
     int64_t s = 0;
     for (auto* b : all) s += (int64_t)b->bytes;
     return s;
@@ -748,7 +758,7 @@ fkadj_status Problem::step_forward(int i, const double* yin, double* yout, doubl
 fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* last, double* out, double* keep) {
     if (n <= 0) return FKADJ_OK;
     const long long stride = (long long)state_elems();
-    if (!sweeping()) {
+    if (run_.id < 0 || !sweeping()) {
         // two states other than src for the steps in between
         double* s0 = src == state_buf(1) ? state_buf(0) : state_buf(1);
         double* s1 = src == state_buf(2) ? state_buf(0) : state_buf(2);
@@ -756,7 +766,16 @@ fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* las
         const double* cur = src;
         for (int k = 0; k < n; ++k) {
             double* o = k == n - 1 ? last : (out ? out + k * stride : ((k & 1) ? s1 : s0));
-            if (fkadj_status s = step_forward(i + k, cur, o, keep ? keep + k * stride : nullptr)) return s;
+            if (sweeping()) {
+                const EStep E = efwd(i + k);
+                const FwdStep r{cur, o, keep ? keep + 3 * k * stride : nullptr, E.p[0], E.p[1], E.p[2], fault()};
+                CK(prof_begin(K_FWD), "profiling event");
+                CK(launch_fwd_tile(P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), r, sms_, st_), "forward step");
+                CK(prof_end(K_FWD), "profiling event");
+                ++launches_;
+            } else if (fkadj_status s = step_forward(i + k, cur, o, keep ? keep + k * stride : nullptr)) {
+                return s;
+            }
             cur = o;
         }
         return FKADJ_OK;
@@ -781,6 +800,16 @@ fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* las
     return FKADJ_OK;
 }
 
+// Steps of a chunk of an adjoint sweep, whose points between the states are
+// made ahead: what 256 MB hold (the launches of a chunk cost about 20 us, so
+// small grids take long ones), at least 2 and at most 64.
+int Problem::sweep_chunk_of(int64_t state_bytes, bool exact) {
+    return (int)std::max<int64_t>(2, std::min<int64_t>(64, (256 << 20) / (state_bytes * (exact ? 3 : 1))));
+}
+int Problem::sweep_chunk() const {
+    return sweep_chunk_of((int64_t)state_bytes(), grad_mode_ == FKADJ_GRAD_EXACT);
+}
+
 fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
                                     const double* stages, double*& z, double*& z2) {
     const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
@@ -788,7 +817,7 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
     auto state = [&](int t) { return t == hi ? y_hi : (t == lo ? y_lo : mid + (t - lo - 1) * sz); };
     for (int top = hi; top > lo;) {
         // a chunk's rows of partial sums (top - 1 down) stay within one window
-        const int n = std::min({top - lo, exact && !stages ? kSweepChunkExact : kSweepChunk, (top - 1) % pwin_ + 1});
+        const int n = std::min({top - lo, sweep_chunk(), (top - 1) % pwin_ + 1});
         AdjRun r{};
         r.zin = z;
         r.zout = z2;
@@ -803,16 +832,13 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
         r.row0 = top - 1;
         r.window = pwin_;
         r.exchange = xchg_.p;
-        r.epoch = epoch_;
         r.fault = fault();
-        epoch_ += (unsigned long long)n;
         r.pts = pts_.as<double>();
         r.pts_step = exact ? 3 : 1;
         if (exact && stages) {
             r.pts = stages + 3 * (long long)(top - 1 - lo) * sz;
             r.pts_step = -3;
         } else if (exact) {
-            epoch_ += (unsigned long long)n;
             for (int k = 0; k < n; ++k)
                 if (fkadj_status s = sweep_forward(top - 1 - k, 1, state(top - 1 - k), state_buf(1), nullptr,
                                                    pts_.as<double>() + 3 * k * sz))
@@ -833,12 +859,29 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
             CK(prof_end(K_MID), "profiling event");
             ++launches_;
         }
-        CK(prof_begin(K_ADJ, n), "profiling event");
-        CK(launch_adj_run(run_, exact, P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), adjf_.as<uint8_t>(), r, st_),
-           "adjoint sweep");
-        CK(prof_end(K_ADJ), "profiling event");
-        ++launches_;
-        std::swap(z, z2);
+        if (run_.id >= 0) {
+            r.epoch = epoch_;  // after a replay's forward sweeps
+            epoch_ += (unsigned long long)n;
+            CK(prof_begin(K_ADJ, n), "profiling event");
+            CK(launch_adj_run(run_, exact, P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), adjf_.as<uint8_t>(), r, st_),
+               "adjoint sweep");
+            CK(prof_end(K_ADJ), "profiling event");
+            ++launches_;
+            std::swap(z, z2);
+        }
+        for (int k = 0; k < n && run_.id < 0; ++k) {
+            const double* p = r.pts + (long long)k * r.pts_step * sz;
+            const double *y1 = state(top - k), *y0 = state(top - k - 1);
+            AdjStep a{z, z2, {y1, p, p, y0}, {nullptr, nullptr, nullptr}, nsbx_, fault()};
+            if (exact) a.y[0] = p + 2 * sz, a.y[1] = p + sz, a.y[2] = p;
+            for (int gr = 0; gr < (exact ? 3 : 1); ++gr) a.row[gr] = prow(gr, top - 1 - k);
+            CK(prof_begin(K_ADJ), "profiling event");
+            CK(launch_adj_tile(exact, P_, g_, gh_.as<double>(), adjf_.as<uint8_t>(), segf_.as<uint8_t>(), a, sms_, st_),
+               "adjoint step");
+            CK(prof_end(K_ADJ), "profiling event");
+            ++launches_;
+            std::swap(z, z2);
+        }
         top -= n;
         // as in the per-step sweeps: a sqrt store reduces at the end of each segment
         if (traj_plan_.policy != FKADJ_CKPT_SQRT && top % pwin_ == 0)
@@ -1065,16 +1108,17 @@ fkadj_status Problem::ensure_traj(const TrajPlan& tp) {
 }
 
 fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
-    if (!zbuf_.p) {
-        CK(zbuf_.alloc(2 * state_bytes()), "alloc adjoint states");
-        CK(cudaMemsetAsync(zbuf_.p, 0xff, zbuf_.bytes, st_), "init adjoint states");
-    }
     const bool sweep = sweeping() && !all_rows;
+    // holes and everything off the grid: 0 for the sweeps, NaN for the preset kernels
+    if (!zbuf_.p || zero_holes_ != sweep) {
+        if (!zbuf_.p) CK(zbuf_.alloc(2 * state_bytes()), "alloc adjoint states");
+        CK(cudaMemsetAsync(zbuf_.p, sweep ? 0 : 0xff, zbuf_.bytes, st_), "init adjoint states");
+        zero_holes_ = sweep;
+    }
     if (sweep) {
         // midpoint states of a chunk, or the stage states of one where the plan keeps none
-        const size_t k = grad_mode_ == FKADJ_GRAD_REF ? (size_t)std::min(kSweepChunk, nt_)
-                         : traj_plan_.keep_f          ? 0
-                                                      : 3 * (size_t)std::min(kSweepChunkExact, nt_);
+        const size_t c = (size_t)std::min(sweep_chunk(), nt_);
+        const size_t k = grad_mode_ == FKADJ_GRAD_REF ? c : (traj_plan_.keep_f ? 0 : 3 * c);
         if (pts_.bytes < k * state_bytes()) {
             CK(pts_.alloc(k * state_bytes()), "alloc adjoint points");
             CK(cudaMemsetAsync(pts_.p, 0xff, pts_.bytes, st_), "init adjoint points");
@@ -1114,27 +1158,22 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
         win = std::min(per_group, c >= kPartialWindow ? c : c * (kPartialWindow / c));
     }
     // Lattice of the partials: 16-cell row segments (16 times as many partials
-    // as 16x16 sub-blocks; the adjoint tiles may then take any height) with
-    // windowed partials, where 64x32 tiles fit the grid into one wave of CTAs,
-    // one per SM, or sweeps could (512 x 512 and below: tiles of the one-wave
-    // height fill the wave, 512^2 x 2000 gradient 132.0 -> 129.4 ms; at 2048 x
-    // 2048, 14 waves, the 16-fold partials cost 1.4 %).  The window then
-    // shrinks, in whole segments under a sqrt store, towards the full rows of
-    // 16x16 partials, but holds a sqrt segment.  The choice depends on the grid
-    // and the device only, never on the store or the launches, so that all give
-    // the same bits.  The 16x16 lattice otherwise: the fused step, the batch
-    // engine's all-rows buffers, and under FKADJ_ZGH_SEGMENTS=0.
+    // as 16x16 sub-blocks; the adjoint tiles may then take any height, and the
+    // sweeps write only the segments with a source) with windowed partials.
+    // The window then shrinks, in whole segments under a sqrt store, towards
+    // the full rows of 16x16 partials, but holds a sqrt segment, or 32 rows:
+    // the reduction runs one CTA per row.  The choice never depends on the
+    // store or the launches, so that all give the same bits.  The 16x16
+    // lattice: the fused step, the batch engine's all-rows buffers, and under
+    // FKADJ_ZGH_SEGMENTS=0.
     const size_t nsb16 = (size_t)nsbx_ * (size_t)nsby_, nsbseg = (size_t)nsbx_ * (size_t)g_.nrows;
     const size_t fit = prow * (nsb16 + 1) / nsbseg / (size_t)groups;  // rows of segment partials within that count
-    const int c_sqrt = std::max(2, (int)std::ceil(std::sqrt((double)nt_)));  // plan_trajectory's stride
-    const bool one_wave = (int64_t)((g_.nrows + 31) / 32) * ((g_.ncols + 63) / 64) <= (int64_t)sms_;
-    bool segs = !all_rows && (forced_path_ < 0 || forced_path_ == ADJ_SPLIT) &&
-                (one_wave || run_shape(g_, sms_).id >= 0);
+    bool segs = !all_rows && (forced_path_ < 0 || forced_path_ == ADJ_SPLIT);
     if (const char* sv = getenv("FKADJ_ZGH_SEGMENTS")) segs = segs && std::atoi(sv) != 0;
     if (segs && (size_t)win > fit) {
         const int c = sqrt_store ? traj_plan_.stride : 1;
         win = (int)std::max<size_t>(std::min<size_t>((size_t)win, fit / (size_t)c * (size_t)c),
-                                    (size_t)(sqrt_store ? c : std::min({win, c_sqrt, kSweepChunk})));
+                                    (size_t)(sqrt_store ? c : std::min(win, 32)));
     }
     if (all_rows) win = (int)prow;
     const size_t nsb = segs ? nsbseg : nsb16;

@@ -174,8 +174,9 @@ public:
     fkadj_status sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
                                const double* stages, double*& z, double*& z2);
     fkadj_status init_sweeps(const int* ai, const std::vector<double>& gh, const std::vector<uint8_t>& wc);
-    // whether sweeps run as one launch (fk_run.h) on this problem
-    bool sweeping() const { return run_.id >= 0 && !run_off_; }
+    // whether this problem's steps are sweeps (fk_run.h): one launch each where
+    // run_.id >= 0, the tile kernels otherwise
+    bool sweeping() const { return swept_ && !run_off_; }
     double* state_buf(int k) const { return work_.as<double>() + (size_t)k * state_elems(); }
     size_t state_elems() const { return (size_t)3 * g_.plane; }
     size_t state_bytes() const { return state_elems() * sizeof(double); }
@@ -285,14 +286,18 @@ private:
     unsigned* fault() const { return fault_.as<unsigned>(); }
     DevBuf cells_;     // geometry flags per padded cell (CELL_*), where the grid is swept
     DevBuf adjf_;      // the adjoint sweeps' flags per padded cell
+    DevBuf segf_;      // per 16-cell row segment: whether it holds a source cell
     DevBuf xchg_;      // the sweeps' edge exchange
     DevBuf pts_;       // points between the states of one chunk of an adjoint sweep
     int sms_ = 0;
-    static constexpr int kSweepChunk = 16, kSweepChunkExact = 8;
-    RunShape run_;     // how the grid is swept (id -1: per-step launches)
+    static int sweep_chunk_of(int64_t state_bytes, bool exact);
+    int sweep_chunk() const;
+    RunShape run_;     // how the grid is swept in one launch (id -1: it does not fit)
+    bool swept_ = false;
+    bool zero_holes_ = false;  // what zbuf_ holds at holes
     unsigned long long epoch_ = 0;  // steps swept so far (the exchange's tags)
-    // per-step launches after all: a sweep met a NaN away from the holes
-    // (FAULT_NAN), which the per-step kernels contain
+    // the preset kernels after all: a sweep met a NaN away from the holes
+    // (FAULT_NAN), which they contain
     bool run_off_ = false;
     bool nan_seen_ = false;
     bool own_sweeps_ = true;  // false for a batch engine's problems, which run batched launches

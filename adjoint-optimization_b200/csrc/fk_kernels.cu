@@ -1321,6 +1321,7 @@ __global__ void k_sum_rows(const double* __restrict__ partial, int ntiles, doubl
     __shared__ double red[8];
     const double* p = partial + (long long)blockIdx.x * ntiles;
     double acc = 0.0;
+#pragma unroll 16
     for (int k = threadIdx.x; k < ntiles; k += 256) acc += p[k];
     const double s = block_sum<256>(acc, red);
     if (threadIdx.x == 0) out[blockIdx.x] = s;

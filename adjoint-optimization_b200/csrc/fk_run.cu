@@ -49,6 +49,7 @@ namespace {
 template <int TX_, int R_, int TYM_>
 struct Shape {
     static constexpr int TX = TX_, R = R_, TYM = TYM_;
+    static constexpr bool RESIDENT = true;  // the tile stays in window A from step to step
     static constexpr int RW = TX + 2 * HALO;  // window width = pitch of every buffer
     // Buffers, three planes each, all addressed in window coordinates (row 0 =
     // 4 rows above the tile): A, the step-start state, rows 0 .. TYM + 7; B,
@@ -65,6 +66,21 @@ struct Shape {
     static_assert(R <= 5, "six flag bits a row in one register");
     static_assert(SMEM_EXACT + 768 <= 232448, "one CTA's shared memory");
     static_assert(THREADS <= 512, "128 registers per thread");
+};
+
+// Tiles of the per-step kernels of larger grids (k_fwd_tile, k_adj_tile): the
+// same stages, with a second window A that takes the next tile's while this
+// one computes, the source read from global memory, and the terms of the z.gh
+// sums in planes of their own (three in the exact mode).
+struct TileShapeBig {
+    static constexpr int TX = 64, R = 4, TYM = 22;
+    static constexpr bool RESIDENT = false;
+    static constexpr int RW = TX + 2 * HALO;
+    static constexpr int PA = (TYM + 8) * RW, PB = (TYM + 6) * RW, PC = (TYM + 4) * RW, TERM = TYM * TX;
+    static constexpr int THREADS = ((RW * ((TYM + 6) / R) + 31) / 32) * 32;
+    static constexpr size_t SMEM = sizeof(double) * (size_t)(3 * (2 * PA + PB + PC) + 3 * TERM);
+    static_assert((TYM + 6) % R == 0 && THREADS <= 512 && SMEM + 256 <= 232448, "one CTA per SM");
+    static_assert(3 * TERM >= 2 * RW, "reads past C stay in the allocation");
 };
 
 // One exchanged value: the state's double and the number of the step it
@@ -212,20 +228,24 @@ __device__ __forceinline__ void fwd_rows(const DevModel& P, const Column& T, con
         const double* pw = Y + k * RW + ((b & CELL_W) ? 1 : -1);
         const double* pe = Y + k * RW + ((b & CELL_E) ? -1 : 1);
         double s[3];
+        double gv = 0.0;
+        if (b & CELL_SOURCE) gv = S::RESIDENT ? G[q0 + k * RW] : __ldg(G + T.o + k * ld);
 #pragma unroll
         for (int f = 0; f < 3; ++f) s[f] = ps[f * PS];
         if (r >= HALO - E && r < HALO + rows + E) {
             double t[3], kk[3];
 #pragma unroll
             for (int f = 0; f < 3; ++f) t[f] = lap4((b & CELL_N) ? s[f] : n[f], s[f], pw[f * PS], pe[f * PS], m[f]);
-            double gv = 0.0;
-            if (b & CELL_SOURCE) gv = G[q0 + k * RW];
             fk_field(P, m, t, Ev, gv, kk[0], kk[1], kk[2]);
             double* a = A + q0 + k * RW;
             if (MODE == 2) {
                 double o[3];
 #pragma unroll
-                for (int f = 0; f < 3; ++f) a[f * S::PA] = o[f] = fma(cD, kk[f], a[f * S::PA] + D[k][f]);
+                for (int f = 0; f < 3; ++f) o[f] = fma(cD, kk[f], a[f * S::PA] + D[k][f]);
+                if (S::RESIDENT) {
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) a[f * S::PA] = o[f];
+                }
                 bad = bad || (isnan(o[0]) && (b & CELL_ACTIVE));
                 if (out) {
 #pragma unroll
@@ -354,8 +374,8 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
 // instead, 250 B a cell and step through L2, and took 20 us for it at 512 x
 // 512.
 //
-// Holes hold 0 in the buffers here (and NaN in every state that leaves the
-// tile): a missing neighbour then adds nothing to the plain sum, and only the
+// Holes and everything off the grid hold 0 here, in the buffers and in z's
+// states: a missing neighbour then adds nothing to the plain sum, and only the
 // neighbours that mirrored this cell are added once more.
 
 // Row k of a column's values of state y (its window's origin), 0 past the tile
@@ -367,6 +387,12 @@ __device__ __forceinline__ void load_point(const Column& T, int k, int rows, int
     for (int f = 0; f < 3; ++f) v[f] = on ? __ldg(y + f * plane + T.o + k * ld) : 0.0;
 }
 
+// A cell's term of a z.gh sum: NaN counts as 0, as does a cell without source
+__device__ __forceinline__ double source_term(unsigned b, double z, double gh) {
+    const double t = z * gh;
+    return (b & CELL_SOURCE) && !isnan(t) ? t : 0.0;
+}
+
 // One backward stage on the tile grown by E cells, for the thread's own cells:
 // k = L^T src + J_F(y)^T src, then in the reference mode
 //   MODE 0: dst = z0 + cA k, D  = cB k
@@ -376,13 +402,14 @@ __device__ __forceinline__ void load_point(const Column& T, int k, int rows, int
 // and k there is scaled by cS = dt/6 (a_4 = dt/6 lambda),
 //   MODE 0: dst = cB z0 + cA k, D  = k;  MODE 1: the same, D += k
 //   MODE 2: z0 <- z0 + (D + k)
-// with z0 in window A.  yv holds the first row of y; `keep` (exact mode, first
-// stage) receives a_3 on u.
+// with z0 in window A.  yv holds the first row of y.  keep: in a resident
+// tile's exact mode, where the first stage leaves a_3 on u; else the planes of
+// the z.gh sums' terms (gh: the source's window origin).
 template <int E, class S, int MODE, int PS, int PT, bool EXACT>
 __device__ __forceinline__ void adj_rows(const DevModel& P, const Column& T, const double* src, double* dst, double* A,
                                          double (&D)[S::R][3], double (&yv)[3], const double* __restrict__ y, int rows,
                                          int ld, long long plane, double cA, double cB, double cS, double* keep,
-                                         double* __restrict__ out, Tagged* __restrict__ x, unsigned long long tag) {
+                                         const double* __restrict__ gh, double* __restrict__ out, Tagged* __restrict__ x, unsigned long long tag) {
     constexpr int RW = S::RW;
     if (T.c < HALO - E || T.c >= HALO + S::TX + E) return;
     const int q0 = T.r0 * RW + T.c;
@@ -398,6 +425,8 @@ __device__ __forceinline__ void adj_rows(const DevModel& P, const Column& T, con
         const unsigned b = bits >> (6 * k);
         double s[3], yn[3];
         if (k + 1 < S::R) load_point<S>(T, k + 1, rows, ld, plane, y, yn);
+        double gv = 0.0;
+        if (!S::RESIDENT && (MODE == 2 || EXACT) && (b & CELL_SOURCE)) gv = __ldg(gh + T.o + k * ld);
 #pragma unroll
         for (int f = 0; f < 3; ++f) s[f] = Z[f * PS + (k + 1) * RW];
         if (r >= HALO - E && r < HALO + rows + E) {
@@ -418,18 +447,20 @@ __device__ __forceinline__ void adj_rows(const DevModel& P, const Column& T, con
             adj_field(P, J, m, t, kk[0], kk[1], kk[2]);
             const bool act = b & CELL_ACTIVE_ADJ;
             double* a = A + q0 + k * RW;
+            const int term = (r - HALO) * S::TX + T.c - HALO;
             if (MODE == 2) {
                 double o[3];
 #pragma unroll
                 for (int f = 0; f < 3; ++f)
                     o[f] = EXACT ? a[f * S::PA] + (D[k][f] + kk[f]) : fma(cB, kk[f], a[f * S::PA] + D[k][f]);
-                if (act) {
+                if (S::RESIDENT && act) {
 #pragma unroll
                     for (int f = 0; f < 3; ++f) a[f * S::PA] = o[f];
                 }
+                if constexpr (!S::RESIDENT && !EXACT) keep[term] = source_term(b, o[0], gv);
                 if (out) {
 #pragma unroll
-                    for (int f = 0; f < 3; ++f) out[f * plane + T.o + k * ld] = act ? o[f] : __longlong_as_double(-1);
+                    for (int f = 0; f < 3; ++f) out[f * plane + T.o + k * ld] = act ? o[f] : 0.0;
                 }
                 if (x && (r < 2 * HALO || r >= rows || T.c < 2 * HALO || T.c >= S::TX)) {
 #pragma unroll
@@ -441,10 +472,20 @@ __device__ __forceinline__ void adj_rows(const DevModel& P, const Column& T, con
                     const double z0 = MODE == 0 ? m[f] : a[f * S::PA];
                     if (EXACT && MODE == 0) kk[f] = cS * kk[f];
                     const double o = EXACT ? fma(cA, kk[f], cB * z0) : fma(cA, kk[f], z0);
-                    if (act) dst[f * PT + q0 + k * RW] = o;
+                    if (!S::RESIDENT) dst[f * PT + q0 + k * RW] = act ? o : 0.0;
+                    else if (act) dst[f * PT + q0 + k * RW] = o;
                     if (EXACT) D[k][f] = MODE == 0 ? kk[f] : D[k][f] + kk[f];
                     else D[k][f] = MODE == 0 ? cB * kk[f] : fma(cB, kk[f], D[k][f]);
-                    if (EXACT && MODE == 0 && f == 0) keep[q0 + k * RW] = o;
+                    if constexpr (EXACT && S::RESIDENT) {
+                        if (MODE == 0 && f == 0) keep[q0 + k * RW] = o;
+                    } else if constexpr (EXACT) {
+                        if (f == 0 && r >= HALO && r < HALO + rows && T.c >= HALO && T.c < HALO + S::TX) {
+                            // b.a4 and a3, then b.(a2 + a3), then b.a1
+                            if (MODE == 0) keep[2 * S::TERM + term] = source_term(b, cS * m[0], gv), keep[S::TERM + term] = o;
+                            else if (E == 2) keep[S::TERM + term] = source_term(b, o + keep[S::TERM + term], gv);
+                            else keep[term] = source_term(b, o, gv);
+                        }
+                    }
                 }
             }
         }
@@ -549,14 +590,6 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     }
     if (!bulk_wait_cta(b, r.fault)) return;
     __syncthreads();
-    for (int q = threadIdx.x; q < (rows + 2 * HALO) * RW; q += blockDim.x) {
-        const int row = q / RW, c = q - row * RW;
-        if (!(adj[off + (long long)row * g.ld + c] & CELL_ACTIVE_ADJ)) {
-#pragma unroll
-            for (int f = 0; f < 3; ++f) A[f * S::PA + q] = 0.0;
-        }
-    }
-    __syncthreads();
     const int nsegs = s_segs;
     // the step's four states (k = 0 is the sweep's first, the latest in time)
     auto yptr = [&](int j) {  // y after j steps back
@@ -577,17 +610,17 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
                              [&](int q) { return ((P.dt / 6.0) * A[q]) * G[q]; });
         adj_rows<3, S, 0, S::PA, S::PB, EXACT>(P, T, A, B, A, D, yv, point(k, 0), rows, g.ld, g.plane,
                                                EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt / 3.0 : 1.0 / 6.0 * P.dt,
-                                               P.dt / 6.0, K3, nullptr, nullptr, 0);
+                                               P.dt / 6.0, K3, nullptr, nullptr, nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 1), yv);
         __syncthreads();
         adj_rows<2, S, 1, S::PB, S::PC, EXACT>(P, T, B, C, A, D, yv, point(k, 1), rows, g.ld, g.plane, 0.5 * P.dt,
                                                EXACT ? P.dt / 3.0 : 2.0 / 6.0 * P.dt, 0.0, nullptr, nullptr, nullptr,
-                                               0);
+                                               nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 2), yv);
         __syncthreads();
         adj_rows<1, S, 1, S::PC, S::PB, EXACT>(P, T, C, B, A, D, yv, point(k, 2), rows, g.ld, g.plane,
                                                EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt / 6.0 : 2.0 / 6.0 * P.dt, 0.0,
-                                               nullptr, nullptr, nullptr, 0);
+                                               nullptr, nullptr, nullptr, nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 3), yv);
         __syncthreads();
         if (EXACT) {
@@ -598,7 +631,7 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
         const unsigned long long tag = r.epoch + k + 1;
         Tagged* x = static_cast<Tagged*>(r.exchange) + (tag & 1) * (3 * g.plane) + off;
         adj_rows<0, S, 2, S::PB, S::PB, EXACT>(P, T, B, nullptr, A, D, yv, point(k, 3), rows, g.ld, g.plane, 0.0,
-                                               1.0 / 6.0 * P.dt, 0.0, nullptr, end ? r.zout + off : nullptr,
+                                               1.0 / 6.0 * P.dt, 0.0, nullptr, nullptr, end ? r.zout + off : nullptr,
                                                end ? nullptr : x, tag);
         if (end) {
             __syncthreads();
@@ -613,6 +646,209 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     }
 }
 
+// --------------------------------------------- per-step tiles, larger grids
+//
+// Where the tiles do not fit the device at once, a step is one launch of one
+// CTA per SM, each taking tiles in turn; a tile's window arrives by bulk
+// copies while the tile before it computes.  The stages are the sweeps'.
+
+// What a tile kernel's CTA goes through: tile i's place and window.
+struct TileWalk {
+    int ntx, tiles, ty;
+    __device__ __forceinline__ int i0(int tile) const { return tile / ntx * ty; }
+    __device__ __forceinline__ int j0(int tile) const { return tile % ntx * TileShapeBig::TX; }
+};
+
+// Issues the copies of the window of `tile` of state y into buffer A (its last
+// readers are past a barrier), a few by every warp: by one warp, it fell 2 us a
+// tile behind the others.  The copies may complete before thread 0 has posted
+// their bytes: the barrier's phase ends with both.
+__device__ __forceinline__ void fetch_tile(const DevGrid& g, const TileWalk& w, int tile, const double* y, double* A,
+                                           uint32_t bar) {
+    using S = TileShapeBig;
+    const int i0 = w.i0(tile), nr = min(w.ty, g.nrows - i0) + 2 * HALO;
+    const double* src = y + (long long)i0 * g.ld + w.j0(tile);
+    bulk_arrive(bar, bulk_bytes<S::RW>(nr));
+    const int t = (threadIdx.x & 31) * (S::THREADS / 32) + (threadIdx.x >> 5);
+    static_assert(3 * (S::TYM + 2 * HALO) <= S::THREADS, "one copy per thread");
+    if (t < 3 * nr) {
+        const int f = t / nr, row = t - f * nr;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        bulk_row<S::RW>(bar, A + f * S::PA + row * S::RW, src + f * g.plane + (long long)row * g.ld);
+    }
+}
+
+// The barrier after a tile's first stage, with the outcome of its window's
+// wait (one for the CTA): where the window did not arrive, as bulk_wait_cta,
+// the fault word is set and the copies in flight (this tile's, and the next
+// one's where it was fetched) waited for once more; the caller returns.
+__device__ __forceinline__ bool window_arrived(bool ok, uint32_t bar, int n, bool next, unsigned* fault) {
+    if (!__syncthreads_or(!ok)) return true;
+    if (threadIdx.x == 0) atomicOr(fault, FAULT_TIMEOUT);
+    bulk_wait(bar + 8 * (n & 1), 1000000000ull, (unsigned)(n >> 1) & 1u);
+    if (next) bulk_wait(bar + 8 * (~n & 1), 1000000000ull, (unsigned)((n + 1) >> 1) & 1u);
+    return false;
+}
+
+// The flags of a thread's rows of a tile, loaded a tile ahead of their use
+struct RowFlags {
+    unsigned f[TileShapeBig::R];
+    __device__ __forceinline__ void load(const DevGrid& g, const TileWalk& w, int tile, const Column& T, int c,
+                                         const uint8_t* __restrict__ cells) {
+        const int i0 = w.i0(tile), rows = min(w.ty, g.nrows - i0);
+        const uint8_t* p = cells + (long long)i0 * g.ld + w.j0(tile) + T.o;
+#pragma unroll
+        for (int k = 0; k < TileShapeBig::R; ++k)
+            f[k] = c >= 1 && c < TileShapeBig::TX + 7 && T.r0 + k < rows + 7 ? __ldg(p + k * g.ld) : 0u;
+    }
+    __device__ __forceinline__ unsigned bits() const {
+        unsigned b = 0;
+#pragma unroll
+        for (int k = 0; k < TileShapeBig::R; ++k) b |= f[k] << (6 * k);
+        return b;
+    }
+};
+
+__device__ __forceinline__ Column tile_column(int ld) {
+    Column T;
+    const int col = threadIdx.x / TileShapeBig::RW;
+    T.c = threadIdx.x - col * TileShapeBig::RW;
+    T.r0 = 1 + col * TileShapeBig::R;
+    T.o = T.r0 * ld + T.c;
+    T.bits = 0;
+    return T;
+}
+
+__global__ void __launch_bounds__(TileShapeBig::THREADS, 1)
+    k_fwd_tile(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
+               const FwdStep r, const TileWalk w) {
+    using S = TileShapeBig;
+    extern __shared__ double4 smem_raw[];
+    __shared__ uint64_t bars[2];
+    double* const W = reinterpret_cast<double*>(smem_raw);
+    double* const B = W + 6 * S::PA - S::RW;
+    double* const C = W + 3 * (2 * S::PA + S::PB) - 2 * S::RW;
+    exp_table_init();
+    const uint32_t bar = bulk_begin(&bars[0]);
+    bulk_begin(&bars[1]);
+    __syncthreads();
+    Column T = tile_column(g.ld);
+    const int c_all = T.c;
+    double D[S::R][3];
+    bool bad = false;
+    int n = 0;
+    RowFlags next;
+    if ((int)blockIdx.x < w.tiles) {
+        fetch_tile(g, w, blockIdx.x, r.src, W, bar);
+        next.load(g, w, blockIdx.x, T, c_all, cells);
+    }
+    const double E0 = __ldg(r.E0), Eh = __ldg(r.Eh), E1 = __ldg(r.E1);
+    for (int tile = blockIdx.x; tile < w.tiles; tile += gridDim.x, ++n) {
+        const int i0 = w.i0(tile), rows = min(w.ty, g.nrows - i0);
+        const long long off = (long long)i0 * g.ld + w.j0(tile);
+        double* A = W + (n & 1) * 3 * S::PA;
+        T.c = T.r0 < rows + 7 ? c_all : -1;
+        T.bits = next.bits();
+        const bool more = tile + (int)gridDim.x < w.tiles;
+        if (more) {
+            fetch_tile(g, w, tile + gridDim.x, r.src, W + (~n & 1) * 3 * S::PA, bar + 8 * (~n & 1));
+            next.load(g, w, tile + gridDim.x, T, c_all, cells);
+        }
+        const bool ok = bulk_wait(bar + 8 * (n & 1), 1000000000ull, (unsigned)(n >> 1) & 1u);
+        const double* ghs = gh + off;
+        auto stage_out = [&](int st) { return r.stages ? r.stages + (long long)st * 3 * g.plane + off : nullptr; };
+        fwd_rows<3, S, 0, S::PA, S::PB>(P, T, A, B, A, ghs, D, rows, g.ld, g.plane, E0, 0.5 * P.dt,
+                                        1.0 / 6.0 * P.dt, stage_out(0), nullptr, 0, bad);
+        if (!window_arrived(ok, bar, n, more, r.fault)) return;
+        fwd_rows<2, S, 1, S::PB, S::PC>(P, T, B, C, A, ghs, D, rows, g.ld, g.plane, Eh, 0.5 * P.dt,
+                                        1.0 / 3.0 * P.dt, stage_out(1), nullptr, 0, bad);
+        __syncthreads();
+        fwd_rows<1, S, 1, S::PC, S::PB>(P, T, C, B, A, ghs, D, rows, g.ld, g.plane, Eh, P.dt,
+                                        1.0 / 3.0 * P.dt, stage_out(2), nullptr, 0, bad);
+        __syncthreads();
+        if (r.dst)
+            fwd_rows<0, S, 2, S::PB, S::PB>(P, T, B, nullptr, A, ghs, D, rows, g.ld, g.plane, E1, 0.0,
+                                            P.dt / 6.0, r.dst + off, nullptr, 0, bad);
+        __syncthreads();  // B and A are free
+    }
+    if (bad) atomicOr(r.fault, FAULT_NAN);
+}
+
+template <bool EXACT>
+__global__ void __launch_bounds__(TileShapeBig::THREADS, 1)
+    k_adj_tile(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ adj,
+               const uint8_t* __restrict__ segs, const AdjStep r, const TileWalk w) {
+    using S = TileShapeBig;
+    extern __shared__ double4 smem_raw[];
+    __shared__ uint64_t bars[2];
+    double* const W = reinterpret_cast<double*>(smem_raw);
+    double* const B = W + 6 * S::PA - S::RW;
+    double* const C = W + 3 * (2 * S::PA + S::PB) - 2 * S::RW;
+    double* const terms = W + 3 * (2 * S::PA + S::PB + S::PC);
+    exp_table_init();
+    const uint32_t bar = bulk_begin(&bars[0]);
+    bulk_begin(&bars[1]);
+    __syncthreads();
+    Column T = tile_column(g.ld);
+    const int c_all = T.c;
+    double D[S::R][3], yv[3];
+    int n = 0;
+    RowFlags next;
+    if ((int)blockIdx.x < w.tiles) {
+        fetch_tile(g, w, blockIdx.x, r.zin, W, bar);
+        next.load(g, w, blockIdx.x, T, c_all, adj);
+    }
+    for (int tile = blockIdx.x; tile < w.tiles; tile += gridDim.x, ++n) {
+        const int i0 = w.i0(tile), j0 = w.j0(tile), rows = min(w.ty, g.nrows - i0);
+        const long long off = (long long)i0 * g.ld + j0;
+        double* A = W + (n & 1) * 3 * S::PA;
+        T.c = T.r0 < rows + 7 ? c_all : -1;
+        T.bits = next.bits();
+        load_point<S>(T, 0, rows, g.ld, g.plane, r.y[0] + off, yv);
+        const bool more = tile + (int)gridDim.x < w.tiles;
+        if (more) {
+            fetch_tile(g, w, tile + gridDim.x, r.zin, W + (~n & 1) * 3 * S::PA, bar + 8 * (~n & 1));
+            next.load(g, w, tile + gridDim.x, T, c_all, adj);
+        }
+        const bool ok = bulk_wait(bar + 8 * (n & 1), 1000000000ull, (unsigned)(n >> 1) & 1u);
+        const double* ghs = gh + off;
+        adj_rows<3, S, 0, S::PA, S::PB, EXACT>(P, T, A, B, A, D, yv, r.y[0] + off, rows, g.ld, g.plane,
+                                               EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt / 3.0 : 1.0 / 6.0 * P.dt,
+                                               P.dt / 6.0, terms, ghs, nullptr, nullptr, 0);
+        load_point<S>(T, 0, rows, g.ld, g.plane, r.y[1] + off, yv);
+        if (!window_arrived(ok, bar, n, more, r.fault)) return;
+        adj_rows<2, S, 1, S::PB, S::PC, EXACT>(P, T, B, C, A, D, yv, r.y[1] + off, rows, g.ld, g.plane, 0.5 * P.dt,
+                                               EXACT ? P.dt / 3.0 : 2.0 / 6.0 * P.dt, 0.0, terms, ghs, nullptr,
+                                               nullptr, 0);
+        load_point<S>(T, 0, rows, g.ld, g.plane, r.y[2] + off, yv);
+        __syncthreads();
+        adj_rows<1, S, 1, S::PC, S::PB, EXACT>(P, T, C, B, A, D, yv, r.y[2] + off, rows, g.ld, g.plane,
+                                               EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt / 6.0 : 2.0 / 6.0 * P.dt, 0.0,
+                                               terms, ghs, nullptr, nullptr, 0);
+        load_point<S>(T, 0, rows, g.ld, g.plane, r.y[3] + off, yv);
+        __syncthreads();
+        adj_rows<0, S, 2, S::PB, S::PB, EXACT>(P, T, B, nullptr, A, D, yv, r.y[3] + off, rows, g.ld, g.plane, 0.0,
+                                               1.0 / 6.0 * P.dt, 0.0, terms, ghs, r.zout + off, nullptr, 0);
+        __syncthreads();
+        // partial sums of the row segments with a source, as segment_terms
+        constexpr int SX = S::TX / 16;
+        const int l = threadIdx.x & 15, h = threadIdx.x >> 4, nh = blockDim.x >> 4;
+        for (int s0 = 0; s0 < rows * SX; s0 += nh) {
+            const int i = s0 + h, row = i / SX, sx = i - row * SX;
+            const long long at = (long long)(i0 + row) * r.nsbx + (j0 / 16 + sx);
+            const bool on = i < rows * SX && __ldg(segs + at);
+            if (!__any_sync(0xffffffffu, on)) continue;
+            for (int gr = 0; gr < (EXACT ? 3 : 1); ++gr) {
+                double s = on ? terms[gr * S::TERM + row * S::TX + sx * 16 + l] : 0.0;
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (on && l == 0) r.row[gr][at] = s;
+            }
+        }
+        if (EXACT) __syncthreads();  // the next tile's first stage writes terms
+    }
+}
+
 // ------------------------------------------------------- midpoint states
 //
 // The midpoint states of r.n backward steps (cu-G:1244-1301) in one launch:
@@ -624,11 +860,17 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
 // waiting for their operands.
 //   y(1/3) = cubic Hermite of (ya, fa, yb, fb) at 1/3,
 //   yh     = partial quartic at 1/2 + (27/64) dt f(y(1/3), E(t + dt/3)).
+// One barrier a step: the y(1/3) buffers alternate, every warp issues a few of
+// the window's copies, and every thread waits for them itself (with barriers at
+// each of these points, 30 % of the warps' time went into them).
 struct MidShape {
-    static constexpr int TX = 64, R = 3, TY = 16, H = 2, RW = TX + 2 * HALO;
+    static constexpr int TX = 64, R = 2, TY = 16, H = 2, RW = TX + 2 * HALO;
+    static constexpr int LW = TX + 2;                 // columns evaluated: the tile and one cell around it
     static constexpr int PW = (TY + 2 * H) * RW;      // a window: rows -2 .. TY + 1
-    static constexpr int THREADS = ((RW * (TY + 2) / R) + 31) / 32 * 32;
-    static constexpr size_t SMEM = sizeof(double) * (size_t)(3 * 3 * PW + 3 * PW + PW);
+    static constexpr int THREADS = (LW * ((TY + 2) / R) + 31) / 32 * 32;
+    static constexpr size_t SMEM = sizeof(double) * (size_t)(3 * 3 * PW + 2 * 3 * PW + PW);
+    static_assert((TY + 2) % R == 0 && THREADS <= 640, "96 registers per thread");
+    static_assert(3 * (TY + 2 * H) <= THREADS, "one window copy per thread");
 };
 
 // f at the thread's cell of row k (window row r) of buffer Y from its column
@@ -658,8 +900,8 @@ __global__ void __launch_bounds__(MidShape::THREADS, 1)
     extern __shared__ double4 smem_raw[];
     __shared__ uint64_t bars[3];
     double* W = reinterpret_cast<double*>(smem_raw);  // three windows in turn
-    double* Y3 = W + 9 * PW;
-    double* G = Y3 + 3 * PW;
+    double* Y3 = W + 9 * PW;                          // two buffers in turn
+    double* G = Y3 + 6 * PW;
     const int i0 = blockIdx.y * S::TY, j0 = blockIdx.x * S::TX;
     const int rows = min(S::TY, g.nrows - i0);
     // window origin: logical (i0 - 2, j0 - 4) = padded (i0 + 2, j0)
@@ -671,57 +913,54 @@ __global__ void __launch_bounds__(MidShape::THREADS, 1)
     bulk_begin(&bars[1]);
     bulk_begin(&bars[2]);
     __syncthreads();
-    auto yptr = [&](int j) {  // y after j steps back
-        return (j == 0 ? r.y_hi : (j == r.n ? r.y_lo : r.y_mid + (long long)(r.n - 1 - j) * r.stride)) + off;
-    };
     const int nr = rows + 2 * S::H;
-    // window of y after j steps back into buffer (j - k0) % 3; its barrier's
-    // parity is (j - k0) / 3 mod 2
+    // the window of y after j steps back into buffer (j - k0) % 3 (as
+    // fetch_tile); its barrier's parity is (j - k0) / 3 mod 2
     auto fetch = [&](int j) {
         const int u = (j - k0) % 3;
+        const double* src =
+            (j == 0 ? r.y_hi : (j == r.n ? r.y_lo : r.y_mid + (long long)(r.n - 1 - j) * r.stride)) + off;
         bulk_arrive(bar + 8 * u, bulk_bytes<RW>(nr));
-        __syncthreads();
-        const double* src = yptr(j);
-        for (int t = threadIdx.x; t < 3 * nr; t += blockDim.x) {
+        const int t = (threadIdx.x & 31) * (S::THREADS / 32) + (threadIdx.x >> 5);
+        if (t < 3 * nr) {
             const int f = t / nr, row = t - f * nr;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             bulk_row<RW>(bar + 8 * u, W + (3 * u + f) * PW + row * RW, src + f * g.plane + (long long)row * g.ld);
         }
     };
     fetch(k0);
     fetch(k0 + 1);
-    const int col = threadIdx.x / RW;
-    const int c = threadIdx.x - col * RW, r0 = 1 + col * R;
-    const bool in = c >= HALO - 1 && c < HALO + S::TX + 1;
+    const int col = threadIdx.x / S::LW;
+    const int c = HALO - 1 + threadIdx.x - col * S::LW, r0 = 1 + col * R;
     unsigned bits = 0;
     double fb[R][3];
 #pragma unroll
     for (int k = 0; k < R; ++k)
-        if (in && r0 + k < rows + 3) {
+        if (r0 + k < rows + 3) {
             bits |= (unsigned)cells[off + (long long)(r0 + k) * g.ld + c] << (6 * k);
             G[(r0 + k) * RW + c] = gh[off + (long long)(r0 + k) * g.ld + c];
         }
     if (!bulk_wait_cta(bar, r.fault)) return;
 #pragma unroll
     for (int k = 0; k < R; ++k)
-        if (in && r0 + k < rows + 3) {
+        if (r0 + k < rows + 3) {
             const int q = (r0 + k) * RW + c;
             mid_field(P, bits >> (6 * k), W + q, G + q, __ldg(r.Et - k0), fb[k]);
         }
     for (int k = k0; k < k1; ++k) {
         const int ub = (k - k0) % 3, ua = (k + 1 - k0) % 3;
-        // the window after next into the buffer that the step before last used
-        if (k + 2 <= k1) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            fetch(k + 2);
-        }
-        if (!bulk_wait_cta(bar + 8 * ua, r.fault, 1000000000ull, (unsigned)((k + 1 - k0) / 3) & 1u)) return;
+        // the window after next into the buffer that the step before last read
+        // (its readers are past the last step's barrier)
+        if (k + 2 <= k1) fetch(k + 2);
+        const double Ea = __ldg(r.Et - k - 1), E3 = __ldg(r.E3 - k);
+        const bool ok = bulk_wait(bar + 8 * ua, 1000000000ull, (unsigned)((k + 1 - k0) / 3) & 1u);
         const double* YA = W + 3 * ua * PW;
         const double* YB = W + 3 * ub * PW;
-        const double Ea = __ldg(r.Et - k - 1);
+        double* T3 = Y3 + 3 * ((k - k0) & 1) * PW;
         double qv[R][3];
 #pragma unroll
         for (int u = 0; u < R; ++u)
-            if (in && r0 + u < rows + 3) {
+            if (r0 + u < rows + 3) {
                 const int q = (r0 + u) * RW + c;
                 double fa[3];
                 mid_field(P, bits >> (6 * u), YA + q, G + q, Ea, fa);
@@ -729,25 +968,30 @@ __global__ void __launch_bounds__(MidShape::THREADS, 1)
                 for (int f = 0; f < 3; ++f) {
                     const double m0 = fa[f] * P.dt, m1 = fb[u][f] * P.dt;
                     const double x0 = YA[f * PW + q], x1 = YB[f * PW + q];
-                    Y3[f * PW + q] = hermite4(hw.c3, x0, m0, x1, m1);
+                    T3[f * PW + q] = hermite4(hw.c3, x0, m0, x1, m1);
                     qv[u][f] = hermite4(hw.c4, x0, m0, x1, m1);
                     fb[u][f] = fa[f];
                 }
             }
-        __syncthreads();
-        const double E3 = __ldg(r.E3 - k);
+        if (__syncthreads_or(!ok)) {
+            // a window did not arrive in time: as bulk_wait_cta, once more for
+            // the copies in flight, then out
+            if (threadIdx.x == 0) atomicOr(r.fault, FAULT_TIMEOUT);
+            for (int j = k + 1; j <= min(k + 2, k1); ++j)
+                bulk_wait(bar + 8 * ((j - k0) % 3), 1000000000ull, (unsigned)((j - k0) / 3) & 1u);
+            return;
+        }
         double* yh = r.yh + (long long)k * r.stride + off;
 #pragma unroll
         for (int u = 0; u < R; ++u)
             if (c >= HALO && c < HALO + S::TX && r0 + u >= S::H && r0 + u < S::H + rows) {
                 const int q = (r0 + u) * RW + c;
                 double m2[3];
-                mid_field(P, bits >> (6 * u), Y3 + q, G + q, E3, m2);
+                mid_field(P, bits >> (6 * u), T3 + q, G + q, E3, m2);
 #pragma unroll
                 for (int f = 0; f < 3; ++f)
                     yh[f * g.plane + (long long)(r0 + u) * g.ld + c] = fma(hw.c2, m2[f] * P.dt, qv[u][f]);
             }
-        __syncthreads();
     }
 }
 
@@ -796,6 +1040,10 @@ size_t run_exchange_bytes(const DevGrid& g) { return 2 * 3 * (size_t)g.plane * s
 
 cudaError_t run_init() {
     cudaError_t e = cudaFuncSetAttribute(k_mid_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MidShape::SMEM);
+    const int big = (int)TileShapeBig::SMEM;
+    if (!e) e = cudaFuncSetAttribute(k_fwd_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (!e) e = cudaFuncSetAttribute(k_adj_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (!e) e = cudaFuncSetAttribute(k_adj_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 #undef X
 #define X(id, a, b, c)                                                                                     \
     if (!e) e = cudaFuncSetAttribute(k_fwd_run<a, b, c>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
@@ -834,6 +1082,37 @@ cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const DevGrid& 
 #undef X
     }
     return cudaErrorInvalidValue;
+}
+
+// Rows per tile of the per-step tile kernels: the fewest waves of CTAs, then
+// the least work per wave (a tile's cost goes with its rows and the halo's).
+static TileWalk tile_walk(const DevGrid& g, int sms) {
+    using S = TileShapeBig;
+    TileWalk w{(g.ncols + S::TX - 1) / S::TX, 0, 0};
+    long long best = -1;
+    for (int ty = HALO; ty <= S::TYM; ++ty) {
+        const int tiles = w.ntx * ((g.nrows + ty - 1) / ty);
+        const long long cost = (long long)((tiles + sms - 1) / sms) * (4 * ty + 12 + 16);
+        if (best < 0 || cost <= best) best = cost, w.ty = ty, w.tiles = tiles;
+    }
+    return w;
+}
+
+cudaError_t launch_fwd_tile(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,
+                            const FwdStep& r, int sms, cudaStream_t st) {
+    using S = TileShapeBig;
+    const TileWalk w = tile_walk(g, sms);
+    k_fwd_tile<<<std::min(sms, w.tiles), S::THREADS, S::SMEM, st>>>(P, g, gh, cells, r, w);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adj_tile(bool exact, const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* adj,
+                            const uint8_t* segs, const AdjStep& r, int sms, cudaStream_t st) {
+    using S = TileShapeBig;
+    const TileWalk w = tile_walk(g, sms);
+    if (exact) k_adj_tile<true><<<std::min(sms, w.tiles), S::THREADS, S::SMEM, st>>>(P, g, gh, adj, segs, r, w);
+    else k_adj_tile<false><<<std::min(sms, w.tiles), S::THREADS, S::SMEM, st>>>(P, g, gh, adj, segs, r, w);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_mid_run(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,

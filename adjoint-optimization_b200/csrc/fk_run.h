@@ -78,6 +78,32 @@ struct AdjRun {
     unsigned long long epoch;
     unsigned* fault;
 };
+// One forward step of a grid that does not fit the device at once: src -> dst
+// (null: not stored) and its stage states Y2, Y3, Y4 to three states in a row
+// (null: not kept).
+struct FwdStep {
+    const double* src;
+    double *dst, *stages;
+    const double *E0, *Eh, *E1;
+    unsigned* fault;
+};
+cudaError_t launch_fwd_tile(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,
+                            const FwdStep& r, int sms, cudaStream_t st);
+
+// One backward step likewise: y are the stages' states; row[0] (exact mode:
+// row[0 .. 2], as AdjRun's groups) the step's row of partial sums.  segs: per
+// row segment of the lattice, whether it holds a source cell.
+struct AdjStep {
+    const double* zin;
+    double* zout;
+    const double* y[4];
+    double* row[3];
+    int nsbx;
+    unsigned* fault;
+};
+cudaError_t launch_adj_tile(bool exact, const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* adj,
+                            const uint8_t* segs, const AdjStep& r, int sms, cudaStream_t st);
+
 // Midpoint states of n backward steps (reference mode), step k's to yh + k *
 // stride; y_hi, y_mid, y_lo as in AdjRun.  Et, E3: the samples at the later end
 // of step 0 and of step 0's third; step k takes Et[-k], Et[-k - 1], E3[-k].

@@ -13,7 +13,7 @@ from test_gpu_edges import _custom
 pytestmark = pytest.mark.gpu
 
 SIZES = [(5, 7), (16, 16), (17, 33), (48, 64), (64, 200), (128, 128), (131, 97), (300, 40), (40, 610), (203, 331),
-         (256, 256), (437, 501), (512, 512), (640, 400), (29 * 18, 64 * 8)]
+         (256, 256), (437, 501), (512, 512), (640, 400), (29 * 18, 64 * 8), (600, 700), (1031, 521)]
 
 
 def _both(monkeypatch, call):
