@@ -590,7 +590,10 @@ fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, 
     CK(segf_.alloc(seg.size()), "alloc segment flags");
     CK(cudaMemcpyAsync(segf_.p, seg.data(), seg.size(), cudaMemcpyHostToDevice, st_), "upload segment flags");
     if (shape.id >= 0) {
-        CK(xchg_.alloc(run_exchange_bytes(g_)), "alloc edge exchange");
+        if (xchg_.alloc(run_exchange_bytes(g_)) != cudaSuccess) {
+            cudaGetLastError();  // no memory for it: the preset kernels
+            return FKADJ_OK;
+        }
         CK(cudaMemsetAsync(xchg_.p, 0, xchg_.bytes, st_), "clear edge exchange");
     }
     run_ = shape;
@@ -599,26 +602,30 @@ fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, 
 }
 
 int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t nnz, int grad_mode, int policy,
-                                bool want_grad) {
+                                bool want_grad, bool sweeps) {
     const int64_t ld = round_up(round_up(ncols, 64) + 2 * HALO, 8);
     const int64_t rows = round_up(nrows, 64) + 2 * HALO;
     const int64_t plane = rows * ld * 8, state = 3 * plane;
-    // geometry (and the sweeps' flags), compact, work, the sweeps' exchange
-    int64_t b = plane + 3 * (plane / 8) + (int64_t)n_num * (8 + 48) + nnz * 12 + 8 * state;
+    const bool exact = grad_mode == FKADJ_GRAD_EXACT;
+    int64_t b = plane + plane / 8 + (int64_t)n_num * (8 + 48) + nnz * 12 + 4 * state;  // geometry, compact, work
+    if (sweeps) b += 3 * (plane / 8) + 4 * state;                                      // flags, edge exchange
     if (!want_grad) return b;
+    const int64_t c = std::max(2, (int)std::ceil(std::sqrt((double)nt)));
     const int64_t nsb = (round_up(ncols, 64) / 16) * (round_up(nrows, 64) / 16);
-    // adjoint pair, partials (all rows of 16x16 ones, or the least window of row segments)
-    b += 2 * state + std::max<int64_t>((int64_t)(3 * nt + 1) * (nsb + 1),
-                                       (grad_mode == FKADJ_GRAD_EXACT ? 3 : 1) * std::min<int64_t>(nt + 1, std::max(32, (int)std::ceil(std::sqrt((double)nt)))) * 16 * nsb) * 8;
-    // stage states of a chunk | midpoint states of a chunk (more than yh and the caches)
-    const bool ex = grad_mode == FKADJ_GRAD_EXACT;
-    b += (int64_t)std::min(nt, sweep_chunk_of(state, ex)) * (ex ? 3 : 1) * state;
+    int64_t partials = (int64_t)(3 * nt + 1) * (nsb + 1);
+    if (sweeps) partials = std::max(partials, (exact ? 3 : 1) * std::min<int64_t>(nt + 1, std::max<int64_t>(32, c)) * 16 * nsb);
+    b += 2 * state + partials * 8;  // adjoint pair, partials
+    if (sweeps)
+        b += (int64_t)std::min(nt, sweep_chunk_of(state, exact)) * (exact ? 3 : 1) * state;  // a chunk's points
+    else
+        b += exact ? 3 * state : state + 27 * plane;  // stages | yh + caches
     if (policy == FKADJ_CKPT_FULL) {
         b += (int64_t)(nt + 1) * state;
+        if (sweeps && exact) b += 3 * (int64_t)nt * state;  // kept stage states
     } else {
-        const int64_t c = std::max(2, (int)std::ceil(std::sqrt((double)nt)));
         b += ((nt + c - 1) / c + 1 + c - 1) * state;
-        b += grad_mode == FKADJ_GRAD_REF ? (c - 1) * state : 3 * c * state;  // kept by the segment recompute
+        if (!exact) b += sweeps ? 0 : (c - 1) * state;  // k1 kept by the segment recompute
+        else if (sweeps) b += 3 * c * state;
     }
     return b;
 }

@@ -102,8 +102,9 @@ public:
     // Device bytes a problem of this size will hold once a job has run
     // (geometry, work states, adjoint work, Jacobian caches, trajectory store
     // under `policy`), for admission control before anything is allocated.
+    // with `sweeps`, what a problem whose steps are sweeps holds (fk_run.h).
     static int64_t estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t nnz, int grad_mode,
-                                  int policy, bool want_grad);
+                                  int policy, bool want_grad, bool sweeps = false);
     Timing last_timing() const { return timing_; }
     // trajectory plan of the last gradient (policy FULL/SQRT/BINOMIAL, 0 = none yet)
     const TrajPlan& last_plan() const { return traj_plan_; }
@@ -131,6 +132,8 @@ public:
         pool_ = pool;
         own_sweeps_ = false;
     }
+    // The preset kernels, which need less device memory (call before init).
+    void no_sweeps() { own_sweeps_ = false; }
     // A problem of a one-shot entry point (call before init): device memory
     // from `pool` (null: cudaMalloc), pinned staging from the process's cache.
     void set_oneshot(cudaMemPool_t pool) {
@@ -300,7 +303,7 @@ private:
     // (FAULT_NAN), which they contain
     bool run_off_ = false;
     bool nan_seen_ = false;
-    bool own_sweeps_ = true;  // false for a batch engine's problems, which run batched launches
+    bool own_sweeps_ = true;  // false for a batch engine's problems, and where memory is short
     DevBuf work_;      // 4 states: two ping-pong, z pair is separate
     DevBuf zbuf_;      // 2 adjoint states
     DevBuf yh_;        // midpoint state
@@ -363,6 +366,12 @@ template <class Call>
 fkadj_status Problem::with_sweeps(Call&& call) {
     nan_seen_ = false;
     fkadj_status s = call();
+    if (s == FKADJ_ERR_NOMEM && sweeping()) {
+        // the preset kernels need less memory
+        for (DevBuf* b : {&xchg_, &pts_}) b->release();
+        swept_ = false;
+        return call();
+    }
     if (!nan_seen_) return s;
     run_off_ = true;
     s = call();

@@ -46,6 +46,8 @@ struct Request {
     std::vector<int64_t> Jc, Ir;
     bool want_grad = true;
     int64_t est = 0;
+    int64_t est_sweeps = 0;  // the same with sweeps
+    bool sweeps = false;     // how it was admitted
     // results
     int state = 0;  // 0 queued, 1 running, 2 done, 3 failed
     fkadj_status status = FKADJ_OK;
@@ -138,6 +140,7 @@ void Server::stop() {
 fkadj_status Server::run_alone(Request& r) {
     auto pb = std::make_unique<Problem>();
     pb->set_oneshot(oneshot_pool(&opt_));
+    if (!r.sweeps) pb->no_sweeps();
     fkadj_options o = opt_;
     o.stream = nullptr;
     o.device = device_;
@@ -177,6 +180,9 @@ void Server::worker() {
             r = reqs_[id].get();
             r->state = 1;
             r->t_admit = host_seconds();
+            // sweeps take more memory than the preset kernels: where it is there
+            r->sweeps = used_ + r->est_sweeps <= budget_;
+            if (r->sweeps) r->est = r->est_sweeps;
             used_ += r->est;
             running_.push_back(id);
             peak_running_ = std::max<int64_t>(peak_running_, (int64_t)running_.size());
@@ -206,6 +212,10 @@ fkadj_status Server::submit(std::unique_ptr<Request> r, int64_t* id) {
     r->est = Problem::estimate_bytes(r->nrows, r->ncols, r->nt, r->n_num, (int64_t)r->Sv.size(), opt_.grad_mode,
                                      opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT,
                                      r->want_grad);
+    r->est_sweeps = Problem::estimate_bytes(r->nrows, r->ncols, r->nt, r->n_num, (int64_t)r->Sv.size(),
+                                            opt_.grad_mode,
+                                            opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT,
+                                            r->want_grad, true);
     if (r->est > budget_) {
         set_error("request does not fit the HBM budget even alone");
         return FKADJ_ERR_NOMEM;
