@@ -99,7 +99,10 @@ static bool g_init_done[64];
 static std::mutex g_oneshot_mu;
 static cudaMemPool_t g_oneshot_pool[64] = {};
 static std::vector<std::pair<size_t, double*>> g_pinned_free;  // (doubles, buffer)
-constexpr size_t kPinnedKeep = 8;
+// a call takes four; several threads' calls (the server's) at once.  Freeing a
+// buffer and pinning it again cost a call 10 to 60 ms where too few were kept
+constexpr size_t kPinnedKeep = 32, kPinnedKeepTotal = (size_t)64 << 20;  // buffers, doubles
+constexpr size_t kPinnedSetup = (size_t)4 << 20;  // doubles: the largest set-up or frame kept in pinned memory
 
 cudaMemPool_t oneshot_pool(const fkadj_options* opt) {
     const char* v = getenv("FKADJ_ONESHOT_POOL");
@@ -141,15 +144,51 @@ static cudaError_t take_pinned(size_t n, double** p, size_t* cap) {
             return cudaSuccess;
         }
     }
-    *cap = n;
-    return cudaMallocHost(p, n * sizeof(double));
+    // whole powers of two: calls of about the same size share their buffers
+    size_t c = (size_t)1 << 14;
+    while (c < n) c *= 2;
+    *cap = c;
+    return cudaMallocHost(p, c * sizeof(double));
+}
+
+// Streams (with a problem's three events) of one-shot calls, kept for the next
+// call on the device: creating and destroying them took 0.15 ms of the
+// smallest call's 0.5.  A stream is given back synchronised.
+struct KeptStream {
+    int device;
+    cudaStream_t st;
+    cudaEvent_t ev[3];
+};
+static std::vector<KeptStream> g_streams_free;
+constexpr size_t kStreamsKeep = 8;
+
+static bool take_stream(int device, cudaStream_t* st, cudaEvent_t* ev) {
+    std::lock_guard<std::mutex> lk(g_oneshot_mu);
+    for (size_t i = 0; i < g_streams_free.size(); ++i)
+        if (g_streams_free[i].device == device) {
+            *st = g_streams_free[i].st;
+            std::copy(g_streams_free[i].ev, g_streams_free[i].ev + 3, ev);
+            g_streams_free.erase(g_streams_free.begin() + i);
+            return true;
+        }
+    return false;
+}
+
+static bool give_stream(int device, cudaStream_t st, cudaEvent_t* ev) {
+    if (!ev[0] || !ev[1] || !ev[2] || cudaStreamSynchronize(st) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lk(g_oneshot_mu);
+    if (g_streams_free.size() >= kStreamsKeep) return false;
+    g_streams_free.push_back({device, st, {ev[0], ev[1], ev[2]}});
+    return true;
 }
 
 static void give_pinned(double* p, size_t cap) {
     if (!p) return;
     {
         std::lock_guard<std::mutex> lk(g_oneshot_mu);
-        if (g_pinned_free.size() < kPinnedKeep) {
+        size_t kept = cap;
+        for (auto& b : g_pinned_free) kept += b.first;
+        if (g_pinned_free.size() < kPinnedKeep && kept <= kPinnedKeepTotal) {
             g_pinned_free.emplace_back(cap, p);
             return;
         }
@@ -172,6 +211,11 @@ fkadj_status release_oneshot_memory() {
     cudaSetDevice(cur);
     for (auto& b : g_pinned_free) cudaFreeHost(b.second);
     g_pinned_free.clear();
+    for (auto& k : g_streams_free) {
+        for (auto& ev : k.ev) cudaEventDestroy(ev);
+        cudaStreamDestroy(k.st);
+    }
+    g_streams_free.clear();
     if (e) {
         set_error(std::string("release cached memory: ") + cudaGetErrorString(e));
         return FKADJ_ERR_CUDA;
@@ -187,21 +231,21 @@ Problem::~Problem() {
         // below): release the buffers first
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
         for (DevBuf* b : all) b->release();
     }
     for (auto& r : prof_pool_) {
         cudaEventDestroy(r.a);
         cudaEventDestroy(r.b);
     }
-    for (auto& e : ev_)
-        if (e) cudaEventDestroy(e);
     drop_graph();
     const auto t1 = clk::now();
+    // a failed call may leave copies to or from the staging in flight: let
+    // them finish before another call takes the buffers
+    if (st_ && (setup_ || (oneshot_ && (Ehost_ || hres_ || frame_)))) cudaStreamSynchronize(st_);
+    give_pinned(setup_, setup_n_);
+    give_pinned(frame_, frame_n_);
     if (oneshot_) {
-        // a failed call may leave copies to or from the staging in flight: let
-        // them finish before another call takes the buffers
-        if (st_ && (Ehost_ || hres_)) cudaStreamSynchronize(st_);
         give_pinned(Ehost_, Ehost_n_);
         give_pinned(hres_, hres_n_);
     } else {
@@ -209,13 +253,19 @@ Problem::~Problem() {
         if (hres_) cudaFreeHost(hres_);
     }
     const auto t2 = clk::now();
+    if (own_stream_ && st_ && oneshot_ && pool_ && give_stream(device_, st_, ev_)) {
+        st_ = nullptr;
+        for (auto& e : ev_) e = nullptr;
+    }
+    for (auto& e : ev_)
+        if (e) cudaEventDestroy(e);
     if (own_stream_ && st_) cudaStreamDestroy(st_);
     delete spline_;
     const auto t3 = clk::now();
     if (verbose_ > 1) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
         size_t bytes = 0;
         for (DevBuf* b : all) bytes += b->bytes;
         for (DevBuf* b : all) b->release();
@@ -387,15 +437,18 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     }
     if (o.stream) {
         st_ = static_cast<cudaStream_t>(o.stream);
+    } else if (oneshot_ && take_stream(device_, &st_, ev_)) {
+        own_stream_ = true;
     } else {
         CK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking), "cudaStreamCreate");
         own_stream_ = true;
     }
-    for (auto& e : ev_) CK(cudaEventCreate(&e), "cudaEventCreate");
+    for (auto& e : ev_)
+        if (!e) CK(cudaEventCreate(&e), "cudaEventCreate");
     if (pool_) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_};
+                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
         for (DevBuf* b : all) b->st = st_, b->pool = pool_;
     }
     {
@@ -404,15 +457,10 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
         graphs_ = st_ != nullptr && st_ != cudaStreamLegacy && st_ != cudaStreamPerThread &&
                   !(ng && ng[0] && ng[0] != '0');
     }
-    size_t fr = 0, tot = 0;
-    CK(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
-    if (pool_) {  // memory the pool holds but no buffer uses is free for this problem too
-        uint64_t reserved = 0, used = 0;
-        if (cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-            cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
-            fr += (size_t)(reserved - used);
+    ckpt_budget_ = o.ckpt_budget_bytes;
+    if (ckpt_budget_ <= 0 && !oneshot_) {  // (asking for the free memory costs 0.1 ms: not in forward calls)
+        if (fkadj_status s = default_budget()) return s;
     }
-    ckpt_budget_ = o.ckpt_budget_bytes > 0 ? o.ckpt_budget_bytes : (int64_t)(0.6 * (double)fr);
 
     g_.nrows = nrows;
     g_.ncols = ncols;
@@ -469,44 +517,102 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
         }
         if (k == 4) autotune_ = false, tuned_ = true, tiles_fixed_ = true;
     }
+    CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "device attribute");
     subblock_lattice(g_, &nsbx_, &nsby_);
     nsb_ = nsbx_ * nsby_;
 
-    // geometry on the padded grid: gh, adjoint stencil weights, compact positions
+    // geometry on the padded grid: gh, adjoint stencil weights, compact
+    // positions, the sweeps' flags; and S as CSR (row sums in ascending column
+    // order).  All of it is made in one pinned block, which the copies to the
+    // device take as it is (small enough ones: pinning a large block costs
+    // more than staging pageable memory).
     const size_t pl = (size_t)g_.plane;
-    std::vector<double> gh(pl, std::nan(""));
-    std::vector<uint8_t> wc(pl, 0);
-    std::vector<long long> pos(n_num);
-    auto act = [&](int i, int j) { return i >= 0 && i < nrows && j >= 0 && j < ncols && ai[i * ncols + j] > 0; };
-    auto weight = [&](int i, int j, int di, int dj) {
-        if (!act(i + di, j + dj)) return 0;
-        return act(i + 2 * di, j + 2 * dj) ? 1 : 2;
-    };
-    const double ghs = p.Du * 2 / p.h;
-    for (int i = 0; i < nrows; ++i)
-        for (int j = 0; j < ncols; ++j) {
-            const int a = ai[i * ncols + j];
-            if (a <= 0) continue;
-            const size_t o2 = (size_t)(i + HALO) * g_.ld + (j + HALO);
-            gh[o2] = ghs * gh_num[a - 1];
-            wc[o2] = (uint8_t)(weight(i, j, -1, 0) | weight(i, j, 1, 0) << 2 | weight(i, j, 0, -1) << 4 |
-                               weight(i, j, 0, 1) << 6);
-            pos[a - 1] = (long long)o2;
+    const int64_t nnz = need_objective ? S_colptr[n_num] : 0;
+    const size_t nseg = (size_t)nsbx_ * nrows;
+    auto words = [](size_t bytes) { return (bytes + 7) / 8; };
+    const size_t need = pl + 3 * words(pl) + words(nseg) + (size_t)n_num + 2 * ((size_t)n_num + 1) +
+                        words((size_t)nnz * sizeof(int)) + (size_t)nnz;
+    std::unique_ptr<double[]> pageable;
+    double* block = nullptr;
+    // (the end of its use is this problem's to wait for: not on a stream that
+    // others queue work on)
+    if (need <= kPinnedSetup && own_stream_) {
+        CK(take_pinned(need, &setup_, &setup_n_), "alloc pinned set-up");
+        block = setup_;
+    } else {
+        pageable.reset(new (std::nothrow) double[need]);
+        block = pageable.get();
+        if (!block) {
+            set_error("host allocation failed");
+            return FKADJ_ERR_NOMEM;
         }
-    if (fkadj_status s = init_sweeps(ai, gh, wc)) return s;
+    }
+    auto carve = [&block](size_t n) {
+        double* p = block;
+        block += n;
+        return p;
+    };
+    double* gh = carve(pl);
+    uint8_t* wc = reinterpret_cast<uint8_t*>(carve(words(pl)));
+    uint8_t* cells = reinterpret_cast<uint8_t*>(carve(words(pl)));
+    uint8_t* adj = reinterpret_cast<uint8_t*>(carve(words(pl)));
+    uint8_t* seg = reinterpret_cast<uint8_t*>(carve(words(nseg)));
+    long long* pos = reinterpret_cast<long long*>(carve(n_num));
+    bool pinched = false;  // an active cell between two opposite holes
+    {
+        std::fill(gh, gh + pl, std::nan(""));
+        std::memset(wc, 0, pl);
+        std::memset(cells, 0, pl);
+        std::memset(adj, 0, pl);
+        std::memset(seg, 0, nseg);
+        const double ghs = p.Du * 2 / p.h;
+        // the mask with two cells of nothing around it
+        const int mw = ncols + 4;
+        std::vector<uint8_t> mask((size_t)(nrows + 4) * mw, 0);
+        for (int i = 0; i < nrows; ++i) {
+            uint8_t* m = mask.data() + (size_t)(i + 2) * mw + 2;
+            for (int j = 0; j < ncols; ++j) m[j] = ai[i * ncols + j] > 0;
+        }
+        for (int i = 0; i < nrows; ++i) {
+            const uint8_t* m = mask.data() + (size_t)(i + 2) * mw + 2;
+            for (int j = 0; j < ncols; ++j, ++m) {
+                if (!*m) continue;
+                const int a = ai[i * ncols + j];
+                const size_t o = (size_t)(i + HALO) * g_.ld + (j + HALO);
+                const unsigned n = m[-mw], s = m[mw], w = m[-1], e = m[1];
+                // transposed weights: 1, or 2 where the neighbour mirrors this cell
+                const unsigned n2 = n & !m[-2 * mw], s2 = s & !m[2 * mw], w2 = w & !m[-2], e2 = e & !m[2];
+                gh[o] = ghs * gh_num[a - 1];
+                const unsigned src = gh[o] != 0.0;
+                wc[o] = (uint8_t)((n + n2) | (s + s2) << 2 | (w + w2) << 4 | (e + e2) << 6);
+                cells[o] = (uint8_t)(CELL_ACTIVE | (n ? 0 : CELL_N) | (s ? 0 : CELL_S) | (w ? 0 : CELL_W) |
+                                     (e ? 0 : CELL_E) | (src ? CELL_SOURCE : 0));
+                adj[o] = (uint8_t)(CELL_ACTIVE_ADJ | (n2 ? CELL_2N : 0) | (s2 ? CELL_2S : 0) | (w2 ? CELL_2W : 0) |
+                                   (e2 ? CELL_2E : 0) | (src ? CELL_SOURCE : 0));
+                if (src) seg[(size_t)i * nsbx_ + j / 16] = 1;
+                pinched = pinched || !(n | s) || !(w | e);
+                pos[a - 1] = (long long)o;
+            }
+        }
+    }
     CK(gh_.alloc(pl * sizeof(double)), "alloc gh");
     CK(wc_.alloc(pl), "alloc weights");
     CK(pos_.alloc((size_t)n_num * sizeof(long long)), "alloc positions");
     // stream-ordered copies (from pageable memory they return once the data is staged)
-    CK(cudaMemcpyAsync(gh_.p, gh.data(), pl * sizeof(double), cudaMemcpyHostToDevice, st_), "upload gh");
-    CK(cudaMemcpyAsync(wc_.p, wc.data(), pl, cudaMemcpyHostToDevice, st_), "upload weights");
-    CK(cudaMemcpyAsync(pos_.p, pos.data(), (size_t)n_num * sizeof(long long), cudaMemcpyHostToDevice, st_),
+    CK(cudaMemcpyAsync(gh_.p, gh, pl * sizeof(double), cudaMemcpyHostToDevice, st_), "upload gh");
+    CK(cudaMemcpyAsync(wc_.p, wc, pl, cudaMemcpyHostToDevice, st_), "upload weights");
+    CK(cudaMemcpyAsync(pos_.p, pos, (size_t)n_num * sizeof(long long), cudaMemcpyHostToDevice, st_),
        "upload positions");
+    if (!pinched) {
+        if (fkadj_status s = init_sweeps(cells, adj, seg)) return s;
+    }
 
     if (need_objective) {
-        // CSC (columns) -> CSR (rows) so that row sums run in ascending column order
-        const int64_t nnz = S_colptr[n_num];
-        std::vector<long long> rp(n_num + 1, 0);
+        long long* rp = reinterpret_cast<long long*>(carve(n_num + 1));
+        long long* fill = reinterpret_cast<long long*>(carve(n_num + 1));
+        double* cv = carve((size_t)nnz);
+        int* ci = reinterpret_cast<int*>(block);
+        std::fill(rp, rp + n_num + 1, 0);
         for (int64_t k = 0; k < nnz; ++k) {
             const int64_t r = S_rowidx[k];
             if (r < 0 || r >= n_num) {
@@ -516,9 +622,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
             rp[r + 1]++;
         }
         for (int r = 0; r < n_num; ++r) rp[r + 1] += rp[r];
-        std::vector<int> ci(nnz);
-        std::vector<double> cv(nnz);
-        std::vector<long long> fill(rp.begin(), rp.end() - 1);
+        std::copy(rp, rp + n_num, fill);
         for (int c = 0; c < n_num; ++c)
             for (int64_t k = S_colptr[c]; k < S_colptr[c + 1]; ++k) {
                 const long long d = fill[S_rowidx[k]]++;
@@ -528,11 +632,10 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
         CK(Srow_.alloc((n_num + 1) * sizeof(long long)), "alloc S");
         CK(Scol_.alloc(std::max<int64_t>(nnz, 1) * sizeof(int)), "alloc S");
         CK(Sval_.alloc(std::max<int64_t>(nnz, 1) * sizeof(double)), "alloc S");
-        CK(cudaMemcpyAsync(Srow_.p, rp.data(), (n_num + 1) * sizeof(long long), cudaMemcpyHostToDevice, st_),
-           "upload S");
+        CK(cudaMemcpyAsync(Srow_.p, rp, (n_num + 1) * sizeof(long long), cudaMemcpyHostToDevice, st_), "upload S");
         if (nnz) {
-            CK(cudaMemcpyAsync(Scol_.p, ci.data(), nnz * sizeof(int), cudaMemcpyHostToDevice, st_), "upload S");
-            CK(cudaMemcpyAsync(Sval_.p, cv.data(), nnz * sizeof(double), cudaMemcpyHostToDevice, st_), "upload S");
+            CK(cudaMemcpyAsync(Scol_.p, ci, nnz * sizeof(int), cudaMemcpyHostToDevice, st_), "upload S");
+            CK(cudaMemcpyAsync(Sval_.p, cv, nnz * sizeof(double), cudaMemcpyHostToDevice, st_), "upload S");
         }
         have_obj_ = true;
     }
@@ -545,50 +648,34 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     CK(work_.alloc(3 * state_bytes()), "alloc states");
     CK(cudaMemsetAsync(work_.p, 0xff, work_.bytes, st_), "init states");
     spline_ = new NakSpline(nt + 1, dt);
+    if (setup_ && !oneshot_) {
+        CK(cudaStreamSynchronize(st_), "synchronize");  // its copies are done
+        give_pinned(setup_, setup_n_);
+        setup_ = nullptr;
+    }
     return FKADJ_OK;
 }
 
 // Whether and how this problem's sweeps run (fk_run.h): with autotuned tiles,
 // where every active cell keeps a neighbour in both directions; one launch per
 // sweep where the grid's tiles fit the device at once, the tile kernels
-// otherwise.  ai: the active index of every cell; gh: the padded source plane;
-// wc: the transposed stencil's weight codes.  FKADJ_SWEEPS=0 in the
-// environment keeps the preset kernels.
-fkadj_status Problem::init_sweeps(const int* ai, const std::vector<double>& gh, const std::vector<uint8_t>& wc) {
-    run_ = RunShape();
-    swept_ = false;
-    CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "device attribute");
+// otherwise.  cells, adj, seg: the sweeps' flags (host).  FKADJ_SWEEPS=0 in
+// the environment keeps the preset kernels.
+fkadj_status Problem::init_sweeps(const uint8_t* cells, const uint8_t* adj, const uint8_t* seg) {
     const char* v = getenv("FKADJ_SWEEPS");
-    if (!autotune_ || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ ||
-        (v && v[0] == '0')) return FKADJ_OK;
+    if (!autotune_ || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ || (v && v[0] == '0')) return FKADJ_OK;
     const char* sv = getenv("FKADJ_ZGH_SEGMENTS");  // the adjoint sweeps write row segments
     if (sv && std::atoi(sv) == 0) return FKADJ_OK;
     int coop = 0;
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_), "device attribute");
     const RunShape shape = coop ? run_shape(g_, sms_) : RunShape();
-    const int ld = g_.ld;
-    std::vector<uint8_t> cells((size_t)g_.plane, 0), adj((size_t)g_.plane, 0), seg((size_t)nsbx_ * g_.nrows, 0);
-    for (int i = 0; i < g_.nrows; ++i)
-        for (int j = 0; j < g_.ncols; ++j) {
-            const int k = i * g_.ncols + j;
-            if (ai[k] <= 0) continue;
-            const size_t o = (size_t)(i + HALO) * ld + (j + HALO);
-            const bool n = i == 0 || ai[k - g_.ncols] <= 0, s = i == g_.nrows - 1 || ai[k + g_.ncols] <= 0;
-            const bool w = j == 0 || ai[k - 1] <= 0, e = j == g_.ncols - 1 || ai[k + 1] <= 0;
-            if ((n && s) || (w && e)) return FKADJ_OK;
-            cells[o] = (uint8_t)(CELL_ACTIVE | (n ? CELL_N : 0) | (s ? CELL_S : 0) | (w ? CELL_W : 0) |
-                                 (e ? CELL_E : 0) | (gh[o] != 0.0 ? CELL_SOURCE : 0));
-            const int c = wc[o];
-            if (gh[o] != 0.0) seg[(size_t)i * nsbx_ + j / 16] = 1;
-            adj[o] = (uint8_t)(CELL_ACTIVE_ADJ | (cells[o] & CELL_SOURCE) | ((c & 3) == 2 ? CELL_2N : 0) | ((c >> 2 & 3) == 2 ? CELL_2S : 0) |
-                               ((c >> 4 & 3) == 2 ? CELL_2W : 0) | ((c >> 6 & 3) == 2 ? CELL_2E : 0));
-        }
-    CK(cells_.alloc(cells.size()), "alloc cell flags");
-    CK(cudaMemcpyAsync(cells_.p, cells.data(), cells.size(), cudaMemcpyHostToDevice, st_), "upload cell flags");
-    CK(adjf_.alloc(adj.size()), "alloc cell flags");
-    CK(cudaMemcpyAsync(adjf_.p, adj.data(), adj.size(), cudaMemcpyHostToDevice, st_), "upload cell flags");
-    CK(segf_.alloc(seg.size()), "alloc segment flags");
-    CK(cudaMemcpyAsync(segf_.p, seg.data(), seg.size(), cudaMemcpyHostToDevice, st_), "upload segment flags");
+    const size_t pl = (size_t)g_.plane, nseg = (size_t)nsbx_ * g_.nrows;
+    CK(cells_.alloc(pl), "alloc cell flags");
+    CK(cudaMemcpyAsync(cells_.p, cells, pl, cudaMemcpyHostToDevice, st_), "upload cell flags");
+    CK(adjf_.alloc(pl), "alloc cell flags");
+    CK(cudaMemcpyAsync(adjf_.p, adj, pl, cudaMemcpyHostToDevice, st_), "upload cell flags");
+    CK(segf_.alloc(nseg), "alloc segment flags");
+    CK(cudaMemcpyAsync(segf_.p, seg, nseg, cudaMemcpyHostToDevice, st_), "upload segment flags");
     if (shape.id >= 0) {
         if (xchg_.alloc(run_exchange_bytes(g_)) != cudaSuccess) {
             cudaGetLastError();  // no memory for it: the preset kernels
@@ -633,7 +720,7 @@ int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t
 int64_t Problem::device_bytes() const {
     const DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_,
                            &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_, &fcache_,
-                           &cells_, &adjf_, &segf_, &xchg_, &pts_};
+                           &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
     int64_t s = 0;
     for (auto* b : all) s += (int64_t)b->bytes;
     return s;
@@ -897,7 +984,21 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
     return FKADJ_OK;
 }
 
+// The state as dense planes in host memory: packed by a kernel, copied through
+// a pinned buffer (three strided copies into pageable memory took 0.15 ms for
+// a 48 x 64 grid, row by row); synchronises.
 fkadj_status Problem::download_grid(const double* d_state, double* host) {
+    const size_t n3 = (size_t)3 * g_.nrows * g_.ncols;
+    if (n3 <= kPinnedSetup && g_.nrows <= 65535) {
+        if (!frame_) CK(take_pinned(n3, &frame_, &frame_n_), "alloc pinned frame");
+        if (dense_.bytes < n3 * sizeof(double)) CK(dense_.alloc(n3 * sizeof(double)), "alloc dense state");
+        CK(launch_pack(g_, d_state, dense_.as<double>(), st_), "pack state");
+        ++launches_;
+        CK(cudaMemcpyAsync(frame_, dense_.p, n3 * sizeof(double), cudaMemcpyDeviceToHost, st_), "download state");
+        CK(cudaStreamSynchronize(st_), "synchronize");
+        std::memcpy(host, frame_, n3 * sizeof(double));
+        return FKADJ_OK;
+    }
     const size_t n = (size_t)g_.nrows * g_.ncols;
     for (int f = 0; f < 3; ++f) {
         const double* src = d_state + (size_t)f * g_.plane + (size_t)HALO * g_.ld + HALO;
@@ -1018,7 +1119,24 @@ fkadj_status Problem::objective_call(const double* Et, const double* y_ini, doub
     return FKADJ_OK;
 }
 
+// 60 % of the free device memory
+fkadj_status Problem::default_budget() {
+    size_t fr = 0, tot = 0;
+    CK(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
+    if (pool_) {  // memory the pool holds but no buffer uses is free for this problem too
+        uint64_t reserved = 0, used = 0;
+        if (cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+            fr += (size_t)(reserved - used);
+    }
+    ckpt_budget_ = (int64_t)(0.6 * (double)fr);
+    return FKADJ_OK;
+}
+
 fkadj_status Problem::plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only) {
+    if (ckpt_budget_ <= 0) {  // a one-shot call's: init leaves it to the gradient
+        if (fkadj_status s = default_budget()) return s;
+    }
     const double sb = (double)state_bytes();
     const int c = std::max(2, (int)std::ceil(std::sqrt((double)nt_)));
     const int sqrt_slots = (nt_ + c - 1) / c + 1 + (c - 1);

@@ -176,7 +176,7 @@ public:
     // states of steps lo .. hi - 1 in a row.
     fkadj_status sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
                                const double* stages, double*& z, double*& z2);
-    fkadj_status init_sweeps(const int* ai, const std::vector<double>& gh, const std::vector<uint8_t>& wc);
+    fkadj_status init_sweeps(const uint8_t* cells, const uint8_t* adj, const uint8_t* seg);
     // whether this problem's steps are sweeps (fk_run.h): one launch each where
     // run_.id >= 0, the tile kernels otherwise
     bool sweeping() const { return swept_ && !run_off_; }
@@ -201,6 +201,7 @@ private:
     // forward step, included); with
     // sqrt_or_full_only (the batch engine, which runs no binomial schedule)
     // BINOMIAL only when SQRT does not fit.
+    fkadj_status default_budget();
     fkadj_status plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only = false);
     int64_t kept_states(const TrajPlan& tp) const;
     fkadj_status ensure_traj(const TrajPlan& tp);
@@ -320,6 +321,11 @@ private:
     double* hres_ = nullptr;   // pinned results: L0 partial sum, then the z.gh rows
     size_t hres_n_ = 0;
     size_t Ehost_n_ = 0;       // capacity of Ehost_ (doubles)
+    double* setup_ = nullptr;  // pinned block of the set-up's uploads
+    size_t setup_n_ = 0;
+    double* frame_ = nullptr;  // pinned staging of a downloaded state
+    size_t frame_n_ = 0;
+    DevBuf dense_;             // a state packed for download
     bool oneshot_ = false;
     bool have_y0_ = false;
 

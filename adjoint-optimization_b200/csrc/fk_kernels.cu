@@ -1351,6 +1351,14 @@ __global__ void k_gather(DevGrid g, const double* __restrict__ y, int n_num,
     yc[2 * n_num + m] = y[2 * g.plane + o];
 }
 
+// Padded grid -> dense planes (NaN at holes).
+__global__ void k_pack(DevGrid g, const double* __restrict__ y, double* __restrict__ out) {
+    const int i = blockIdx.y, f = blockIdx.z;
+    const double* src = y + f * g.plane + (long long)(i + HALO) * g.ld + HALO;
+    double* dst = out + ((long long)f * g.nrows + i) * g.ncols;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < g.ncols; j += gridDim.x * blockDim.x) dst[j] = src[j];
+}
+
 // Objective at T: for each field f, zc_f = -gamma_f * (S y_f) with S in CSR
 // (row sums in ascending column order, the order of the reference's CSC
 // accumulation, cu-G:1514-1522); per-block partials of y_f . zc_f.
@@ -1775,6 +1783,13 @@ cudaError_t launch_scatter(const DevGrid& g, const double* yc, int n_num, const 
 cudaError_t launch_gather(const DevGrid& g, const double* y, int n_num, const long long* pos, double* yc,
                           cudaStream_t st) {
     k_gather<<<(n_num + 255) / 256, 256, 0, st>>>(g, y, n_num, pos, yc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pack(const DevGrid& g, const double* y, double* out, cudaStream_t st) {
+    // rows past the grid limit of 65535 go by the strided copies instead
+    if (g.nrows > 65535) return cudaErrorInvalidValue;
+    k_pack<<<dim3((g.ncols + 255) / 256, g.nrows, 3), 256, 0, st>>>(g, y, out);
     return cudaGetLastError();
 }
 

@@ -174,6 +174,8 @@ cudaError_t launch_scatter(const DevGrid& g, const double* yc, int n_num, const 
                            double* y, cudaStream_t st);
 cudaError_t launch_gather(const DevGrid& g, const double* y, int n_num, const long long* pos, double* yc,
                           cudaStream_t st);
+// Dense planes of a state, for download (at most 65535 rows)
+cudaError_t launch_pack(const DevGrid& g, const double* y, double* out, cudaStream_t st);
 int objective_blocks(int n_num);
 cudaError_t launch_objective(const double* yc, int n_num, const long long* rowptr, const int* colidx,
                              const double* val, const double gamma[3], double* zc, double* partial,
