@@ -116,7 +116,8 @@ fkadj_status BatchEngine::init(const fkadj_options* opt) {
 fkadj_status BatchEngine::add_problem(const fkadj_params& p, double dt, int nt, const int* ai, int nrows, int ncols,
                                       int n_num, const double* gh_num, const double* gamma, int64_t S_ncol,
                                       const int64_t* S_colptr, const int64_t* S_rowidx, const double* S_val,
-                                      double alpha, int grad_mode, int ckpt_policy, int64_t ckpt_budget, int* id) {
+                                      double alpha, int grad_mode, int ckpt_policy, int64_t ckpt_budget, int* id,
+                                      bool sweeps) {
     fkadj_options o = opt_;
     o.stream = st_;
     o.grad_mode = grad_mode;
@@ -124,7 +125,7 @@ fkadj_status BatchEngine::add_problem(const fkadj_params& p, double dt, int nt, 
     o.ckpt_budget_bytes = ckpt_budget;
     o.tile = tiles_[0] + 1;  // fixed preset: no per-problem autotune inside a batch
     auto pb = std::make_unique<Problem>();
-    pb->use_pool(pool_);
+    pb->use_pool(pool_, sweeps && !(opt_.tile > 0 && opt_.tile <= tile_count()));
     const bool need_obj = gamma && S_colptr;
     fkadj_status s = pb->init(p, dt, nt, ai, nrows, ncols, n_num, gh_num, gamma, S_ncol, S_colptr, S_rowidx,
                               S_val, alpha, &o, need_obj);
@@ -186,6 +187,39 @@ int64_t BatchEngine::device_bytes() const {
     return s;
 }
 
+// Stores, work buffers, initial state and plan of a job, from its first step.
+fkadj_status BatchEngine::prepare_job(Job& j, const double* y_ini) {
+    Problem& P = *probs_[j.prob];
+    fkadj_status s;
+    j.swept = P.sweeping();
+    j.cur_c = 0;
+    j.have_fcarry = j.have_jcarry = j.finishing = false;
+    if (j.want_grad) {
+        if ((s = P.plan_trajectory(j.tp, true))) return s;
+        if (j.tp.policy == FKADJ_CKPT_BINOMIAL) {
+            set_error("batched jobs store full or sqrt trajectories; the binomial schedule runs in the "
+                      "standalone engine (raise ckpt_budget_bytes or use fkadj_problem_grad)");
+            return FKADJ_ERR_NOMEM;
+        }
+        // k1 = f(y) kept by the segment recompute (sqrt store, reference mode),
+        // or the stage states (sweeps, exact mode); the full store evaluates
+        // them (keeping them there multiplies the store)
+        if (j.tp.policy != FKADJ_CKPT_SQRT) j.tp.keep_f = false;
+        if ((s = P.ensure_traj(j.tp))) return s;
+        if ((s = P.ensure_adjoint_work(!j.swept))) return s;  // the tick kernels' rows are all reduced at the end
+        if ((s = P.upload_state(y_ini, P.slot(0)))) return s;
+        j.cur = P.slot(0);
+        j.z = P.zbuf_.as<double>();
+        j.z2 = j.z + P.state_elems();
+    } else {
+        j.tp = TrajPlan{};
+        j.tp.policy = 0;
+        if ((s = P.upload_state(y_ini, P.state_buf(0)))) return s;
+        j.cur = P.state_buf(0);
+    }
+    return build_plan(j);
+}
+
 fkadj_status BatchEngine::build_plan(Job& j) {
     Problem& P = *probs_[j.prob];
     const int nt = P.nt_;
@@ -204,7 +238,9 @@ fkadj_status BatchEngine::build_plan(Job& j) {
         } else {
             for (int k = K - 1; k >= 0; --k) {
                 const int s0 = k * c, s1 = std::min(s0 + c, nt);
-                for (int t = s0; t < s1 - 1; ++t) j.plan.push_back({Action::RECOMP, t});
+                // where stage states are kept, those of the segment's last step too
+                const int e = j.swept && exact && j.tp.keep_f ? s1 : s1 - 1;
+                for (int t = s0; t < e; ++t) j.plan.push_back({Action::RECOMP, t});
                 if (exact)
                     for (int t = s1 - 1; t >= s0; --t) j.plan.push_back({Action::EXADJ, t});
                 else
@@ -245,30 +281,16 @@ fkadj_status BatchEngine::submit(int prob, const double* Et, const double* y_ini
     j->want_grad = want_grad;
     j->t_submit = host_seconds();
     fkadj_status s;
-    if ((s = P.prepare_E(Et, false))) return s;  // batched kernels take E by value
+    if ((s = P.prepare_E(Et, P.sweeping()))) return s;  // the tick kernels take E by value
     j->Et.assign(Et, Et + P.nt_ + 1);
-    if (want_grad) {
-        if ((s = P.plan_trajectory(j->tp, true))) return s;
-        if (j->tp.policy == FKADJ_CKPT_BINOMIAL) {
-            set_error("batched jobs store full or sqrt trajectories; the binomial schedule runs in the "
-                      "standalone engine (raise ckpt_budget_bytes or use fkadj_problem_grad)");
-            return FKADJ_ERR_NOMEM;
-        }
-        // k1 = f(y) kept by the segment recompute (sqrt store, reference mode);
-        // the full store evaluates it (keeping it there doubles the store)
-        if (j->tp.policy != FKADJ_CKPT_SQRT) j->tp.keep_f = false;
-        if ((s = P.ensure_traj(j->tp))) return s;
-        if ((s = P.ensure_adjoint_work(true))) return s;  // the batch reduces all rows at the end
-        if ((s = P.upload_state(y_ini, P.slot(0)))) return s;
-        j->cur = P.slot(0);
-        j->z = P.zbuf_.as<double>();
-        j->z2 = j->z + P.state_elems();
-    } else {
-        j->tp.policy = 0;
-        if ((s = P.upload_state(y_ini, P.state_buf(0)))) return s;
-        j->cur = P.state_buf(0);
+    s = prepare_job(*j, y_ini);
+    if (s == FKADJ_ERR_NOMEM && P.sweeping()) {  // the tick kernels need less memory
+        for (DevBuf* b : {&P.xchg_, &P.pts_, &P.kf_}) b->release();
+        P.traj_plan_ = TrajPlan();
+        P.swept_ = false;
+        s = prepare_job(*j, y_ini);
     }
-    if ((s = build_plan(*j))) return s;
+    if (s) return s;
     j->h_out = take_pinned((size_t)j->rows + 2, &j->h_cap);  // [0] L0 sum, [1..rows], fault word
     if (!j->h_out) {
         set_error("pinned results: out of host memory");
@@ -296,18 +318,25 @@ fkadj_status BatchEngine::host_action(Job& j, const Action& a) {
                 "scatter z");
             ++launches_;
             if (!exact) {
-                BCK(launch_dot_gh(P.g_, j.z, P.gh_.as<double>(), P.partial_.as<double>() + (size_t)P.nt_ * nsb,
-                                  P.nsbx_, P.nsby_, st_),
+                BCK(launch_dot_gh(P.g_, j.z, P.gh_.as<double>(),
+                                  j.swept ? P.prow(0, P.nt_) : P.partial_.as<double>() + (size_t)P.nt_ * nsb, P.nsbx_,
+                                  P.nsby_, st_, P.segs_),
                     "z.gh");
                 ++launches_;
+                if (j.swept && (j.tp.policy == FKADJ_CKPT_SQRT || P.nt_ % P.pwin_ == 0)) {
+                    BCK(P.flush_range(0, P.nt_, 1), "reduce z.gh");
+                    ++launches_;
+                }
             }
         }
         return FKADJ_OK;
     }
     // FINISH: reductions and results to pinned memory
     if (j.want_grad) {
-        BCK(launch_sum_rows(P.partial_.as<double>(), j.rows, P.nsb_, P.zgh_.as<double>(), st_), "reduce");
-        ++launches_;
+        if (!j.swept) {
+            BCK(launch_sum_rows(P.partial_.as<double>(), j.rows, P.nsb_, P.zgh_.as<double>(), st_), "reduce");
+            ++launches_;
+        }
         BCK(cudaMemcpyAsync(j.h_out + 1, P.zgh_.p, sizeof(double) * j.rows, cudaMemcpyDeviceToHost, st_),
             "download");
     }
@@ -494,6 +523,12 @@ fkadj_status BatchEngine::finish_poll(Job& j) {
     if (q != cudaSuccess) return fail(q, "job completion");
     Problem& P = *probs_[j.prob];
     const int nt = P.nt_;
+    if (j.swept && *reinterpret_cast<const unsigned*>(j.h_out + j.rows + 1) == FAULT_NAN) {
+        // a NaN state: once more with the tick kernels, which contain it
+        P.run_off_ = true;
+        return prepare_job(j, nullptr);
+    }
+    P.run_off_ = false;
     const double l0 = -j.h_out[0];
     double le = 0;
     for (int i = 0; i <= nt; ++i) le += j.Et[i] * j.Et[i];
@@ -541,7 +576,7 @@ fkadj_status BatchEngine::tick(int* active) {
         for (int id : active_) {
             Problem& P = *probs_[jobs_[id]->prob];
             const int64_t c = (int64_t)P.g_.nrows * P.g_.ncols;
-            if (jobs_[id]->want_grad && c > cells) cells = c, best = jobs_[id]->prob;
+            if (jobs_[id]->want_grad && !jobs_[id]->swept && c > cells) cells = c, best = jobs_[id]->prob;
         }
         if (best >= 0) {
             Problem& P = *probs_[best];
@@ -561,7 +596,7 @@ fkadj_status BatchEngine::tick(int* active) {
         }
     }
     // finished jobs and host actions first; `ready` jobs have a device action next
-    std::vector<int> still, ready;
+    std::vector<int> still, ready, swept;
     still.reserve(active_.size());
     for (int id : active_) {
         Job& j = *jobs_[id];
@@ -578,9 +613,10 @@ fkadj_status BatchEngine::tick(int* active) {
             if (a.kind == Action::FINISH) break;
         }
         still.push_back(id);
-        if (!j.finishing && j.pc < j.plan.size()) ready.push_back(id);
+        if (!j.finishing && j.pc < j.plan.size()) (j.swept ? swept : ready).push_back(id);
     }
     active_.swap(still);
+    if (!swept.empty() && (s = sweep_tick(swept))) return s;
     int K = 1;
     if (block_graphs_ && !ready.empty()) {
         int m = kBlockMax;
@@ -589,7 +625,7 @@ fkadj_status BatchEngine::tick(int* active) {
     }
     if (K >= 2) {
         if ((s = launch_block(K, ready))) return s;
-    } else {
+    } else if (!ready.empty() || swept.empty()) {
         t_fwd_->n = t_fwd_->tiles = 0;
         t_mid_->n = t_mid_->tiles = 0;
         t_adj_->n = t_adj_->tiles = 0;
@@ -602,6 +638,144 @@ fkadj_status BatchEngine::tick(int* active) {
         ++ticks_;
     }
     if (active) *active = (int)active_.size();
+    return FKADJ_OK;
+}
+
+// Calls launch(P, jobs, n) for each group of problems with one model.
+template <class Job_, class Launch>
+fkadj_status BatchEngine::by_model(std::vector<std::pair<Problem*, Job_>>& v, Launch&& launch) {
+    std::vector<Job_> group;
+    while (!v.empty()) {
+        Problem* P = v[0].first;
+        group.clear();
+        size_t kept = 0;
+        for (auto& e : v) {
+            if (!std::memcmp(&e.first->P_, &P->P_, sizeof P->P_)) group.push_back(e.second);
+            else v[kept++] = e;
+        }
+        v.resize(kept);
+        BCK(launch(*P, group.data(), (int)group.size()), "batched sweeps");
+    }
+    return FKADJ_OK;
+}
+
+// One tick of the jobs that run as sweeps (each has a device action next): a
+// run of forward steps of every job that has some next, the problems' sweeps
+// sharing launches (launch_fwd_jobs), then a chunk of backward steps of every
+// job that has those next, likewise.  A recomputed segment is taken whole; the
+// jobs in their forward sweep take as many steps as the longest of those, up
+// to kBlockMax, so that a launch's jobs end together.
+fkadj_status BatchEngine::sweep_tick(const std::vector<int>& ready) {
+    fkadj_status s;
+    auto run_of = [&](const Job& j) {  // actions of the next one's kind, at most kBlockMax
+        size_t k = j.pc;
+        while (k < j.plan.size() && k < j.pc + kBlockMax && j.plan[k].kind == j.plan[j.pc].kind) ++k;
+        return (int)(k - j.pc);
+    };
+    int m = 0;
+    for (int id : ready)
+        if (jobs_[id]->plan[jobs_[id]->pc].kind == Action::RECOMP) m = std::max(m, run_of(*jobs_[id]));
+    if (m == 0) m = kBlockMax;
+    std::vector<std::pair<Problem*, FwdJob>> fwd;
+    auto forward = [&](Problem& P, int i, int n, const double* src, double* last, double* out, double* keep, int first,
+                       int every) -> fkadj_status {
+        if (P.run_.id < 0) {
+            launches_ += n;
+            return P.sweep_forward(i, n, src, last, out, keep, first, every);
+        }
+        fwd.emplace_back(&P, P.forward_job(i, n, src, last, out, keep, first, every));
+        return FKADJ_OK;
+    };
+    auto launch_forward = [&]() {
+        return by_model(fwd, [&](Problem& P, const FwdJob* q, int n) {
+            return launch_fwd_jobs(P.P_, q, n, P.sms_, st_, &launches_);
+        });
+    };
+    for (int id : ready) {
+        Job& j = *jobs_[id];
+        Problem& P = *probs_[j.prob];
+        const Action a = j.plan[j.pc];
+        if (a.kind != Action::FWD && a.kind != Action::RECOMP) continue;
+        const int n = std::min(run_of(j), m), i = a.idx, c = j.tp.stride, nt = P.nt_;
+        double* last = j.cur == P.state_buf(1) ? P.state_buf(2) : P.state_buf(1);
+        if (a.kind == Action::RECOMP) {  // states s0 + 1 .. s1 - 1 to the segment's slots
+            const int k = i / c, s0 = k * c, s1 = std::min(s0 + c, nt);
+            if (i + n < s1) last = P.segslot(i + n - s0 - 1);
+            s = forward(P, i, n, i == s0 ? P.slot(k) : P.segslot(i - s0 - 1), last, P.segslot(i - s0),
+                        P.grad_mode_ == FKADJ_GRAD_EXACT && j.tp.keep_f ? P.fslot(3 * (i - s0)) : nullptr, 1, 1);
+        } else if (!j.want_grad) {
+            s = forward(P, i, n, j.cur, last, nullptr, nullptr, 1, 1);
+        } else {  // every c-th state and y(T) to the store
+            if (i + n == nt) last = P.slot(j.tp.nslots - 1);
+            else if ((i + n) % c == 0) last = P.slot((i + n) / c);
+            s = forward(P, i, n, j.cur, last, P.slot(i / c + 1), nullptr, c - i % c, c);
+        }
+        if (s) return s;
+        if (a.kind == Action::FWD) {
+            j.cur = last;
+            if (i + n == nt) j.yT = last;
+        }
+        j.pc += n;
+    }
+    if ((s = launch_forward())) return s;
+    struct Back {
+        Job* j;
+        int top, n;
+    };
+    std::vector<Back> back;
+    std::vector<std::pair<Problem*, MidJob>> mid;
+    std::vector<std::pair<Problem*, AdjJob>> adj[2];
+    for (int id : ready) {
+        Job& j = *jobs_[id];
+        Problem& P = *probs_[j.prob];
+        const Action a = j.plan[j.pc];
+        if (a.kind != Action::ADJ && a.kind != Action::EXADJ) continue;
+        const bool exact = a.kind == Action::EXADJ, full = j.tp.policy == FKADJ_CKPT_FULL;
+        const int top = exact ? a.idx + 1 : a.idx, c = j.tp.stride;
+        const int k = full ? 0 : (top - 1) / c, lo = k * c, hi = full ? P.nt_ : std::min(lo + c, P.nt_);
+        const double *y_hi = full ? P.slot(hi) : P.slot(k + 1), *y_lo = P.slot(k);
+        const double* mids = full ? P.slot(1) : P.segslot(0);
+        const double* stages = exact && j.tp.keep_f ? P.fslot(0) : nullptr;
+        auto state = [&](int t) { return t == hi ? y_hi : (t == lo ? y_lo : mids + (size_t)(t - lo - 1) * P.state_elems()); };
+        Problem::AdjointChunk q = P.adjoint_chunk(top, hi, lo, y_hi, mids, y_lo, stages, j.z, j.z2, kBlockMax);
+        const int n = q.n;
+        if (P.run_.id < 0) {
+            const int64_t l0 = P.launches_;
+            if ((s = P.sweep_adjoint(top, top - n, state(top), state(top - n + 1), state(top - n),
+                                     stages ? stages + 3 * (size_t)(top - n - lo) * P.state_elems() : nullptr, j.z, j.z2)))
+                return s;
+            launches_ += P.launches_ - l0;
+        } else {
+            if (q.replay && (s = forward(P, top - n, n, state(top - n), P.state_buf(1), nullptr, P.pts_.as<double>(), 1, 1)))
+                return s;
+            if (!exact) mid.emplace_back(&P, q.mid);
+            P.take_tags(q);
+            adj[exact].emplace_back(&P, q.adj);
+            std::swap(j.z, j.z2);
+        }
+        j.pc += n;
+        back.push_back({&j, top, n});
+    }
+    if ((s = launch_forward())) return s;
+    if ((s = by_model(mid, [&](Problem& P, const MidJob* q, int n) {
+             return launch_mid_jobs(P.P_, P.hw_, q, n, P.sms_, st_, &launches_);
+         })))
+        return s;
+    for (int exact = 0; exact < 2; ++exact)
+        if ((s = by_model(adj[exact], [&](Problem& P, const AdjJob* q, int n) {
+                 return launch_adj_jobs(exact != 0, P.P_, q, n, P.sms_, st_, &launches_);
+             })))
+            return s;
+    // the chunks' rows of z.gh sums
+    for (const Back& b : back) {
+        Problem& P = *probs_[b.j->prob];
+        const bool exact = P.grad_mode_ == FKADJ_GRAD_EXACT, sqrt_store = b.j->tp.policy == FKADJ_CKPT_SQRT;
+        const int row = b.top - b.n;
+        if (!sqrt_store && (row % P.pwin_ != 0 || P.run_.id < 0)) continue;
+        for (int g = 0; g < (exact ? 3 : 1); ++g, ++launches_)
+            BCK(sqrt_store ? P.flush_range(g, row, b.n) : P.flush_rows(g, row, exact ? P.nt_ : P.nt_ + 1), "reduce z.gh");
+    }
+    ++ticks_;
     return FKADJ_OK;
 }
 

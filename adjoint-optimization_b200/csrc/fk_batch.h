@@ -42,6 +42,7 @@ struct Job {
     int cur_c = 0;
     bool have_fcarry = false, have_jcarry = false;  // f(y) / J(y) carried from the previous backward step
     bool finishing = false, done = false;
+    bool swept = false;  // advanced by sweeps (fk_run.h), else by the tick kernels
     fkadj_status status = FKADJ_OK;
     double* h_out = nullptr;  // pinned: [0] sum for L0, [1..rows] reductions
     size_t h_cap = 0;         // doubles in h_out (a buffer of the engine's pool)
@@ -62,7 +63,7 @@ public:
     fkadj_status add_problem(const fkadj_params& p, double dt, int nt, const int* active_index, int nrows,
                              int ncols, int n_num, const double* gh_num, const double* gamma, int64_t S_ncol,
                              const int64_t* S_colptr, const int64_t* S_rowidx, const double* S_val, double alpha,
-                             int grad_mode, int ckpt_policy, int64_t ckpt_budget, int* id);
+                             int grad_mode, int ckpt_policy, int64_t ckpt_budget, int* id, bool sweeps = true);
     fkadj_status remove_problem(int id);
 
     // Queues a job; the initial state is uploaded now (y_ini may be null to
@@ -87,7 +88,11 @@ public:
 
 private:
     fkadj_status fail(cudaError_t e, const char* what);
+    fkadj_status prepare_job(Job& j, const double* y_ini);
     fkadj_status build_plan(Job& j);
+    fkadj_status sweep_tick(const std::vector<int>& ready);
+    template <class Job_, class Launch>
+    fkadj_status by_model(std::vector<std::pair<Problem*, Job_>>& v, Launch&& launch);
     fkadj_status host_action(Job& j, const Action& a);
     fkadj_status tick_action(Job& j, const Action& a);
     fkadj_status finish_poll(Job& j);

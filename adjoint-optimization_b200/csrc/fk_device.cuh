@@ -32,6 +32,7 @@ struct DevModel {
     double eq;          // exp(-2 ksm (u_c - u_v)): e^{-2ksm(u-u_v)} = eq * e^{-2ksm(u-u_c)}
     double cu, cv, cw;  // D / h^2
     double dt;
+    double dt_6, dt_3;  // dt / 6, dt / 3: a division in the kernels is a subroutine
     // constant factors of the Jacobian (fk_jacT)
     double two_ksm;       // 2 ksm: dp/du = 2 ksm p (1 - p)
     double kfk2_rsi;      // 2 k_fk / tau_si

@@ -58,6 +58,8 @@ static DevModel make_model(const fkadj_params& p, double dt) {
     M.cv = p.Dv / (p.h * p.h);
     M.cw = p.Dw / (p.h * p.h);
     M.dt = dt;
+    M.dt_6 = dt / 6.0;
+    M.dt_3 = dt / 3.0;
     M.two_ksm = 2.0 * p.ksm;
     M.kfk2_rsi = 2.0 * p.k_fk / p.tau_si;
     M.two_ksm_dv12 = 2.0 * p.ksm * (p.tau_v2_minus - p.tau_v1_minus);
@@ -243,15 +245,16 @@ Problem::~Problem() {
     // a failed call may leave copies to or from the staging in flight: let
     // them finish before another call takes the buffers
     if (st_ && (setup_ || (oneshot_ && (Ehost_ || hres_ || frame_)))) cudaStreamSynchronize(st_);
+    if (eup_) {
+        cudaEventSynchronize(eup_);
+        cudaEventDestroy(eup_);
+    }
     give_pinned(setup_, setup_n_);
     give_pinned(frame_, frame_n_);
-    if (oneshot_) {
-        give_pinned(Ehost_, Ehost_n_);
-        give_pinned(hres_, hres_n_);
-    } else {
-        if (Ehost_) cudaFreeHost(Ehost_);
-        if (hres_) cudaFreeHost(hres_);
-    }
+    if (oneshot_ || shared_) give_pinned(Ehost_, Ehost_n_);
+    else if (Ehost_) cudaFreeHost(Ehost_);
+    if (oneshot_) give_pinned(hres_, hres_n_);
+    else if (hres_) cudaFreeHost(hres_);
     const auto t2 = clk::now();
     if (own_stream_ && st_ && oneshot_ && pool_ && give_stream(device_, st_, ev_)) {
         st_ = nullptr;
@@ -663,7 +666,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
 // the environment keeps the preset kernels.
 fkadj_status Problem::init_sweeps(const uint8_t* cells, const uint8_t* adj, const uint8_t* seg) {
     const char* v = getenv("FKADJ_SWEEPS");
-    if (!autotune_ || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ || (v && v[0] == '0')) return FKADJ_OK;
+    if (!(autotune_ || shared_) || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ || (v && v[0] == '0')) return FKADJ_OK;
     const char* sv = getenv("FKADJ_ZGH_SEGMENTS");  // the adjoint sweeps write row segments
     if (sv && std::atoi(sv) == 0) return FKADJ_OK;
     int coop = 0;
@@ -748,11 +751,14 @@ fkadj_status Problem::prepare_E(const double* Et, bool upload) {
     const size_t n = (size_t)3 * nt_ + 1;
     if (!Ed_.p) {
         CK(Ed_.alloc(n * sizeof(double)), "alloc E tables");
-        if (oneshot_)
+        if (oneshot_ || shared_)
             CK(take_pinned(n, &Ehost_, &Ehost_n_), "alloc pinned E tables");
         else
             CK(cudaMallocHost(&Ehost_, n * sizeof(double)), "alloc pinned E tables");
+        if (shared_) CK(cudaEventCreateWithFlags(&eup_, cudaEventDisableTiming), "event");
         ++buf_gen_;
+    } else if (shared_) {  // the stream is other problems' too
+        CK(cudaEventSynchronize(eup_), "the previous upload");
     } else {
         CK(cudaStreamSynchronize(st_), "synchronize");  // the previous upload is done with the staging
     }
@@ -760,6 +766,7 @@ fkadj_status Problem::prepare_E(const double* Et, bool upload) {
     std::copy(Eh_.begin(), Eh_.end(), Ehost_ + nt_ + 1);
     std::copy(E3_.begin(), E3_.end(), Ehost_ + 2 * nt_ + 1);
     CK(cudaMemcpyAsync(Ed_.p, Ehost_, n * sizeof(double), cudaMemcpyHostToDevice, st_), "upload E tables");
+    if (eup_) CK(cudaEventRecord(eup_, st_), "event");
     return FKADJ_OK;
 }
 
@@ -849,7 +856,28 @@ fkadj_status Problem::step_forward(int i, const double* yin, double* yout, doubl
     return FKADJ_OK;
 }
 
-fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* last, double* out, double* keep) {
+FwdJob Problem::forward_job(int i, int n, const double* src, double* last, double* out, double* keep, int first,
+                            int every) {
+    FwdRun r{};
+    r.src = src;
+    r.last = last;
+    r.out = out;
+    r.stages = keep;
+    r.stride = (long long)state_elems();
+    r.n = n;
+    r.first = first;
+    r.every = every;
+    r.Et = etab() + i;
+    r.Eh = etab() + (nt_ + 1) + i;
+    r.exchange = xchg_.p;
+    r.epoch = epoch_;
+    r.fault = fault();
+    epoch_ += (unsigned long long)n;
+    return {g_, gh_.as<double>(), cells_.as<uint8_t>(), r};
+}
+
+fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* last, double* out, double* keep, int first,
+                                    int every) {
     if (n <= 0) return FKADJ_OK;
     const long long stride = (long long)state_elems();
     if (run_.id < 0 || !sweeping()) {
@@ -859,7 +887,9 @@ fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* las
         if (last == ((n & 1) ? s1 : s0)) std::swap(s0, s1);
         const double* cur = src;
         for (int k = 0; k < n; ++k) {
-            double* o = k == n - 1 ? last : (out ? out + k * stride : ((k & 1) ? s1 : s0));
+            const int m = k + 1 - first;
+            double* o = k == n - 1 ? last
+                                   : (out && m >= 0 && m % every == 0 ? out + m / every * stride : ((k & 1) ? s1 : s0));
             if (sweeping()) {
                 const EStep E = efwd(i + k);
                 const FwdStep r{cur, o, keep ? keep + 3 * k * stride : nullptr, E.p[0], E.p[1], E.p[2], fault()};
@@ -874,21 +904,8 @@ fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* las
         }
         return FKADJ_OK;
     }
-    FwdRun r{};
-    r.src = src;
-    r.last = last;
-    r.out = out;
-    r.stages = keep;
-    r.stride = stride;
-    r.n = n;
-    r.Et = etab() + i;
-    r.Eh = etab() + (nt_ + 1) + i;
-    r.exchange = xchg_.p;
-    r.epoch = epoch_;
-    r.fault = fault();
-    epoch_ += (unsigned long long)n;
     CK(prof_begin(K_FWD, n), "profiling event");
-    CK(launch_fwd_run(run_, P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), r, st_), "forward sweep");
+    CK(launch_fwd_run(run_, P_, forward_job(i, n, src, last, out, keep, first, every), st_), "forward sweep");
     CK(prof_end(K_FWD), "profiling event");
     ++launches_;
     return FKADJ_OK;
@@ -904,61 +921,81 @@ int Problem::sweep_chunk() const {
     return sweep_chunk_of((int64_t)state_bytes(), grad_mode_ == FKADJ_GRAD_EXACT);
 }
 
+// The next chunk of a backward sweep from state hi to lo, at most `most`
+// steps: its adjoint job, and what makes its points between the states: the
+// midpoint job (reference mode) or a replay (exact mode without kept stages),
+// whose launch comes first.
+Problem::AdjointChunk Problem::adjoint_chunk(int top, int hi, int lo, const double* y_hi, const double* mid,
+                                             const double* y_lo, const double* stages, const double* z, double* z2,
+                                             int most) {
+    const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
+    const long long sz = (long long)state_elems();
+    auto state = [&](int t) { return t == hi ? y_hi : (t == lo ? y_lo : mid + (t - lo - 1) * sz); };
+    // a chunk's rows of partial sums (top - 1 down) stay within one window
+    const int n = std::min({top - lo, most, sweep_chunk(), (top - 1) % pwin_ + 1});
+    AdjRun r{};
+    r.zin = z;
+    r.zout = z2;
+    r.y_hi = state(top);
+    r.y_mid = mid + (long long)(top - n - lo) * sz;
+    r.y_lo = state(top - n);
+    r.stride = sz;
+    r.n = n;
+    r.partial = partial_.as<double>();
+    r.nsb = nsb_;
+    r.nsbx = nsbx_;
+    r.row0 = top - 1;
+    r.window = pwin_;
+    r.exchange = xchg_.p;
+    r.fault = fault();
+    r.pts = pts_.as<double>();
+    r.pts_step = 1;
+    AdjointChunk c{};
+    c.n = n;
+    if (exact) {
+        r.pts_step = -3;
+        r.pts = stages ? stages + 3 * (long long)(top - 1 - lo) * sz : pts_.as<double>() + 3 * (n - 1) * sz;
+        c.replay = !stages;
+    } else {
+        MidRun m{};
+        m.y_hi = r.y_hi;
+        m.y_mid = r.y_mid;
+        m.y_lo = r.y_lo;
+        m.yh = pts_.as<double>();
+        m.stride = sz;
+        m.n = n;
+        m.Et = etab() + top;
+        m.E3 = etab() + (2 * nt_ + 1) + top - 1;
+        m.fault = fault();
+        c.mid = {g_, gh_.as<double>(), cells_.as<uint8_t>(), m};
+    }
+    c.adj = {g_, gh_.as<double>(), cells_.as<uint8_t>(), adjf_.as<uint8_t>(), r};
+    return c;
+}
+
 fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
                                     const double* stages, double*& z, double*& z2) {
     const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
     const long long sz = (long long)state_elems();
     auto state = [&](int t) { return t == hi ? y_hi : (t == lo ? y_lo : mid + (t - lo - 1) * sz); };
     for (int top = hi; top > lo;) {
-        // a chunk's rows of partial sums (top - 1 down) stay within one window
-        const int n = std::min({top - lo, sweep_chunk(), (top - 1) % pwin_ + 1});
-        AdjRun r{};
-        r.zin = z;
-        r.zout = z2;
-        r.y_hi = state(top);
-        r.y_mid = mid + (long long)(top - n - lo) * sz;
-        r.y_lo = state(top - n);
-        r.stride = sz;
-        r.n = n;
-        r.partial = partial_.as<double>();
-        r.nsb = nsb_;
-        r.nsbx = nsbx_;
-        r.row0 = top - 1;
-        r.window = pwin_;
-        r.exchange = xchg_.p;
-        r.fault = fault();
-        r.pts = pts_.as<double>();
-        r.pts_step = exact ? 3 : 1;
-        if (exact && stages) {
-            r.pts = stages + 3 * (long long)(top - 1 - lo) * sz;
-            r.pts_step = -3;
-        } else if (exact) {
-            for (int k = 0; k < n; ++k)
-                if (fkadj_status s = sweep_forward(top - 1 - k, 1, state(top - 1 - k), state_buf(1), nullptr,
-                                                   pts_.as<double>() + 3 * k * sz))
-                    return s;
-        } else {
-            MidRun m{};
-            m.y_hi = r.y_hi;
-            m.y_mid = r.y_mid;
-            m.y_lo = r.y_lo;
-            m.yh = pts_.as<double>();
-            m.stride = sz;
-            m.n = n;
-            m.Et = etab() + top;
-            m.E3 = etab() + (2 * nt_ + 1) + top - 1;
-            m.fault = fault();
+        AdjointChunk c = adjoint_chunk(top, hi, lo, y_hi, mid, y_lo, stages, z, z2, nt_);
+        AdjRun& r = c.adj.r;
+        const int n = c.n;
+        if (c.replay) {
+            // from the chunk's lowest state up, every step's stages
+            if (fkadj_status s = sweep_forward(top - n, n, state(top - n), state_buf(1), nullptr, pts_.as<double>()))
+                return s;
+        } else if (!exact) {
             CK(prof_begin(K_MID, n), "profiling event");
-            CK(launch_mid_run(P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), hw_, m, sms_, st_), "adjoint midpoints");
+            CK(launch_mid_run(P_, hw_, c.mid, sms_, st_), "adjoint midpoints");
             CK(prof_end(K_MID), "profiling event");
             ++launches_;
         }
         if (run_.id >= 0) {
-            r.epoch = epoch_;  // after a replay's forward sweeps
-            epoch_ += (unsigned long long)n;
+            take_tags(c);  // after a replay's
             CK(prof_begin(K_ADJ, n), "profiling event");
-            CK(launch_adj_run(run_, exact, P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), adjf_.as<uint8_t>(), r, st_),
-               "adjoint sweep");
+            CK(launch_adj_run(run_, exact, P_, c.adj, st_), "adjoint sweep");
             CK(prof_end(K_ADJ), "profiling event");
             ++launches_;
             std::swap(z, z2);
@@ -1242,7 +1279,9 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
     }
     if (sweep) {
         // midpoint states of a chunk, or the stage states of one where the plan keeps none
-        const size_t c = (size_t)std::min(sweep_chunk(), nt_);
+        // (chunks do not cross the segments of a sqrt store)
+        const int seg = traj_plan_.policy == FKADJ_CKPT_SQRT ? traj_plan_.stride : nt_;
+        const size_t c = (size_t)std::min({sweep_chunk(), nt_, seg});
         const size_t k = grad_mode_ == FKADJ_GRAD_REF ? c : (traj_plan_.keep_f ? 0 : 3 * c);
         if (pts_.bytes < k * state_bytes()) {
             CK(pts_.alloc(k * state_bytes()), "alloc adjoint points");
@@ -1719,15 +1758,17 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
     if (tp.policy == FKADJ_CKPT_FULL) {
         if ((s = sweep_forward(0, nt, slot(0), slot(nt), slot(1), tp.keep_f ? fslot(0) : nullptr))) return s;
         cur = slot(nt);
+    } else if (!binomial) {  // every c-th state and y(T)
+        if ((s = sweep_forward(0, nt, slot(0), slot(K), slot(1), nullptr, c, c))) return s;
+        cur = slot(K);
     } else {
-        // binomial: the forward sweep stores the schedule's spine; its k-th state
-        // goes to the k-th slot the reversal takes (free slots are taken from the
-        // back of nslots-1 .. 2), y(T) to slot 1; sqrt: every c-th state and y(T)
-        const std::vector<int> spine = binomial ? binomial_spine(nt, tp.nslots - 2) : std::vector<int>();
+        // the forward sweep stores the schedule's spine; its k-th state goes to
+        // the k-th slot the reversal takes (free slots are taken from the back
+        // of nslots-1 .. 2), y(T) to slot 1
+        const std::vector<int> spine = binomial_spine(nt, tp.nslots - 2);
         for (int i = 0, k = 0; i < nt; ++k) {
-            int stop = nt;
-            if (binomial ? k < (int)spine.size() : i + c < nt) stop = binomial ? spine[k] : i + c;
-            double* out = binomial ? (stop == nt ? slot(1) : slot(2 + k)) : slot(k + 1);
+            const int stop = k < (int)spine.size() ? spine[k] : nt;
+            double* out = stop == nt ? slot(1) : slot(2 + k);
             if ((s = sweep_forward(i, stop - i, cur, out))) return s;
             cur = out;
             i = stop;

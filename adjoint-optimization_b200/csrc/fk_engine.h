@@ -127,10 +127,12 @@ public:
     enum AdjPath { ADJ_SPLIT = 0, ADJ_FUSED = 1, ADJ_FUSED_RECOMPUTE = 2 };
     int adjoint_path() const { return adj_path_; }
     int fused_tile() const { return tkf_; }
-    // Stream-ordered device memory from `pool` (call before init).
-    void use_pool(cudaMemPool_t pool) {
+    // A batch engine's problem: stream-ordered device memory from `pool`; with
+    // `sweeps`, sweeps whatever its fixed tile (call before init).
+    void use_pool(cudaMemPool_t pool, bool sweeps) {
         pool_ = pool;
-        own_sweeps_ = false;
+        shared_ = true;
+        own_sweeps_ = sweeps;
     }
     // The preset kernels, which need less device memory (call before init).
     void no_sweeps() { own_sweeps_ = false; }
@@ -163,13 +165,29 @@ public:
     // standalone kernels read (the batched kernels take E by value).
     fkadj_status prepare_E(const double* Et, bool upload = true);
     fkadj_status step_forward(int i, const double* yin, double* yout, double* k1 = nullptr);
-    // n forward steps from step i, src -> last; the states between go to out +
-    // k * state_elems() (k = 0 .. n-2) when out is non-null; `keep` receives per
-    // step k1 = f of the state before it (reference mode: per-step launches) or
-    // the three stage states (exact mode: sweeps).  One launch where the grid
-    // is swept (sweeping()), n launches otherwise.
+    // n forward steps from step i, src -> last; of the states between, those
+    // after `first` steps and every `every` more go to out, out +
+    // state_elems(), ... when out is non-null; `keep` receives per step k1 = f
+    // of the state before it (reference mode: per-step launches) or the three
+    // stage states (exact mode: sweeps).  One launch where the grid is swept
+    // (sweeping()), n launches otherwise.
     fkadj_status sweep_forward(int i, int n, const double* src, double* last, double* out = nullptr,
-                               double* keep = nullptr);
+                               double* keep = nullptr, int first = 1, int every = 1);
+    // The same as a job of a launch (its exchange tags are taken: launch jobs
+    // in the order they were made).
+    FwdJob forward_job(int i, int n, const double* src, double* last, double* out, double* keep, int first, int every);
+    struct AdjointChunk {
+        int n;        // steps
+        bool replay;  // the points come from a forward sweep of the same steps into pts_
+        MidJob mid;   // ... or from this (reference mode)
+        AdjJob adj;   // its exchange tags are still to be taken (take_tags)
+    };
+    AdjointChunk adjoint_chunk(int top, int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
+                               const double* stages, const double* z, double* z2, int most);
+    void take_tags(AdjointChunk& c) {
+        c.adj.r.epoch = epoch_;
+        epoch_ += (unsigned long long)c.n;
+    }
     // Backward steps hi .. lo + 1 of a swept problem, z -> z (the pair is
     // swapped as it goes): y_hi, y_lo the states at both ends, mid the states
     // lo + 1 .. hi - 1 in a row, stages (exact mode; null: replayed) the stage
@@ -304,7 +322,9 @@ private:
     // (FAULT_NAN), which they contain
     bool run_off_ = false;
     bool nan_seen_ = false;
-    bool own_sweeps_ = true;  // false for a batch engine's problems, and where memory is short
+    bool own_sweeps_ = true;  // false where memory is short
+    bool shared_ = false;     // a batch engine's problem
+    cudaEvent_t eup_ = nullptr;  // of such a problem: its E tables' upload
     DevBuf work_;      // 4 states: two ping-pong, z pair is separate
     DevBuf zbuf_;      // 2 adjoint states
     DevBuf yh_;        // midpoint state

@@ -397,7 +397,7 @@ __device__ __forceinline__ void fwd_step_tile(const DevModel& P, const DevGrid& 
                                 rows, nullptr);
     fwd_stage<1, TX, TY, NT, 1, PF>(P, A, B, D, y0g, ghs, g.ld, g.plane, Eh, dt * 1.0, 1.0 / 3.0 * dt, nullptr, s4,
                                 rows, nullptr);
-    fwd_stage<0, TX, TY, NT, 2, PF>(P, B, A, D, y0g, ghs, g.ld, g.plane, E1, 0.0, dt * 1.0 / 6.0, yout + off, nullptr,
+    fwd_stage<0, TX, TY, NT, 2, PF>(P, B, A, D, y0g, ghs, g.ld, g.plane, E1, 0.0, P.dt_6, yout + off, nullptr,
                                 rows, nullptr);
 }
 
@@ -1130,7 +1130,7 @@ __device__ __forceinline__ void adj_exact_tile(const DevModel& P, const DevGrid&
                                         nullptr, nullptr, phase))
         return;
     const double dt = P.dt;
-    const double c6 = dt / 6.0, c3 = dt / 3.0, c2 = dt * 0.5;
+    const double c6 = P.dt_6, c3 = P.dt_3, c2 = dt * 0.5;
     const long long sst = 3 * g.plane;
     // the first stage takes g(a4) = c6 g(lambda), a4 = c6 lambda
     exact_stage<3, TX, TY, NT, 0, PF>(P, g, A, B, D, lam, wc, stages + 2 * sst, off, c3, dt, nullptr, T3, rows, c6);

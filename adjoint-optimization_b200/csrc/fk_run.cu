@@ -29,6 +29,8 @@
 #include "fk_run.h"
 
 #include <algorithm>
+#include <utility>
+#include <vector>
 
 #include "fk_bulk.cuh"
 
@@ -81,6 +83,25 @@ struct TileShapeBig {
     static constexpr size_t SMEM = sizeof(double) * (size_t)(3 * (2 * PA + PB + PC) + 3 * TERM);
     static_assert((TYM + 6) % R == 0 && THREADS <= 512 && SMEM + 256 <= 232448, "one CTA per SM");
     static_assert(3 * TERM >= 2 * RW, "reads past C stay in the allocation");
+};
+
+// The jobs of a launch, in the order of their tiles.  A kernel of several
+// copies its CTA's job to shared memory first (take): indexed where they lie,
+// among the parameters, one instance ended in an illegal instruction.
+constexpr int kRunJobs = 16;
+template <class Job>
+struct RunJobs {
+    int n;
+    Job job[kRunJobs];
+    // *j <- the job of a tile; ends with the CTA synchronised
+    __device__ __forceinline__ void take(int tile, Job* j) const {
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int q = 0; q < kRunJobs; ++q)
+                if (q < n && tile >= job[q].tile0 && (q + 1 >= n || tile < job[min(q + 1, kRunJobs - 1)].tile0)) *j = job[q];
+        }
+        __syncthreads();
+    }
 };
 
 // One exchanged value: the state's double and the number of the step it
@@ -279,11 +300,14 @@ double o[3];
 // tile).  The exchange area is two 3-plane grids of Tagged, used in turn: a
 // tile writes step k + 2's edges over step k's only after it has read its
 // neighbours' step k + 1, which they published after they had read step k.
-template <int TX, int R, int TYM>
-__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
-    k_fwd_run(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
-              const FwdRun r, int ty) {
-    using S = Shape<TX, R, TYM>;
+template <class S>
+__device__ __forceinline__ void fwd_run(const DevModel& P, const FwdJob& J) {
+    constexpr int TX = S::TX, R = S::R;
+    const DevGrid& g = J.g;
+    const FwdRun& r = J.r;
+    const double* __restrict__ gh = J.gh;
+    const uint8_t* __restrict__ cells = J.cells;
+    const int ty = J.ty;
     constexpr int RW = S::RW;
     extern __shared__ double4 smem_raw[];
     __shared__ uint64_t bar;
@@ -291,13 +315,13 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     double* B = A + 3 * S::PA - RW;
     double* C = A + 3 * (S::PA + S::PB) - 2 * RW;
     double* G = A + 3 * (S::PA + S::PB + S::PC) - RW;
-    const int bx = blockIdx.x, by = blockIdx.y;
+    const int tile = blockIdx.x - J.tile0, by = tile / J.ntx, bx = tile - by * J.ntx;
     const int i0 = by * ty, j0 = bx * TX;
     const int rows = min(ty, g.nrows - i0);
     const long long off = (long long)i0 * g.ld + j0;  // window origin: logical (i0 - 4, j0 - 4)
 
     int2* ring = reinterpret_cast<int2*>(G + RW + S::PB);
-    const int nring = ring_table<S>(ring, g.ld, rows, i0, j0, g.nrows, (int)gridDim.x * TX);
+    const int nring = ring_table<S>(ring, g.ld, rows, i0, j0, g.nrows, J.ntx * TX);
     exp_table_init();
     const uint32_t b = bulk_begin(&bar);
     __syncthreads();
@@ -347,9 +371,13 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
         const unsigned long long tag = r.epoch + k + 1;
         Tagged* x = static_cast<Tagged*>(r.exchange) + (tag & 1) * (3 * g.plane) + off;
         {
-            double* out = end ? r.last : (r.out ? r.out + k * r.stride : nullptr);
+            double* out = end ? r.last : nullptr;
+            if (!end && r.out && k + 1 >= r.first) {
+                const int m = (k + 1 - r.first) / r.every;
+                if (m * r.every == k + 1 - r.first) out = r.out + m * r.stride;
+            }
             fwd_rows<0, S, 2, S::PB, S::PB>(P, T, B, nullptr, A, G, D, rows, g.ld, g.plane, __ldg(r.Et + k + 1), 0.0,
-                                            P.dt / 6.0, out ? out + off : nullptr, end ? nullptr : x, tag, bad);
+                                            P.dt_6, out ? out + off : nullptr, end ? nullptr : x, tag, bad);
         }
         if (end) break;
         if (!read_ring<S>(A, ring, nring, x, tag, g.plane, r.fault)) return;
@@ -359,6 +387,19 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     // neighbour for missing), this sweep lets it spread.  The host repeats the
     // call with them.
     if (bad) atomicOr(r.fault, FAULT_NAN);
+}
+
+template <int TX, int R, int TYM>
+__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1) k_fwd_run(const DevModel P, const FwdJob j) {
+    fwd_run<Shape<TX, R, TYM>>(P, j);
+}
+
+template <int TX, int R, int TYM>
+__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
+    k_fwd_jobs(const DevModel P, const RunJobs<FwdJob> jobs) {
+    __shared__ FwdJob j;
+    jobs.take(blockIdx.x, &j);
+    fwd_run<Shape<TX, R, TYM>>(P, j);
 }
 
 // ------------------------------------------------------------ adjoint sweeps
@@ -535,11 +576,15 @@ __device__ __forceinline__ void segment_terms(const uint16_t* list, int count, d
     }
 }
 
-template <int TX, int R, int TYM, bool EXACT>
-__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
-    k_adj_run(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
-              const uint8_t* __restrict__ adj, const AdjRun r, int ty) {
-    using S = Shape<TX, R, TYM>;
+template <class S, bool EXACT>
+__device__ __forceinline__ void adj_run(const DevModel& P, const AdjJob& J) {
+    constexpr int TX = S::TX, R = S::R, TYM = S::TYM;
+    const DevGrid& g = J.g;
+    const AdjRun& r = J.r;
+    const double* __restrict__ gh = J.gh;
+    const uint8_t* __restrict__ cells = J.cells;
+    const uint8_t* __restrict__ adj = J.adj;
+    const int ty = J.ty;
     constexpr int RW = S::RW;
     extern __shared__ double4 smem_raw[];
     __shared__ uint64_t bar;
@@ -551,11 +596,11 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     double* G = A + 3 * (S::PA + S::PB + S::PC) - RW;
     int2* ring = reinterpret_cast<int2*>(G + RW + S::PB);
     double* K3 = reinterpret_cast<double*>(ring + S::RING) - RW;  // a_3 on u (exact mode), rows 1 ..
-    const int bx = blockIdx.x, by = blockIdx.y;
+    const int tile = blockIdx.x - J.tile0, by = tile / J.ntx, bx = tile - by * J.ntx;
     const int i0 = by * ty, j0 = bx * TX;
     const int rows = min(ty, g.nrows - i0);
     const long long off = (long long)i0 * g.ld + j0;
-    const int nring = ring_table<S>(ring, g.ld, rows, i0, j0, g.nrows, (int)gridDim.x * TX);
+    const int nring = ring_table<S>(ring, g.ld, rows, i0, j0, g.nrows, J.ntx * TX);
     exp_table_init();
     if (threadIdx.x == 0) s_segs = 0;
     const uint32_t b = bulk_begin(&bar);
@@ -607,19 +652,19 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     for (int k = 0; k < r.n; ++k) {
         if (EXACT)
             segment_terms<S>(segs, nsegs, partial(2, k), i0, j0, r.nsbx,
-                             [&](int q) { return ((P.dt / 6.0) * A[q]) * G[q]; });
+                             [&](int q) { return ((P.dt_6) * A[q]) * G[q]; });
         adj_rows<3, S, 0, S::PA, S::PB, EXACT>(P, T, A, B, A, D, yv, point(k, 0), rows, g.ld, g.plane,
-                                               EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt / 3.0 : 1.0 / 6.0 * P.dt,
-                                               P.dt / 6.0, K3, nullptr, nullptr, nullptr, 0);
+                                               EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt_3 : 1.0 / 6.0 * P.dt,
+                                               P.dt_6, K3, nullptr, nullptr, nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 1), yv);
         __syncthreads();
         adj_rows<2, S, 1, S::PB, S::PC, EXACT>(P, T, B, C, A, D, yv, point(k, 1), rows, g.ld, g.plane, 0.5 * P.dt,
-                                               EXACT ? P.dt / 3.0 : 2.0 / 6.0 * P.dt, 0.0, nullptr, nullptr, nullptr,
+                                               EXACT ? P.dt_3 : 2.0 / 6.0 * P.dt, 0.0, nullptr, nullptr, nullptr,
                                                nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 2), yv);
         __syncthreads();
         adj_rows<1, S, 1, S::PC, S::PB, EXACT>(P, T, C, B, A, D, yv, point(k, 2), rows, g.ld, g.plane,
-                                               EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt / 6.0 : 2.0 / 6.0 * P.dt, 0.0,
+                                               EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt_6 : 2.0 / 6.0 * P.dt, 0.0,
                                                nullptr, nullptr, nullptr, nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, point(k, 3), yv);
         __syncthreads();
@@ -644,6 +689,19 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
         if (!EXACT)
             segment_terms<S>(segs, nsegs, partial(0, k), i0, j0, r.nsbx, [&](int q) { return A[q] * G[q]; });
     }
+}
+
+template <int TX, int R, int TYM, bool EXACT>
+__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1) k_adj_run(const DevModel P, const AdjJob j) {
+    adj_run<Shape<TX, R, TYM>, EXACT>(P, j);
+}
+
+template <int TX, int R, int TYM, bool EXACT>
+__global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
+    k_adj_jobs(const DevModel P, const RunJobs<AdjJob> jobs) {
+    __shared__ AdjJob j;
+    jobs.take(blockIdx.x, &j);
+    adj_run<Shape<TX, R, TYM>, EXACT>(P, j);
 }
 
 // --------------------------------------------- per-step tiles, larger grids
@@ -768,7 +826,7 @@ __global__ void __launch_bounds__(TileShapeBig::THREADS, 1)
         __syncthreads();
         if (r.dst)
             fwd_rows<0, S, 2, S::PB, S::PB>(P, T, B, nullptr, A, ghs, D, rows, g.ld, g.plane, E1, 0.0,
-                                            P.dt / 6.0, r.dst + off, nullptr, 0, bad);
+                                            P.dt_6, r.dst + off, nullptr, 0, bad);
         __syncthreads();  // B and A are free
     }
     if (bad) atomicOr(r.fault, FAULT_NAN);
@@ -813,17 +871,17 @@ __global__ void __launch_bounds__(TileShapeBig::THREADS, 1)
         const bool ok = bulk_wait(bar + 8 * (n & 1), 1000000000ull, (unsigned)(n >> 1) & 1u);
         const double* ghs = gh + off;
         adj_rows<3, S, 0, S::PA, S::PB, EXACT>(P, T, A, B, A, D, yv, r.y[0] + off, rows, g.ld, g.plane,
-                                               EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt / 3.0 : 1.0 / 6.0 * P.dt,
-                                               P.dt / 6.0, terms, ghs, nullptr, nullptr, 0);
+                                               EXACT ? P.dt : 0.5 * P.dt, EXACT ? P.dt_3 : 1.0 / 6.0 * P.dt,
+                                               P.dt_6, terms, ghs, nullptr, nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, r.y[1] + off, yv);
         if (!window_arrived(ok, bar, n, more, r.fault)) return;
         adj_rows<2, S, 1, S::PB, S::PC, EXACT>(P, T, B, C, A, D, yv, r.y[1] + off, rows, g.ld, g.plane, 0.5 * P.dt,
-                                               EXACT ? P.dt / 3.0 : 2.0 / 6.0 * P.dt, 0.0, terms, ghs, nullptr,
+                                               EXACT ? P.dt_3 : 2.0 / 6.0 * P.dt, 0.0, terms, ghs, nullptr,
                                                nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, r.y[2] + off, yv);
         __syncthreads();
         adj_rows<1, S, 1, S::PC, S::PB, EXACT>(P, T, C, B, A, D, yv, r.y[2] + off, rows, g.ld, g.plane,
-                                               EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt / 6.0 : 2.0 / 6.0 * P.dt, 0.0,
+                                               EXACT ? 0.5 * P.dt : P.dt, EXACT ? P.dt_6 : 2.0 / 6.0 * P.dt, 0.0,
                                                terms, ghs, nullptr, nullptr, 0);
         load_point<S>(T, 0, rows, g.ld, g.plane, r.y[3] + off, yv);
         __syncthreads();
@@ -892,21 +950,24 @@ __device__ __forceinline__ void mid_field(const DevModel& P, unsigned b, const d
     fk_field(P, y, t, E, gv, kk[0], kk[1], kk[2]);
 }
 
-__global__ void __launch_bounds__(MidShape::THREADS, 1)
-    k_mid_run(const DevModel P, const DevGrid g, const double* __restrict__ gh, const uint8_t* __restrict__ cells,
-              const HermiteW hw, const MidRun r, int per) {
+__device__ __forceinline__ void mid_run(const DevModel& P, const HermiteW& hw, const MidJob& J) {
     using S = MidShape;
+    const DevGrid& g = J.g;
+    const MidRun& r = J.r;
+    const double* __restrict__ gh = J.gh;
+    const uint8_t* __restrict__ cells = J.cells;
     constexpr int RW = S::RW, PW = S::PW, R = S::R;
     extern __shared__ double4 smem_raw[];
     __shared__ uint64_t bars[3];
     double* W = reinterpret_cast<double*>(smem_raw);  // three windows in turn
     double* Y3 = W + 9 * PW;                          // two buffers in turn
     double* G = Y3 + 6 * PW;
-    const int i0 = blockIdx.y * S::TY, j0 = blockIdx.x * S::TX;
+    const int bx = (blockIdx.x - J.tile0) % J.ntx, t0 = (blockIdx.x - J.tile0) / J.ntx;
+    const int i0 = t0 % J.nty * S::TY, j0 = bx * S::TX;
     const int rows = min(S::TY, g.nrows - i0);
     // window origin: logical (i0 - 2, j0 - 4) = padded (i0 + 2, j0)
     const long long off = (long long)(i0 + HALO - S::H) * g.ld + j0;
-    const int k0 = blockIdx.z * per, k1 = min(k0 + per, r.n);  // steps k0 .. k1 - 1
+    const int k0 = t0 / J.nty * J.per, k1 = min(k0 + J.per, r.n);  // steps k0 .. k1 - 1
     if (k0 >= k1) return;
     exp_table_init();
     const uint32_t bar = bulk_begin(&bars[0]);
@@ -995,73 +1056,189 @@ __global__ void __launch_bounds__(MidShape::THREADS, 1)
     }
 }
 
+__global__ void __launch_bounds__(MidShape::THREADS, 1) k_mid_run(const DevModel P, const HermiteW hw, const MidJob j) {
+    mid_run(P, hw, j);
+}
+
+__global__ void __launch_bounds__(MidShape::THREADS, 1)
+    k_mid_jobs(const DevModel P, const HermiteW hw, const RunJobs<MidJob> jobs) {
+    __shared__ MidJob j;
+    jobs.take(blockIdx.x, &j);
+    mid_run(P, hw, j);
+}
+
 }  // namespace
 
 #define X(id, a, b, c) \
     case id: { using S = Shape<a, b, c>; DO(S); } break;
 
+constexpr int kRunShapes = 6;
+struct ShapeInfo {
+    int tx, R, tym, rw, threads;
+    // a step's cost on tiles of `rows` rows: per stage, the evaluations (a
+    // warp's row, by FP64 issue) or the depth of a thread's column, whichever
+    // is longer
+    double cost(int rows) const {
+        double c = 0;
+        for (int e = 3; e >= 0; --e) c += std::max((double)rw * (rows + 2 * e) / 32.0 * 62.0, R * 420.0);
+        return c;
+    }
+    int threads_for(int rows) const { return std::min(threads, (rw * ((rows + 6 + R - 1) / R) + 31) / 32 * 32); }
+};
+static ShapeInfo shape_info(int id) {
+    switch (id) {
+#define DO(S) return {S::TX, S::R, S::TYM, S::RW, S::THREADS}
+        FKADJ_RUN_LIST(X)
+#undef DO
+    }
+    return {};
+}
+
 RunShape run_shape(const DevGrid& g, int sms) {
     RunShape best;
     double best_cost = 0;
-    for (int id = 0; id < 6; ++id) {
-        int tx = 0, R = 0, tym = 0, rw = 0, threads = 0;
-        switch (id) {
-#define DO(S) tx = S::TX, R = S::R, tym = S::TYM, rw = S::RW, threads = S::THREADS
-            FKADJ_RUN_LIST(X)
-#undef DO
-        }
-        const int ntx = (g.ncols + tx - 1) / tx;
+    for (int id = 0; id < kRunShapes; ++id) {
+        const ShapeInfo f = shape_info(id);
+        const int ntx = (g.ncols + f.tx - 1) / f.tx;
         if (ntx > sms) continue;
         // at least 4 rows: a tile's halo is its direct neighbours' cells
         const int rows = std::max(HALO, (g.nrows + sms / ntx - 1) / (sms / ntx));
-        if (rows > tym) continue;
-        // a step's cost: per stage, the evaluations (a warp's row, by FP64
-        // issue) or the depth of a thread's column, whichever is longer
-        double cost = 0;
-        for (int e = 3; e >= 0; --e) {
-            const double warps = (double)rw * (rows + 2 * e) / 32.0;
-            cost += std::max(warps * 62.0, R * 420.0);
-        }
+        if (rows > f.tym) continue;
+        const double cost = f.cost(rows);
         if (best.id < 0 || cost < best_cost) {
             best_cost = cost;
-            best.id = id;
-            best.tx = tx;
-            best.rows = rows;
-            best.ntx = ntx;
-            best.nty = (g.nrows + rows - 1) / rows;
-            const int need = rw * ((rows + 6 + R - 1) / R);
-            best.threads = std::min(threads, (need + 31) / 32 * 32);
+            best = {id, f.tx, rows, ntx, (g.nrows + rows - 1) / rows, f.threads_for(rows)};
         }
     }
     return best;
+}
+
+// How n problems' tiles share launches of at most `sms` tiles and kRunJobs
+// problems: their shape, each one's launch, and the rows of a tile in each.
+struct RunPacking {
+    int id = -1, bins = 0;
+    std::vector<int> bin, rows;
+    double cost = 0;
+};
+
+// The packing of shape `id`, or bins = 0 where a grid does not fit in it: the
+// largest problem to the emptiest of as few launches as hold them all, then
+// in each launch as few rows a tile as still fit.
+template <class Job>
+static RunPacking pack_shape(const Job* j, int n, int id, int sms) {
+    const ShapeInfo f = shape_info(id);
+    auto tiles = [&](int q, int rows) {
+        return ((j[q].g.ncols + f.tx - 1) / f.tx) * ((j[q].g.nrows + rows - 1) / rows);
+    };
+    RunPacking p;
+    std::vector<int> order(n);
+    long long total = 0;
+    for (int q = 0; q < n; ++q) {
+        order[q] = q;
+        total += tiles(q, f.tym);
+        if (tiles(q, f.tym) > sms) return p;
+    }
+    std::sort(order.begin(), order.end(), [&](int a, int b) { return tiles(a, f.tym) > tiles(b, f.tym); });
+    std::vector<int> load, count;
+    for (int bins = std::max((int)((total + sms - 1) / sms), (n + kRunJobs - 1) / kRunJobs);; ++bins) {
+        load.assign(bins, 0);
+        count.assign(bins, 0);
+        p.bin.assign(n, 0);
+        bool fits = true;
+        for (int q : order) {
+            int b = -1;
+            for (int c = 0; c < bins; ++c)
+                if (count[c] < kRunJobs && (b < 0 || load[c] < load[b])) b = c;
+            load[b] += tiles(q, f.tym);
+            ++count[b];
+            p.bin[q] = b;
+            fits = fits && load[b] <= sms;
+        }
+        if (!fits) continue;  // ends at one problem per launch at the latest
+        p.bins = bins;
+        break;
+    }
+    p.id = id;
+    for (int b = 0; b < p.bins; ++b) {
+        int rows = f.tym;
+        for (; rows > HALO; --rows) {
+            int t = 0;
+            for (int q = 0; q < n; ++q)
+                if (p.bin[q] == b) t += tiles(q, rows - 1);
+            if (t > sms) break;
+        }
+        p.rows.push_back(rows);
+        p.cost += f.cost(rows);
+    }
+    return p;
+}
+
+// Runs n jobs packed: launch(id, jobs of one launch, threads, tiles).  Where
+// no shape takes all the grids, in two parts (run_shape has one for each).
+template <class Job, class Launch>
+static cudaError_t run_packed(const Job* j, int n, int sms, Launch&& launch) {
+    if (n <= 0) return cudaSuccess;
+    RunPacking best;
+    for (int id = 0; id < kRunShapes; ++id) {
+        RunPacking p = pack_shape(j, n, id, sms);
+        if (p.bins > 0 && (best.bins == 0 || p.cost < best.cost)) best = std::move(p);
+    }
+    if (best.bins == 0) {
+        if (n == 1) return cudaErrorInvalidValue;
+        const cudaError_t e = run_packed(j, n / 2, sms, launch);
+        return e ? e : run_packed(j + n / 2, n - n / 2, sms, launch);
+    }
+    const ShapeInfo f = shape_info(best.id);
+    for (int b = 0; b < best.bins; ++b) {
+        RunJobs<Job> jobs;
+        jobs.n = 0;
+        int tiles = 0;
+        for (int q = 0; q < n; ++q) {
+            if (best.bin[q] != b) continue;
+            Job& k = jobs.job[jobs.n++];
+            k = j[q];
+            const int nty = (k.g.nrows + best.rows[b] - 1) / best.rows[b];
+            k.ty = std::max(HALO, (k.g.nrows + nty - 1) / nty);
+            k.ntx = (k.g.ncols + f.tx - 1) / f.tx;
+            k.tile0 = tiles;
+            tiles += k.ntx * ((k.g.nrows + k.ty - 1) / k.ty);
+        }
+        if (const cudaError_t e = launch(best.id, jobs, f.threads_for(best.rows[b]), tiles)) return e;
+    }
+    return cudaSuccess;
 }
 
 size_t run_exchange_bytes(const DevGrid& g) { return 2 * 3 * (size_t)g.plane * sizeof(Tagged); }
 
 cudaError_t run_init() {
     cudaError_t e = cudaFuncSetAttribute(k_mid_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MidShape::SMEM);
+    if (!e) e = cudaFuncSetAttribute(k_mid_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MidShape::SMEM);
     const int big = (int)TileShapeBig::SMEM;
     if (!e) e = cudaFuncSetAttribute(k_fwd_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (!e) e = cudaFuncSetAttribute(k_adj_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (!e) e = cudaFuncSetAttribute(k_adj_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 #undef X
-#define X(id, a, b, c)                                                                                     \
-    if (!e) e = cudaFuncSetAttribute(k_fwd_run<a, b, c>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     (int)Shape<a, b, c>::SMEM);                                            \
-    if (!e) e = cudaFuncSetAttribute(k_adj_run<a, b, c, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     (int)Shape<a, b, c>::SMEM);                                            \
-    if (!e) e = cudaFuncSetAttribute(k_adj_run<a, b, c, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     (int)Shape<a, b, c>::SMEM_EXACT);
+#define N_(K, smem) \
+    if (!e) e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem))
+#define X(id, a, b, c)                                                    \
+    N_((k_fwd_run<a, b, c>), (Shape<a, b, c>::SMEM));                  \
+    N_((k_fwd_jobs<a, b, c>), (Shape<a, b, c>::SMEM));           \
+    N_((k_adj_run<a, b, c, false>), (Shape<a, b, c>::SMEM));           \
+    N_((k_adj_jobs<a, b, c, false>), (Shape<a, b, c>::SMEM));    \
+    N_((k_adj_run<a, b, c, true>), (Shape<a, b, c>::SMEM_EXACT));      \
+    N_((k_adj_jobs<a, b, c, true>), (Shape<a, b, c>::SMEM_EXACT));
     FKADJ_RUN_LIST(X)
 #undef X
+#undef N_
     return e;
 }
 
-template <class K, class... Args>
-static cudaError_t launch_run(K kernel, const RunShape& s, size_t smem, cudaStream_t st, Args&&... args) {
+template <class K, class Jobs>
+static cudaError_t launch_run(K kernel, int tiles, int threads, size_t smem, cudaStream_t st, const DevModel& P,
+                              const Jobs& jobs) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(s.ntx, s.nty);
-    cfg.blockDim = dim3(s.threads);
+    cfg.gridDim = dim3(tiles);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -1069,19 +1246,69 @@ static cudaError_t launch_run(K kernel, const RunShape& s, size_t smem, cudaStre
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, P, jobs);
 }
 
-cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const DevGrid& g, const double* gh,
-                           const uint8_t* cells, const FwdRun& r, cudaStream_t st) {
-    if (r.n <= 0) return cudaSuccess;
+template <class Job>
+static Job placed(const RunShape& s, Job j) {
+    j.ty = s.rows;
+    j.ntx = s.ntx;
+    j.tile0 = 0;
+    return j;
+}
+
+cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const FwdJob& j, cudaStream_t st) {
+    if (j.r.n <= 0) return cudaSuccess;
     switch (s.id) {
 #define X(id, a, b, c) \
-    case id: return launch_run(k_fwd_run<a, b, c>, s, Shape<a, b, c>::SMEM, st, P, g, gh, cells, r, s.rows);
+    case id: return launch_run(k_fwd_run<a, b, c>, s.tiles(), s.threads, Shape<a, b, c>::SMEM, st, P, placed(s, j));
         FKADJ_RUN_LIST(X)
 #undef X
     }
     return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_adj_run(const RunShape& s, bool exact, const DevModel& P, const AdjJob& j, cudaStream_t st) {
+    if (j.r.n <= 0) return cudaSuccess;
+    const AdjJob q = placed(s, j);
+    switch (s.id) {
+#define X(id, a, b, c)                                                                                                 \
+    case id:                                                                                                           \
+        return exact ? launch_run(k_adj_run<a, b, c, true>, s.tiles(), s.threads, Shape<a, b, c>::SMEM_EXACT, st, P, q) \
+                     : launch_run(k_adj_run<a, b, c, false>, s.tiles(), s.threads, Shape<a, b, c>::SMEM, st, P, q);
+        FKADJ_RUN_LIST(X)
+#undef X
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_fwd_jobs(const DevModel& P, const FwdJob* j, int n, int sms, cudaStream_t st, int64_t* launches) {
+    return run_packed(j, n, sms, [&](int id, const RunJobs<FwdJob>& jobs, int threads, int tiles) {
+        ++*launches;
+        switch (id) {
+#define X(id, a, b, c) \
+    case id: return launch_run(k_fwd_jobs<a, b, c>, tiles, threads, Shape<a, b, c>::SMEM, st, P, jobs);
+            FKADJ_RUN_LIST(X)
+#undef X
+        }
+        return cudaErrorInvalidValue;
+    });
+}
+
+cudaError_t launch_adj_jobs(bool exact, const DevModel& P, const AdjJob* j, int n, int sms, cudaStream_t st,
+                            int64_t* launches) {
+    return run_packed(j, n, sms, [&](int id, const RunJobs<AdjJob>& jobs, int threads, int tiles) {
+        ++*launches;
+        switch (id) {
+#define X(id, a, b, c)                                                                                           \
+    case id:                                                                                                     \
+        return exact ? launch_run(k_adj_jobs<a, b, c, true>, tiles, threads, Shape<a, b, c>::SMEM_EXACT, st, P, jobs) \
+                     : launch_run(k_adj_jobs<a, b, c, false>, tiles, threads, Shape<a, b, c>::SMEM, st, P, jobs);
+            FKADJ_RUN_LIST(X)
+#undef X
+        }
+        return cudaErrorInvalidValue;
+    });
 }
 
 // Rows per tile of the per-step tile kernels: the fewest waves of CTAs, then
@@ -1115,38 +1342,48 @@ cudaError_t launch_adj_tile(bool exact, const DevModel& P, const DevGrid& g, con
     return cudaGetLastError();
 }
 
-cudaError_t launch_mid_run(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,
-                           const HermiteW& hw, const MidRun& r, int sms, cudaStream_t st) {
-    if (r.n <= 0) return cudaSuccess;
+// Fills in where a midpoint job's tiles lie from tile0 on; returns its CTAs.
+// Runs of steps per CTA: the fewest evaluations (per steps cost 2 per + 1)
+// over whole waves of CTAs, one per SM.
+static int place_mid(MidJob& j, int tile0, int sms) {
     using S = MidShape;
-    const int ntx = (g.ncols + S::TX - 1) / S::TX, nty = (g.nrows + S::TY - 1) / S::TY, tiles = ntx * nty;
-    // runs of steps: the fewest evaluations (per steps cost 2 per + 1) over
-    // whole waves of CTAs, one per SM
-    int per = r.n;
+    j.ntx = (j.g.ncols + S::TX - 1) / S::TX;
+    j.nty = (j.g.nrows + S::TY - 1) / S::TY;
+    j.tile0 = tile0;
+    const int tiles = j.ntx * j.nty;
     long long best = -1;
-    for (int p = 1; p <= r.n; ++p) {
-        const long long ctas = (long long)tiles * ((r.n + p - 1) / p);
+    for (int p = 1; p <= j.r.n; ++p) {
+        const long long ctas = (long long)tiles * ((j.r.n + p - 1) / p);
         const long long cost = (ctas + sms - 1) / sms * (2 * p + 1);
-        if (best < 0 || cost <= best) best = cost, per = p;
+        if (best < 0 || cost <= best) best = cost, j.per = p;
     }
-    k_mid_run<<<dim3(ntx, nty, (r.n + per - 1) / per), S::THREADS, S::SMEM, st>>>(P, g, gh, cells, hw, r, per);
+    return tiles * ((j.r.n + j.per - 1) / j.per);
+}
+
+cudaError_t launch_mid_run(const DevModel& P, const HermiteW& hw, const MidJob& j, int sms, cudaStream_t st) {
+    if (j.r.n <= 0) return cudaSuccess;
+    MidJob q = j;
+    const int ctas = place_mid(q, 0, sms);
+    k_mid_run<<<ctas, MidShape::THREADS, MidShape::SMEM, st>>>(P, hw, q);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adj_run(const RunShape& s, bool exact, const DevModel& P, const DevGrid& g, const double* gh,
-                           const uint8_t* cells, const uint8_t* adj, const AdjRun& r, cudaStream_t st) {
-    if (r.n <= 0) return cudaSuccess;
-    switch (s.id) {
-#define X(id, a, b, c)                                                                                            \
-    case id:                                                                                                      \
-        return exact ? launch_run(k_adj_run<a, b, c, true>, s, Shape<a, b, c>::SMEM_EXACT, st, P, g, gh, cells, adj, \
-                                  r, s.rows)                                                                      \
-                     : launch_run(k_adj_run<a, b, c, false>, s, Shape<a, b, c>::SMEM, st, P, g, gh, cells, adj, r, \
-                                  s.rows);
-        FKADJ_RUN_LIST(X)
-#undef X
+cudaError_t launch_mid_jobs(const DevModel& P, const HermiteW& hw, const MidJob* j, int n, int sms, cudaStream_t st,
+                            int64_t* launches) {
+    for (int q0 = 0; q0 < n; q0 += kRunJobs) {
+        RunJobs<MidJob> jobs;
+        jobs.n = std::min(kRunJobs, n - q0);
+        int ctas = 0;
+        // each job as though it shared the device evenly with the others
+        for (int q = 0; q < jobs.n; ++q) {
+            jobs.job[q] = j[q0 + q];
+            ctas += place_mid(jobs.job[q], ctas, std::max(1, sms / jobs.n));
+        }
+        ++*launches;
+        k_mid_jobs<<<ctas, MidShape::THREADS, MidShape::SMEM, st>>>(P, hw, jobs);
+        if (const cudaError_t e = cudaGetLastError()) return e;
     }
-    return cudaErrorInvalidValue;
+    return cudaSuccess;
 }
 
 }  // namespace fkadj

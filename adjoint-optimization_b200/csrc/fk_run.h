@@ -36,24 +36,22 @@ cudaError_t run_init();
 size_t run_exchange_bytes(const DevGrid& g);
 
 // One forward sweep of n steps from state src.  The state after step k
-// (0-based) goes to `last` for k = n - 1, else to out + k * stride when out is
-// non-null.  None of them is src.
+// (0-based) goes to `last` for k = n - 1; of the others, when out is non-null,
+// those after `first` steps and every `every` more go to out, out + stride,
+// and so on.  None of them is src.
 struct FwdRun {
     const double* src;
     double* last;
     double* out;
     double* stages;         // stage states Y2, Y3, Y4 of step k to stages + (3 k + 0 .. 2) * stride (null: not kept)
     long long stride;
-    int n;
+    int n, first, every;
     const double *Et, *Eh;  // samples: step k takes Et[k], Eh[k], Et[k + 1]
     void* exchange;
     unsigned long long epoch;  // steps of all the sweeps before this one: the exchange's tags are never reset
     unsigned* fault;
 };
 constexpr unsigned FAULT_TIMEOUT = 1, FAULT_NAN = 2;
-
-cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const DevGrid& g, const double* gh,
-                           const uint8_t* cells, const FwdRun& r, cudaStream_t st);
 
 // One backward sweep of n steps from zin (z, resp. lambda, at the later end) to
 // zout, two distinct states.  Step k takes the state from the later end back:
@@ -78,6 +76,56 @@ struct AdjRun {
     unsigned long long epoch;
     unsigned* fault;
 };
+// Midpoint states of n backward steps (reference mode), step k's to yh + k *
+// stride; y_hi, y_mid, y_lo as in AdjRun.  Et, E3: the samples at the later end
+// of step 0 and of step 0's third; step k takes Et[-k], Et[-k - 1], E3[-k].
+struct MidRun {
+    const double *y_hi, *y_mid, *y_lo;
+    double* yh;
+    long long stride;
+    int n;
+    const double *Et, *E3;
+    unsigned* fault;
+};
+// The sweeps of one launch: a problem's grid and tables, its sweep, and where
+// its tiles lie (filled in by the launch functions).  Sweeps of several
+// problems of one model share a launch where their tiles fit the device
+// together; none waits for another's.
+struct FwdJob {
+    DevGrid g;
+    const double* gh;
+    const uint8_t* cells;
+    FwdRun r;
+    int ty, ntx, tile0;
+};
+struct AdjJob {
+    DevGrid g;
+    const double* gh;
+    const uint8_t *cells, *adj;
+    AdjRun r;
+    int ty, ntx, tile0;
+};
+struct MidJob {
+    DevGrid g;
+    const double* gh;
+    const uint8_t* cells;
+    MidRun r;
+    int per, ntx, nty, tile0;
+};
+
+// One problem's sweep, cut as s.
+cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const FwdJob& j, cudaStream_t st);
+cudaError_t launch_adj_run(const RunShape& s, bool exact, const DevModel& P, const AdjJob& j, cudaStream_t st);
+cudaError_t launch_mid_run(const DevModel& P, const HermiteW& hw, const MidJob& j, int sms, cudaStream_t st);
+
+// n problems' sweeps (each grid fits the device: run_shape), in as few
+// launches as their tiles need; adds those to *launches.
+cudaError_t launch_fwd_jobs(const DevModel& P, const FwdJob* j, int n, int sms, cudaStream_t st, int64_t* launches);
+cudaError_t launch_adj_jobs(bool exact, const DevModel& P, const AdjJob* j, int n, int sms, cudaStream_t st,
+                            int64_t* launches);
+cudaError_t launch_mid_jobs(const DevModel& P, const HermiteW& hw, const MidJob* j, int n, int sms, cudaStream_t st,
+                            int64_t* launches);
+
 // One forward step of a grid that does not fit the device at once: src -> dst
 // (null: not stored) and its stage states Y2, Y3, Y4 to three states in a row
 // (null: not kept).
@@ -103,21 +151,5 @@ struct AdjStep {
 };
 cudaError_t launch_adj_tile(bool exact, const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* adj,
                             const uint8_t* segs, const AdjStep& r, int sms, cudaStream_t st);
-
-// Midpoint states of n backward steps (reference mode), step k's to yh + k *
-// stride; y_hi, y_mid, y_lo as in AdjRun.  Et, E3: the samples at the later end
-// of step 0 and of step 0's third; step k takes Et[-k], Et[-k - 1], E3[-k].
-struct MidRun {
-    const double *y_hi, *y_mid, *y_lo;
-    double* yh;
-    long long stride;
-    int n;
-    const double *Et, *E3;
-    unsigned* fault;
-};
-cudaError_t launch_mid_run(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,
-                           const HermiteW& hw, const MidRun& r, int sms, cudaStream_t st);
-cudaError_t launch_adj_run(const RunShape& s, bool exact, const DevModel& P, const DevGrid& g, const double* gh,
-                           const uint8_t* cells, const uint8_t* adj, const AdjRun& r, cudaStream_t st);
 
 }  // namespace fkadj

@@ -236,7 +236,7 @@ fkadj_status Server::admit(Request& r) {
     const int policy = opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT;
     fkadj_status s = eng_->add_problem(r.p, r.dt, r.nt, r.ai.data(), r.nrows, r.ncols, r.n_num, r.gh.data(),
                                        r.gamma.data(), r.n_num, r.Jc.data(), r.Ir.data(), r.Sv.data(), r.alpha,
-                                       opt_.grad_mode, policy, budget_, &pid);
+                                       opt_.grad_mode, policy, budget_, &pid, r.sweeps);
     if (s) return s;
     int job = -1;
     s = eng_->submit(pid, r.Et.data(), r.y0.data(), r.want_grad, &job);
@@ -277,6 +277,8 @@ void Server::loop() {
             while (!queue_.empty() && (int)running_.size() < kBatchMaxItems) {
                 Request& r = *reqs_[queue_.front()];
                 if (used_ + r.est > budget_ && !running_.empty()) break;
+                r.sweeps = used_ + r.est_sweeps <= budget_;
+                if (r.sweeps) r.est = r.est_sweeps;
                 lk.unlock();
                 fkadj_status s = admit(r);
                 lk.lock();
