@@ -324,7 +324,9 @@ fkadj_status BatchEngine::host_action(Job& j, const Action& a) {
                     "z.gh");
                 ++launches_;
                 if (j.swept && (j.tp.policy == FKADJ_CKPT_SQRT || P.nt_ % P.pwin_ == 0)) {
-                    BCK(P.flush_range(0, P.nt_, 1), "reduce z.gh");
+                    SumList l;
+                    P.sum_range(l, P.nt_, 1);
+                    BCK(launch_sum_list(l, st_), "reduce z.gh");
                     ++launches_;
                 }
             }
@@ -767,13 +769,23 @@ fkadj_status BatchEngine::sweep_tick(const std::vector<int>& ready) {
              })))
             return s;
     // the chunks' rows of z.gh sums
+    SumList sums;
     for (const Back& b : back) {
         Problem& P = *probs_[b.j->prob];
-        const bool exact = P.grad_mode_ == FKADJ_GRAD_EXACT, sqrt_store = b.j->tp.policy == FKADJ_CKPT_SQRT;
+        const bool sqrt_store = b.j->tp.policy == FKADJ_CKPT_SQRT;
         const int row = b.top - b.n;
         if (!sqrt_store && (row % P.pwin_ != 0 || P.run_.id < 0)) continue;
-        for (int g = 0; g < (exact ? 3 : 1); ++g, ++launches_)
-            BCK(sqrt_store ? P.flush_range(g, row, b.n) : P.flush_rows(g, row, exact ? P.nt_ : P.nt_ + 1), "reduce z.gh");
+        if (sums.n + 3 > SumList::kMax) {
+            BCK(launch_sum_list(sums, st_), "reduce z.gh");
+            sums = SumList();
+            ++launches_;
+        }
+        if (sqrt_store) P.sum_range(sums, row, b.n);
+        else P.sum_window(sums, row);
+    }
+    if (sums.n) {
+        BCK(launch_sum_list(sums, st_), "reduce z.gh");
+        ++launches_;
     }
     ++ticks_;
     return FKADJ_OK;

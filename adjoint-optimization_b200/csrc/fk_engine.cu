@@ -1016,7 +1016,7 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
         top -= n;
         // as in the per-step sweeps: a sqrt store reduces at the end of each segment
         if (traj_plan_.policy != FKADJ_CKPT_SQRT && top % pwin_ == 0)
-            for (int g = 0; g < (exact ? 3 : 1); ++g) CK(flush_rows(g, top, exact ? nt_ : nt_ + 1), "reduce z.gh");
+            CK(flush_rows(top), "reduce z.gh");
     }
     return FKADJ_OK;
 }
@@ -1688,7 +1688,7 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
         // rows t .. t+pwin-1 of the three groups are complete (a sqrt store
         // reduces at the end of each segment instead)
         if (tp.policy != FKADJ_CKPT_SQRT && t % pwin_ == 0)
-            for (int g = 0; g < 3; ++g) CK(flush_rows(g, t, nt), "reduce z.gh");
+            CK(flush_rows(t), "reduce z.gh");
         return FKADJ_OK;
     };
     const bool sweep = sweeping();
@@ -1724,26 +1724,35 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
         }
         for (int t = s1 - 1; t >= s0 && !sweep; --t)
             if ((s = back(t, st(t)))) return s;
-        for (int g = 0; g < 3; ++g) CK(flush_range(g, s0, s1 - s0), "reduce z.gh");
+        CK(flush_range(s0, s1 - s0), "reduce z.gh");
         if ((s = segment_launch())) return s;
     }
     return FKADJ_OK;
 }
 
-cudaError_t Problem::flush_rows(int g, int row, int rows_g) {
-    ++launches_;
-    const int n = std::min(pwin_, rows_g - row);
-    return launch_sum_rows(partial_.as<double>() + (size_t)g * pwin_ * nsb_, n, nsb_,
-                           zgh_.as<double>() + (size_t)g * nt_ + row, st_);
+void Problem::sum_window(SumList& l, int row) const {
+    const int n = std::min(pwin_, (groups() == 3 ? nt_ : nt_ + 1) - row);
+    for (int g = 0; g < groups(); ++g)
+        l.add(partial_.as<double>() + (size_t)g * pwin_ * nsb_, n, nsb_, zgh_.as<double>() + (size_t)g * nt_ + row);
 }
 
-// Reduces rows row0 .. row0+n-1 of group g into zgh; they must not wrap around
-// the window (a sqrt segment's rows, with the window a whole number of
-// segments).
-cudaError_t Problem::flush_range(int g, int row0, int n) {
+void Problem::sum_range(SumList& l, int row0, int n) const {
+    for (int g = 0; g < groups(); ++g)
+        l.add(prow(g, row0), n, nsb_, zgh_.as<double>() + (size_t)g * nt_ + row0);
+}
+
+cudaError_t Problem::flush_rows(int row) {
     ++launches_;
-    return launch_sum_rows(partial_.as<double>() + ((size_t)g * pwin_ + (size_t)(row0 % pwin_)) * nsb_, n, nsb_,
-                           zgh_.as<double>() + (size_t)g * nt_ + row0, st_);
+    SumList l;
+    sum_window(l, row);
+    return launch_sum_list(l, st_);
+}
+
+cudaError_t Problem::flush_range(int row0, int n) {
+    ++launches_;
+    SumList l;
+    sum_range(l, row0, n);
+    return launch_sum_list(l, st_);
 }
 
 fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_out) {
@@ -1797,8 +1806,8 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
         CK(launch_scatter(g_, zc_.as<double>(), n_num_, pos_.as<long long>(), 1.0, z, st_), "scatter z");
         CK(launch_dot_gh(g_, z, gh_.as<double>(), prow(0, nt), nsbx_, nsby_, st_, segs_), "z.gh");
         launches_ += 2;
-        if (tp.policy == FKADJ_CKPT_SQRT) CK(flush_range(0, nt, 1), "reduce z.gh");
-        else if (nt % pwin_ == 0) CK(flush_rows(0, nt, nt + 1), "reduce z.gh");
+        if (tp.policy == FKADJ_CKPT_SQRT) CK(flush_range(nt, 1), "reduce z.gh");
+        else if (nt % pwin_ == 0) CK(flush_rows(nt), "reduce z.gh");
     }
     // ---- backward sweep (cu-G:1866-1908)
     // Work carried from backward step i to step i-1 (computed once, same
@@ -1831,7 +1840,7 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
                "fused adjoint step");
             CK(prof_end(K_ADJ), "profiling event");
             launches_ += 1;
-            if (!seg_rows && (i - 1) % pwin_ == 0) CK(flush_rows(0, i - 1, nt + 1), "reduce z.gh");
+            if (!seg_rows && (i - 1) % pwin_ == 0) CK(flush_rows(i - 1), "reduce z.gh");
             std::swap(z, z2);
             cur_c = nxt;
             have_fcarry = fa == nullptr;
@@ -1856,7 +1865,7 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
            "adjoint step");
         CK(prof_end(K_ADJ), "profiling event");
         launches_ += 2;
-        if (!seg_rows && (i - 1) % pwin_ == 0) CK(flush_rows(0, i - 1, nt + 1), "reduce z.gh");
+        if (!seg_rows && (i - 1) % pwin_ == 0) CK(flush_rows(i - 1), "reduce z.gh");
         std::swap(z, z2);
         cur_c = nxt;
         have_fcarry = fa == nullptr;
@@ -1912,7 +1921,7 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
             }
             for (int i = s1; i > s0 && !sweep; --i)
                 if ((s = back_step(i, st(i - 1), st(i), kept(i - 1), kept(i)))) return s;
-            CK(flush_range(0, s0, s1 - s0), "reduce z.gh");  // rows s0 .. s1-1
+            CK(flush_range(s0, s1 - s0), "reduce z.gh");  // rows s0 .. s1-1
             if ((s = segment_launch())) return s;
         }
     }

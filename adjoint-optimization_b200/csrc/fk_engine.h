@@ -237,9 +237,15 @@ private:
     double* prow(int g, int row) const {
         return partial_.as<double>() + ((size_t)g * pwin_ + (size_t)(row % pwin_)) * nsb_;
     }
-    // reduces the rows row .. row+pwin-1 (clipped to rows_g) of group g into zgh
-    cudaError_t flush_rows(int g, int row, int rows_g);
-    cudaError_t flush_range(int g, int row0, int n);
+    int groups() const { return grad_mode_ == FKADJ_GRAD_EXACT ? 3 : 1; }
+    // Adds to l, per group of partial sums, the reduction into zgh of the
+    // window of rows from `row` on (clipped to the group's rows), or of rows
+    // row0 .. row0+n-1; the latter must not wrap around the window (a sqrt
+    // segment's rows, with the window a whole number of segments).
+    void sum_window(SumList& l, int row) const;
+    void sum_range(SumList& l, int row0, int n) const;
+    cudaError_t flush_rows(int row);
+    cudaError_t flush_range(int row0, int n);
     static constexpr int kPartialWindow = 512;
     fkadj_status download_grid(const double* d_state, double* host_dense);
     double* slot(int k) const { return traj_.as<double>() + (size_t)k * state_elems(); }

@@ -170,6 +170,22 @@ cudaError_t launch_adj_fused(int tile, const DevModel& P, const DevGrid& g, cons
 cudaError_t launch_dot_gh(const DevGrid& g, const double* z, const double* gh, double* row, int nsbx, int nsby,
                           cudaStream_t st, bool segments = false);
 cudaError_t launch_sum_rows(const double* partial, int rows, int ntiles, double* out, cudaStream_t st);
+// Several such blocks of rows in one launch.
+struct SumList {
+    static constexpr int kMax = 16;
+    struct Block {
+        const double* partial;
+        double* out;
+        int ntiles, row0;  // row0: rows of the blocks before it
+    };
+    int n = 0, rows = 0;
+    Block block[kMax];
+    void add(const double* partial, int nrows, int ntiles, double* out) {
+        block[n++] = {partial, out, ntiles, rows};
+        rows += nrows;
+    }
+};
+cudaError_t launch_sum_list(const SumList& l, cudaStream_t st);
 cudaError_t launch_scatter(const DevGrid& g, const double* yc, int n_num, const long long* pos, double scale,
                            double* y, cudaStream_t st);
 cudaError_t launch_gather(const DevGrid& g, const double* y, int n_num, const long long* pos, double* yc,

@@ -1342,28 +1342,38 @@ cudaError_t launch_adj_tile(bool exact, const DevModel& P, const DevGrid& g, con
     return cudaGetLastError();
 }
 
-// Fills in where a midpoint job's tiles lie from tile0 on; returns its CTAs.
-// Runs of steps per CTA: the fewest evaluations (per steps cost 2 per + 1)
-// over whole waves of CTAs, one per SM.
-static int place_mid(MidJob& j, int tile0, int sms) {
+// Fills in where n midpoint jobs' tiles lie, one after the other; returns
+// their CTAs.  Runs of steps per CTA: the fewest evaluations (per steps cost 2
+// per + 1) over whole waves of CTAs, one per SM.
+static int place_mid(MidJob* j, int n, int sms) {
     using S = MidShape;
-    j.ntx = (j.g.ncols + S::TX - 1) / S::TX;
-    j.nty = (j.g.nrows + S::TY - 1) / S::TY;
-    j.tile0 = tile0;
-    const int tiles = j.ntx * j.nty;
-    long long best = -1;
-    for (int p = 1; p <= j.r.n; ++p) {
-        const long long ctas = (long long)tiles * ((j.r.n + p - 1) / p);
-        const long long cost = (ctas + sms - 1) / sms * (2 * p + 1);
-        if (best < 0 || cost <= best) best = cost, j.per = p;
+    int most = 1, per = 1;
+    for (int q = 0; q < n; ++q) {
+        j[q].ntx = (j[q].g.ncols + S::TX - 1) / S::TX;
+        j[q].nty = (j[q].g.nrows + S::TY - 1) / S::TY;
+        most = std::max(most, j[q].r.n);
     }
-    return tiles * ((j.r.n + j.per - 1) / j.per);
+    auto ctas = [&](int q, int p) { return j[q].ntx * j[q].nty * ((j[q].r.n + p - 1) / p); };
+    long long best = -1;
+    for (int p = 1; p <= most; ++p) {
+        long long c = 0;
+        for (int q = 0; q < n; ++q) c += ctas(q, p);
+        const long long cost = (c + sms - 1) / sms * (2 * p + 1);
+        if (best < 0 || cost <= best) best = cost, per = p;
+    }
+    int tile0 = 0;
+    for (int q = 0; q < n; ++q) {
+        j[q].per = per;
+        j[q].tile0 = tile0;
+        tile0 += ctas(q, per);
+    }
+    return tile0;
 }
 
 cudaError_t launch_mid_run(const DevModel& P, const HermiteW& hw, const MidJob& j, int sms, cudaStream_t st) {
     if (j.r.n <= 0) return cudaSuccess;
     MidJob q = j;
-    const int ctas = place_mid(q, 0, sms);
+    const int ctas = place_mid(&q, 1, sms);
     k_mid_run<<<ctas, MidShape::THREADS, MidShape::SMEM, st>>>(P, hw, q);
     return cudaGetLastError();
 }
@@ -1373,12 +1383,8 @@ cudaError_t launch_mid_jobs(const DevModel& P, const HermiteW& hw, const MidJob*
     for (int q0 = 0; q0 < n; q0 += kRunJobs) {
         RunJobs<MidJob> jobs;
         jobs.n = std::min(kRunJobs, n - q0);
-        int ctas = 0;
-        // each job as though it shared the device evenly with the others
-        for (int q = 0; q < jobs.n; ++q) {
-            jobs.job[q] = j[q0 + q];
-            ctas += place_mid(jobs.job[q], ctas, std::max(1, sms / jobs.n));
-        }
+        std::copy(j + q0, j + q0 + jobs.n, jobs.job);
+        const int ctas = place_mid(jobs.job, jobs.n, sms);
         ++*launches;
         k_mid_jobs<<<ctas, MidShape::THREADS, MidShape::SMEM, st>>>(P, hw, jobs);
         if (const cudaError_t e = cudaGetLastError()) return e;
