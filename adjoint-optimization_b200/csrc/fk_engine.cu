@@ -974,7 +974,7 @@ Problem::AdjointChunk Problem::adjoint_chunk(int top, int hi, int lo, const doub
 }
 
 fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
-                                    const double* stages, double*& z, double*& z2) {
+                                    const double* stages, double*& z, double*& z2, double* replayed) {
     const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
     const long long sz = (long long)state_elems();
     auto state = [&](int t) { return t == hi ? y_hi : (t == lo ? y_lo : mid + (t - lo - 1) * sz); };
@@ -984,7 +984,7 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
         const int n = c.n;
         if (c.replay) {
             // from the chunk's lowest state up, every step's stages
-            if (fkadj_status s = sweep_forward(top - n, n, state(top - n), state_buf(1), nullptr, pts_.as<double>()))
+            if (fkadj_status s = sweep_forward(top - n, n, state(top - n), state_buf(1), replayed, pts_.as<double>()))
                 return s;
         } else if (!exact) {
             CK(prof_begin(K_MID, n), "profiling event");
@@ -1622,9 +1622,15 @@ int64_t binomial_recompute_steps(int nt, int free_slots) {
 // checkpoint.  The walk of a part [a, b) with checkpoint m is: advance y_a to
 // y_m into a free slot, reverse [m, b), give the slot back, reverse [a, m).  It
 // runs from an explicit stack: with many slots the chain of right parts is as
-// long as the horizon.
+// long as the horizon.  visit(j, n, y_j, y_j+1) takes steps j + n - 1 .. j: one
+// (y_j+1 null), or a swept problem's part of two, y_j+1 null where it is not
+// stored.  The pair's replay in the exact mode is one forward sweep, which
+// gives y_j+1 on the way (three steps before, the advance to it among them),
+// and its backward steps share their launch.
 fkadj_status Problem::reverse_binomial(int nt, double* y0, std::vector<double*>& free,
-                                       const std::function<fkadj_status(int, const double*)>& visit) {
+                                       const std::function<fkadj_status(int, int, const double*, const double*)>&
+                                           visit) {
+    const bool pairs = sweeping();
     struct Task {
         enum { REVERSE, RETURN_SLOT } kind;
         int a, b;
@@ -1641,17 +1647,20 @@ fkadj_status Problem::reverse_binomial(int nt, double* y0, std::vector<double*>&
             continue;
         }
         const int a = k.a, b = k.b;
-        if (b - a == 1) {
-            if ((s = visit(a, k.ya))) return s;
+        if (b - a == 1 || (pairs && b - a == 2)) {
+            // (the spine's y_{a+1} lies in the slot this walk would take for it)
+            const double* y1 = b - a == 2 && k.spine && !free.empty() ? free.back() : nullptr;
+            if ((s = visit(a, b - a, k.ya, y1))) return s;
             continue;
         }
         if (free.empty()) {  // no snapshot left: replay from y_a for every state
             double* scr = segslot(0);
-            for (int j = b - 1; j > a; --j) {
-                if ((s = advance(a, j, k.ya, scr))) return s;
-                if ((s = visit(j, scr))) return s;
+            for (int j = b; j > a;) {
+                const int n = pairs && j - a > 1 ? 2 : 1;
+                j -= n;
+                if (j > a && (s = advance(a, j, k.ya, scr))) return s;
+                if ((s = visit(j, n, j > a ? scr : k.ya, nullptr))) return s;
             }
-            if ((s = visit(a, k.ya))) return s;
             continue;
         }
         const int m = binomial_split(a, b, (int)free.size());
@@ -1702,8 +1711,13 @@ fkadj_status Problem::grad_exact_backward(const TrajPlan& tp, double* lam, doubl
     if (tp.policy == FKADJ_CKPT_BINOMIAL) {
         std::vector<double*> free;
         for (int k = tp.nslots - 1; k >= 2; --k) free.push_back(slot(k));
-        return reverse_binomial(nt, slot(0), free, [&](int t, const double* y) {
-            return sweep ? sweep_adjoint(t + 1, t, y, nullptr, y, nullptr, lam, lam2) : back(t, y);
+        return reverse_binomial(nt, slot(0), free, [&](int t, int n, const double* y, const double* y1) {
+            if (!sweep) return back(t, y);
+            double* mid = y1 || n == 1 ? nullptr : state_buf(2);
+            // (rows t + 1 and t of the partial sums in different windows: two chunks, the first from y1)
+            if (mid && (t + 1) % pwin_ == 0)
+                if (fkadj_status e = advance(t, t + 1, y, mid)) return e;
+            return sweep_adjoint(t + n, t, y, y1 ? y1 : mid, y, nullptr, lam, lam2, mid);
         });
     }
     for (int k = K - 1; k >= 0; --k) {
@@ -1883,9 +1897,14 @@ fkadj_status Problem::grad_sequence(const TrajPlan& tp, bool exact, double** yT_
         for (int k = tp.nslots - 1; k >= 2; --k) free.push_back(slot(k));
         const double* prev = slot(1);  // y(T)
         double* keep = state_buf(0);
-        auto visit = [&](int j, const double* yj) -> fkadj_status {
-            fkadj_status r = sweep ? sweep_adjoint(j + 1, j, prev, nullptr, yj, nullptr, z, z2)
-                                   : back_step(j + 1, yj, prev, nullptr, nullptr);
+        auto visit = [&](int j, int n, const double* yj, const double* y1) -> fkadj_status {
+            fkadj_status r = FKADJ_OK;
+            if (n == 2 && !y1) {
+                if ((r = advance(j, j + 1, yj, state_buf(2)))) return r;
+                y1 = state_buf(2);
+            }
+            r = sweep ? sweep_adjoint(j + n, j, prev, y1, yj, nullptr, z, z2)
+                      : back_step(j + 1, yj, prev, nullptr, nullptr);
             if (r) return r;
             CK(cudaMemcpyAsync(keep, yj, state_bytes(), cudaMemcpyDeviceToDevice, st_), "keep state");
             prev = keep;

@@ -191,9 +191,10 @@ public:
     // Backward steps hi .. lo + 1 of a swept problem, z -> z (the pair is
     // swapped as it goes): y_hi, y_lo the states at both ends, mid the states
     // lo + 1 .. hi - 1 in a row, stages (exact mode; null: replayed) the stage
-    // states of steps lo .. hi - 1 in a row.
+    // states of steps lo .. hi - 1 in a row.  replayed: where a replay leaves
+    // the states between (mid, where they are not there yet).
     fkadj_status sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
-                               const double* stages, double*& z, double*& z2);
+                               const double* stages, double*& z, double*& z2, double* replayed = nullptr);
     fkadj_status init_sweeps(const uint8_t* cells, const uint8_t* adj, const uint8_t* seg);
     // whether this problem's steps are sweeps (fk_run.h): one launch each where
     // run_.id >= 0, the tile kernels otherwise
@@ -228,7 +229,7 @@ private:
     fkadj_status grad_exact_backward(const TrajPlan& tp, double* lam, double* lam2);
     fkadj_status advance(int a, int m, const double* src, double* dst);
     fkadj_status reverse_binomial(int nt, double* y0, std::vector<double*>& free,
-                                  const std::function<fkadj_status(int, const double*)>& visit);
+                                  const std::function<fkadj_status(int, int, const double*, const double*)>& visit);
     // all_rows: keep the z.gh partials of every step (the batch engine);
     // otherwise a window of kPartialWindow rows reduced as the sweep goes.
     fkadj_status ensure_adjoint_work(bool all_rows = false);

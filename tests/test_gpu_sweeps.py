@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from fkadj import _lib, api, workloads as W
+from fkadj.batch import Batch
 from test_gpu_edges import _custom
 
 pytestmark = pytest.mark.gpu
@@ -138,3 +139,62 @@ def test_nan_input_stays_where_single_steps_keep_it(monkeypatch, field):
     y0[field * inst.n_num + inst.n_num // 2] = np.nan
     (_, yf0), (_, yf1) = _both(monkeypatch, lambda: _forward(inst, 0, y0=y0))
     _same(yf0, yf1)
+
+
+@pytest.mark.parametrize("mode", [_lib.GRAD_REF, _lib.GRAD_EXACT])
+def test_pairs_of_the_binomial_store_on_a_grid_of_several_waves(mode):
+    inst = W.make_instance(600, 9, ncols=700, seed=9, n_obstacles=100, intervals=3)
+    sb = 3 * 8 * (640 + 8) * (704 + 8)
+
+    def call(pol, b):
+        with api.Problem(inst, opts=api.options(grad_mode=mode, ckpt_policy=pol, ckpt_budget_bytes=b)) as pb:
+            return pb.grad(inst.Et, inst.y0)["gradE"]
+    full = call(_lib.CKPT_FULL, 0)
+    for states in (3, 4, 6):
+        assert np.array_equal(call(_lib.CKPT_BINOMIAL, states * sb), full), states
+
+
+@pytest.mark.parametrize("store", [_lib.CKPT_FULL, _lib.CKPT_SQRT])
+@pytest.mark.parametrize("mode", [_lib.GRAD_REF, _lib.GRAD_EXACT])
+def test_batched_sweeps_give_the_bits_of_single_problems(mode, store):
+    """More problems than one launch takes, of two models, from one tile to the
+    whole device and beyond; among them one without a gradient, one with cells
+    between two holes (these fall, and the objective with them) and one with a
+    NaN among its inputs."""
+    sizes = [(5, 7), (16, 16), (300, 40), (40, 610), (131, 97), (512, 512), (600, 700), (256, 256), (64, 200)] + \
+        [(48 + k, 64 + 3 * k) for k in range(12)]
+    insts = [W.make_instance(r, 7 + 5 * (k % 9), ncols=c, dt=0.02 if k % 3 else 0.01, seed=k, intervals=4,
+                             n_obstacles=max(1, r * c // 2500), alpha=0.1,
+                             r_range=(0.02, 0.1) if min(r, c) > 30 else (0.01, 0.02))
+             for k, (r, c) in enumerate(sizes)]
+    mask = np.ones((70, 90), bool)
+    mask[10, 10] = mask[12, 10] = False
+    insts.append(_custom(mask, 30))
+    bad = np.array(insts[4].y0)
+    bad[insts[4].n_num // 2] = np.nan
+    opts = api.options(grad_mode=mode, ckpt_policy=store)
+
+    def single(x):
+        with api.Problem(x, opts=opts) as pb:
+            return pb.grad(x.Et, x.y0)
+    want = [single(x) for x in insts[:-1]]
+    with pytest.raises(_lib.FkadjError) as fallen:
+        single(insts[-1])
+    with Batch() as b:
+        ids = [b.add_problem(x, grad_mode=mode, ckpt_policy=store) for x in insts]
+        for repeat in range(2):
+            jobs = [b.submit(p, x.Et, bad if k == 4 and repeat == 0 else x.y0, want_grad=k != 2)
+                    for k, (p, x) in enumerate(zip(ids, insts))]
+            b.run()
+            with pytest.raises(_lib.FkadjError) as e:
+                b.result(jobs[-1])
+            assert e.value.status == fallen.value.status
+            for k, (j, w) in enumerate(zip(jobs, want)):
+                if k == 4 and repeat == 0:
+                    with pytest.raises(_lib.FkadjError):
+                        b.result(j)
+                    continue
+                r = b.result(j)
+                assert r["Lcost"] == w["Lcost"], (k, repeat)
+                if k != 2:
+                    assert np.array_equal(r["gradE"], w["gradE"]), (k, repeat)
