@@ -40,13 +40,24 @@ namespace {
 
 // Kernel instances (id, TX, R, TYM): tiles of TX columns and up to TYM rows;
 // TYM + 6 is a multiple of R (the first stage's region, TYM + 6 rows of it).
+// A grid takes the one of least cost among those whose tiles fit the device
+// (ShapeInfo::cost), and so do a batch's launches.  Forward and backward us a
+// step with each (a dash: does not fit):
+//             64x5x29    64x3x15   32x3x30   32x2x18   16x2x34   16x1x14
+//   128x128   6.6 13.3   5.2 8.0   4.5 7.5   3.7 6.5   3.9 6.5   3.2 5.0
+//   256x256   7.7 15.2   5.9 9.4   5.7 9.5   5.6 9.0   5.9 9.4      -
+//   320x320   8.4 16.9   7.1 10.9  6.9 11.0     -         -         -
+//   437x501  11.0 19.1      -         -         -         -         -
+// and between the last two 64x4x22: 384x384 8.9 16.9 -> 8.2 14.0.
 #define FKADJ_RUN_LIST(X) \
     X(0, 64, 5, 29)       \
     X(1, 64, 3, 15)       \
     X(2, 32, 3, 30)       \
     X(3, 32, 2, 18)       \
     X(4, 16, 2, 34)       \
-    X(5, 16, 1, 14)
+    X(5, 16, 1, 14)       \
+    X(6, 64, 4, 22)       \
+    X(7, 32, 4, 42)
 
 template <int TX_, int R_, int TYM_>
 struct Shape {
@@ -1072,15 +1083,15 @@ __global__ void __launch_bounds__(MidShape::THREADS, 1)
 #define X(id, a, b, c) \
     case id: { using S = Shape<a, b, c>; DO(S); } break;
 
-constexpr int kRunShapes = 6;
+constexpr int kRunShapes = 8;
 struct ShapeInfo {
     int tx, R, tym, rw, threads;
     // a step's cost on tiles of `rows` rows: per stage, the evaluations (a
     // warp's row, by FP64 issue) or the depth of a thread's column, whichever
-    // is longer
+    // is longer, and something for the depth in any case
     double cost(int rows) const {
         double c = 0;
-        for (int e = 3; e >= 0; --e) c += std::max((double)rw * (rows + 2 * e) / 32.0 * 62.0, R * 420.0);
+        for (int e = 3; e >= 0; --e) c += std::max((double)rw * (rows + 2 * e) / 32.0 * 62.0, R * 420.0) + R * 40.0;
         return c;
     }
     int threads_for(int rows) const { return std::min(threads, (rw * ((rows + 6 + R - 1) / R) + 31) / 32 * 32); }
