@@ -2300,12 +2300,7 @@ void fkadj_problem_tiles(const fkadj_problem* pb, int out[4], int shapes[12]) {
     if (!pb || !out) return;
     for (int k = 0; k < 4; ++k) {
         out[k] = pb->impl.tile(k);
-        if (shapes) {
-            const fkadj::TileShape t = fkadj::tile_shape(out[k]);
-            shapes[3 * k] = t.tx;
-            shapes[3 * k + 1] = pb->impl.tile_rows(k);
-            shapes[3 * k + 2] = t.nt;
-        }
+        if (shapes) pb->impl.launched_tile(k, shapes + 3 * k);
     }
 }
 

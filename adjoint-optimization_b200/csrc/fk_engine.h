@@ -151,6 +151,12 @@ public:
     int tile_rows(int kind) const {
         return ty_[kind] > 0 && (kind != T_ADJ || segs_) ? ty_[kind] : tile_shape(tk_[kind]).ty;
     }
+    // columns, rows and threads of a kind's tiles as launched
+    void launched_tile(int kind, int tile[3]) const {
+        if (sweeping()) return run_tile(g_, run_, sms_, kind == T_MID, tile);
+        const TileShape t = tile_shape(tk_[kind]);
+        tile[0] = t.tx, tile[1] = tile_rows(kind), tile[2] = t.nt;
+    }
     // Times every tile preset of every kernel kind on the current initial
     // state (a few launches each) and keeps the fastest per kind.  Results do
     // not depend on the choice (fixed-order reductions).

@@ -1336,6 +1336,14 @@ static TileWalk tile_walk(const DevGrid& g, int sms) {
     return w;
 }
 
+void run_tile(const DevGrid& g, const RunShape& s, int sms, bool midpoint, int tile[3]) {
+    const int mid[3] = {MidShape::TX, MidShape::TY, MidShape::THREADS};
+    const int run[3] = {s.tx, s.rows, s.threads};
+    const int big[3] = {TileShapeBig::TX, tile_walk(g, sms).ty, TileShapeBig::THREADS};
+    const int* t = midpoint ? mid : (s.id >= 0 ? run : big);
+    std::copy(t, t + 3, tile);
+}
+
 cudaError_t launch_fwd_tile(const DevModel& P, const DevGrid& g, const double* gh, const uint8_t* cells,
                             const FwdStep& r, int sms, cudaStream_t st) {
     using S = TileShapeBig;

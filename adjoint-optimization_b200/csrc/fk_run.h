@@ -28,6 +28,10 @@ struct RunShape {
     int tiles() const { return ntx * nty; }
 };
 
+// Tiles of a swept grid's launches: columns, rows, threads of a sweep (s.id >=
+// 0) or of the tile kernels, or of the midpoint kernel.
+void run_tile(const DevGrid& g, const RunShape& s, int sms, bool midpoint, int tile[3]);
+
 // The shape for grid g on a device with `sms` multiprocessors (id -1: none).
 RunShape run_shape(const DevGrid& g, int sms);
 cudaError_t run_init();

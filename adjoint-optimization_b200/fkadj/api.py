@@ -212,7 +212,7 @@ class Problem:
         return {n: (shp[3 * k], shp[3 * k + 1], shp[3 * k + 2]) for k, n in enumerate(names)}
 
     def kernel_time(self, kernel: int):
-        """(average ms per launch, samples) of kernel 0 forward step,
+        """(average ms per step, steps timed) of kernel 0 forward step,
         1 adjoint midpoint, 2 adjoint step, over the last call."""
         ms, n = C.c_double(), C.c_int64()
         self._L.fkadj_problem_kernel_time(self._h, int(kernel), C.byref(ms), C.byref(n))

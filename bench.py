@@ -45,39 +45,27 @@ for _p in (PKG, os.path.join(ROOT, "oracle")):
 METRIC = "fwd+adjoint gradients/s at 512^2"
 UNIT = "gradients/s"
 
-# bytes per dense cell per launch the kernels move as designed (one RK4 step)
-BYTES_PER_CELL = {0: 56.0,    # forward step: read y (24) + gh (8), write y (24)
-                  1: 160.0,   # adjoint midpoint: read y_{i-1}, y_i (48) + f(y_{i-1}), f(y_i) (48) + gh (8),
-                              #   write J(yh) (56; yh itself is not stored while the J(yh) cache is read)
-                  2: 249.0}   # adjoint step: read z (24) + J(y_i), J(yh) (112) + y_{i-1} (24) + gh (8)
-                              #   + weight code (1), write z (24) + J(y_{i-1}) (56)
-# DRAM bytes per cell of one k_fwd_step launch measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum, caches flushed before the launch) at 512x512.  The reads
-# (33 B/cell: y 24 + gh 8 + halo) reach DRAM; the 24 B/cell of writes stay in the
-# 126 MB L2.
-FWD_TRAFFIC_PER_CELL = 8654848 / 262144
-KERNEL_NAMES = {0: "k_fwd_step", 1: "k_adj_mid", 2: "k_adj_step"}
-# fused reference-adjoint step (midpoint + four stages in one launch): read z, y_{i-1}, y_i (72) + kept f(y_{i-1}),
-# f(y_i) (48) + gh (8) + weight and stencil codes (2), write z (24); with the J_F(y)^T cache also read J(y_i) and
-# write J(y_{i-1}) (56 each)
-FUSED_BYTES_PER_CELL = {"fused": 266.0, "fused-recompute": 154.0}
-# discrete-exact adjoint step (--mode exact): read lambda (24), y (24), the three stage states (72), gh (8),
-# weight code (1); write lambda (24)
-EXACT_BYTES_PER_CELL = 153.0
-# FP64 flops per vector-field evaluation of the forward step (stage update included), counted by ncu
-# (2 x DFMA + DMUL + DADD thread instructions) at 512x512: 585.1 per cell on 64x29 tiles of the
-# 64x32/640 preset, whose launch makes 1216384 evaluations (fwd_evaluations)
-FWD_FLOPS_PER_EVAL = 585.1 * 262144 / 1216384
-# the same capture's FP64 pipe activity (sm__pipe_fp64_cycles_active, % of active cycles) and launch duration:
-# DMUL, DADD and compare instructions occupy the pipe as a DFMA does, so the pipe is busier than the flop rate
-# says; scaled to the live launch time it estimates the pipe's activity in the replayed graph
-FWD_FP64_PIPE_NCU = (0.400, 0.019936)  # (fraction, ms of the serialised launch)
+# bytes per dense cell and step the sweeps move through global memory as designed; the tiles stay in shared memory
+# from step to step, their edges' exchange stays in L2
+BYTES_PER_CELL = {0: 24.0,    # forward sweep: write y where it is stored (the recompute of a segment: every step)
+                  1: 48.0,    # midpoints: read y_{i-1} (24; y_i is the step before's), write yh (24)
+                  2: 48.0}    # adjoint sweep: read yh and y_{i-1} (48; y_i is the step before's)
+KERNEL_NAMES = {0: "k_fwd_run", 1: "k_mid_run", 2: "k_adj_run"}
+# discrete-exact sweeps (--mode exact): the recompute writes the three stage states too, the adjoint sweep reads
+# them and y
+EXACT_BYTES_PER_CELL = 96.0
+# DRAM bytes per cell and step of k_fwd_run (a recompute that stores every state) measured by ncu
+# (dram__bytes_read.sum + dram__bytes_write.sum) at 512x512
+FWD_TRAFFIC_PER_CELL = (9973504 + 160473344) / (33 * 262144)
+# FP64 flops per vector-field evaluation of the forward sweep (stage update included), counted by ncu
+# (2 x DFMA + DMUL + DADD thread instructions) at 512x512
+FWD_FLOPS_PER_EVAL = (2 * 1786145856 + 683922624 + 788625024) / (33 * 1216384)
 
 
 def fwd_evaluations(nrows, ncols, tx, ty):
-    """Vector-field evaluations of one forward-step launch: stage s of a tile
-    runs on the tile grown by 4 - s cells (temporal blocking); bottom-row tiles
-    stop at the grid's edge."""
+    """Vector-field evaluations of one forward step: stage s of a tile runs on
+    the tile grown by 4 - s cells (temporal blocking); bottom-row tiles stop at
+    the grid's edge."""
     n = 0
     for i0 in range(0, nrows, ty):
         rows = min(ty, nrows - i0)
@@ -326,8 +314,7 @@ def run_ours(args):
     barrier()
     ms = gmax(ev0.elapsed_time(ev1))
     value = replica_value(world, args.steps, ms)
-    # the last timed gradient's forward sweep: CUDA events on the engine stream around its nt back-to-back
-    # k_fwd_step launches (recorded inside the replayed graph)
+    # the last timed gradient's forward sweep: CUDA events on the engine stream around its launches
     fwd_sweep_ms = pb.last_timing["fwd_ms"]
 
     # roofline: sampled per-kernel device times in one more gradient
@@ -340,24 +327,19 @@ def run_ours(args):
         # forward sweep + recompute + one stage replay per backward step; the
         # discrete adjoint step in the adjoint slot; no midpoint kernel
         per_grad = {0: 2 * inst.nt + recompute, 2: inst.nt}
-        names[2], nbytes[2] = "k_adj_exact", EXACT_BYTES_PER_CELL
+        names[2], nbytes[2] = "k_adj_run (exact)", EXACT_BYTES_PER_CELL
     else:
         per_grad = {0: inst.nt + recompute, 1: inst.nt, 2: inst.nt}
-        adj = pb.adjoint_kernel
-        if adj["path"] != "split":  # one fused launch per backward step: no midpoint kernel
-            per_grad = {0: inst.nt + recompute, 2: inst.nt}
-            names[2], nbytes[2] = "k_adj_fused", FUSED_BYTES_PER_CELL[adj["path"]]
     kt = {k: pb.kernel_time(k) for k in per_grad}
     tiles = pb.tiles
     share = {k: kt[k][0] * per_grad[k] for k in kt}
     dom = max(share, key=share.get)
     cells = inst.nrows * inst.ncols
-    # the dominant kernel's live average launch: for the forward step, its sweep in the timed region / nt;
-    # otherwise the sampled launches of the profiling gradient (each bracketed by its own events, which
-    # adds the gap a graph replay hides: an upper bound)
+    # the dominant kernel's time per step: for the forward step, its sweep in the timed region / nt; otherwise the
+    # profiling gradient's launches, each bracketed by its own events
     fwd_live_ms = fwd_sweep_ms / inst.nt
     avg_ms, avg_src = ((fwd_live_ms, "forward sweep of the last timed gradient / nt (CUDA events)") if dom == 0
-                       else (kt[dom][0], "sampled launches, each bracketed by CUDA events"))
+                       else (kt[dom][0], "launches bracketed by CUDA events, per step"))
     achieved = nbytes[dom] * cells / (avg_ms / 1000.0) / 1e9
     peak, peak_kind = peaks()
     roof = {"bound": "hbm", "kernel": names[dom], "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -368,29 +350,21 @@ def run_ours(args):
             "time_share": {names[k]: share[k] / sum(share.values()) for k in share},
             "tiles": {k: list(v) for k, v in tiles.items()
                       if (k == "adj_exact") == (args.mode == "exact") or k == "fwd_step"},
-            "adjoint_path": pb.adjoint_kernel,
-            "note": "FP64 bound: a vector-field evaluation costs 2 exp (table-driven, 11 FP64 "
-                    "instructions each), 4 reciprocals (estimate + one cubic refinement) and ~50 "
-                    "FMA-class operations, 126 FP64 flops, 4.6 evaluations per cell-step; the HBM fraction "
-                    "is reported against the copy peak"}
+            "launches": "a sweep of steps each (kernel_ms_bracketed is per step)",
+            "note": "FP64 bound: a vector-field evaluation costs 81 FP64 instructions, about 4.6 evaluations per "
+                    "cell-step with the tiles' halo; the HBM fraction is reported against the copy peak"}
     # the forward step against the FP64 roof (the bound it is nearer to)
     ftx, fty, _ = tiles["fwd_step"]
     fl = FWD_FLOPS_PER_EVAL * fwd_evaluations(inst.nrows, inst.ncols, ftx, fty)
     mhz = clocks.get("sm_mhz") or 1965.0
     fpeak = 148 * 128 * mhz * 1e6 / 1e12
-    roof["fp64"] = {"kernel": "k_fwd_step", "achieved": fl / (fwd_live_ms / 1000.0) / 1e12, "peak": fpeak,
+    roof["fp64"] = {"kernel": names[0], "achieved": fl / (fwd_live_ms / 1000.0) / 1e12, "peak": fpeak,
                     "unit": "TFLOP/s", "frac": fl / (fwd_live_ms / 1000.0) / 1e12 / fpeak, "avg_launch_ms": fwd_live_ms,
                     "flops_per_launch": fl, "peak_source": "148 SMs x 64 DFMA/clock x 2 at the sampled SM clock",
                     "flops_source": "ncu-counted FP64 instructions per evaluation at 512x512"}
-    if inst.nrows == 512 and inst.ncols == 512 and (ftx, fty) == (64, 29):
-        frac_ncu, ms_ncu = FWD_FP64_PIPE_NCU
-        roof["fp64"]["pipe_active"] = {
-            "ncu": frac_ncu, "ncu_launch_ms": ms_ncu, "live_estimate": min(1.0, frac_ncu * ms_ncu / fwd_live_ms),
-            "what": "FP64 pipe busy fraction: ncu capture of one serialised launch of the same preset, and that "
-                    "scaled to the live launch time"}
     if roof["traffic"] is None and dom == 0 and FWD_TRAFFIC_PER_CELL:
         roof["traffic"] = FWD_TRAFFIC_PER_CELL * cells
-        roof["traffic_source"] = "ncu capture of one k_fwd_step launch at 512x512 (dram read + write)"
+        roof["traffic_source"] = "ncu capture of k_fwd_run at 512x512 (dram read + write), per step"
     roof = binding_roof(roof)
     sqrt_bytes = pb.device_bytes
     pb.close()
@@ -403,7 +377,7 @@ def run_ours(args):
                                 grad_mode=gmode)
             with api.Problem(inst, opts=fopts) as pf:
                 pf.grad(Et, inst.y0)
-                pf.grad(Et)  # the second call captures the gradient's graph: outside the timed region
+                pf.grad(Et)  # buffers are allocated by now: outside the timed region
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 torch.cuda.synchronize()
                 e0.record(stream)
@@ -530,12 +504,12 @@ def serve_and_batch(args):
                "sequential_warm_gradients_per_s": r["sequential_warm_throughput_req_s"],
                "what": "every gradient submitted at once to the server (concurrent single-instance solves, one "
                        "stream each, admission by device footprint)"}
-    ticks["what"] = "one BatchEngine: every tick's steps of all jobs in one persistent launch per kernel kind"
+    ticks["what"] = "one BatchEngine: every job's sweeps, packed into shared launches"
     best = max((streams, ticks), key=lambda x: x["speedup"])
     batched = {"count": len(insts), "sides": ticks["sides"], "nt_range": ticks["nt_range"],
                "scale": (f"{args.batch_count} of the 64 uneven instances, sides <= {args.serve_max_side}, "
                          f"horizons x{args.serve_nt_scale}"),
-               "sequential": "one resident problem at a time, each gradient a replayed graph",
+               "sequential": "one resident problem at a time",
                "speedup": best["speedup"], "streams": streams, "persistent_kernels": ticks}
     return served, plain, batched
 

@@ -162,7 +162,8 @@ int64_t fkadj_problem_last_launches(const fkadj_problem *pb);
  * reference, which keeps every state in host memory, cu-G:1658-1664):
  * out[0] policy (fkadj_ckpt_policy FULL/SQRT/BINOMIAL; 0 before the first
  * gradient), out[1] stored state slots, out[2] segment / scratch slots,
- * out[3] forward steps the backward sweep recomputes. */
+ * out[3] forward steps the backward sweep recomputes under the store's
+ * schedule (a BINOMIAL store's parts of two steps may take fewer). */
 void fkadj_problem_last_plan(const fkadj_problem *pb, int64_t out[4]);
 
 /* How the reference-mode backward step runs (no counterpart in the reference,
@@ -175,15 +176,17 @@ void fkadj_problem_last_plan(const fkadj_problem *pb, int64_t out[4]);
 void fkadj_problem_adjoint_kernel(const fkadj_problem *pb, int out[4]);
 
 /* Sampled per-kernel device time: when enabled, CUDA events bracket about one
- * in (nt/100) launches of each kernel kind during the following calls.
- * kernel: 0 forward step, 1 adjoint midpoint, 2 adjoint step.  Reports the
- * average milliseconds per launch of the last call and the sample count.
+ * in (nt/100) launches of a single step, and every launch of a sweep of steps,
+ * of each kernel kind during the following calls.  kernel: 0 forward step, 1
+ * adjoint midpoint, 2 adjoint step.  Reports the average milliseconds per step
+ * of the last call and the number of steps timed.
  * No reference counterpart (the reference has no timers besides tic/toc in
  * src/cuda/simple_grad_desc.m:80-86). */
 void fkadj_problem_set_profiling(fkadj_problem *pb, int enable);
 /* Tile presets in use (autotuned or fixed) for the forward step, adjoint
  * midpoint, adjoint step and exact adjoint step: out[k] = preset index, with
- * (tx, ty, threads) of each preset in shapes[3k..3k+2] when shapes != NULL. */
+ * (tx, ty, threads) of the tiles as launched in shapes[3k..3k+2] when shapes !=
+ * NULL (a problem that sweeps does not run its presets). */
 void fkadj_problem_tiles(const fkadj_problem *pb, int out[4], int shapes[12]);
 void fkadj_problem_kernel_time(const fkadj_problem *pb, int kernel, double *avg_ms, int64_t *samples);
 
