@@ -4,7 +4,7 @@
 // replayed graph, of which about 4 us are the launch boundary and the tile
 // loads, and the rest runs the FP64 pipe half busy.  Where the grid's tiles
 // fit the device at once (one CTA per SM), a whole sweep runs as one
-// cooperative launch instead: each CTA keeps its tile in shared memory from
+// cooperative launch instead (11.0 us a step): each CTA keeps its tile in shared memory from
 // step to step and exchanges only the 4-cell edges with its eight neighbours
 // through L2, waiting for its own neighbours and no one else.
 //
@@ -421,10 +421,15 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
 // twice, y_{i-1}; the exact mode: the step's stage states Y4, Y3, Y2 and y_s).
 // The sweep therefore is k_fwd_run's with the Jacobian evaluated at a state
 // read from global memory, one row ahead of its use.  Evaluating J on the
-// halo again (4.6 times a cell and step) costs 380 FP64 instructions a cell;
+// halo again (4.6 times a cell and step) costs 490 FP64 instructions a cell;
 // the per-step kernels read the seven entries cached by other kernels
-// instead, 250 B a cell and step through L2, and took 20 us for it at 512 x
-// 512.
+// instead, 250 B a cell and step through L2.  At 512 x 512 a step takes 19.8
+// us, 20 with the caches, but the kernel that made them (14 us a step) is now
+// k_mid_run (6.6 us); at 256 x 256 9.0 us, at 128 x 128 4.6.  Of the 19.8 us
+// the FP64 pipe is busy 42 %; 16 warps wait on fixed latencies, the points'
+// loads, the exchange and the barriers.  (Keeping J(yh) of the second stage
+// for the third, through an L2 scratch, took 17 % of the FP64 instructions
+// away and 1 % of the time: the 286 KB a step cost the SM's port as much.)
 //
 // Holes and everything off the grid hold 0 here, in the buffers and in z's
 // states: a missing neighbour then adds nothing to the plain sum, and only the
@@ -719,7 +724,12 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
 //
 // Where the tiles do not fit the device at once, a step is one launch of one
 // CTA per SM, each taking tiles in turn; a tile's window arrives by bulk
-// copies while the tile before it computes.  The stages are the sweeps'.
+// copies while the tile before it computes.  The stages are the sweeps'.  FP64
+// issue and fixed latencies bound them (pipe 48 % busy forward, 41 % exact
+// backward at 1536 x 1536, which also waits on DRAM for its points).  Forward,
+// backward and exact backward us a step, with the preset kernels and here:
+// 1024 x 768 52 and 43, 85 and 66; 2048 x 2048 218 and 199, 367 and 319, 405
+// and 335.  (Prefetching the next tile's points into L2: 353 for the 335.)
 
 // What a tile kernel's CTA goes through: tile i's place and window.
 struct TileWalk {
@@ -926,7 +936,8 @@ __global__ void __launch_bounds__(TileShapeBig::THREADS, 1)
 // in time: the state and f of a step's later end are the earlier end of the
 // step before it, so each step costs two evaluations and one window load,
 // issued a step ahead.  Per-step launches took 14 us a step at 512 x 512,
-// waiting for their operands.
+// waiting for their operands; this takes 6.6 (2048 x 2048: 207 and 133), the
+// FP64 pipe 50 % and the issue slots 64 % busy.
 //   y(1/3) = cubic Hermite of (ya, fa, yb, fb) at 1/3,
 //   yh     = partial quartic at 1/2 + (27/64) dt f(y(1/3), E(t + dt/3)).
 // One barrier a step: the y(1/3) buffers alternate, every warp issues a few of
@@ -1124,6 +1135,11 @@ RunShape run_shape(const DevGrid& g, int sms) {
     return best;
 }
 
+// Launches of several problems: each cooperative launch occupies the device for
+// as long as its longest sweep, and two do not overlap, so small grids one
+// after the other leave most SMs idle.  Ten uneven gradients to 256 x 256 x
+// 150: 16.1 ms a step at a time with the tick kernels, 8.1 packed.
+//
 // How n problems' tiles share launches of at most `sms` tiles and kRunJobs
 // problems: their shape, each one's launch, and the rows of a tile in each.
 struct RunPacking {
