@@ -29,6 +29,7 @@
 #include "fk_run.h"
 
 #include <algorithm>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
 // the per-step kernels read the seven entries cached by other kernels
 // instead, 250 B a cell and step through L2.  At 512 x 512 a step takes 19.8
 // us, 20 with the caches, but the kernel that made them (14 us a step) is now
-// k_mid_run (6.6 us); at 256 x 256 9.0 us, at 128 x 128 4.6.  Of the 19.8 us
+// k_mid_run (6.6 us); at 256 x 256 8.6 us, at 128 x 128 4.6.  Of the 19.8 us
 // the FP64 pipe is busy 42 %; 16 warps wait on fixed latencies, the points'
 // loads, the exchange and the barriers.  (Keeping J(yh) of the second stage
 // for the third, through an L2 scratch, took 17 % of the FP64 instructions
@@ -592,11 +593,17 @@ __device__ __forceinline__ void segment_terms(const uint16_t* list, int count, d
     }
 }
 
-template <class S, bool EXACT>
+// COPY: the job's parts in registers instead of read where they are needed.
+// That ends the spills of 20 to 36 bytes of the instances with two and five
+// rows a thread (exact mode 512 x 512 22.0 -> 20.9 us a step, 203 x 331 9.8 ->
+// 9.1; reference mode 256 x 256 8.9 -> 8.6, 512 x 512 the same), but costs the exact
+// instances that did not spill (384 x 384 15.7 -> 16.2) and, from shared
+// memory, a batch (8.05 -> 8.24 ms).
+template <class S, bool EXACT, bool COPY>
 __device__ __forceinline__ void adj_run(const DevModel& P, const AdjJob& J) {
     constexpr int TX = S::TX, R = S::R, TYM = S::TYM;
-    const DevGrid& g = J.g;
-    const AdjRun& r = J.r;
+    std::conditional_t<COPY, const DevGrid, const DevGrid&> g = J.g;
+    std::conditional_t<COPY, const AdjRun, const AdjRun&> r = J.r;
     const double* __restrict__ gh = J.gh;
     const uint8_t* __restrict__ cells = J.cells;
     const uint8_t* __restrict__ adj = J.adj;
@@ -709,7 +716,7 @@ __device__ __forceinline__ void adj_run(const DevModel& P, const AdjJob& J) {
 
 template <int TX, int R, int TYM, bool EXACT>
 __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1) k_adj_run(const DevModel P, const AdjJob j) {
-    adj_run<Shape<TX, R, TYM>, EXACT>(P, j);
+    adj_run<Shape<TX, R, TYM>, EXACT, !EXACT || R == 2 || R == 5>(P, j);
 }
 
 template <int TX, int R, int TYM, bool EXACT>
@@ -717,7 +724,7 @@ __global__ void __launch_bounds__(Shape<TX, R, TYM>::THREADS, 1)
     k_adj_jobs(const DevModel P, const RunJobs<AdjJob> jobs) {
     __shared__ AdjJob j;
     jobs.take(blockIdx.x, &j);
-    adj_run<Shape<TX, R, TYM>, EXACT>(P, j);
+    adj_run<Shape<TX, R, TYM>, EXACT, false>(P, j);
 }
 
 // --------------------------------------------- per-step tiles, larger grids
