@@ -233,7 +233,7 @@ Problem::~Problem() {
         // below): release the buffers first
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
+                         &fcache_, &Ed_, &flags_, &xchg_, &pts_, &dense_};
         for (DevBuf* b : all) b->release();
     }
     for (auto& r : prof_pool_) {
@@ -244,7 +244,7 @@ Problem::~Problem() {
     const auto t1 = clk::now();
     // a failed call may leave copies to or from the staging in flight: let
     // them finish before another call takes the buffers
-    if (st_ && (setup_ || (oneshot_ && (Ehost_ || hres_ || frame_)))) cudaStreamSynchronize(st_);
+    if (st_ && (setup_ || frame_ || (oneshot_ && (Ehost_ || hres_)))) cudaStreamSynchronize(st_);
     if (eup_) {
         cudaEventSynchronize(eup_);
         cudaEventDestroy(eup_);
@@ -268,7 +268,7 @@ Problem::~Problem() {
     if (verbose_ > 1) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
+                         &fcache_, &Ed_, &flags_, &xchg_, &pts_, &dense_};
         size_t bytes = 0;
         for (DevBuf* b : all) bytes += b->bytes;
         for (DevBuf* b : all) b->release();
@@ -451,7 +451,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     if (pool_) {
         DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_, &fault_,
                          &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_,
-                         &fcache_, &Ed_, &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
+                         &fcache_, &Ed_, &flags_, &xchg_, &pts_, &dense_};
         for (DevBuf* b : all) b->st = st_, b->pool = pool_;
     }
     {
@@ -526,9 +526,11 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
 
     // geometry on the padded grid: gh, adjoint stencil weights, compact
     // positions, the sweeps' flags; and S as CSR (row sums in ascending column
-    // order).  All of it is made in one pinned block, which the copies to the
-    // device take as it is (small enough ones: pinning a large block costs
-    // more than staging pageable memory).
+    // order).  All of it is made in one block: in one-shot calls a pinned one, kept
+    // from call to call, which the copies to the device take as it is (small
+    // enough ones).  Resident problems stage pageable memory: pinning 32 MB
+    // takes 13 ms, which the first one would pay (437 x 501: the first problem
+    // of a process 57-71 ms, with pinned blocks 66-109, later ones 10 either way).
     const size_t pl = (size_t)g_.plane;
     const int64_t nnz = need_objective ? S_colptr[n_num] : 0;
     const size_t nseg = (size_t)nsbx_ * nrows;
@@ -539,7 +541,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     double* block = nullptr;
     // (the end of its use is this problem's to wait for: not on a stream that
     // others queue work on)
-    if (need <= kPinnedSetup && own_stream_) {
+    if (need <= kPinnedSetup && own_stream_ && oneshot_) {
         CK(take_pinned(need, &setup_, &setup_n_), "alloc pinned set-up");
         block = setup_;
     } else {
@@ -607,7 +609,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     CK(cudaMemcpyAsync(pos_.p, pos, (size_t)n_num * sizeof(long long), cudaMemcpyHostToDevice, st_),
        "upload positions");
     if (!pinched) {
-        if (fkadj_status s = init_sweeps(cells, adj, seg)) return s;
+        if (fkadj_status s = init_sweeps(cells)) return s;
     }
 
     if (need_objective) {
@@ -651,11 +653,6 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
     CK(work_.alloc(3 * state_bytes()), "alloc states");
     CK(cudaMemsetAsync(work_.p, 0xff, work_.bytes, st_), "init states");
     spline_ = new NakSpline(nt + 1, dt);
-    if (setup_ && !oneshot_) {
-        CK(cudaStreamSynchronize(st_), "synchronize");  // its copies are done
-        give_pinned(setup_, setup_n_);
-        setup_ = nullptr;
-    }
     return FKADJ_OK;
 }
 
@@ -664,9 +661,10 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
 // sweep where the grid's tiles fit the device at once, the tile kernels
 // otherwise.  Where both run, forward and backward us a step with the sweep
 // and with the tile kernels: 256 x 256 5.6 9.0 and 12.8 16.9, 384 x 384 8.2
-// 14.0 and 14.8 21.0, 437 x 501 11.0 19.1 and 21.0 31.3.  cells, adj, seg: the sweeps' flags (host).  FKADJ_SWEEPS=0 in
-// the environment keeps the preset kernels.
-fkadj_status Problem::init_sweeps(const uint8_t* cells, const uint8_t* adj, const uint8_t* seg) {
+// 14.0 and 14.8 21.0, 437 x 501 11.0 19.1 and 21.0 31.3.  flags (host): the
+// sweeps' cell flags, adjoint flags and segment flags, in a row.
+// FKADJ_SWEEPS=0 in the environment keeps the preset kernels.
+fkadj_status Problem::init_sweeps(const uint8_t* flags) {
     const char* v = getenv("FKADJ_SWEEPS");
     if (!(autotune_ || shared_) || forced_path_ >= 0 || jcache_mode_ != 2 || !own_sweeps_ || (v && v[0] == '0')) return FKADJ_OK;
     const char* sv = getenv("FKADJ_ZGH_SEGMENTS");  // the adjoint sweeps write row segments
@@ -674,13 +672,10 @@ fkadj_status Problem::init_sweeps(const uint8_t* cells, const uint8_t* adj, cons
     int coop = 0;
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_), "device attribute");
     const RunShape shape = coop ? run_shape(g_, sms_) : RunShape();
-    const size_t pl = (size_t)g_.plane, nseg = (size_t)nsbx_ * g_.nrows;
-    CK(cells_.alloc(pl), "alloc cell flags");
-    CK(cudaMemcpyAsync(cells_.p, cells, pl, cudaMemcpyHostToDevice, st_), "upload cell flags");
-    CK(adjf_.alloc(pl), "alloc cell flags");
-    CK(cudaMemcpyAsync(adjf_.p, adj, pl, cudaMemcpyHostToDevice, st_), "upload cell flags");
-    CK(segf_.alloc(nseg), "alloc segment flags");
-    CK(cudaMemcpyAsync(segf_.p, seg, nseg, cudaMemcpyHostToDevice, st_), "upload segment flags");
+    const size_t nseg = (size_t)nsbx_ * g_.nrows;
+    // the three as they lie one after the other in the set-up's block
+    CK(flags_.alloc(2 * flag_bytes() + nseg), "alloc cell flags");
+    CK(cudaMemcpyAsync(flags_.p, flags, flags_.bytes, cudaMemcpyHostToDevice, st_), "upload cell flags");
     if (shape.id >= 0) {
         if (xchg_.alloc(run_exchange_bytes(g_)) != cudaSuccess) {
             cudaGetLastError();  // no memory for it: the preset kernels
@@ -725,7 +720,7 @@ int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t
 int64_t Problem::device_bytes() const {
     const DevBuf* all[] = {&gh_, &wc_, &pos_, &Srow_, &Scol_, &Sval_, &yc_, &zc_, &opart_, &osum_,
                            &work_, &zbuf_, &yh_, &partial_, &zgh_, &traj_, &seg_, &kf_, &y0res_, &stg_, &jcache_, &fcache_,
-                           &cells_, &adjf_, &segf_, &xchg_, &pts_, &dense_};
+                           &flags_, &xchg_, &pts_, &dense_};
     int64_t s = 0;
     for (auto* b : all) s += (int64_t)b->bytes;
     return s;
@@ -875,7 +870,7 @@ FwdJob Problem::forward_job(int i, int n, const double* src, double* last, doubl
     r.epoch = epoch_;
     r.fault = fault();
     epoch_ += (unsigned long long)n;
-    return {g_, gh_.as<double>(), cells_.as<uint8_t>(), r};
+    return {g_, gh_.as<double>(), flags_.as<uint8_t>(), r};
 }
 
 fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* last, double* out, double* keep, int first,
@@ -896,7 +891,7 @@ fkadj_status Problem::sweep_forward(int i, int n, const double* src, double* las
                 const EStep E = efwd(i + k);
                 const FwdStep r{cur, o, keep ? keep + 3 * k * stride : nullptr, E.p[0], E.p[1], E.p[2], fault()};
                 CK(prof_begin(K_FWD), "profiling event");
-                CK(launch_fwd_tile(P_, g_, gh_.as<double>(), cells_.as<uint8_t>(), r, sms_, st_), "forward step");
+                CK(launch_fwd_tile(P_, g_, gh_.as<double>(), flags_.as<uint8_t>(), r, sms_, st_), "forward step");
                 CK(prof_end(K_FWD), "profiling event");
                 ++launches_;
             } else if (fkadj_status s = step_forward(i + k, cur, o, keep ? keep + k * stride : nullptr)) {
@@ -969,9 +964,9 @@ Problem::AdjointChunk Problem::adjoint_chunk(int top, int hi, int lo, const doub
         m.Et = etab() + top;
         m.E3 = etab() + (2 * nt_ + 1) + top - 1;
         m.fault = fault();
-        c.mid = {g_, gh_.as<double>(), cells_.as<uint8_t>(), m};
+        c.mid = {g_, gh_.as<double>(), flags_.as<uint8_t>(), m};
     }
-    c.adj = {g_, gh_.as<double>(), cells_.as<uint8_t>(), adjf_.as<uint8_t>(), r};
+    c.adj = {g_, gh_.as<double>(), flags_.as<uint8_t>(), adj_flags(), r};
     return c;
 }
 
@@ -1009,7 +1004,7 @@ fkadj_status Problem::sweep_adjoint(int hi, int lo, const double* y_hi, const do
             if (exact) a.y[0] = p + 2 * sz, a.y[1] = p + sz, a.y[2] = p;
             for (int gr = 0; gr < (exact ? 3 : 1); ++gr) a.row[gr] = prow(gr, top - 1 - k);
             CK(prof_begin(K_ADJ), "profiling event");
-            CK(launch_adj_tile(exact, P_, g_, gh_.as<double>(), adjf_.as<uint8_t>(), segf_.as<uint8_t>(), a, sms_, st_),
+            CK(launch_adj_tile(exact, P_, g_, gh_.as<double>(), adj_flags(), segment_flags(), a, sms_, st_),
                "adjoint step");
             CK(prof_end(K_ADJ), "profiling event");
             ++launches_;
@@ -1036,6 +1031,8 @@ fkadj_status Problem::download_grid(const double* d_state, double* host) {
         CK(cudaMemcpyAsync(frame_, dense_.p, n3 * sizeof(double), cudaMemcpyDeviceToHost, st_), "download state");
         CK(cudaStreamSynchronize(st_), "synchronize");
         std::memcpy(host, frame_, n3 * sizeof(double));
+        give_pinned(frame_, frame_n_);  // (kept while no call needs it: pinning 8 MB takes 3.6 ms)
+        frame_ = nullptr;
         return FKADJ_OK;
     }
     const size_t n = (size_t)g_.nrows * g_.ncols;

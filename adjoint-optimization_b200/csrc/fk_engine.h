@@ -201,7 +201,7 @@ public:
     // the states between (mid, where they are not there yet).
     fkadj_status sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
                                const double* stages, double*& z, double*& z2, double* replayed = nullptr);
-    fkadj_status init_sweeps(const uint8_t* cells, const uint8_t* adj, const uint8_t* seg);
+    fkadj_status init_sweeps(const uint8_t* flags);
     // whether this problem's steps are sweeps (fk_run.h): one launch each where
     // run_.id >= 0, the tile kernels otherwise
     bool sweeping() const { return swept_ && !run_off_; }
@@ -319,9 +319,11 @@ private:
     DevBuf gh_, wc_, pos_, Srow_, Scol_, Sval_, yc_, zc_, opart_, osum_;
     DevBuf fault_;     // this problem's fault word: set by a step kernel whose bounded wait expired
     unsigned* fault() const { return fault_.as<unsigned>(); }
-    DevBuf cells_;     // geometry flags per padded cell (CELL_*), where the grid is swept
-    DevBuf adjf_;      // the adjoint sweeps' flags per padded cell
-    DevBuf segf_;      // per 16-cell row segment: whether it holds a source cell
+    DevBuf flags_;     // where the grid is swept: geometry flags per padded cell (CELL_*), the adjoint
+                       // sweeps' flags likewise, and per 16-cell row segment whether it holds a source cell
+    size_t flag_bytes() const { return ((size_t)g_.plane + 7) / 8 * 8; }
+    const uint8_t* adj_flags() const { return flags_.as<uint8_t>() + flag_bytes(); }
+    const uint8_t* segment_flags() const { return flags_.as<uint8_t>() + 2 * flag_bytes(); }
     DevBuf xchg_;      // the sweeps' edge exchange
     DevBuf pts_;       // points between the states of one chunk of an adjoint sweep
     int sms_ = 0;

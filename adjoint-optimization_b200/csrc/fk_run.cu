@@ -289,7 +289,7 @@ __device__ __forceinline__ void fwd_rows(const DevModel& P, const Column& T, con
                     for (int f = 0; f < 3; ++f) put_tagged(x + f * plane + T.o + k * ld, o[f], tag);
                 }
             } else {
-double o[3];
+                double o[3];
 #pragma unroll
                 for (int f = 0; f < 3; ++f) {
                     const double y0 = MODE == 0 ? m[f] : a[f * S::PA];
