@@ -149,8 +149,10 @@ static cudaError_t take_pinned(size_t n, double** p, size_t* cap) {
     // whole powers of two: calls of about the same size share their buffers
     size_t c = (size_t)1 << 14;
     while (c < n) c *= 2;
-    *cap = c;
-    return cudaMallocHost(p, c * sizeof(double));
+    const cudaError_t e = cudaMallocHost(p, c * sizeof(double));
+    *cap = e ? 0 : c;
+    if (e) *p = nullptr;
+    return e;
 }
 
 // Streams (with a problem's three events) of one-shot calls, kept for the next
@@ -746,13 +748,17 @@ fkadj_status Problem::prepare_E(const double* Et, bool upload) {
     if (!upload) return FKADJ_OK;
     // device tables [Et | Eh | E3] for the kernels (through pinned staging)
     const size_t n = (size_t)3 * nt_ + 1;
-    if (!Ed_.p) {
-        CK(Ed_.alloc(n * sizeof(double)), "alloc E tables");
-        if (oneshot_ || shared_)
-            CK(take_pinned(n, &Ehost_, &Ehost_n_), "alloc pinned E tables");
-        else
-            CK(cudaMallocHost(&Ehost_, n * sizeof(double)), "alloc pinned E tables");
-        if (shared_) CK(cudaEventCreateWithFlags(&eup_, cudaEventDisableTiming), "event");
+    if (!e_ready_) {
+        // (what an earlier call that ran out of memory left is kept)
+        if (!Ed_.p) CK(Ed_.alloc(n * sizeof(double)), "alloc E tables");
+        if (!Ehost_) {
+            if (oneshot_ || shared_)
+                CK(take_pinned(n, &Ehost_, &Ehost_n_), "alloc pinned E tables");
+            else
+                CK(cudaMallocHost(&Ehost_, n * sizeof(double)), "alloc pinned E tables");
+        }
+        if (shared_ && !eup_) CK(cudaEventCreateWithFlags(&eup_, cudaEventDisableTiming), "event");
+        e_ready_ = true;
         ++buf_gen_;
     } else if (shared_) {  // the stream is other problems' too
         CK(cudaEventSynchronize(eup_), "the previous upload");
@@ -1253,6 +1259,7 @@ fkadj_status Problem::ensure_traj(const TrajPlan& tp) {
     traj_.release();
     seg_.release();
     kf_.release();
+    traj_plan_ = TrajPlan();  // no plan's buffers until all of them are there
     CK(traj_.alloc((size_t)tp.nslots * state_bytes()), "alloc trajectory");
     CK(cudaMemsetAsync(traj_.p, 0xff, traj_.bytes, st_), "init trajectory");
     if (tp.seg_slots) {
@@ -1287,19 +1294,19 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
             CK(cudaMemsetAsync(pts_.p, 0xff, pts_.bytes, st_), "init adjoint points");
         }
     }
-    if (grad_mode_ == FKADJ_GRAD_REF && !sweep && !yh_.p) {
-        CK(yh_.alloc(state_bytes()), "alloc midpoint state");
-        CK(cudaMemsetAsync(yh_.p, 0xff, yh_.bytes, st_), "init midpoint state");
+    // each buffer by itself: an earlier call may have run out of memory between two of them
+    auto filled = [&](DevBuf& b, size_t bytes) {
+        if (b.p) return cudaSuccess;
+        const cudaError_t e = b.alloc(bytes);
+        return e ? e : cudaMemsetAsync(b.p, 0xff, bytes, st_);
+    };
+    if (grad_mode_ == FKADJ_GRAD_REF && !sweep) {
+        CK(filled(yh_, state_bytes()), "alloc midpoint state");
         // Jacobian caches J(y) x2 and J(yh) (7 planes each), f(y) carry x2 (3 planes each)
-        CK(jcache_.alloc(21 * (size_t)g_.plane * sizeof(double)), "alloc Jacobian cache");
-        CK(cudaMemsetAsync(jcache_.p, 0xff, jcache_.bytes, st_), "init Jacobian cache");
-        CK(fcache_.alloc(6 * (size_t)g_.plane * sizeof(double)), "alloc f cache");
-        CK(cudaMemsetAsync(fcache_.p, 0xff, fcache_.bytes, st_), "init f cache");
+        CK(filled(jcache_, 21 * (size_t)g_.plane * sizeof(double)), "alloc Jacobian cache");
+        CK(filled(fcache_, 6 * (size_t)g_.plane * sizeof(double)), "alloc f cache");
     }
-    if (grad_mode_ == FKADJ_GRAD_EXACT && !sweep && !stg_.p) {
-        CK(stg_.alloc(3 * state_bytes()), "alloc stage states");
-        CK(cudaMemsetAsync(stg_.p, 0xff, stg_.bytes, st_), "init stage states");
-    }
+    if (grad_mode_ == FKADJ_GRAD_EXACT && !sweep) CK(filled(stg_, 3 * state_bytes()), "alloc stage states");
     // z.gh partials, one row of nsb sub-block sums per row of results.  The
     // standalone sweep keeps a window of kPartialWindow rows per group (the
     // exact mode has three groups of nt rows, the reference mode one of nt+1)
@@ -2038,6 +2045,7 @@ fkadj_status Problem::grad_call(const double* Et, const double* y_ini, double* L
         } else {
             if (hres_) cudaFreeHost(hres_);
             hres_ = nullptr;
+            hres_n_ = 0;
             CK(cudaMallocHost(&hres_, (prow + 1) * sizeof(double)), "alloc pinned results");
             hres_n_ = prow + 1;
         }

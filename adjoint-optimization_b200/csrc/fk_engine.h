@@ -356,6 +356,7 @@ private:
     double* hres_ = nullptr;   // pinned results: L0 partial sum, then the z.gh rows
     size_t hres_n_ = 0;
     size_t Ehost_n_ = 0;       // capacity of Ehost_ (doubles)
+    bool e_ready_ = false;     // the E tables' buffers are there
     double* setup_ = nullptr;  // pinned block of the set-up's uploads
     size_t setup_n_ = 0;
     double* frame_ = nullptr;  // pinned staging of a downloaded state

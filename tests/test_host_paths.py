@@ -1,0 +1,173 @@
+"""Host paths that only a failing call reaches, run without a GPU: the
+library's objects linked with a stand-in for the CUDA runtime
+(fake_cudart.cpp) whose kernels do nothing, whose device memory can run out at
+any allocation and whose cooperative launches can be refused.  Every buffer a
+sweep is handed must lie in live device memory."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from fkadj import _lib, api, batch, serve, workloads as W
+from fkadj.batch import Batch
+from fkadj.serve import Server
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+PKG = _lib.PKG_DIR
+MODES = [_lib.GRAD_REF, _lib.GRAD_EXACT]
+STORES = [_lib.CKPT_FULL, _lib.CKPT_SQRT, _lib.CKPT_BINOMIAL]
+FAULT_NAN = 2
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    subprocess.run(["make", "-s", "-C", PKG, "-j4", "lib"], check=True)
+    tmp = tmp_path_factory.mktemp("fake")
+    obj, lib = str(tmp / "fake.o"), str(tmp / "libfkadj_fake.so")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", f"-I{cuda}/include", "-c", "-o", obj,
+                    os.path.join(HERE, "fake_cudart.cpp")], check=True)
+    objs = [os.path.join(PKG, "_build", f"fk_{n}.o")
+            for n in ("kernels", "run", "engine", "spline", "noalloc", "batch", "serve", "matio")]
+    # its own definitions of the runtime, whatever the process has loaded
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", lib, *objs, obj, "-lpthread", "-lz"],
+                   check=True)
+    return lib
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    for v in ("FKADJ_SWEEPS", "FKADJ_TILES", "FKADJ_ADJ_PATH", "FKADJ_JCACHE", "FKADJ_ZGH_SEGMENTS",
+              "FKADJ_SERVE_MODE", "FKADJ_SERVE_STREAMS", "FKADJ_ONESHOT_POOL"):
+        monkeypatch.delenv(v, raising=False)
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "LIB_PATH", fake_path)
+    monkeypatch.setattr(batch, "_bound", False)
+    monkeypatch.setattr(serve, "_bound", False)
+    L = _lib.load()
+    for n in ("allocations", "in_use", "peak", "bad_spans"):
+        getattr(L, f"fake_{n}").restype = C.c_int64
+    L.fake_launches.restype = C.c_int64
+    L.fake_launches.argtypes = [C.c_char_p]
+    L.fake_first_bad.restype = C.c_char_p
+    L.fake_reset.argtypes = [C.c_int64]
+    L.fake_fail_allocations.argtypes = [C.c_int64, C.c_int64]
+    L.fake_fail_host_allocation.argtypes = [C.c_int64]
+    L.fake_fault.argtypes = [C.c_char_p, C.c_uint, C.c_int]
+    _lib.check(L.fkadj_release_cached_memory())
+    L.fake_reset(0)
+    yield L
+    assert L.fake_bad_spans() == 0, L.fake_first_bad().decode()
+    L.fake_reset(0)
+
+
+def _inst(rows=40, cols=72, nt=24, **kw):
+    return W.make_instance(rows, nt, ncols=cols, seed=1, n_obstacles=3, intervals=3, alpha=0.1, **kw)
+
+
+def _state_bytes(inst):
+    return 3 * 8 * (-(-inst.nrows // 64) * 64 + 8) * (-(-inst.ncols // 64) * 64 + 8)
+
+
+def _opts(inst, mode=_lib.GRAD_REF, store=_lib.CKPT_AUTO, states=0):
+    return api.options(grad_mode=mode, ckpt_policy=store, ckpt_budget_bytes=int(states * _state_bytes(inst)))
+
+
+def _sweeps(L):
+    return L.fake_launches(b"k_fwd_run") + L.fake_launches(b"k_fwd_jobs")
+
+
+@pytest.mark.parametrize("store", STORES)
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("rows,cols,nt", [(5, 7, 3), (40, 72, 24), (131, 97, 37), (300, 200, 70), (640, 900, 9)])
+def test_sweeps_stay_in_their_buffers(fake, rows, cols, nt, mode, store):
+    inst = _inst(rows, cols, nt)
+    with api.Problem(inst, opts=_opts(inst, mode, store, 6 if store == _lib.CKPT_BINOMIAL else 0)) as pb:
+        for y in (inst.y0, None):
+            pb.grad(inst.Et, y, return_yf=True)
+        pb.objective(inst.Et)
+    if store != _lib.CKPT_BINOMIAL:
+        with Batch() as b:
+            ids = [b.add_problem(inst, grad_mode=mode, ckpt_policy=store) for _ in range(3)]
+            for j in [b.submit(p, inst.Et, inst.y0, want_grad=k != 1) for k, p in enumerate(ids)]:
+                b.run()
+                b.result(j)
+    assert fake.fake_launches(b"k_fwd_step") == 0 and fake.fake_launches(b"k_batch") == 0
+    assert _sweeps(fake) > 0 or fake.fake_launches(b"k_fwd_tile") > 0
+
+
+@pytest.mark.parametrize("sweeps,n_failing", [("1", 1), ("1", 1000), ("0", 1)])
+@pytest.mark.parametrize("store", STORES[:2])
+@pytest.mark.parametrize("mode", MODES)
+def test_a_failed_allocation_leaves_no_missing_buffer(fake, monkeypatch, mode, store, sweeps, n_failing):
+    """Allocations of a first gradient fail from any one on: the call gives its
+    result without sweeps or reports the lack of memory, and the next one finds
+    every buffer that a problem of its kind holds."""
+    inst = _inst()
+    opts = _opts(inst, mode, store)
+
+    def held(v):
+        monkeypatch.setenv("FKADJ_SWEEPS", v)
+        before = fake.fake_in_use()
+        with api.Problem(inst, opts=opts) as pb:
+            fake.fake_fail_allocations(-1, 0)
+            pb.grad(inst.Et, inst.y0)
+            return fake.fake_in_use() - before, fake.fake_allocations()
+    preset, swept = held("0"), held("1")
+    monkeypatch.setenv("FKADJ_SWEEPS", sweeps)
+    for k in range((swept if sweeps == "1" else preset)[1]):
+        before = fake.fake_in_use()
+        with api.Problem(inst, opts=opts) as pb:
+            fake.fake_fail_allocations(k, n_failing)
+            try:
+                pb.grad(inst.Et, inst.y0)
+            except _lib.FkadjError as e:
+                assert e.status == _lib.ERR_NOMEM
+            fake.fake_fail_allocations(-1, 0)
+            pb.grad(inst.Et, inst.y0)
+            runs = fake.fake_launches(b"k_adj_run")
+            pb.grad(inst.Et)
+            want = swept if fake.fake_launches(b"k_adj_run") > runs else preset
+            assert fake.fake_in_use() - before >= want[0], k
+
+
+@pytest.mark.parametrize("k", range(4))
+def test_a_failed_change_of_the_store_is_made_again(fake, k):
+    """The repeat after a NaN takes another store (no kept stage states); where
+    its allocation fails, the next call must not take the old plan for done."""
+    inst = _inst()
+    with api.Problem(inst, opts=_opts(inst, _lib.GRAD_EXACT, _lib.CKPT_SQRT)) as pb:
+        pb.grad(inst.Et, inst.y0)
+        fake.fake_fault(b"k_fwd_run", FAULT_NAN, 1)
+        fake.fake_fail_allocations(k, 1)
+        try:
+            pb.grad(inst.Et)
+        except _lib.FkadjError as e:
+            assert e.status == _lib.ERR_NOMEM
+        fake.fake_fail_allocations(-1, 0)
+        pb.grad(inst.Et)
+
+
+@pytest.mark.parametrize("k", range(4))
+def test_a_failed_pinned_allocation_leaves_no_missing_buffer(fake, k):
+    inst = _inst()
+    with api.Problem(inst) as pb:
+        fake.fake_fail_host_allocation(k)
+        try:
+            pb.grad(inst.Et, inst.y0, return_yf=True)
+        except _lib.FkadjError as e:
+            assert e.status == _lib.ERR_NOMEM
+        fake.fake_fail_host_allocation(-1)
+        pb.grad(inst.Et, inst.y0, return_yf=True)
+    with Server(hbm_budget_bytes=1 << 30) as sv:
+        fake.fake_fail_host_allocation(k)
+        rid = sv.submit(inst)
+        try:
+            sv.wait(rid)
+        except _lib.FkadjError as e:
+            assert e.status == _lib.ERR_NOMEM
+        fake.fake_fail_host_allocation(-1)
+        rid = sv.submit(inst)
+        assert sv.wait(rid)
