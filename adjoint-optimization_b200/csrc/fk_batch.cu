@@ -194,9 +194,12 @@ fkadj_status BatchEngine::prepare_job(Job& j, const double* y_ini) {
     j.swept = P.sweeping();
     j.cur_c = 0;
     j.have_fcarry = j.have_jcarry = j.finishing = false;
+    P.refused_ = false;
+    if (j.swept && (s = P.ensure_exchange())) return s;
     if (j.want_grad) {
         if ((s = P.plan_trajectory(j.tp, true))) return s;
         if (j.tp.policy == FKADJ_CKPT_BINOMIAL) {
+            P.refused_ = true;
             set_error("batched jobs store full or sqrt trajectories; the binomial schedule runs in the "
                       "standalone engine (raise ckpt_budget_bytes or use fkadj_problem_grad)");
             return FKADJ_ERR_NOMEM;
@@ -284,11 +287,12 @@ fkadj_status BatchEngine::submit(int prob, const double* Et, const double* y_ini
     if ((s = P.prepare_E(Et, P.sweeping()))) return s;  // the tick kernels take E by value
     j->Et.assign(Et, Et + P.nt_ + 1);
     s = prepare_job(*j, y_ini);
-    if (s == FKADJ_ERR_NOMEM && P.sweeping()) {  // the tick kernels need less memory
-        for (DevBuf* b : {&P.xchg_, &P.pts_, &P.kf_}) b->release();
-        P.traj_plan_ = TrajPlan();
+    if (s == FKADJ_ERR_NOMEM && P.sweeping() && !P.refused_) {
+        // the tick kernels need less memory; as in Problem::with_sweeps
+        P.drop_sweep_buffers();
         P.swept_ = false;
         s = prepare_job(*j, y_ini);
+        if (s == FKADJ_ERR_NOMEM) P.swept_ = true;
     }
     if (s) return s;
     j->h_out = take_pinned((size_t)j->rows + 2, &j->h_cap);  // [0] L0 sum, [1..rows], fault word

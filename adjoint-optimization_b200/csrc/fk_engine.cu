@@ -678,15 +678,19 @@ fkadj_status Problem::init_sweeps(const uint8_t* flags) {
     // the three as they lie one after the other in the set-up's block
     CK(flags_.alloc(2 * flag_bytes() + nseg), "alloc cell flags");
     CK(cudaMemcpyAsync(flags_.p, flags, flags_.bytes, cudaMemcpyHostToDevice, st_), "upload cell flags");
-    if (shape.id >= 0) {
-        if (xchg_.alloc(run_exchange_bytes(g_)) != cudaSuccess) {
-            cudaGetLastError();  // no memory for it: the preset kernels
-            return FKADJ_OK;
-        }
-        CK(cudaMemsetAsync(xchg_.p, 0, xchg_.bytes, st_), "clear edge exchange");
-    }
     run_ = shape;
     swept_ = true;
+    const fkadj_status s = ensure_exchange();
+    if (s == FKADJ_ERR_NOMEM) swept_ = false;  // the preset kernels
+    return s == FKADJ_ERR_NOMEM ? FKADJ_OK : s;
+}
+
+// The edge exchange of a problem that sweeps in one launch: its tags count on
+// from sweep to sweep, and none equals the zeros it starts from.
+fkadj_status Problem::ensure_exchange() {
+    if (!sweeping() || run_.id < 0 || xchg_.p) return FKADJ_OK;
+    CK(xchg_.alloc(run_exchange_bytes(g_)), "alloc edge exchange");
+    CK(cudaMemsetAsync(xchg_.p, 0, xchg_.bytes, st_), "clear edge exchange");
     return FKADJ_OK;
 }
 
@@ -1229,6 +1233,7 @@ fkadj_status Problem::plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only) {
     }
     const double need = (double)(tp.nslots + tp.seg_slots) * sb;
     if (ckpt_policy_ != FKADJ_CKPT_FULL && need > (double)ckpt_budget_) {
+        refused_ = true;
         set_error("trajectory store does not fit the checkpoint budget");
         return FKADJ_ERR_NOMEM;
     }

@@ -202,6 +202,11 @@ public:
     fkadj_status sweep_adjoint(int hi, int lo, const double* y_hi, const double* mid, const double* y_lo,
                                const double* stages, double*& z, double*& z2, double* replayed = nullptr);
     fkadj_status init_sweeps(const uint8_t* flags);
+    fkadj_status ensure_exchange();
+    // What only sweeps use.  (Kept stage states go with the plan: ensure_traj.)
+    void drop_sweep_buffers() {
+        for (DevBuf* b : {&xchg_, &pts_}) b->release();
+    }
     // whether this problem's steps are sweeps (fk_run.h): one launch each where
     // run_.id >= 0, the tile kernels otherwise
     bool sweeping() const { return swept_ && !run_off_; }
@@ -337,6 +342,7 @@ private:
     // (FAULT_NAN), which they contain
     bool run_off_ = false;
     bool nan_seen_ = false;
+    bool refused_ = false;     // the last plan: refused by the caller's budget, whatever memory there is
     bool own_sweeps_ = true;  // false where memory is short
     bool shared_ = false;     // a batch engine's problem
     cudaEvent_t eup_ = nullptr;  // of such a problem: its E tables' upload
@@ -406,13 +412,17 @@ private:
 
 template <class Call>
 fkadj_status Problem::with_sweeps(Call&& call) {
-    nan_seen_ = false;
-    fkadj_status s = call();
-    if (s == FKADJ_ERR_NOMEM && sweeping()) {
-        // the preset kernels need less memory
-        for (DevBuf* b : {&xchg_, &pts_}) b->release();
+    nan_seen_ = refused_ = false;
+    fkadj_status s = ensure_exchange();
+    if (!s) s = call();
+    if (s == FKADJ_ERR_NOMEM && sweeping() && !refused_) {
+        // the preset kernels need less memory; where they lack it too, sweeps
+        // were not what it was short for
+        drop_sweep_buffers();
         swept_ = false;
-        return call();
+        s = call();
+        if (s == FKADJ_ERR_NOMEM) swept_ = true;
+        return s;
     }
     if (!nan_seen_) return s;
     run_off_ = true;

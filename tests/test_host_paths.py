@@ -171,3 +171,46 @@ def test_a_failed_pinned_allocation_leaves_no_missing_buffer(fake, k):
         fake.fake_fail_host_allocation(-1)
         rid = sv.submit(inst)
         assert sv.wait(rid)
+
+
+def _refused(fake, inst, call):
+    runs = _sweeps(fake)
+    with pytest.raises(_lib.FkadjError) as e:
+        call()
+    assert e.value.status == _lib.ERR_NOMEM
+    assert _sweeps(fake) == runs and fake.fake_launches(b"k_fwd_step") == 0
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_a_refused_budget_leaves_the_sweeps_on(fake, mode):
+    """A gradient whose store does not fit the caller's budget fails before
+    any device work; the problem's objectives go on as sweeps."""
+    inst = _inst()
+    with api.Problem(inst, opts=_opts(inst, mode, _lib.CKPT_SQRT, 2)) as pb:
+        for n in range(1, 3):
+            _refused(fake, inst, lambda: pb.grad(inst.Et, inst.y0))
+            pb.objective(inst.Et, inst.y0)
+            assert _sweeps(fake) == n
+    with Batch() as b:
+        for states, store in ((2, _lib.CKPT_SQRT), (6, _lib.CKPT_BINOMIAL)):  # the latter is not a batch's
+            p = b.add_problem(inst, grad_mode=mode, ckpt_policy=store, ckpt_budget_bytes=states * _state_bytes(inst))
+            _refused(fake, inst, lambda: b.submit(p, inst.Et, inst.y0))
+            runs = _sweeps(fake)
+            j = b.submit(p, inst.Et, inst.y0, want_grad=False)
+            b.run()
+            b.result(j)
+            assert _sweeps(fake) > runs and fake.fake_launches(b"k_batch_fwd") == 0
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_sweeps_come_back_where_the_preset_kernels_lacked_memory_too(fake, mode):
+    inst = _inst()
+    with api.Problem(inst, opts=_opts(inst, mode, _lib.CKPT_SQRT)) as pb:
+        fake.fake_fail_allocations(0, 1000)
+        with pytest.raises(_lib.FkadjError) as e:
+            pb.grad(inst.Et, inst.y0)
+        assert e.value.status == _lib.ERR_NOMEM
+        fake.fake_fail_allocations(-1, 0)
+        steps = fake.fake_launches(b"k_fwd_step")
+        pb.grad(inst.Et, inst.y0)
+        assert fake.fake_launches(b"k_adj_run") > 0 and fake.fake_launches(b"k_fwd_step") == steps
