@@ -530,9 +530,19 @@ fkadj_status BatchEngine::finish_poll(Job& j) {
     Problem& P = *probs_[j.prob];
     const int nt = P.nt_;
     if (j.swept && *reinterpret_cast<const unsigned*>(j.h_out + j.rows + 1) == FAULT_NAN) {
-        // a NaN state: once more with the tick kernels, which contain it
+        // a NaN state: once more with the tick kernels, which contain it, and
+        // with their buffers in place of the sweeps'.  Where the device lacks
+        // the memory, this job fails and the others go on.
         P.run_off_ = true;
-        return prepare_job(j, nullptr);
+        P.drop_sweep_buffers();
+        const fkadj_status s = prepare_job(j, nullptr);
+        if (s != FKADJ_ERR_NOMEM) return s;
+        P.run_off_ = false;
+        j.status = s;
+        j.gradE.clear();
+        j.done = true;
+        j.t_done = host_seconds();
+        return FKADJ_OK;
     }
     P.run_off_ = false;
     const double l0 = -j.h_out[0];

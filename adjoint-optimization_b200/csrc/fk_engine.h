@@ -425,8 +425,16 @@ fkadj_status Problem::with_sweeps(Call&& call) {
         return s;
     }
     if (!nan_seen_) return s;
+    // once more with the preset kernels.  A one-shot problem (the server's)
+    // never holds both paths' buffers; a resident one gives the sweeps' up
+    // only where the device lacks the memory (the next call sweeps again)
     run_off_ = true;
+    if (oneshot_) drop_sweep_buffers();
     s = call();
+    if (s == FKADJ_ERR_NOMEM && !refused_ && (xchg_.p || pts_.p)) {
+        drop_sweep_buffers();
+        s = call();
+    }
     run_off_ = false;
     return s;
 }

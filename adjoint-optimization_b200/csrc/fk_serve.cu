@@ -46,7 +46,7 @@ struct Request {
     std::vector<int64_t> Jc, Ir;
     bool want_grad = true;
     int64_t est = 0;
-    int64_t est_sweeps = 0;  // the same with sweeps
+    int64_t est_sweeps = 0;  // the same with sweeps, and where a NaN has the preset kernels repeat it
     bool sweeps = false;     // how it was admitted
     // results
     int state = 0;  // 0 queued, 1 running, 2 done, 3 failed
@@ -216,6 +216,7 @@ fkadj_status Server::submit(std::unique_ptr<Request> r, int64_t* id) {
                                             opt_.grad_mode,
                                             opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT,
                                             r->want_grad, true);
+    r->est_sweeps = std::max(r->est_sweeps, r->est);
     if (r->est > budget_) {
         set_error("request does not fit the HBM budget even alone");
         return FKADJ_ERR_NOMEM;

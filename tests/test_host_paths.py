@@ -214,3 +214,51 @@ def test_sweeps_come_back_where_the_preset_kernels_lacked_memory_too(fake, mode)
         steps = fake.fake_launches(b"k_fwd_step")
         pb.grad(inst.Et, inst.y0)
         assert fake.fake_launches(b"k_adj_run") > 0 and fake.fake_launches(b"k_fwd_step") == steps
+
+
+@pytest.mark.parametrize("want_grad", [True, False])
+@pytest.mark.parametrize("store", STORES[:2])
+@pytest.mark.parametrize("mode", MODES)
+def test_a_batched_job_that_cannot_be_repeated_fails_alone(fake, mode, store, want_grad):
+    """A NaN among one job's inputs, and no memory for the tick kernels'
+    buffers: that job reports it, the others give their results, and both
+    problems take new jobs (as sweeps)."""
+    inst = _inst()
+    with Batch() as b:
+        ids = [b.add_problem(inst, grad_mode=mode, ckpt_policy=store) for _ in range(2)]
+        jobs = [b.submit(ids[0], inst.Et, inst.y0, want_grad=want_grad), b.submit(ids[1], inst.Et, inst.y0)]
+        fake.fake_fault(b"k_fwd_jobs", FAULT_NAN, 1)  # the first problem's
+        while not b.done(jobs[1]):
+            b.tick()
+            fake.fake_fail_allocations(0, 1000)
+        if want_grad:
+            with pytest.raises(_lib.FkadjError) as e:
+                b.run()
+                b.result(jobs[0])
+            assert e.value.status == _lib.ERR_NOMEM
+        else:  # an objective needs no more buffers
+            b.run()
+            b.result(jobs[0])
+        b.result(jobs[1])
+        fake.fake_fail_allocations(-1, 0)
+        ticks = fake.fake_launches(b"k_batch")
+        for j in [b.submit(p, inst.Et, inst.y0) for p in ids]:
+            b.run()
+            assert b.result(j)["gradE"].size == inst.nt + 1
+        assert fake.fake_launches(b"k_batch") == ticks
+
+
+@pytest.mark.parametrize("store", STORES)
+@pytest.mark.parametrize("mode", MODES)
+def test_a_repeat_without_memory_takes_the_sweeps_buffers(fake, mode, store):
+    inst = _inst()
+    with api.Problem(inst, opts=_opts(inst, mode, store, 6 if store == _lib.CKPT_BINOMIAL else 0)) as pb:
+        pb.grad(inst.Et, inst.y0)
+        for _ in range(2):
+            runs = fake.fake_launches(b"k_adj_run")
+            fake.fake_fault(b"k_fwd_run", FAULT_NAN, 1)
+            fake.fake_fail_allocations(0, 1)
+            pb.grad(inst.Et)
+            fake.fake_fail_allocations(-1, 0)
+            pb.grad(inst.Et)
+            assert fake.fake_launches(b"k_adj_run") >= runs + 2
