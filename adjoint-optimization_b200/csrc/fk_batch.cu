@@ -25,6 +25,7 @@ double host_seconds() {
 fkadj_status BatchEngine::fail(cudaError_t e, const char* what) {
     set_error(std::string(what) + ": " + cudaGetErrorString(e));
     cudaGetLastError();
+    no_coop_ = no_coop_ || e == cudaErrorCooperativeLaunchTooLarge;
     return e == cudaErrorMemoryAllocation ? FKADJ_ERR_NOMEM : FKADJ_ERR_CUDA;
 }
 
@@ -130,6 +131,7 @@ fkadj_status BatchEngine::add_problem(const fkadj_params& p, double dt, int nt, 
     fkadj_status s = pb->init(p, dt, nt, ai, nrows, ncols, n_num, gh_num, gamma, S_ncol, S_colptr, S_rowidx,
                               S_val, alpha, &o, need_obj);
     if (s) return s;
+    if (no_coop_) pb->no_run();
     BatchInstance bi;
     bi.P = pb->P_;
     bi.g = pb->g_;
@@ -523,6 +525,18 @@ fkadj_status BatchEngine::tick_action(Job& j, const Action& a) {
     return FKADJ_OK;
 }
 
+// The job from its first step again; out of memory, it is done with that status.
+fkadj_status BatchEngine::restart_job(Job& j) {
+    const fkadj_status s = prepare_job(j, nullptr);
+    if (s != FKADJ_ERR_NOMEM) return s;
+    probs_[j.prob]->run_off_ = false;
+    j.status = s;
+    j.gradE.clear();
+    j.done = true;
+    j.t_done = host_seconds();
+    return FKADJ_OK;
+}
+
 fkadj_status BatchEngine::finish_poll(Job& j) {
     const cudaError_t q = cudaEventQuery(j.ev);
     if (q == cudaErrorNotReady) return FKADJ_OK;
@@ -535,14 +549,7 @@ fkadj_status BatchEngine::finish_poll(Job& j) {
         // the memory, this job fails and the others go on.
         P.run_off_ = true;
         P.drop_sweep_buffers();
-        const fkadj_status s = prepare_job(j, nullptr);
-        if (s != FKADJ_ERR_NOMEM) return s;
-        P.run_off_ = false;
-        j.status = s;
-        j.gradE.clear();
-        j.done = true;
-        j.t_done = host_seconds();
-        return FKADJ_OK;
+        return restart_job(j);
     }
     P.run_off_ = false;
     const double l0 = -j.h_out[0];
@@ -632,7 +639,23 @@ fkadj_status BatchEngine::tick(int* active) {
         if (!j.finishing && j.pc < j.plan.size()) (j.swept ? swept : ready).push_back(id);
     }
     active_.swap(still);
-    if (!swept.empty() && (s = sweep_tick(swept))) return s;
+    if (!swept.empty()) {
+        const bool first = !no_coop_;
+        s = sweep_tick(swept);
+        if (s && first && no_coop_) {
+            // a cooperative launch was refused (Problem::no_run): all problems
+            // by the tile kernels from here on, these jobs from their start
+            for (auto& p : probs_)
+                if (p) p->no_run();
+            for (int id : swept)
+                if ((s = restart_job(*jobs_[id]))) return s;
+            active_.erase(std::remove_if(active_.begin(), active_.end(), [&](int id) { return jobs_[id]->done; }),
+                          active_.end());
+            if (active) *active = (int)active_.size();
+            return FKADJ_OK;
+        }
+        if (s) return s;
+    }
     int K = 1;
     if (block_graphs_ && !ready.empty()) {
         int m = kBlockMax;

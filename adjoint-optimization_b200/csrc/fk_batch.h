@@ -89,6 +89,7 @@ public:
 private:
     fkadj_status fail(cudaError_t e, const char* what);
     fkadj_status prepare_job(Job& j, const double* y_ini);
+    fkadj_status restart_job(Job& j);
     fkadj_status build_plan(Job& j);
     fkadj_status sweep_tick(const std::vector<int>& ready);
     template <class Job_, class Launch>
@@ -103,6 +104,7 @@ private:
     cudaMemPool_t pool_ = nullptr;  // device memory of the engine's problems
     int tiles_[4] = {0, 0, 0, 0};  // fwd, mid, adj presets; fused preset (fused_shape)
     int adj_path_ = 0;             // reference-adjoint path (Problem::AdjPath), from the autotuner
+    bool no_coop_ = false;      // a cooperative launch was refused as too large (Problem::no_run)
     bool tuned_ = false;        // presets fixed (options.tile > 0) or autotuned
     HermiteW hw_{};
     std::vector<std::unique_ptr<Problem>> probs_;

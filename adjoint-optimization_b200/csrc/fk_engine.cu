@@ -380,6 +380,7 @@ fkadj_status Problem::segment_launch() {
 fkadj_status Problem::fail_cuda(cudaError_t e, const char* what) {
     set_error(std::string(what) + ": " + cudaGetErrorString(e));
     cudaGetLastError();
+    no_coop_ = e == cudaErrorCooperativeLaunchTooLarge;
     return e == cudaErrorMemoryAllocation ? FKADJ_ERR_NOMEM : FKADJ_ERR_CUDA;
 }
 

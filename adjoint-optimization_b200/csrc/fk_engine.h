@@ -203,6 +203,14 @@ public:
                                const double* stages, double*& z, double*& z2, double* replayed = nullptr);
     fkadj_status init_sweeps(const uint8_t* flags);
     fkadj_status ensure_exchange();
+    // Sweeps as launches of the tile kernels from here on (the same bits): the
+    // device refused a cooperative launch of the grid's tiles, a CTA per SM (a
+    // stream may see fewer SMs than the device has).
+    void no_run() {
+        no_coop_ = false;
+        run_ = RunShape();
+        xchg_.release();
+    }
     // What only sweeps use.  (Kept stage states go with the plan: ensure_traj.)
     void drop_sweep_buffers() {
         for (DevBuf* b : {&xchg_, &pts_}) b->release();
@@ -342,6 +350,7 @@ private:
     // (FAULT_NAN), which they contain
     bool run_off_ = false;
     bool nan_seen_ = false;
+    bool no_coop_ = false;     // a cooperative launch was refused as too large
     bool refused_ = false;     // the last plan: refused by the caller's budget, whatever memory there is
     bool own_sweeps_ = true;  // false where memory is short
     bool shared_ = false;     // a batch engine's problem
@@ -415,6 +424,10 @@ fkadj_status Problem::with_sweeps(Call&& call) {
     nan_seen_ = refused_ = false;
     fkadj_status s = ensure_exchange();
     if (!s) s = call();
+    if (no_coop_) {
+        no_run();
+        s = call();
+    }
     if (s == FKADJ_ERR_NOMEM && sweeping() && !refused_) {
         // the preset kernels need less memory; where they lack it too, sweeps
         // were not what it was short for

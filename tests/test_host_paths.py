@@ -262,3 +262,29 @@ def test_a_repeat_without_memory_takes_the_sweeps_buffers(fake, mode, store):
             fake.fake_fail_allocations(-1, 0)
             pb.grad(inst.Et)
             assert fake.fake_launches(b"k_adj_run") >= runs + 2
+
+
+@pytest.mark.parametrize("store", STORES[:2])
+@pytest.mark.parametrize("mode", MODES)
+def test_a_refused_cooperative_launch_gives_way_to_tile_kernels(fake, mode, store):
+    """A stream that sees fewer SMs than the device has refuses a CTA per SM."""
+    inst = _inst()
+    fake.fake_refuse_cooperative(1)
+    call = (inst.Et, inst.dt, inst.nt, inst.y0, inst.active_index, inst.ncols, inst.nrows, inst.ghost)
+    api.fk_forward_Et(*call, 5, params=inst.params)
+    api.fk_grad_Et(*call, inst.gamma, inst.S, inst.alpha, params=inst.params, opts=_opts(inst, mode, store))
+    with api.Problem(inst, opts=_opts(inst, mode, store)) as pb:
+        pb.grad(inst.Et, inst.y0)
+        steps = fake.fake_launches(b"k_fwd_tile")
+        pb.objective(inst.Et)
+        assert fake.fake_launches(b"k_fwd_tile") == steps + inst.nt
+    with Batch() as b:
+        jobs = [b.submit(b.add_problem(inst, grad_mode=mode, ckpt_policy=store), inst.Et, inst.y0, want_grad=k > 0)
+                for k in range(3)]
+        b.run()
+        jobs.append(b.submit(b.add_problem(inst, grad_mode=mode, ckpt_policy=store), inst.Et, inst.y0))
+        b.run()
+        for j in jobs:
+            b.result(j)
+    assert fake.fake_launches(b"k_adj_tile") > 0
+    assert _sweeps(fake) == 0 and fake.fake_launches(b"k_fwd_step") == 0 and fake.fake_launches(b"k_batch") == 0
