@@ -101,6 +101,14 @@ __device__ __forceinline__ bool bulk_wait(uint32_t bar, uint64_t limit_ns = 1000
     return false;
 }
 
+// Waits once more, bounded, for windows first .. last of a ring of N barriers
+// in a row (window j arrives on barrier j % N): what a CTA that gives up does
+// before it returns, for all of its windows still in flight.
+template <int N>
+__device__ __forceinline__ void bulk_drain(uint32_t bars, int first, int last, uint64_t limit_ns = 1000000000ull) {
+    for (int j = first; j <= last; ++j) bulk_wait(bars + 8 * (j % N), limit_ns, (unsigned)(j / N) & 1u);
+}
+
 // bulk_wait for all threads of a CTA, with one outcome for all of them: true
 // when the posted bytes arrived.  When the wait expired in any thread, thread
 // 0 sets *fault (when non-null), the CTA waits once more, again bounded, for

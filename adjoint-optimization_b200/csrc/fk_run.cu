@@ -771,8 +771,7 @@ __device__ __forceinline__ void fetch_tile(const DevGrid& g, const TileWalk& w, 
 __device__ __forceinline__ bool window_arrived(bool ok, uint32_t bar, int n, bool next, unsigned* fault) {
     if (!__syncthreads_or(!ok)) return true;
     if (threadIdx.x == 0) atomicOr(fault, FAULT_TIMEOUT);
-    bulk_wait(bar + 8 * (n & 1), 1000000000ull, (unsigned)(n >> 1) & 1u);
-    if (next) bulk_wait(bar + 8 * (~n & 1), 1000000000ull, (unsigned)((n + 1) >> 1) & 1u);
+    bulk_drain<2>(bar, n, next ? n + 1 : n);
     return false;
 }
 
@@ -1030,7 +1029,10 @@ __device__ __forceinline__ void mid_run(const DevModel& P, const HermiteW& hw, c
             bits |= (unsigned)cells[off + (long long)(r0 + k) * g.ld + c] << (6 * k);
             G[(r0 + k) * RW + c] = gh[off + (long long)(r0 + k) * g.ld + c];
         }
-    if (!bulk_wait_cta(bar, r.fault)) return;
+    if (!bulk_wait_cta(bar, r.fault)) {
+        bulk_drain<3>(bar, 1, 1);  // the second window is in flight too
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < R; ++k)
         if (r0 + k < rows + 3) {
@@ -1067,8 +1069,7 @@ __device__ __forceinline__ void mid_run(const DevModel& P, const HermiteW& hw, c
             // a window did not arrive in time: as bulk_wait_cta, once more for
             // the copies in flight, then out
             if (threadIdx.x == 0) atomicOr(r.fault, FAULT_TIMEOUT);
-            for (int j = k + 1; j <= min(k + 2, k1); ++j)
-                bulk_wait(bar + 8 * ((j - k0) % 3), 1000000000ull, (unsigned)((j - k0) / 3) & 1u);
+            bulk_drain<3>(bar, k + 1 - k0, min(k + 2, k1) - k0);
             return;
         }
         double* yh = r.yh + (long long)k * r.stride + off;
