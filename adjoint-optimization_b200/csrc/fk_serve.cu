@@ -125,7 +125,11 @@ fkadj_status Server::start(const fkadj_options* opt, int64_t budget) {
 }
 
 void Server::stop() {
-    stop_ = true;
+    {
+        // (under the lock: a worker that has just found nothing to do would miss the notice)
+        std::lock_guard<std::mutex> lk(mu_);
+        stop_ = true;
+    }
     cv_.notify_all();
     for (auto& w : workers_)
         if (w.joinable()) w.join();

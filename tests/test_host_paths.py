@@ -6,6 +6,7 @@ sweep is handed must lie in live device memory."""
 import ctypes as C
 import os
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -288,3 +289,16 @@ def test_a_refused_cooperative_launch_gives_way_to_tile_kernels(fake, mode, stor
             b.result(j)
     assert fake.fake_launches(b"k_adj_tile") > 0
     assert _sweeps(fake) == 0 and fake.fake_launches(b"k_fwd_step") == 0 and fake.fake_launches(b"k_batch") == 0
+
+
+def test_a_server_stops_while_its_workers_go_to_sleep(fake_path, tmp_path):
+    """In a process of its own, which must end."""
+    slow = str(tmp_path / "slow_wait.so")
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", slow, os.path.join(HERE, "slow_wait.cpp"), "-ldl"], check=True)
+    code = ("import time\n"
+            "from fkadj.serve import Server\n"
+            "sv = Server(hbm_budget_bytes=1 << 30)\n"
+            "time.sleep(0.02)\n"
+            "sv.close()\n")
+    env = dict(os.environ, FKADJ_LIB=fake_path, LD_PRELOAD=slow, PYTHONPATH=PKG, OPENBLAS_NUM_THREADS="1")
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=60)
