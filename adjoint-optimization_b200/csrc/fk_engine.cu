@@ -695,20 +695,35 @@ fkadj_status Problem::ensure_exchange() {
     return FKADJ_OK;
 }
 
+int64_t Problem::padded_state_bytes(int nrows, int ncols) {
+    const int64_t ld = round_up(round_up(ncols, 64) + 2 * HALO, 8);
+    return 3 * 8 * ld * (round_up(nrows, 64) + 2 * HALO);
+}
+
+int64_t Problem::estimate_slack(int nrows, int ncols, int nt, int n_num, int grad_mode, int policy, bool want_grad) {
+    // row pointers of S, blocks of the objective's sum, pulse tables, words
+    int64_t b = 8 * ((int64_t)n_num + 1) + 8 * objective_blocks(n_num) + 8 * (3 * (int64_t)nt + 1) + 1024;
+    if (!want_grad) return b;
+    // the window of z.gh partials on row segments beyond all rows on the 16x16 lattice (the batch engine's)
+    const bool exact = grad_mode == FKADJ_GRAD_EXACT;
+    const size_t nsbx = round_up(ncols, 64) / 16, nsb16 = nsbx * (round_up(nrows, 64) / 16), nsbseg = nsbx * nrows;
+    const int c = policy == FKADJ_CKPT_FULL ? 0 : std::max(2, (int)std::ceil(std::sqrt((double)nt)));
+    const int64_t window = (int64_t)(exact ? 3 : 1) * partial_window(nt, exact, c, nsb16, nsbseg, true) * (int64_t)nsbseg;
+    return b + 8 * std::max<int64_t>(0, window - (int64_t)(3 * nt + 1) * (int64_t)nsb16);
+}
+
 int64_t Problem::estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t nnz, int grad_mode, int policy,
                                 bool want_grad, bool sweeps) {
-    const int64_t ld = round_up(round_up(ncols, 64) + 2 * HALO, 8);
-    const int64_t rows = round_up(nrows, 64) + 2 * HALO;
-    const int64_t plane = rows * ld * 8, state = 3 * plane;
+    const int64_t state = padded_state_bytes(nrows, ncols), plane = state / 3;
     const bool exact = grad_mode == FKADJ_GRAD_EXACT;
     int64_t b = plane + plane / 8 + (int64_t)n_num * (8 + 48) + nnz * 12 + 4 * state;  // geometry, compact, work
-    if (sweeps) b += 3 * (plane / 8) + 4 * state;                                      // flags, edge exchange
+    b += estimate_slack(nrows, ncols, nt, n_num, grad_mode, policy, want_grad);
+    if (sweeps) b += 3 * (plane / 8) + 4 * state;  // flags, edge exchange
     if (!want_grad) return b;
     const int64_t c = std::max(2, (int)std::ceil(std::sqrt((double)nt)));
     const int64_t nsb = (round_up(ncols, 64) / 16) * (round_up(nrows, 64) / 16);
-    int64_t partials = (int64_t)(3 * nt + 1) * (nsb + 1);
-    if (sweeps) partials = std::max(partials, (exact ? 3 : 1) * std::min<int64_t>(nt + 1, std::max<int64_t>(32, c)) * 16 * nsb);
-    b += 2 * state + partials * 8;  // adjoint pair, partials
+    // adjoint pair, partials
+    b += 2 * state + (int64_t)(3 * nt + 1) * (nsb + 1) * 8;
     if (sweeps)
         b += (int64_t)std::min(nt, sweep_chunk_of(state, exact)) * (exact ? 3 : 1) * state;  // a chunk's points
     else
@@ -1281,6 +1296,23 @@ fkadj_status Problem::ensure_traj(const TrajPlan& tp) {
     return FKADJ_OK;
 }
 
+// Rows per group in the window of z.gh partials of a standalone sweep (see
+// ensure_adjoint_work); stride: a sqrt store's, 0 otherwise.
+int Problem::partial_window(int nt, bool exact, int stride, size_t nsb16, size_t nsbseg, bool segs) {
+    const int per_group = exact ? nt : nt + 1;
+    int win = std::min(per_group, kPartialWindow);
+    if (stride > 0)
+        win = std::min(per_group, stride >= kPartialWindow ? stride : stride * (kPartialWindow / stride));
+    // rows of segment partials within the full rows of 16x16 partials
+    const size_t fit = (size_t)(3 * nt + 1) * (nsb16 + 1) / nsbseg / (size_t)(exact ? 3 : 1);
+    if (segs && (size_t)win > fit) {
+        const int c = stride > 0 ? stride : 1;
+        win = (int)std::max<size_t>(std::min<size_t>((size_t)win, fit / (size_t)c * (size_t)c),
+                                    (size_t)(stride > 0 ? c : std::min(win, 32)));
+    }
+    return win;
+}
+
 fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
     const bool sweep = sweeping() && !all_rows;
     // holes and everything off the grid: 0 for the sweeps, NaN for the preset kernels
@@ -1326,13 +1358,6 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
     // segment's rows never wrap around it.
     const size_t prow = (size_t)(3 * nt_ + 1);
     const int groups = grad_mode_ == FKADJ_GRAD_EXACT ? 3 : 1;
-    const int per_group = grad_mode_ == FKADJ_GRAD_EXACT ? nt_ : nt_ + 1;
-    const bool sqrt_store = traj_plan_.policy == FKADJ_CKPT_SQRT && traj_plan_.stride > 0;
-    int win = std::min(per_group, kPartialWindow);
-    if (sqrt_store) {
-        const int c = traj_plan_.stride;
-        win = std::min(per_group, c >= kPartialWindow ? c : c * (kPartialWindow / c));
-    }
     // Lattice of the partials: 16-cell row segments (16 times as many partials
     // as 16x16 sub-blocks; the adjoint tiles may then take any height, and the
     // sweeps write only the segments with a source) with windowed partials.
@@ -1343,14 +1368,10 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
     // lattice: the fused step, the batch engine's all-rows buffers, and under
     // FKADJ_ZGH_SEGMENTS=0.
     const size_t nsb16 = (size_t)nsbx_ * (size_t)nsby_, nsbseg = (size_t)nsbx_ * (size_t)g_.nrows;
-    const size_t fit = prow * (nsb16 + 1) / nsbseg / (size_t)groups;  // rows of segment partials within that count
     bool segs = !all_rows && (forced_path_ < 0 || forced_path_ == ADJ_SPLIT);
     if (const char* sv = getenv("FKADJ_ZGH_SEGMENTS")) segs = segs && std::atoi(sv) != 0;
-    if (segs && (size_t)win > fit) {
-        const int c = sqrt_store ? traj_plan_.stride : 1;
-        win = (int)std::max<size_t>(std::min<size_t>((size_t)win, fit / (size_t)c * (size_t)c),
-                                    (size_t)(sqrt_store ? c : std::min(win, 32)));
-    }
+    const int stride = traj_plan_.policy == FKADJ_CKPT_SQRT ? traj_plan_.stride : 0;
+    int win = partial_window(nt_, grad_mode_ == FKADJ_GRAD_EXACT, stride, nsb16, nsbseg, segs);
     if (all_rows) win = (int)prow;
     const size_t nsb = segs ? nsbseg : nsb16;
     const size_t pbytes = (all_rows ? prow : (size_t)groups * win) * nsb * sizeof(double);

@@ -99,10 +99,17 @@ public:
                       double* gradE, double* yf);
 
     int64_t device_bytes() const;
+    // The part of estimate_bytes that refuses no request: small tables, and
+    // what the window of z.gh partials on row segments takes beyond all rows on
+    // the 16x16 lattice.
+    static int64_t estimate_slack(int nrows, int ncols, int nt, int n_num, int grad_mode, int policy, bool want_grad);
+    // Bytes of one state of a grid as it lies on the device (3 padded planes).
+    static int64_t padded_state_bytes(int nrows, int ncols);
     // Device bytes a problem of this size will hold once a job has run
     // (geometry, work states, adjoint work, Jacobian caches, trajectory store
     // under `policy`), for admission control before anything is allocated.
-    // with `sweeps`, what a problem whose steps are sweeps holds (fk_run.h).
+    // With `sweeps`, what a problem whose steps are sweeps holds (fk_run.h).  A
+    // FULL store without k1 kept beside the states (TrajPlan::keep_f).
     static int64_t estimate_bytes(int nrows, int ncols, int nt, int n_num, int64_t nnz, int grad_mode,
                                   int policy, bool want_grad, bool sweeps = false);
     Timing last_timing() const { return timing_; }
@@ -267,6 +274,7 @@ private:
     cudaError_t flush_rows(int row);
     cudaError_t flush_range(int row0, int n);
     static constexpr int kPartialWindow = 512;
+    static int partial_window(int nt, bool exact, int stride, size_t nsb16, size_t nsbseg, bool segs);
     fkadj_status download_grid(const double* d_state, double* host_dense);
     double* slot(int k) const { return traj_.as<double>() + (size_t)k * state_elems(); }
     double* segslot(int k) const { return seg_.as<double>() + (size_t)k * state_elems(); }

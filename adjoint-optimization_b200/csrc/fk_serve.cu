@@ -45,9 +45,10 @@ struct Request {
     std::vector<double> gh, gamma, Sv, Et, y0;
     std::vector<int64_t> Jc, Ir;
     bool want_grad = true;
-    int64_t est = 0;
+    int64_t est = 0;         // device bytes it is charged for
     int64_t est_sweeps = 0;  // the same with sweeps, and where a NaN has the preset kernels repeat it
     bool sweeps = false;     // how it was admitted
+    bool keep_f = false;     // its full store holds k1 beside the states (a worker's request)
     // results
     int state = 0;  // 0 queued, 1 running, 2 done, 3 failed
     fkadj_status status = FKADJ_OK;
@@ -150,6 +151,8 @@ fkadj_status Server::run_alone(Request& r) {
     o.device = device_;
     o.ckpt_policy = opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT;
     o.ckpt_budget_bytes = budget_;
+    if (o.ckpt_policy == FKADJ_CKPT_FULL && opt_.grad_mode == FKADJ_GRAD_REF && !r.keep_f)
+        o.ckpt_budget_bytes = (r.nt + 1) * Problem::padded_state_bytes(r.nrows, r.ncols);  // the states alone
     fkadj_status s = pb->init(r.p, r.dt, r.nt, r.ai.data(), r.nrows, r.ncols, r.n_num, r.gh.data(), r.gamma.data(),
                               r.n_num, r.Jc.data(), r.Ir.data(), r.Sv.data(), r.alpha, &o, true);
     if (s) return s;
@@ -213,18 +216,25 @@ void Server::worker() {
 
 fkadj_status Server::submit(std::unique_ptr<Request> r, int64_t* id) {
     r->t_submit = host_seconds();
-    r->est = Problem::estimate_bytes(r->nrows, r->ncols, r->nt, r->n_num, (int64_t)r->Sv.size(), opt_.grad_mode,
-                                     opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT,
-                                     r->want_grad);
-    r->est_sweeps = Problem::estimate_bytes(r->nrows, r->ncols, r->nt, r->n_num, (int64_t)r->Sv.size(),
-                                            opt_.grad_mode,
-                                            opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT,
-                                            r->want_grad, true);
-    r->est_sweeps = std::max(r->est_sweeps, r->est);
-    if (r->est > budget_) {
+    const int policy = opt_.ckpt_policy == FKADJ_CKPT_FULL ? FKADJ_CKPT_FULL : FKADJ_CKPT_SQRT;
+    auto estimate = [&](bool sweeps) {
+        return Problem::estimate_bytes(r->nrows, r->ncols, r->nt, r->n_num, (int64_t)r->Sv.size(), opt_.grad_mode,
+                                       policy, r->want_grad, sweeps);
+    };
+    r->est = estimate(false);
+    // a request that fits but for this is not refused: it runs alone
+    const int64_t slack =
+        Problem::estimate_slack(r->nrows, r->ncols, r->nt, r->n_num, opt_.grad_mode, policy, r->want_grad);
+    if (r->est - slack > budget_) {
         set_error("request does not fit the HBM budget even alone");
         return FKADJ_ERR_NOMEM;
     }
+    if (streams_ && r->want_grad && policy == FKADJ_CKPT_FULL && opt_.grad_mode == FKADJ_GRAD_REF) {
+        const int64_t kept = r->nt * Problem::padded_state_bytes(r->nrows, r->ncols);
+        r->keep_f = r->est + kept <= budget_;
+        if (r->keep_f) r->est += kept;
+    }
+    r->est_sweeps = std::max(estimate(true), r->est);
     {
         std::lock_guard<std::mutex> lk(mu_);
         r->id = next_id_++;

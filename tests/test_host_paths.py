@@ -14,12 +14,14 @@ import pytest
 from fkadj import _lib, api, batch, serve, workloads as W
 from fkadj.batch import Batch
 from fkadj.serve import Server
+from test_gpu_edges import _custom as custom_mask
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = _lib.PKG_DIR
 MODES = [_lib.GRAD_REF, _lib.GRAD_EXACT]
 STORES = [_lib.CKPT_FULL, _lib.CKPT_SQRT, _lib.CKPT_BINOMIAL]
 FAULT_NAN = 2
+ESTIMATE = "_ZN5fkadj7Problem14estimate_bytesEiiiiliibb"
 
 
 @pytest.fixture(scope="module")
@@ -302,3 +304,36 @@ def test_a_server_stops_while_its_workers_go_to_sleep(fake_path, tmp_path):
             "sv.close()\n")
     env = dict(os.environ, FKADJ_LIB=fake_path, LD_PRELOAD=slow, PYTHONPATH=PKG, OPENBLAS_NUM_THREADS="1")
     subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=60)
+
+
+@pytest.mark.parametrize("mask", ["open", "pinched"])
+@pytest.mark.parametrize("nan", [False, True])
+@pytest.mark.parametrize("store", STORES[:2])
+@pytest.mark.parametrize("mode", MODES)
+def test_a_served_request_stays_within_the_budget(fake, monkeypatch, mode, store, nan, mask):
+    """The server's estimate bounds the device memory a request takes, with
+    sweeps or without (a cell between two holes), repeated after a NaN or not,
+    for budgets from the least that holds the estimate on; on a large grid with
+    a short horizon the partial sums' window is what counts."""
+    estimate = getattr(fake, ESTIMATE)
+    estimate.restype = C.c_int64
+    estimate.argtypes = [C.c_int] * 4 + [C.c_int64, C.c_int, C.c_int, C.c_bool, C.c_bool]
+    for rows, cols, nt in ((40, 72, 24), (131, 97, 90), (640, 500, 24)):
+        if mask == "pinched":
+            m = np.ones((rows, cols), bool)
+            m[10, 10] = m[12, 10] = False
+            inst = custom_mask(m, nt)
+        else:
+            inst = _inst(rows, cols, nt)
+        least = [estimate(rows, cols, nt, inst.n_num, inst.S.nnz, mode, store, g, False) for g in (True, False)]
+        for budget in [least[0], least[0] + 5 * _state_bytes(inst), 2 * least[0], 8 * least[0]]:
+            with Server(opts=_opts(inst, mode, store), hbm_budget_bytes=budget) as sv:
+                for grad in (True, False):
+                    _lib.check(fake.fkadj_release_cached_memory())
+                    fake.fake_reset(0)
+                    base = fake.fake_in_use()
+                    if nan:
+                        fake.fake_fault(b"k_fwd_", FAULT_NAN, 1)
+                    assert sv.wait(sv.submit(inst, want_grad=grad), 60)
+                    assert fake.fake_peak() - base <= budget, (rows, cols, nt, budget / least[0], grad)
+                assert sv.stats["failed"] == 0
