@@ -59,6 +59,15 @@ struct Request {
     int prob = -1, job = -1;
 };
 
+// Whether a request is admitted with sweeps, which take more memory than the
+// preset kernels: where that fits beside the running ones (`used` bytes), and
+// where it does not keep out the next waiting request (next bytes; < 0: none)
+// that would be admitted beside it otherwise.
+bool admit_sweeps(int64_t budget, int64_t used, int64_t est, int64_t est_sweeps, int64_t next) {
+    const bool keeps_out = next >= 0 && used + est_sweeps + next > budget && used + est + next <= budget;
+    return used + est_sweeps <= budget && !keeps_out;
+}
+
 class Server {
 public:
     ~Server() { stop(); }
@@ -74,6 +83,8 @@ private:
     void loop();
     void worker();
     fkadj_status admit(Request& r);
+    // device bytes of the k-th waiting request with the preset kernels, -1: none
+    int64_t waiting(size_t k) { return k < queue_.size() ? reqs_[queue_[k]]->est : -1; }
     fkadj_status run_alone(Request& r);
     bool streams_ = true;
     int nworkers_ = 4;
@@ -187,8 +198,7 @@ void Server::worker() {
             r = reqs_[id].get();
             r->state = 1;
             r->t_admit = host_seconds();
-            // sweeps take more memory than the preset kernels: where it is there
-            r->sweeps = used_ + r->est_sweeps <= budget_;
+            r->sweeps = admit_sweeps(budget_, used_, r->est, r->est_sweeps, waiting(0));
             if (r->sweeps) r->est = r->est_sweeps;
             used_ += r->est;
             running_.push_back(id);
@@ -292,7 +302,7 @@ void Server::loop() {
             while (!queue_.empty() && (int)running_.size() < kBatchMaxItems) {
                 Request& r = *reqs_[queue_.front()];
                 if (used_ + r.est > budget_ && !running_.empty()) break;
-                r.sweeps = used_ + r.est_sweeps <= budget_;
+                r.sweeps = admit_sweeps(budget_, used_, r.est, r.est_sweeps, waiting(1));
                 if (r.sweeps) r.est = r.est_sweeps;
                 lk.unlock();
                 fkadj_status s = admit(r);

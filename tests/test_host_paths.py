@@ -21,6 +21,7 @@ PKG = _lib.PKG_DIR
 MODES = [_lib.GRAD_REF, _lib.GRAD_EXACT]
 STORES = [_lib.CKPT_FULL, _lib.CKPT_SQRT, _lib.CKPT_BINOMIAL]
 FAULT_NAN = 2
+ADMIT = "_ZN5fkadj12admit_sweepsElllll"
 ESTIMATE = "_ZN5fkadj7Problem14estimate_bytesEiiiiliibb"
 
 
@@ -337,3 +338,16 @@ def test_a_served_request_stays_within_the_budget(fake, monkeypatch, mode, store
                     assert sv.wait(sv.submit(inst, want_grad=grad), 60)
                     assert fake.fake_peak() - base <= budget, (rows, cols, nt, budget / least[0], grad)
                 assert sv.stats["failed"] == 0
+
+
+@pytest.mark.parametrize("budget,used,est,est_sweeps,following,want", [
+    (100, 0, 40, 60, -1, True), (100, 0, 40, 100, -1, True), (100, 0, 40, 101, -1, False),
+    (100, 40, 40, 60, -1, True), (100, 41, 40, 60, -1, False),
+    (100, 0, 40, 60, 40, True),     # both fit
+    (100, 0, 40, 61, 40, False),    # the next one fits beside the preset kernels only
+    (100, 0, 40, 61, 61, True)])    # the next one waits either way
+def test_sweeps_do_not_keep_the_next_request_out(fake, budget, used, est, est_sweeps, following, want):
+    admit = getattr(fake, ADMIT)
+    admit.restype = C.c_bool
+    admit.argtypes = [C.c_int64] * 5
+    assert admit(budget, used, est, est_sweeps, following) == want
