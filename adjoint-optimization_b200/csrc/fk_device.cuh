@@ -106,9 +106,11 @@ __device__ __forceinline__ double fk_rcp_finite(double x) {
 // exact gradient 512^2 x 500 29.9 -> 28.3 ms, 2048^2 x 24 24.2 -> 22.8 ms.
 // Within 1.2 ulp of e^x for x in [-707, 692]; it saturates instead of
 // overflowing: the result stays in [2^-1020, 2^1000) (m is clamped), so the
-// smoothed steps need no cap of their own.  A NaN argument gives NaN; beyond
-// |s d| = 2^51 (a state that has blown up) and at infinities the value is
-// unspecified.
+// smoothed steps need no cap of their own.  K is read from the sum's low word:
+// beyond |s d| = 2^31 (at the steps' slope of 100, |u| above 4.6e5: a state
+// that has blown up) the value is one of that range, but not always the limit
+// on the argument's side; beyond 2^51 and at infinities it is unspecified.  A
+// NaN argument gives NaN.
 __shared__ double fk_exp2_tab[16];
 // 2^(j/16), j = 0..15
 __constant__ double kExp2Tab[16] = {
