@@ -1195,6 +1195,34 @@ fkadj_status Problem::default_budget() {
     return FKADJ_OK;
 }
 
+// What a backward step under the binomial store costs a swept problem beside
+// one under the sqrt store with all it needs at hand, in forward steps: the
+// reference mode's launches for two steps in place of a chunk's, and the copy
+// of the state kept between them; the exact mode's replay, which gives the
+// state between the two as well, and launches.  (Grids that do not fit the
+// device at once launch per step either way.)  From full gradients, ms with
+// the sqrt and the binomial store by the states in the budget:
+//                              fewest       a half      all but a few
+//   256 x 256 x 400             8.6 17.5    8.6 17.2     8.6 16.9
+//     exact                    10.4 15.5    8.3 14.8     8.3 14.1
+//   512 x 512 x 400            20.0 29.4   20.0 27.8    20.0 26.0
+//     exact                    22.6 27.0   18.1 25.1    18.1 23.5
+//   700 x 600 x 300            33.0 37.5   33.1 34.4    33.2 30.6
+//     exact                    39.5 37.7   31.5 34.1    31.5 30.6
+//   1024 x 768 x 200           32.9 38.0   32.9 35.3    32.9 31.7
+//     exact                    38.0 37.3   30.5 34.7    30.5 31.4
+//   2048 x 2048 x 60           50.6 52.8   50.6 50.4    50.6 46.0
+//     exact                    55.3 51.8   55.3 49.5    45.1 45.5
+// A forward step of these takes 5.3, 11.1, 28, 39 and 196 us.
+// *forward_us: the step it is counted in.
+double Problem::binomial_step_cost(double* forward_us) const {
+    const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
+    const double cells = (double)g_.nrows * g_.ncols;
+    *forward_us = run_.id >= 0 ? 3.0 + 31e-6 * cells : 6.0 + 46e-6 * cells;
+    if (run_.id >= 0) return exact ? 1.0 + 14.0 / *forward_us : 26.0 / *forward_us;
+    return exact ? 0.9 : 0.3 + 12.0 / *forward_us;
+}
+
 fkadj_status Problem::plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only) {
     if (ckpt_budget_ <= 0) {  // a one-shot call's: init leaves it to the gradient
         if (fkadj_status s = default_budget()) return s;
@@ -1212,17 +1240,30 @@ fkadj_status Problem::plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only) {
         } else if ((double)sqrt_slots * sb <= (double)ckpt_budget_) {
             pol = FKADJ_CKPT_SQRT;
             if (!sqrt_or_full_only && bino_fit >= 2) {
-                // recomputed forward steps: sqrt recomputes every segment but its
-                // first state; the binomial reversal what binomial_recompute_steps
-                // counts, plus (reference mode) the work the sqrt store saves each
-                // backward step (k1 kept beside the segment, no state copy per
-                // visit): measured on B200 at 512^2 x 20000 as 15.5 us per
-                // backward step, 0.9 of a forward step
+                // In forward steps: sqrt recomputes every segment but its first
+                // state, the binomial reversal what binomial_recompute_steps
+                // counts, plus (reference mode) the work the sqrt store saves
+                // the preset kernels each backward step (k1 kept beside the
+                // segment, no state copy per visit): 15.5 us at 512^2 x 20000,
+                // 0.9 of a forward step
                 const int K = (nt_ + c - 1) / c;
-                const double sqrt_cost = (double)(nt_ - K);
-                const double bino_cost = (double)binomial_recompute_steps(nt_, bino_slots - 2) +
-                                         (grad_mode_ == FKADJ_GRAD_REF ? 0.9 * nt_ : 0.0);
-                if (bino_cost < sqrt_cost) pol = FKADJ_CKPT_BINOMIAL;
+                const double sqrt_steps = (double)(nt_ - K);
+                const double bino_steps = (double)binomial_recompute_steps(nt_, bino_slots - 2);
+                const bool exact = grad_mode_ == FKADJ_GRAD_EXACT;
+                double gain = sqrt_steps - bino_steps - (exact ? 0.0 : 0.9 * nt_);  // of BINOMIAL
+                if (swept_) {
+                    // sweeps: each store's own work per backward step; the sqrt
+                    // store replays too where no stage states fit (exact mode)
+                    double us = 0;
+                    const bool replays = exact && (double)(sqrt_slots + 3 * c) * sb > (double)ckpt_budget_;
+                    const double swept_gain =
+                        sqrt_steps + (replays ? nt_ : 0) - bino_steps - nt_ * binomial_step_cost(&us);
+                    // (on small grids the first figure keeps the choice where
+                    // the two differ by less than 2 ms: the plans that callers
+                    // of short gradients know stay)
+                    if (run_.id < 0 || std::fabs(swept_gain) * us > 2000.0) gain = swept_gain;
+                }
+                if (gain > 0) pol = FKADJ_CKPT_BINOMIAL;
             }
         } else {
             pol = FKADJ_CKPT_BINOMIAL;

@@ -240,12 +240,12 @@ private:
     // a call that sweeps, repeated with per-step launches where check_fault found FAULT_NAN
     template <class Call> fkadj_status with_sweeps(Call&& call);
     // Resolves the checkpoint policy.  AUTO takes FULL when the budget holds
-    // every state, else whichever of SQRT and BINOMIAL fits and recomputes
-    // fewer forward steps (costed in forward-step equivalents, the binomial
-    // reference-mode reversal's extra per-step work, measured at 0.9 of a
-    // forward step, included); with
-    // sqrt_or_full_only (the batch engine, which runs no binomial schedule)
-    // BINOMIAL only when SQRT does not fit.
+    // every state, else whichever of SQRT and BINOMIAL fits and costs less,
+    // counted in forward-step equivalents (the work of each per backward step
+    // included); with sqrt_or_full_only (the batch
+    // engine, which runs no binomial schedule) BINOMIAL only when SQRT does not
+    // fit.
+    double binomial_step_cost(double* forward_us) const;
     fkadj_status default_budget();
     fkadj_status plan_trajectory(TrajPlan& tp, bool sqrt_or_full_only = false);
     int64_t kept_states(const TrajPlan& tp) const;
