@@ -676,7 +676,10 @@ fkadj_status Problem::init_sweeps(const uint8_t* flags) {
     const RunShape shape = coop ? run_shape(g_, sms_) : RunShape();
     const size_t nseg = (size_t)nsbx_ * g_.nrows;
     // the three as they lie one after the other in the set-up's block
-    CK(flags_.alloc(2 * flag_bytes() + nseg), "alloc cell flags");
+    if (flags_.alloc(2 * flag_bytes() + nseg) != cudaSuccess) {
+        cudaGetLastError();  // no memory for them: the preset kernels
+        return FKADJ_OK;
+    }
     CK(cudaMemcpyAsync(flags_.p, flags, flags_.bytes, cudaMemcpyHostToDevice, st_), "upload cell flags");
     run_ = shape;
     swept_ = true;

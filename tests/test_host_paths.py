@@ -388,3 +388,29 @@ def test_a_process_prepares_the_sweep_kernels_it_launches(fake_path):
             "    assert n() == [1, 1, 1, 0, 0, 0, 0], n()\n")
     env = dict(os.environ, FKADJ_LIB=fake_path, PYTHONPATH=PKG)
     subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=60)
+
+
+def test_a_problem_without_memory_for_the_flags_or_the_exchange_is_made_all_the_same(fake, monkeypatch):
+    """What the preset kernels need is asked for; nothing is left behind where that fails."""
+    inst = _inst()
+
+    def made(k):
+        before = fake.fake_in_use()
+        fake.fake_fail_allocations(k, 1)
+        try:
+            with api.Problem(inst) as pb:
+                n = fake.fake_allocations()
+                fake.fake_fail_allocations(-1, 0)
+                pb.grad(inst.Et, inst.y0)
+                return n
+        except _lib.FkadjError as e:
+            assert e.status == _lib.ERR_NOMEM
+        finally:
+            fake.fake_fail_allocations(-1, 0)
+            assert fake.fake_in_use() == before
+    monkeypatch.setenv("FKADJ_SWEEPS", "0")
+    preset = made(-1)
+    monkeypatch.delenv("FKADJ_SWEEPS")
+    swept = made(-1)
+    assert swept == preset + 2
+    assert sum(made(k) is not None for k in range(swept)) == 2
