@@ -2,15 +2,24 @@
 //
 // Each job (one objective or one gradient of one resident Problem) is a fixed
 // program of actions: nt forward steps, the objective at T, the backward sweep
-// (with sqrt-checkpoint segment recomputes), and a final reduction.  A tick
-// takes the next action of every active job and runs them as at most three
-// launches -- all forward-type steps, all midpoint steps, all adjoint steps of
-// every job -- through the batched persistent kernels (k_batch_*), whose work
-// queues reach the device in one small copy per tick.  Jobs of different grid
-// sizes and horizons therefore
-// share every launch, small grids fill the GPU together, and a job finishing or
-// starting changes only the next tick's queue.  The reference has no batching
-// (one instance per MATLAB call, simple_grad_desc.m:82).
+// (with sqrt-checkpoint segment recomputes), and a final reduction.
+//
+// A tick takes a run of actions of every active job whose problem sweeps
+// (sweep_tick): up to kBlockMax forward steps, or a recomputed segment, then a
+// chunk of backward steps with its midpoints.  The runs of all jobs of one
+// model share launches (launch_fwd_jobs and so on, fk_run.h), their tiles
+// packed into as few as hold them.
+//
+// Of the other jobs (fixed presets, a cell between two holes, the repeat after
+// a NaN, short memory) a tick takes the next action each, as at most three
+// launches -- all forward-type steps, all midpoint steps, all adjoint steps --
+// through the batched persistent kernels (k_batch_*), whose work queues reach
+// the device in one small copy; runs of such ticks replay as graphs.
+//
+// Jobs of different grid sizes and horizons therefore share launches, small
+// grids fill the GPU together, and a job finishing or starting changes only
+// the next tick.  The reference has no batching (one instance per MATLAB call,
+// simple_grad_desc.m:82).
 #pragma once
 
 #include <cstdint>

@@ -1,6 +1,9 @@
-// fk_kernels.cu -- sm_100a kernels of the FK forward / adjoint engine.
+// fk_kernels.cu -- sm_100a kernels of the FK forward / adjoint engine that
+// launch per step (presets), and the reductions, layout and objective kernels.
 //
-// Every time step is one fused launch.  A CTA owns a TX x TY tile of the grid,
+// The steps run here where a problem does not sweep (fk_run.cu): fixed presets,
+// a cell between two opposite holes, a NaN to contain, short memory.  A step
+// then is one fused launch.  A CTA owns a TX x TY tile of the grid,
 // stages the tile plus a HALO-wide ring of each field into shared memory once,
 // and runs all four RK stages out of shared memory: stage s is evaluated on the
 // tile grown by (4 - s) cells, so the halo shrinks by one cell per stage and no

@@ -1146,8 +1146,8 @@ static cudaError_t run_packed(const Job* j, int n, int sms, Launch&& launch) {
 size_t run_exchange_bytes(const DevGrid& g) { return 2 * 3 * (size_t)g.plane * sizeof(Tagged); }
 
 // Lets kernel K take its dynamic shared memory, once per device.  By the
-// launch that needs it: all instances at once, which loads them, held the
-// first problem of a process 45 ms.
+// launch that needs it: all instances at once, which loads them, held
+// the first problem of a process up by 45 ms.
 template <auto K>
 static cudaError_t allow_smem(size_t smem) {
     static std::atomic<uint64_t> done{0};

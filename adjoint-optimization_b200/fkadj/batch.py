@@ -1,8 +1,8 @@
 """Batched execution of many independent FK problems (C ABI fkadj_batch_*).
 
-Every tick advances every running job by one step; the steps of all jobs run
-as at most three launches of the persistent batched kernels, so instances of
-different grid sizes and horizons fill the GPU together.
+Every tick advances every running job by a run of steps (by one step where a
+problem does not sweep), and the runs of all jobs share launches, so instances
+of different grid sizes and horizons fill the GPU together.
 """
 from __future__ import annotations
 

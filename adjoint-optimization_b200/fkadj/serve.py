@@ -1,8 +1,9 @@
 """Continuous-batching request server (C ABI fkadj_server_*).
 
-A worker thread inside the library owns the GPU; requests submitted from any
-thread are admitted between ticks by device-memory footprint and share the
-batched launches with the requests already running.
+Requests submitted from any thread are admitted in arrival order by
+device-memory footprint and run by a pool of worker threads inside the library,
+each on a stream of its own, or (FKADJ_SERVE_MODE=ticks) by one batch engine
+whose launches they share.
 """
 from __future__ import annotations
 
