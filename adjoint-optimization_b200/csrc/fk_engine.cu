@@ -437,6 +437,7 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
         std::lock_guard<std::mutex> lk(g_init_mu);
         if (device_ < 64 && !g_init_done[device_]) {
             CK(kernels_init(), "kernel attribute setup");
+            CK(run_init(), "kernel attribute setup");
             g_init_done[device_] = true;
         }
     }

@@ -29,7 +29,6 @@
 #include "fk_run.h"
 
 #include <algorithm>
-#include <atomic>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -1019,7 +1018,6 @@ static ShapeInfo shape_info(int id) {
 #define DO(S) return {S::TX, S::R, S::TYM, S::RW, S::THREADS}
         FKADJ_RUN_LIST(X)
 #undef DO
-#undef X
     }
     return {};
 }
@@ -1145,25 +1143,32 @@ static cudaError_t run_packed(const Job* j, int n, int sms, Launch&& launch) {
 
 size_t run_exchange_bytes(const DevGrid& g) { return 2 * 3 * (size_t)g.plane * sizeof(Tagged); }
 
-// Lets kernel K take its dynamic shared memory, once per device.  By the
-// launch that needs it: all instances at once, which loads them, held
-// the first problem of a process up by 45 ms.
-template <auto K>
-static cudaError_t allow_smem(size_t smem) {
-    static std::atomic<uint64_t> done{0};
-    int device = 0;
-    if (const cudaError_t e = cudaGetDevice(&device)) return e;
-    const uint64_t bit = device < 64 ? 1ull << device : 0;
-    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (!e) done.fetch_or(bit, std::memory_order_relaxed);
+cudaError_t run_init() {
+    cudaError_t e = cudaFuncSetAttribute(k_mid_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MidShape::SMEM);
+    if (!e) e = cudaFuncSetAttribute(k_mid_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MidShape::SMEM);
+    const int big = (int)TileShapeBig::SMEM;
+    if (!e) e = cudaFuncSetAttribute(k_fwd_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (!e) e = cudaFuncSetAttribute(k_adj_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (!e) e = cudaFuncSetAttribute(k_adj_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+#undef X
+#define N_(K, smem) \
+    if (!e) e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem))
+#define X(id, a, b, c)                                                    \
+    N_((k_fwd_run<a, b, c>), (Shape<a, b, c>::SMEM));                  \
+    N_((k_fwd_jobs<a, b, c>), (Shape<a, b, c>::SMEM));           \
+    N_((k_adj_run<a, b, c, false>), (Shape<a, b, c>::SMEM));           \
+    N_((k_adj_jobs<a, b, c, false>), (Shape<a, b, c>::SMEM));    \
+    N_((k_adj_run<a, b, c, true>), (Shape<a, b, c>::SMEM_EXACT));      \
+    N_((k_adj_jobs<a, b, c, true>), (Shape<a, b, c>::SMEM_EXACT));
+    FKADJ_RUN_LIST(X)
+#undef X
+#undef N_
     return e;
 }
 
-template <auto K, class Jobs>
-static cudaError_t launch_run(int tiles, int threads, size_t smem, cudaStream_t st, const DevModel& P,
+template <class K, class Jobs>
+static cudaError_t launch_run(K kernel, int tiles, int threads, size_t smem, cudaStream_t st, const DevModel& P,
                               const Jobs& jobs) {
-    if (const cudaError_t e = allow_smem<K>(smem)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles);
     cfg.blockDim = dim3(threads);
@@ -1174,7 +1179,7 @@ static cudaError_t launch_run(int tiles, int threads, size_t smem, cudaStream_t 
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, K, P, jobs);
+    return cudaLaunchKernelEx(&cfg, kernel, P, jobs);
 }
 
 template <class Job>
@@ -1189,7 +1194,7 @@ cudaError_t launch_fwd_run(const RunShape& s, const DevModel& P, const FwdJob& j
     if (j.r.n <= 0) return cudaSuccess;
     switch (s.id) {
 #define X(id, a, b, c) \
-    case id: return launch_run<k_fwd_run<a, b, c>>(s.tiles(), s.threads, Shape<a, b, c>::SMEM, st, P, placed(s, j));
+    case id: return launch_run(k_fwd_run<a, b, c>, s.tiles(), s.threads, Shape<a, b, c>::SMEM, st, P, placed(s, j));
         FKADJ_RUN_LIST(X)
 #undef X
     }
@@ -1202,8 +1207,8 @@ cudaError_t launch_adj_run(const RunShape& s, bool exact, const DevModel& P, con
     switch (s.id) {
 #define X(id, a, b, c)                                                                                                 \
     case id:                                                                                                           \
-        return exact ? launch_run<k_adj_run<a, b, c, true>>(s.tiles(), s.threads, Shape<a, b, c>::SMEM_EXACT, st, P, q) \
-                     : launch_run<k_adj_run<a, b, c, false>>(s.tiles(), s.threads, Shape<a, b, c>::SMEM, st, P, q);
+        return exact ? launch_run(k_adj_run<a, b, c, true>, s.tiles(), s.threads, Shape<a, b, c>::SMEM_EXACT, st, P, q) \
+                     : launch_run(k_adj_run<a, b, c, false>, s.tiles(), s.threads, Shape<a, b, c>::SMEM, st, P, q);
         FKADJ_RUN_LIST(X)
 #undef X
     }
@@ -1215,7 +1220,7 @@ cudaError_t launch_fwd_jobs(const DevModel& P, const FwdJob* j, int n, int sms, 
         ++*launches;
         switch (id) {
 #define X(id, a, b, c) \
-    case id: return launch_run<k_fwd_jobs<a, b, c>>(tiles, threads, Shape<a, b, c>::SMEM, st, P, jobs);
+    case id: return launch_run(k_fwd_jobs<a, b, c>, tiles, threads, Shape<a, b, c>::SMEM, st, P, jobs);
             FKADJ_RUN_LIST(X)
 #undef X
         }
@@ -1230,8 +1235,8 @@ cudaError_t launch_adj_jobs(bool exact, const DevModel& P, const AdjJob* j, int 
         switch (id) {
 #define X(id, a, b, c)                                                                                           \
     case id:                                                                                                     \
-        return exact ? launch_run<k_adj_jobs<a, b, c, true>>(tiles, threads, Shape<a, b, c>::SMEM_EXACT, st, P, jobs) \
-                     : launch_run<k_adj_jobs<a, b, c, false>>(tiles, threads, Shape<a, b, c>::SMEM, st, P, jobs);
+        return exact ? launch_run(k_adj_jobs<a, b, c, true>, tiles, threads, Shape<a, b, c>::SMEM_EXACT, st, P, jobs) \
+                     : launch_run(k_adj_jobs<a, b, c, false>, tiles, threads, Shape<a, b, c>::SMEM, st, P, jobs);
             FKADJ_RUN_LIST(X)
 #undef X
         }
@@ -1265,7 +1270,6 @@ cudaError_t launch_fwd_tile(const DevModel& P, const DevGrid& g, const double* g
                             const FwdStep& r, int sms, cudaStream_t st) {
     using S = TileShapeBig;
     const TileWalk w = tile_walk(g, sms);
-    if (const cudaError_t e = allow_smem<k_fwd_tile>(S::SMEM)) return e;
     k_fwd_tile<<<std::min(sms, w.tiles), S::THREADS, S::SMEM, st>>>(P, g, gh, cells, r, w);
     return cudaGetLastError();
 }
@@ -1274,8 +1278,6 @@ cudaError_t launch_adj_tile(bool exact, const DevModel& P, const DevGrid& g, con
                             const uint8_t* segs, const AdjStep& r, int sms, cudaStream_t st) {
     using S = TileShapeBig;
     const TileWalk w = tile_walk(g, sms);
-    if (const cudaError_t e = exact ? allow_smem<k_adj_tile<true>>(S::SMEM) : allow_smem<k_adj_tile<false>>(S::SMEM))
-        return e;
     if (exact) k_adj_tile<true><<<std::min(sms, w.tiles), S::THREADS, S::SMEM, st>>>(P, g, gh, adj, segs, r, w);
     else k_adj_tile<false><<<std::min(sms, w.tiles), S::THREADS, S::SMEM, st>>>(P, g, gh, adj, segs, r, w);
     return cudaGetLastError();
@@ -1313,15 +1315,12 @@ cudaError_t launch_mid_run(const DevModel& P, const HermiteW& hw, const MidJob& 
     if (j.r.n <= 0) return cudaSuccess;
     MidJob q = j;
     const int ctas = place_mid(&q, 1, sms);
-    if (const cudaError_t e = allow_smem<k_mid_run>(MidShape::SMEM)) return e;
     k_mid_run<<<ctas, MidShape::THREADS, MidShape::SMEM, st>>>(P, hw, q);
     return cudaGetLastError();
 }
 
 cudaError_t launch_mid_jobs(const DevModel& P, const HermiteW& hw, const MidJob* j, int n, int sms, cudaStream_t st,
                             int64_t* launches) {
-    if (n <= 0) return cudaSuccess;
-    if (const cudaError_t e = allow_smem<k_mid_jobs>(MidShape::SMEM)) return e;
     for (int q0 = 0; q0 < n; q0 += kRunJobs) {
         RunJobs<MidJob> jobs;
         jobs.n = std::min(kRunJobs, n - q0);

@@ -34,6 +34,7 @@ void run_tile(const DevGrid& g, const RunShape& s, int sms, bool midpoint, int t
 
 // The shape for grid g on a device with `sms` multiprocessors (id -1: none).
 RunShape run_shape(const DevGrid& g, int sms);
+cudaError_t run_init();
 
 // Bytes of the exchange area of grid g's sweeps (zeroed once; see k_fwd_run).
 size_t run_exchange_bytes(const DevGrid& g);

@@ -35,7 +35,6 @@ struct Tables {
     std::map<uintptr_t, size_t> live;          // device allocations
     std::map<const void*, void*> symbols;
     std::map<std::string, int64_t> launches;
-    std::map<const void*, int> smem;           // dynamic shared memory allowed
 };
 Tables& tables() {
     static Tables* t = new Tables;
@@ -223,13 +222,6 @@ int64_t fake_launches(const char* kernel) {
         if (l.first.find(kernel) != std::string::npos) n += l.second;
     return n;
 }
-// kernels whose shared memory was allowed: each is loaded by that
-int64_t fake_prepared(const char* kernel) {
-    Lock lk(tables().mu);
-    int64_t n = 0;
-    for (auto& f : tables().smem) n += tables().names[f.first].find(kernel) != std::string::npos;
-    return n;
-}
 int64_t fake_bad_spans() { Lock lk(tables().mu); return bad; }
 const char* fake_first_bad() { return first_bad.c_str(); }
 
@@ -259,12 +251,7 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
     *static_cast<void**>(st) = pushed.st;
     return cudaSuccess;
 }
-static bool allowed(const void* f, size_t smem) {
-    Lock lk(tables().mu);
-    return smem <= 48 << 10 || (size_t)tables().smem[f] >= smem;
-}
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t smem, cudaStream_t) {
-    if (!allowed(f, smem)) return cudaErrorInvalidValue;
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t) {
     launched(f, args);
     return cudaSuccess;
 }
@@ -272,15 +259,10 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
     for (unsigned k = 0; k < c->numAttrs; ++k)
         if (c->attrs[k].id == cudaLaunchAttributeCooperative && c->attrs[k].val.cooperative && refuse_cooperative)
             return cudaErrorCooperativeLaunchTooLarge;
-    if (!allowed(f, c->dynamicSmemBytes)) return cudaErrorInvalidValue;
     launched(f, args);
     return cudaSuccess;
 }
-cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
-    Lock lk(tables().mu);
-    if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) tables().smem[f] = v;
-    return cudaSuccess;
-}
+cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) {
     *n = 1;
     return cudaSuccess;

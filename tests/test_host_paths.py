@@ -370,26 +370,6 @@ def test_auto_takes_the_store_that_sweeps_cost_less(fake, rows, cols, nt, mode, 
         assert pb.last_plan["policy"] == want
 
 
-def test_a_process_prepares_the_sweep_kernels_it_launches(fake_path):
-    """Each one at its first launch: allowing a kernel its shared memory loads
-    it, and all 53 of them held the first problem of a process up by 45 ms."""
-    code = ("import ctypes as C\n"
-            "from fkadj import _lib, api, workloads as W\n"
-            "L = _lib.load()\n"
-            "n = lambda: [int(L.fake_prepared(k)) for k in (b'k_fwd_run', b'k_adj_run', b'k_mid_run', b'k_fwd_jobs',\n"
-            "             b'k_adj_jobs', b'k_mid_jobs', b'_tile')]\n"
-            "inst = W.make_instance(40, 24, ncols=72, seed=1, n_obstacles=3, intervals=3)\n"
-            "with api.Problem(inst) as pb:\n"
-            "    assert sum(n()) == 0, n()\n"
-            "    pb.objective(inst.Et, inst.y0)\n"
-            "    assert n() == [1, 0, 0, 0, 0, 0, 0], n()\n"
-            "    pb.grad(inst.Et)\n"
-            "    pb.grad(inst.Et)\n"
-            "    assert n() == [1, 1, 1, 0, 0, 0, 0], n()\n")
-    env = dict(os.environ, FKADJ_LIB=fake_path, PYTHONPATH=PKG)
-    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=60)
-
-
 def test_a_problem_without_memory_for_the_flags_or_the_exchange_is_made_all_the_same(fake, monkeypatch):
     """What the preset kernels need is asked for; nothing is left behind where that fails."""
     inst = _inst()
