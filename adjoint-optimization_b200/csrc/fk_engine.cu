@@ -1413,7 +1413,8 @@ fkadj_status Problem::ensure_adjoint_work(bool all_rows) {
     // FKADJ_ZGH_SEGMENTS=0.
     const size_t nsb16 = (size_t)nsbx_ * (size_t)nsby_, nsbseg = (size_t)nsbx_ * (size_t)g_.nrows;
     bool segs = !all_rows && (forced_path_ < 0 || forced_path_ == ADJ_SPLIT);
-    if (const char* sv = getenv("FKADJ_ZGH_SEGMENTS")) segs = segs && std::atoi(sv) != 0;
+    // (a problem that sweeps was made without it: init_sweeps)
+    if (const char* sv = sweep ? nullptr : getenv("FKADJ_ZGH_SEGMENTS")) segs = segs && std::atoi(sv) != 0;
     const int stride = traj_plan_.policy == FKADJ_CKPT_SQRT ? traj_plan_.stride : 0;
     int win = partial_window(nt_, grad_mode_ == FKADJ_GRAD_EXACT, stride, nsb16, nsbseg, segs);
     if (all_rows) win = (int)prow;

@@ -117,6 +117,7 @@ struct Check {
         states(r.y_lo, 1, "y_lo");
         states(r.y_mid, r.n - 1, "y_mid");
         for (int k = 0; k < r.n; ++k) states(r.pts + (long long)k * r.pts_step * r.stride, exact ? 3 : 1, "pts");
+        if (r.nsb < (long long)r.nsbx * g.nrows && bad++ == 0) first_bad = kernel + " rows of partial sums";
         table(r.partial, sizeof(double) * (exact ? 3 : 1) * r.window * r.nsb, "partial");
         table(r.exchange, run_exchange_bytes(g), "exchange");
         fault(r.fault);

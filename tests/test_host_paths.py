@@ -394,3 +394,14 @@ def test_a_problem_without_memory_for_the_flags_or_the_exchange_is_made_all_the_
     swept = made(-1)
     assert swept == preset + 2
     assert sum(made(k) is not None for k in range(swept)) == 2
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_the_lattice_of_a_swept_problem_stays_what_it_was_made_with(fake, monkeypatch, mode):
+    """FKADJ_ZGH_SEGMENTS=0 keeps a problem made under it from sweeping; set
+    later, it must not shrink the rows that the sweeps write."""
+    inst = _inst()
+    with api.Problem(inst, opts=_opts(inst, mode)) as pb:
+        monkeypatch.setenv("FKADJ_ZGH_SEGMENTS", "0")
+        pb.grad(inst.Et, inst.y0)
+        assert fake.fake_launches(b"k_adj_run") > 0
