@@ -663,8 +663,8 @@ fkadj_status Problem::init(const fkadj_params& p, double dt, int nt, const int* 
 // where every active cell keeps a neighbour in both directions; one launch per
 // sweep where the grid's tiles fit the device at once, the tile kernels
 // otherwise.  Where both run, forward and backward us a step with the sweep
-// and with the tile kernels: 256 x 256 5.6 9.0 and 12.8 16.9, 384 x 384 8.2
-// 14.0 and 14.8 21.0, 437 x 501 11.0 19.1 and 21.0 31.3.  flags (host): the
+// and with the tile kernels: 256 x 256 5.4 8.5 and 12.8 16.6, 384 x 384 8.1
+// 14.2 and 14.5 20.7, 437 x 501 11.0 19.2 and 20.5 30.8.  flags (host): the
 // sweeps' cell flags, adjoint flags and segment flags, in a row.
 // FKADJ_SWEEPS=0 in the environment keeps the preset kernels.
 fkadj_status Problem::init_sweeps(const uint8_t* flags) {

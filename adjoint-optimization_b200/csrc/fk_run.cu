@@ -45,12 +45,13 @@ namespace {
 // A grid takes the one of least cost among those whose tiles fit the device
 // (ShapeInfo::cost), and so do a batch's launches.  Forward and backward us a
 // step with each (a dash: does not fit):
-//             64x5x29    64x3x15   32x3x30   32x2x18   16x2x34   16x1x14
-//   128x128   6.6 13.3   5.2 8.0   4.5 7.5   3.7 6.5   3.9 6.5   3.2 5.0
-//   256x256   7.7 15.2   5.9 9.4   5.7 9.5   5.6 9.0   5.9 9.4      -
-//   320x320   8.4 16.9   7.1 10.9  6.9 11.0     -         -         -
-//   437x501  11.0 19.1      -         -         -         -         -
-// and between the last two 64x4x22: 384x384 8.9 16.9 -> 8.2 14.0.
+//             64x5x29    64x4x22   64x3x15   32x3x30   32x2x18   16x2x34   16x1x14
+//   128x128   6.5 13.5   6.0 11.0  5.0 8.1   4.3 7.0   3.5 5.8   3.7 6.1   3.0 4.6
+//   256x256   7.6 15.3   6.3 12.0  5.8 9.5   5.6 9.3   5.4 8.5   5.7 9.0      -
+//   320x320   8.3 16.8   7.2 13.2  7.0 11.0  6.8 10.9     -         -         -
+//   384x384   8.8 17.0   8.2 14.2     -         -         -         -         -
+//   437x501  11.0 19.2      -         -         -         -         -         -
+// (32x4x42, not listed, is level with 64x4x22 at 384x384: 8.3 14.1.)
 #define FKADJ_RUN_LIST(X) \
     X(0, 64, 5, 29)       \
     X(1, 64, 3, 15)       \
